@@ -289,6 +289,15 @@ __global__ void __launch_bounds__(256) k_fluid_finish(StepArgs a) {
 // time_step.f90:152-161 / :222-236 (advance_state in solid.cuh) as its own kernel.
 __global__ void __launch_bounds__(256) k_advance(AdvArgs a) { advance_state(a); }
 
+// 1 / |k|^2 per mode, correctly rounded (0 at k = 0), from the rounded squares the kernels add
+__global__ void k_recip_k2(double* rk2, const double* ky2, double scalex, int hx, int nyh) {
+    const int n = hx * nyh;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int kx = i / nyh, ky = i - kx * nyh;
+        rk2[i] = i == 0 ? 0.0 : 1.0 / __dadd_rn(__dmul_rn((double)(kx * kx), scalex), ky2[ky]);
+    }
+}
+
 // ---- the packed Temperton layout (ABI boundary only) ---------------------------------
 // unpack: fk (Fortran (0:nx-1,0:ny-1)) -> S[kx][ky]   (cof_fftw33.f90:214-233)
 template <typename R>
@@ -436,7 +445,7 @@ struct fsibe_ctx {
     SizeKernels<float> kxf{}, kyf{};
     void* phys[PH_N] = {};
     void* spec[SP_N] = {};
-    void *twX = nullptr, *twR = nullptr, *twY = nullptr;
+    void *twX = nullptr, *twR = nullptr, *twY = nullptr, *tw64 = nullptr;
     DevScalars* S = nullptr;
     double* red = nullptr;
     double* beam[B_N] = {};
@@ -457,6 +466,9 @@ struct fsibe_ctx {
     float2* etabf = nullptr;
     int* dcut = nullptr;          // dealiasing cut per kx
     float* kxw = nullptr;         // (float)(kx kxs), kx in [0, hx]: the FP32 kernels' wavenumbers
+    double* kmode = nullptr;      // FP64 form: kx 2 pi / xl [hx+1], signed ky 2 pi / yl [ny], ky^2 (2 pi / yl)^2 [ny/2+1]
+    double* rk2 = nullptr;        // FP64 form: 1 / |k|^2 [hx][ny/2+1]
+    int enorm = 0;                // log2 (1 / (nx ny))
     int kcut = 0;                 // first kx whose row is entirely removed by the 2/3 rule
     double* dscratch = nullptr;   // 2*nx*ny doubles (ABI transfers, packed arrays)
     double* dscratch2 = nullptr;  // nx*ny doubles
@@ -550,6 +562,22 @@ static std::string g_err;
 
 static bool pow2_ok(int n) { return n >= 32 && n <= 4096 && (n & (n - 1)) == 0; }
 
+// a fraction times 2^62 in two balanced 32-bit halves (fft_fx.cuh); a low half of -2^31, whose
+// negative has no 32-bit value, moves one unit up
+__host__ __device__ static inline void fx_halves(long long v, int& hi, int& lo) {
+    if ((int)v == INT32_MIN) ++v;
+    lo = (int)v;
+    hi = (int)((v - (long long)lo) >> 32);
+}
+static void make_table(std::vector<int4>& out, long n, long count) {
+    const long double pi_l = 3.141592653589793238462643383279502884L, one = 4611686018427387904.0L;
+    out.resize(count);
+    for (long m = 0; m < count; ++m) {
+        const long double a = 2.0L * pi_l * (long double)m / (long double)n;
+        fx_halves(llroundl(cosl(a) * one), out[m].x, out[m].y);
+        fx_halves(llroundl(-sinl(a) * one), out[m].z, out[m].w);
+    }
+}
 template <typename T>
 static void make_table(std::vector<T>& out, long n, long count) {
     const long double pi_l = 3.141592653589793238462643383279502884L;
@@ -572,15 +600,19 @@ static KArgs<R> kargs(fsibe_ctx* c) {
     for (int i = 0; i < PH_N; ++i) *ph[i] = reinterpret_cast<R*>(c->phys[i]);
     C2<R>** sp[] = {&a.W, &a.M, &a.Wlo, &a.A, &a.B, &a.Tu, &a.Tv, &a.Tw, &a.Tsa, &a.Tsb, &a.Tdx, &a.Tdy, &a.P1, &a.P2, &a.Tq, &a.spec0, &a.spec1};
     for (int i = 0; i < SP_N; ++i) *sp[i] = reinterpret_cast<C2<R>*>(c->spec[i]);
-    a.twX = reinterpret_cast<const C2<R>*>(c->twX);
-    a.twR = reinterpret_cast<const C2<R>*>(c->twR);
-    a.twY = reinterpret_cast<const C2<R>*>(c->twY);
+    a.twX = reinterpret_cast<const TwF<R>*>(c->twX);
+    a.twR = reinterpret_cast<const TwF<R>*>(c->twR);
+    a.twY = reinterpret_cast<const TwF<R>*>(c->twY);
+    a.twX64 = reinterpret_cast<const C2<R>*>(c->tw64);
+    a.twR64 = a.twX64 ? a.twX64 + c->g.hx : nullptr;
     a.S = c->S;
     a.red = c->red;
     a.etab = c->etab;
     a.etabf = c->etabf;
     a.dcut = c->dcut;
     a.kxw = c->kxw;
+    a.kxd = c->kmode; a.kyd = a.kxd + c->g.hx + 1; a.ky2 = a.kyd + c->g.ny; a.rk2 = c->rk2;
+    a.enorm = c->enorm;
     a.kcut = c->kcut;
     a.spg = reinterpret_cast<const R*>(c->spg);
     a.s10 = reinterpret_cast<const R*>(c->s10);
@@ -1524,7 +1556,7 @@ int fsibe_destroy(fsibe_ctx* c) {
     for (void* p : c->phys) if (p) cudaFree(p);
     for (void* p : c->spec) if (p) cudaFree(p);
     for (double* p : c->beam) if (p) cudaFree(p);
-    void* others[] = {c->twX, c->twR, c->twY, c->S, c->red, c->oo, c->ws, c->pred, c->minv, c->minv_rse, c->d1d, c->fgeo, c->fgij, c->clws, c->prims, c->primg, c->nprims,
+    void* others[] = {c->twX, c->twR, c->twY, c->tw64, c->S, c->red, c->oo, c->ws, c->pred, c->minv, c->minv_rse, c->d1d, c->kmode, c->rk2, c->fgeo, c->fgij, c->clws, c->prims, c->primg, c->nprims,
                       c->rect, c->counter, c->fterm, c->rows, c->dscratch, c->dscratch2, c->etab, c->etabf, c->dcut, c->kxw,
                       c->bg, c->frame, c->spg, c->s10, c->s10_dudx, c->rect_full, c->snap};
     for (void* p : others) if (p) cudaFree(p);
@@ -1682,6 +1714,19 @@ int fsibe_create(const fsibe_params* p, fsibe_ctx** out) {
         for (int kx = 0; kx <= p->nx / 2; ++kx) kw[kx] = (float)((double)kx * g.kxs);
         cudaMemcpy(c->kxw, kw.data(), 4 * kw.size(), cudaMemcpyHostToDevice);
     }
+    for (size_t m = NN; m > 1; m >>= 1) --c->enorm;
+    if (!c->fp32) {
+        const int nyh = p->ny / 2 + 1;
+        std::vector<double> km(g.hx + 1 + p->ny + nyh);
+        double *kxd = km.data(), *kyd = kxd + g.hx + 1, *ky2 = kyd + p->ny;
+        for (int kx = 0; kx <= g.hx; ++kx) kxd[kx] = (double)kx * g.kxs;
+        for (int ky = 0; ky < p->ny; ++ky) kyd[ky] = (double)signed_k(ky, p->ny) * g.kys;
+        for (int ky = 0; ky < nyh; ++ky) ky2[ky] = (double)(ky * ky) * g.scaley;
+        ALLOC(c->kmode, 8 * km.size());
+        ALLOC(c->rk2, 8 * (size_t)g.hx * nyh);
+        cudaMemcpy(c->kmode, km.data(), 8 * km.size(), cudaMemcpyHostToDevice);
+        k_recip_k2<<<256, 256>>>(c->rk2, c->kmode + g.hx + 1 + p->ny, g.scalex, g.hx, nyh);
+    }
     {
         // 2/3 rule (dealiase_mask.f90:9-26), evaluated with the reference's FP64 expression:
         // dcut[kx] = smallest |ky| that is removed
@@ -1737,10 +1782,19 @@ int fsibe_create(const fsibe_params* p, fsibe_ctx** out) {
         cudaMemcpy(c->twR, tR.data(), 8 * tR.size(), cudaMemcpyHostToDevice);
         cudaMemcpy(c->twY, tY.data(), 8 * tY.size(), cudaMemcpyHostToDevice);
     } else {
-        std::vector<double2> tX, tR, tY;
+        std::vector<int4> tX, tR, tY;
+        make_table(tY, p->ny, p->ny);
         make_table(tX, p->nx / 2, p->nx / 2);
         make_table(tR, p->nx, p->nx / 2 + 1);
-        make_table(tY, p->ny, p->ny);
+        if (p->nx == 4096) {  // the step's rows of this length take the same fractions in doubles (step_fp)
+            std::vector<double2> d;
+            for (const auto* tab : {&tX, &tR})
+                for (const int4& w : *tab)
+                    d.push_back(make_double2(std::ldexp((double)(((long long)w.x << 32) + w.y), -62),
+                                             std::ldexp((double)(((long long)w.z << 32) + w.w), -62)));
+            ALLOC(c->tw64, 16 * d.size());
+            cudaMemcpy(c->tw64, d.data(), 16 * d.size(), cudaMemcpyHostToDevice);
+        }
         ALLOC(c->twX, 16 * tX.size()); ALLOC(c->twR, 16 * tR.size()); ALLOC(c->twY, 16 * tY.size());
         cudaMemcpy(c->twX, tX.data(), 16 * tX.size(), cudaMemcpyHostToDevice);
         cudaMemcpy(c->twR, tR.data(), 16 * tR.size(), cudaMemcpyHostToDevice);
@@ -3137,22 +3191,17 @@ std::mutex g_static_mu;
 
 int static_log2_index(int n) { int i = 0; while ((32 << i) < n) ++i; return i; }
 
-__global__ void k_static_twiddles(double2* twY, int ny, double2* twX, int hx, double2* twR, int nx) {
+__global__ void k_static_twiddles(int4* twY, int ny, int4* twX, int hx, int4* twR, int nx) {
     const int total = ny + hx + hx + 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        int4* out = i < ny ? twY + i : (i < ny + hx ? twX + (i - ny) : twR + (i - ny - hx));
+        const int m = i < ny ? i : (i < ny + hx ? i - ny : i - ny - hx), n = i < ny ? ny : (i < ny + hx ? hx : nx);
         double s, c;
-        if (i < ny) {
-            sincospi(2.0 * (double)i / (double)ny, &s, &c);
-            twY[i] = make_double2(c, -s);
-        } else if (i < ny + hx) {
-            const int m = i - ny;
-            sincospi(2.0 * (double)m / (double)hx, &s, &c);
-            twX[m] = make_double2(c, -s);
-        } else {
-            const int m = i - ny - hx;
-            sincospi(2.0 * (double)m / (double)nx, &s, &c);
-            twR[m] = make_double2(c, -s);
-        }
+        sincospi(2.0 * (double)m / (double)n, &s, &c);
+        int4 w;
+        fx_halves(__double2ll_rn(c * 4611686018427387904.0), w.x, w.y);
+        fx_halves(__double2ll_rn(-s * 4611686018427387904.0), w.z, w.w);
+        *out = w;
     }
 }
 }  // namespace
@@ -3225,14 +3274,15 @@ extern "C" int fsibe_coftxy_static(const double* f_dev, double* fk_dev, int32_t 
     const int hx = nx / 2;
     double2* T = reinterpret_cast<double2*>(base);
     double2* Sx = reinterpret_cast<double2*>(base + FSIBE_STATIC_MAX_CELLS);
-    double2* twY = reinterpret_cast<double2*>(base + 2 * FSIBE_STATIC_MAX_CELLS);
-    double2* twX = twY + ny;
-    double2* twR = twX + hx;
+    int4* twY = reinterpret_cast<int4*>(base + 2 * FSIBE_STATIC_MAX_CELLS);
+    int4* twX = twY + ny;
+    int4* twR = twX + hx;
     k_static_twiddles<<<16, 256, 0, st>>>(twY, ny, twX, hx, twR, nx);
     KArgs<double> a;
     std::memset(&a, 0, sizeof(a));
     a.g.nx = nx; a.g.ny = ny; a.g.hx = hx;
     a.g.inv_nxny = 1.0 / ((double)nx * (double)ny);
+    for (int m = nx * ny; m > 1; m >>= 1) --a.enorm;
     a.phys0 = const_cast<double*>(f_dev);
     a.spec0 = T;
     a.spec1 = Sx;

@@ -46,6 +46,11 @@ template <typename R> struct C2T;
 template <> struct C2T<double> { typedef double2 type; };
 template <> struct C2T<float> { typedef float2 type; };
 template <typename R> using C2 = typename C2T<R>::type;
+// a twiddle's type: FP32 the complex value; the FP64 form's transforms are fixed point (fft_fx.cuh)
+// and take cos and sin as 62-bit fractions in balanced 32-bit halves (c hi, c lo, s hi, s lo)
+template <typename R> struct TwT { typedef C2<R> type; };
+template <> struct TwT<double> { typedef int4 type; };
+template <typename R> using TwF = typename TwT<R>::type;
 
 template <typename R> __host__ __device__ __forceinline__ C2<R> mk(R x, R y) { C2<R> r; r.x = x; r.y = y; return r; }
 template <typename R> __device__ __forceinline__ C2<R> cadd(C2<R> a, C2<R> b) { return mk<R>(a.x + b.x, a.y + b.y); }

@@ -1,15 +1,16 @@
-// fft.cuh -- block-level Stockham FFT engine for power-of-two lengths.
+// fft.cuh -- block-level Stockham FFT engine for power-of-two lengths (FP32, and the
+// time step's FP64 rows of 4096 real values; the FP64 form's other transforms are fft_fx.cuh's, on
+// the same data layout).
 //
-// A length-N complex sequence lives in shared memory (padded with pad8) and is transformed
-// in place by a group of G = N/8 threads.  Each stage is a radix-8 Stockham pass (radix 4
-// or 2 for the last stage when log2 N is not a multiple of 3): every thread loads its
-// butterfly inputs into registers, the block synchronises, and the outputs are written to
-// their autosorted positions.  Twiddles come from a table W_N^m = exp(-2 pi i m/N) computed
-// on the host in long double and rounded once to the storage type.
+// A length-N complex sequence is transformed by a group of G = N/8 threads that hold it in
+// registers.  Each stage is a radix-8 Stockham pass (radix 4 or 2 for the last stage when log2 N
+// is not a multiple of 3); between stages the outputs go to their autosorted positions in a
+// shared-memory row (padded with pad8).  Twiddles come from a table W_N^m = exp(-2 pi i m/N)
+// computed on the host in long double and rounded once to the storage type.
 //
 // Forward = exp(-i..), inverse = exp(+i..), both unnormalised (like FFTW).
 #pragma once
-#include "common.cuh"
+#include "fft_fx.cuh"
 
 namespace fsibe {
 
@@ -61,125 +62,12 @@ __device__ __forceinline__ void dftp(C2<R>* v) {
     else dft2<R, INV>(v);
 }
 
-// One Stockham stage of radix P; NS = product of the radices already applied.
-template <typename R, int N, int P, int NS, bool INV>
-__device__ __forceinline__ void fft_stage(C2<R>* buf, const C2<R>* __restrict__ tw, int t) {
-    constexpr int G = N / 8, B = N / P, PER = 8 / P;
-    C2<R> v[8];
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int j = t + q * G;
-#pragma unroll
-        for (int r = 0; r < P; ++r) v[q * P + r] = buf[pad8(j + r * B)];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int j = t + q * G;
-        const int k = j & (NS - 1);
-        if constexpr (NS > 1) {
-#pragma unroll
-            for (int r = 1; r < P; ++r) {
-                C2<R> w = __ldg(&tw[r * k * (N / (NS * P))]);
-                if (INV) w.y = -w.y;
-                v[q * P + r] = cmul<R>(v[q * P + r], w);
-            }
-        }
-        dftp<R, P, INV>(v + q * P);
-        const int base = (j - k) * P + k;
-#pragma unroll
-        for (int r = 0; r < P; ++r) buf[pad8(base + r * NS)] = v[q * P + r];
-    }
-    __syncthreads();
-}
-
-template <typename R, int N, bool INV, int NS = 1>
-__device__ __forceinline__ void fft_run(C2<R>* buf, const C2<R>* __restrict__ tw, int t) {
-    if constexpr (NS * 8 <= N) {
-        fft_stage<R, N, 8, NS, INV>(buf, tw, t);
-        fft_run<R, N, INV, NS * 8>(buf, tw, t);
-    } else if constexpr (NS * 4 == N) {
-        fft_stage<R, N, 4, NS, INV>(buf, tw, t);
-    } else if constexpr (NS * 2 == N) {
-        fft_stage<R, N, 2, NS, INV>(buf, tw, t);
-    }
-}
-
-// In-place transform of buf (padded, natural order). All threads of the block must call it;
-// the caller synchronises before (data written by other threads) -- the routine ends synced.
-template <typename R, int N, bool INV>
-__device__ __forceinline__ void block_fft(C2<R>* buf, const C2<R>* __restrict__ tw, int t) {
-    static_assert(N >= 16 && (N & (N - 1)) == 0, "power-of-two length >= 16");
-    fft_run<R, N, INV>(buf, tw, t);
-}
-
-// NB independent transforms of the same length at buf + b * bstride, b < NB, stage by stage:
-// each stage loads all NB butterflies, synchronises once, and shares its twiddles between the
-// NB transforms.  Each transform's arithmetic is exactly that of block_fft.
-template <typename R, int N, int P, int NS, bool INV, int NB>
-__device__ __forceinline__ void fft_stage_m(C2<R>* buf, int bstride, const C2<R>* __restrict__ tw, int t) {
-    constexpr int G = N / 8, B = N / P, PER = 8 / P;
-    C2<R> v[NB][8];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int j = t + q * G;
-#pragma unroll
-            for (int r = 0; r < P; ++r) v[b][q * P + r] = buf[b * bstride + pad8(j + r * B)];
-        }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int j = t + q * G;
-        const int k = j & (NS - 1);
-        if constexpr (NS > 1) {
-#pragma unroll
-            for (int r = 1; r < P; ++r) {
-                C2<R> w = __ldg(&tw[r * k * (N / (NS * P))]);
-                if (INV) w.y = -w.y;
-#pragma unroll
-                for (int b = 0; b < NB; ++b) v[b][q * P + r] = cmul<R>(v[b][q * P + r], w);
-            }
-        }
-        const int base = (j - k) * P + k;
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            dftp<R, P, INV>(v[b] + q * P);
-#pragma unroll
-            for (int r = 0; r < P; ++r) buf[b * bstride + pad8(base + r * NS)] = v[b][q * P + r];
-        }
-    }
-    __syncthreads();
-}
-
-template <typename R, int N, bool INV, int NB, int NS = 1>
-__device__ __forceinline__ void fft_run_m(C2<R>* buf, int bstride, const C2<R>* __restrict__ tw, int t) {
-    if constexpr (NS * 8 <= N) {
-        fft_stage_m<R, N, 8, NS, INV, NB>(buf, bstride, tw, t);
-        fft_run_m<R, N, INV, NB, NS * 8>(buf, bstride, tw, t);
-    } else if constexpr (NS * 4 == N) {
-        fft_stage_m<R, N, 4, NS, INV, NB>(buf, bstride, tw, t);
-    } else if constexpr (NS * 2 == N) {
-        fft_stage_m<R, N, 2, NS, INV, NB>(buf, bstride, tw, t);
-    }
-}
-
-// NB in-place transforms (padded, natural order) at buf + b * bstride; the same contract as
-// block_fft.
-template <typename R, int N, bool INV, int NB>
-__device__ __forceinline__ void block_fft_m(C2<R>* buf, int bstride, const C2<R>* __restrict__ tw, int t) {
-    static_assert(N >= 16 && (N & (N - 1)) == 0, "power-of-two length >= 16");
-    fft_run_m<R, N, INV, NB>(buf, bstride, tw, t);
-}
-
 // ---- transforms of values held in registers ------------------------------------------------
 // A thread of the G = N/8 owns elements t + m G (m < 8) of each of the NB sequences.  These are
 // exactly the inputs of its first-stage butterfly and the outputs of its last-stage
 // butterflies, so a transform whose inputs are computed in registers and whose outputs go to
 // registers needs shared memory only between stages: stages - 1 exchanges instead of a load and
-// a store per stage plus the staging in and out.  Each stage's arithmetic (twiddles, radix-P
-// butterfly, operation order) is that of fft_stage_m, so the results are bitwise the same.
+// a store per stage plus the staging in and out.
 
 // The butterflies of one stage on v[b][q P + r] (input r of butterfly q, j = t + q G), b < NB
 // of the NBA rows of v.
@@ -251,13 +139,15 @@ __device__ __forceinline__ void fft_reg_run(C2<R> (&v)[NBA][8], C2<R>* buf, int 
 // NB transforms of the sequences v[b][m] = element t + m (N/8), b < NB (of the NBA rows of v);
 // buf + b * bstride are NB padded shared-memory rows for the exchanges, free when this is
 // called (the caller synchronises after their last use); they are free again on return.  All
-// threads of the block call it.
+// threads of the block call it.  FP64: the result is scaled by 2^ex (fft_fx.cuh); FP32 leaves the
+// scale to the caller (ex is not used).
 template <typename R, int N, bool INV, int NB, int NBA>
 __device__ __forceinline__ void block_fft_reg_m(C2<R> (&v)[NBA][8], C2<R>* buf, int bstride,
-                                                const C2<R>* __restrict__ tw, int t) {
+                                                const TwF<R>* __restrict__ tw, int t, int ex = 0) {
     static_assert(N >= 16 && (N & (N - 1)) == 0, "power-of-two length >= 16");
     static_assert(NB >= 1 && NB <= NBA, "NB of the NBA rows");
-    fft_reg_run<R, N, INV, NB, 1, NBA>(v, buf, bstride, tw, t);
+    if constexpr (sizeof(R) == 8) fx_fft_reg<N, INV, NB>(v, buf, bstride, tw, t, ex);
+    else fft_reg_run<R, N, INV, NB, 1, NBA>(v, buf, bstride, tw, t);
 }
 
 // ---- paired transforms (FP32): a thread owns two adjacent butterflies -----------------------
@@ -381,66 +271,11 @@ __device__ __forceinline__ void block_fft2_m(float2 (&v)[NBA][16], float4* buf, 
 // A real row x[0..2H) is handled as z[m] = x[2m] + i x[2m+1], m < H, transformed with a
 // length-H complex FFT.  twr[k] = exp(-2 pi i k / 2H), k <= H.
 
-// After the forward length-H FFT of z (in buf): X[k], k in [0,H), in place.  The Nyquist bin
-// X[H] is dropped (the reference's filtering).  Pairs (k, H-k) handled by the same thread.
-template <typename R, int H>
-__device__ __forceinline__ void r2c_split(C2<R>* buf, const C2<R>* __restrict__ twr, int t) {
-    constexpr int G = H / 8;
-    // pairs k = 1 .. H/2-1, plus k = 0 and k = H/2 handled by thread 0
-    for (int k = 1 + t; k < H / 2; k += G) {
-        const C2<R> zk = buf[pad8(k)], zm = buf[pad8(H - k)];
-        const C2<R> wk = __ldg(&twr[k]), wm = __ldg(&twr[H - k]);
-        // X[k] = 1/2 (zk + conj zm) + w^k (zk - conj zm)/(2i)
-        C2<R> e = mk<R>((R)0.5 * (zk.x + zm.x), (R)0.5 * (zk.y - zm.y));
-        C2<R> d = mk<R>(zk.x - zm.x, zk.y + zm.y);           // zk - conj zm
-        C2<R> o = mk<R>((R)0.5 * d.y, (R)-0.5 * d.x);         // d / (2i)
-        C2<R> Xk = cadd<R>(e, cmul<R>(wk, o));
-        // X[H-k] = 1/2 (zm + conj zk) + w^(H-k) (zm - conj zk)/(2i)
-        C2<R> e2 = mk<R>((R)0.5 * (zm.x + zk.x), (R)0.5 * (zm.y - zk.y));
-        C2<R> d2 = mk<R>(zm.x - zk.x, zm.y + zk.y);
-        C2<R> o2 = mk<R>((R)0.5 * d2.y, (R)-0.5 * d2.x);
-        C2<R> Xm = cadd<R>(e2, cmul<R>(wm, o2));
-        buf[pad8(k)] = Xk;
-        buf[pad8(H - k)] = Xm;
-    }
-    if (t == 0) {
-        C2<R> z0 = buf[pad8(0)];
-        buf[pad8(0)] = mk<R>(z0.x + z0.y, (R)0);
-        C2<R> zh = buf[pad8(H / 2)];
-        buf[pad8(H / 2)] = mk<R>(zh.x, -zh.y);
-    }
-    __syncthreads();
-}
-
-// Before the inverse length-H FFT: X[k], k in [0,H) (X[H] = 0, Im X[0] ignored) -> Z'[k] so
-// that z = IFFT_H(Z') gives x[2m] = Re z[m], x[2m+1] = Im z[m] (unnormalised c2r).
-template <typename R, int H>
-__device__ __forceinline__ void c2r_merge(C2<R>* buf, const C2<R>* __restrict__ twr, int t) {
-    constexpr int G = H / 8;
-    for (int k = 1 + t; k < H / 2; k += G) {
-        const C2<R> xk = buf[pad8(k)], xm = buf[pad8(H - k)];
-        const C2<R> wk = __ldg(&twr[k]), wm = __ldg(&twr[H - k]);
-        // Z'[k] = (xk + conj xm) + i (xk - conj xm) conj(w^k)
-        C2<R> e = mk<R>(xk.x + xm.x, xk.y - xm.y);
-        C2<R> o = cmul<R>(mk<R>(xk.x - xm.x, xk.y + xm.y), mk<R>(wk.x, -wk.y));
-        C2<R> Zk = mk<R>(e.x - o.y, e.y + o.x);
-        C2<R> e2 = mk<R>(xm.x + xk.x, xm.y - xk.y);
-        C2<R> o2 = cmul<R>(mk<R>(xm.x - xk.x, xm.y + xk.y), mk<R>(wm.x, -wm.y));
-        C2<R> Zm = mk<R>(e2.x - o2.y, e2.y + o2.x);
-        buf[pad8(k)] = Zk;
-        buf[pad8(H - k)] = Zm;
-    }
-    if (t == 0) {
-        C2<R> x0 = buf[pad8(0)];
-        buf[pad8(0)] = mk<R>(x0.x, x0.x);
-        C2<R> xh = buf[pad8(H / 2)];
-        buf[pad8(H / 2)] = mk<R>((R)2 * xh.x, (R)-2 * xh.y);
-    }
-    __syncthreads();
-}
-
-// r2c_split and c2r_merge of NB rows at buf + b * bstride (each row's arithmetic unchanged;
-// the twiddles are loaded once for all rows).
+// r2c_split_m, after the forward length-H FFT of z (NB rows at buf + b * bstride): X[k], k in
+// [0, H), in place; the Nyquist bin X[H] is dropped (the reference's filtering).  c2r_merge_m,
+// before the inverse length-H FFT: X[k], k in [0, H) (X[H] = 0, Im X[0] ignored) -> Z'[k] so that
+// z = IFFT_H(Z') gives x[2m] = Re z[m], x[2m+1] = Im z[m] (unnormalised c2r).  Pairs (k, H-k) are
+// handled by the same thread.
 template <typename R, int H, int NB>
 __device__ __forceinline__ void r2c_split_m(C2<R>* buf, int bstride, const C2<R>* __restrict__ twr, int t) {
     constexpr int G = H / 8;

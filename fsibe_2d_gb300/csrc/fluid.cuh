@@ -34,7 +34,8 @@ struct KArgs {
     R *u, *v, *mask, *mvx, *mvy, *vor_mean, *press, *sa, *sb, *phys0;
     // half spectra C2<R>[hx][ny]
     C2<R> *W, *M, *Wlo, *A, *B, *Tu, *Tv, *Tw, *Tsa, *Tsb, *Tdx, *Tdy, *P1, *P2, *Tq, *spec0, *spec1;
-    const C2<R> *twX, *twR, *twY;
+    const TwF<R> *twX, *twR, *twY;
+    const C2<R> *twX64, *twR64;  // FP64, nx = 4096: the x tables in doubles (step_fp)
     DevScalars* S;
     double* red;
     const double* etab;   // integrating factor per direction: exp(coefx kx^2) [hx], exp(coefy ky^2) [ny/2+1]
@@ -42,6 +43,12 @@ struct KArgs {
     const int* dcut;      // 2/3-rule: modes with |ky| >= dcut[kx] are removed (dealiase_mask.f90:9-26)
     const float* kxw;     // FP32 form: (float)(kx kxs) for kx in [0, hx], formed on the host (the
                           // kernels' FP64 product and conversion per element, without the FP64 pipe)
+    // FP64 form: per-mode constants from the host, so that no kernel forms them on the FP64 pipe
+    const double* kxd;    // kx 2 pi / xl, kx in [0, hx]
+    const double* kyd;    // signed ky 2 pi / yl, ky in [0, ny)
+    const double* ky2;    // ky^2 (2 pi / yl)^2, ky in [0, ny/2]
+    const double* rk2;    // 1 / |k|^2 correctly rounded, [hx][ny/2 + 1] (0 at k = 0)
+    int enorm;            // log2 of the normalisation 1/(nx ny)
     int kcut;             // rows kx >= kcut hold no dealiased mode (dcut = 0): exact zeros after the update
     int viscous, pressure_on, penalize, op;
     int explicit_step;    // 1 on the Euler start-up step (the host's flag: nl_x runs beside k_step_begin)
@@ -83,11 +90,29 @@ __device__ __forceinline__ double col_reduce_ff(const float* col, int n, bool mx
     return mx ? (double)s : (double)s + (double)c;
 }
 
-// kx 2 pi / xl in the kernels' type: FP32 from the host's table, FP64 as the product
+// kx 2 pi / xl in the kernels' type, from the host's tables
 template <typename R> __device__ __forceinline__ R kx_wave(const KArgs<R>& a, int kx) {
     if constexpr (kIsF32<R>) return a.kxw[kx];
-    else return (double)kx * a.g.kxs;
+    else return __ldg(&a.kxd[kx]);
 }
+// signed ky 2 pi / yl in the kernels' type
+template <typename R> __device__ __forceinline__ R ky_wave(const KArgs<R>& a, int ky, int ks) {
+    if constexpr (kIsF32<R>) return (R)ks * (R)a.g.kys;
+    else return __ldg(&a.kyd[ky]);
+}
+// s / |k|^2 of mode (kx, |ky| = ka) in the FP64 form (poisson.f90:159-162 divides): the correctly
+// rounded quotient by the tabled reciprocal, three FP64 instructions a component where a division
+// takes ten (and its SMSP's FP64 pipe 660 cycles).  With this, the wavenumber tables and the sums
+// left out away from the mask: 1024^2 k_nl_y 181 -> 160 us, k_press_x 153 -> 104, k_press_y 70 -> 49
+__device__ __forceinline__ double2 over_k2(const KArgs<double>& a, double2 s, double kx2, int kx, int ka) {
+    const double k2 = __dadd_rn(kx2, __ldg(&a.ky2[ka])), r = __ldg(&a.rk2[(size_t)kx * (a.g.ny / 2 + 1) + ka]);
+    return make_double2(div_cr(s.x, k2, r), div_cr(s.y, k2, r));
+}
+// a value that is zero (of either sign), without an FP64 comparison
+__device__ __forceinline__ bool is_zero(double x) {
+    return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
 
 // k_nl_x's parts.  The advection part needs no mask, so it can run beside the mask kernels;
 // the penalization part then adds the mask's term on the rows of the mask's box alone
@@ -139,7 +164,7 @@ __device__ __forceinline__ void ff_update(float wh, float wl, float d, float Eh,
 // Operators the generic inverse-y kernel applies before the transform.
 enum SpecOp { OP_ID = 0, OP_DX = 1, OP_DY = 2, OP_U = 3, OP_V = 4, OP_UX = 5 };  // OP_UX: du/dx
 
-__device__ __forceinline__ int signed_k(int k, int n) { return (k <= n / 2) ? k : k - n; }
+__host__ __device__ __forceinline__ int signed_k(int k, int n) { return (k <= n / 2) ? k : k - n; }
 
 template <typename R, int H, int TRV = 0>
 struct XRows {
@@ -188,39 +213,12 @@ __device__ __forceinline__ void load_tileT_dx(C2<R>* buf, const C2<R>* __restric
     }
 }
 
-// inverse x transform of one row buffer (after load + __syncthreads)
-template <typename R, int H>
-__device__ __forceinline__ void row_c2r(C2<R>* rb, const C2<R>* __restrict__ twR, const C2<R>* __restrict__ twX, int t) {
-    c2r_merge<R, H>(rb, twR, t);
-    block_fft<R, H, true>(rb, twX, t);
-}
-
-template <typename R, int H>
-__device__ __forceinline__ void row_r2c(C2<R>* rb, const C2<R>* __restrict__ twR, const C2<R>* __restrict__ twX, int t) {
-    block_fft<R, H, false>(rb, twX, t);
-    r2c_split<R, H>(rb, twR, t);
-}
-
-// NB rows at rb + b * bstride at once (their stages share synchronisations and twiddles)
-template <typename R, int H, int NB>
-__device__ __forceinline__ void row_c2r_m(C2<R>* rb, int bstride, const C2<R>* __restrict__ twR,
-                                          const C2<R>* __restrict__ twX, int t) {
-    c2r_merge_m<R, H, NB>(rb, bstride, twR, t);
-    block_fft_m<R, H, true, NB>(rb, bstride, twX, t);
-}
-template <typename R, int H, int NB>
-__device__ __forceinline__ void row_r2c_m(C2<R>* rb, int bstride, const C2<R>* __restrict__ twR,
-                                          const C2<R>* __restrict__ twX, int t) {
-    block_fft_m<R, H, false, NB>(rb, bstride, twX, t);
-    r2c_split_m<R, H, NB>(rb, bstride, twR, t);
-}
-
-// row_c2r_m with the transform's output in registers: v[b][q] = element t + q (H/8) of row b
-// (the row buffers are free on return).  The merge runs in shared memory, the transform's
-// stages exchange through it; the arithmetic is row_c2r_m's.
+// The inverse x transform of NB rows at rb + b * bstride (loaded and synchronised), their stages
+// together, with the output in registers: v[b][q] = element t + q (H/8) of row b (the row buffers
+// are free on return).  The merge runs in shared memory, the transform's stages exchange through it.
 template <typename R, int H, int NB, int NBA>
-__device__ __forceinline__ void row_c2r_reg(C2<R>* rb, int bstride, const C2<R>* __restrict__ twR,
-                                            const C2<R>* __restrict__ twX, int t, C2<R> (&v)[NBA][8]) {
+__device__ __forceinline__ void row_c2r_fp(C2<R>* rb, int bstride, const C2<R>* __restrict__ twR,
+                                           const C2<R>* __restrict__ twX, int t, C2<R> (&v)[NBA][8]) {
     constexpr int G = H / 8;
     c2r_merge_m<R, H, NB>(rb, bstride, twR, t);
 #pragma unroll
@@ -228,21 +226,50 @@ __device__ __forceinline__ void row_c2r_reg(C2<R>* rb, int bstride, const C2<R>*
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[b][q] = rb[b * bstride + pad8(t + q * G)];
     __syncthreads();
-    block_fft_reg_m<R, H, true, NB>(v, rb, bstride, twX, t);
+    fft_reg_run<R, H, true, NB, 1>(v, rb, bstride, twX, t);
 }
-// row_r2c_m of rows given in registers (v[b][q] = element t + q (H/8)); the rows must be free
-// (synchronised after their last use).  The result is in the row buffers, as from row_r2c_m.
+// The forward x transform of rows given in registers (v[b][q] = element t + q (H/8)); the row
+// buffers must be free (synchronised after their last use) and hold the half spectra on return.
 template <typename R, int H, int NB, int NBA>
-__device__ __forceinline__ void row_r2c_reg(C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, const C2<R>* __restrict__ twR,
-                                            const C2<R>* __restrict__ twX, int t) {
+__device__ __forceinline__ void row_r2c_fp(C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, const C2<R>* __restrict__ twR,
+                                           const C2<R>* __restrict__ twX, int t) {
     constexpr int G = H / 8;
-    block_fft_reg_m<R, H, false, NB>(v, rb, bstride, twX, t);
+    fft_reg_run<R, H, false, NB, 1>(v, rb, bstride, twX, t);
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
         for (int q = 0; q < 8; ++q) rb[b * bstride + pad8(t + q * G)] = v[b][q];
     __syncthreads();
     r2c_split_m<R, H, NB>(rb, bstride, twR, t);
+}
+// The two in the precision form's engine: the floating-point stages in FP32, fixed point in FP64.
+template <typename R, int H, int NB, int NBA>
+__device__ __forceinline__ void row_c2r_reg(C2<R>* rb, int bstride, const TwF<R>* __restrict__ twR,
+                                            const TwF<R>* __restrict__ twX, int t, C2<R> (&v)[NBA][8]) {
+    if constexpr (kIsF32<R>) row_c2r_fp<R, H, NB>(rb, bstride, twR, twX, t, v);
+    else fx_c2r_reg<H, NB>(rb, bstride, twR, twX, t, v);
+}
+template <typename R, int H, int NB, int NBA>
+__device__ __forceinline__ void row_r2c_reg(C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, const TwF<R>* __restrict__ twR,
+                                            const TwF<R>* __restrict__ twX, int t) {
+    if constexpr (kIsF32<R>) row_r2c_fp<R, H, NB>(v, rb, bstride, twR, twX, t);
+    else fx_r2c_reg<H, NB>(v, rb, bstride, twR, twX, t);
+}
+// The same in the time step's fused kernels.  FP64 rows of 4096 real values (H = 2048) keep the
+// FP64 stages there.  Fixed point is the more exact at that length too (4096^2, three steps: the
+// pressure within 3.7e-16 of the CPU's, 4.0e-16 with the FP64 stages), but at 4096^2 the pressure
+// jump at the beam's free end is what is left of two values 2 10^7 times as large, one or two units
+// of their last place, and the comparison on record at that size holds that last place.
+template <typename R, int H> constexpr bool step_fp() { return kIsF32<R> || H == 2048; }
+template <typename R, int H, int NB, int NBA>
+__device__ __forceinline__ void step_c2r(const KArgs<R>& a, C2<R>* rb, int bstride, int t, C2<R> (&v)[NBA][8]) {
+    if constexpr (sizeof(R) == 8 && step_fp<R, H>()) row_c2r_fp<R, H, NB>(rb, bstride, a.twR64, a.twX64, t, v);
+    else row_c2r_reg<R, H, NB>(rb, bstride, a.twR, a.twX, t, v);
+}
+template <typename R, int H, int NB, int NBA>
+__device__ __forceinline__ void step_r2c(const KArgs<R>& a, C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, int t) {
+    if constexpr (sizeof(R) == 8 && step_fp<R, H>()) row_r2c_fp<R, H, NB>(v, rb, bstride, a.twR64, a.twX64, t);
+    else row_r2c_reg<R, H, NB>(v, rb, bstride, a.twR, a.twX, t);
 }
 
 template <typename R>
@@ -272,10 +299,10 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xfwd(KArgs<R> a) {
     C2<R>* rb = buf + r * X::PL;
     const size_t boff = blockIdx.y * a.bstride;
     const C2<R>* f2 = reinterpret_cast<const C2<R>*>(a.phys0) + boff + (size_t)(iy0 + r) * H;
+    C2<R> f[1][8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) rb[pad8(t + q * X::G)] = f2[t + q * X::G];
-    __syncthreads();
-    row_r2c<R, H>(rb, a.twR, a.twX, t);
+    for (int q = 0; q < 8; ++q) f[0][q] = f2[t + q * X::G];
+    row_r2c_reg<R, H, 1>(f, rb, 0, a.twR, a.twX, t);
     C2<R>* T = a.spec0 + boff;
     for (int i = threadIdx.x; i < H * X::TR; i += blockDim.x) {
         const int rr = i % X::TR, kx = i / X::TR;
@@ -296,10 +323,11 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xinv(KArgs<R> a) {
     load_tileT<R, H, X::TR, X::PL>(buf, a.spec0 + boff, ny, iy0);
     cp_async_wait_f();
     __syncthreads();
-    row_c2r<R, H>(rb, a.twR, a.twX, t);
+    C2<R> f[1][8];
+    row_c2r_reg<R, H, 1>(rb, 0, a.twR, a.twX, t, f);
     C2<R>* f2 = reinterpret_cast<C2<R>*>(a.phys0) + boff + (size_t)(iy0 + r) * H;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) f2[t + q * X::G] = rb[pad8(t + q * X::G)];
+    for (int q = 0; q < 8; ++q) f2[t + q * X::G] = f[0][q];
 }
 
 // forward y of spec0 (T) -> spec1 (S), scaled by 1/(nx ny), ky = ny/2 zeroed
@@ -311,17 +339,16 @@ __global__ void __launch_bounds__(NY / 8) k_yfwd(KArgs<R> a) {
     const int kx = blockIdx.x, t = threadIdx.x;
     const size_t boff = blockIdx.y * a.bstride;
     const C2<R>* in = a.spec0 + boff + (size_t)kx * NY;
+    C2<R> f[1][8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) buf[pad8(t + q * G)] = in[t + q * G];
-    __syncthreads();
-    block_fft<R, NY, false>(buf, a.twY, t);
-    const R norm = (R)a.g.inv_nxny;
+    for (int q = 0; q < 8; ++q) f[0][q] = in[t + q * G];
+    block_fft_reg_m<R, NY, false, 1>(f, buf, 0, a.twY, t, a.enorm);
+    const R norm = kIsF32<R> ? (R)a.g.inv_nxny : (R)1;  // (FP64: scaled by the transform)
     C2<R>* out = a.spec1 + boff + (size_t)kx * NY;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int ky = t + q * G;
-        C2<R> z = buf[pad8(ky)];
-        out[ky] = (ky == NY / 2) ? mk<R>(0, 0) : cscale<R>(z, norm);
+        out[ky] = (ky == NY / 2) ? mk<R>(0, 0) : (kIsF32<R> ? cscale<R>(f[0][q], norm) : f[0][q]);
     }
 }
 
@@ -335,6 +362,7 @@ __global__ void __launch_bounds__(NY / 8) k_yinv(KArgs<R> a) {
     const size_t boff = blockIdx.y * a.bstride;
     const C2<R>* in = a.spec1 + boff + (size_t)kx * NY;
     const Geometry& g = a.g;
+    C2<R> f[1][8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int ky = t + q * G;
@@ -352,13 +380,12 @@ __global__ void __launch_bounds__(NY / 8) k_yinv(KArgs<R> a) {
             }
         }
         if (ky == NY / 2) o = mk<R>(0, 0);
-        buf[pad8(ky)] = o;
+        f[0][q] = o;
     }
-    __syncthreads();
-    block_fft<R, NY, true>(buf, a.twY, t);
+    block_fft_reg_m<R, NY, true, 1>(f, buf, 0, a.twY, t);
     C2<R>* out = a.spec0 + boff + (size_t)kx * NY;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) out[t + q * G] = buf[pad8(t + q * G)];
+    for (int q = 0; q < 8; ++q) out[t + q * G] = f[0][q];
 }
 
 // ======================================================================================
@@ -378,8 +405,8 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_vel_x(KArgs<R> a) {
     load_tileT<R, H, X::TR, X::PL>(bufB, a.Tv, ny, iy0);
     cp_async_wait_f();
     __syncthreads();
-    row_c2r<R, H>(bufA + r * X::PL, a.twR, a.twX, t);
-    row_c2r<R, H>(bufB + r * X::PL, a.twR, a.twX, t);
+    C2<R> uv[2][8];
+    row_c2r_reg<R, H, 2>(bufA + r * X::PL, X::TR * X::PL, a.twR, a.twX, t, uv);
     const R U = (R)a.S->mean_u_next, V = (R)a.S->mean_v_next;
     const int iy = iy0 + r;
     C2<R>* u2 = reinterpret_cast<C2<R>*>(a.u) + (size_t)iy * H;
@@ -388,7 +415,7 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_vel_x(KArgs<R> a) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int m = t + q * X::G;
-        C2<R> ur = bufA[r * X::PL + pad8(m)], vr = bufB[r * X::PL + pad8(m)];
+        C2<R> ur = uv[0][q], vr = uv[1][q];
         C2<R> uu = mk<R>(ur.x + U, ur.y + U);
         C2<R> vv = mk<R>(-vr.x + V, -vr.y + V);
         if constexpr (kIsF32<R>) {  // FP32 form keeps the k=0 mean flow out of the stored field
@@ -464,7 +491,7 @@ __device__ __forceinline__ void nl_x_tile(const KArgs<R>& a, const int iy0) {
         load_tileT<R, H, X::TR, X::PL>(bufB, a.Tdy, ny, iy0, kin);
         cp_async_wait_f();
         __syncthreads();
-        row_c2r_reg<R, H, 2>(ra, BS, a.twR, a.twX, t, dxy);  // both together, to registers
+        step_c2r<R, H, 2>(a, ra, BS, t, dxy);  // both together, to registers
     }
     // the vorticity sponge: the vorticity itself (x inverse of Tw, the inverse-y transform of the
     // state that k_nl_y left), for the term -F(mask_sponge omega) of cal_nlk
@@ -474,7 +501,7 @@ __device__ __forceinline__ void nl_x_tile(const KArgs<R>& a, const int iy0) {
         load_tileT<R, H, X::TR, X::PL>(bufA, a.Tw, ny, iy0, kin);
         cp_async_wait_f();
         __syncthreads();
-        row_c2r_reg<R, H, 1>(ra, BS, a.twR, a.twX, t, om);
+        step_c2r<R, H, 1>(a, ra, BS, t, om);
     }
     const int iy = iy0 + r;
     const size_t roff = (size_t)iy * H;
@@ -505,9 +532,15 @@ __device__ __forceinline__ void nl_x_tile(const KArgs<R>& a, const int iy0) {
             }
         }
         if (pen) {
-            const C2<R> kk = k2[m], mx = x2[m], my = y2[m];
-            pxv[q] = mk<R>(-kk.x * (uu.x - mx.x), -kk.y * (uu.y - mx.y));
-            pyv[q] = mk<R>(-kk.x * (vv.x - my.x), -kk.y * (vv.y - my.y));
+            const C2<R> kk = k2[m];
+            if (kIsF32<R> || !(is_zero(kk.x) && is_zero(kk.y))) {
+                const C2<R> mx = x2[m], my = y2[m];
+                pxv[q] = mk<R>(-kk.x * (uu.x - mx.x), -kk.y * (uu.y - mx.y));
+                pyv[q] = mk<R>(-kk.x * (vv.x - my.x), -kk.y * (vv.y - my.y));
+            } else {  // outside the mask: no term, and none of its FP64 arithmetic
+                pxv[q] = mk<R>(0, 0);
+                pyv[q] = mk<R>(0, 0);
+            }
             if constexpr (SPG == 2) {
                 const C2<R> si = reinterpret_cast<const C2<R>*>(a.s10)[roff + m];
                 pxv[q] = mk<R>(pxv[q].x + si.x, pxv[q].y + si.y);
@@ -522,17 +555,17 @@ __device__ __forceinline__ void nl_x_tile(const KArgs<R>& a, const int iy0) {
     if constexpr (PART == NL_WHOLE) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) { fw[0][q] = wv[q]; fw[1][q] = pyv[q]; fw[2][q] = pxv[q]; }
-        row_r2c_reg<R, H, 3>(fw, ra, BS, a.twR, a.twX, t);  // into buffers A, B and C together
+        step_r2c<R, H, 3>(a, fw, ra, BS, t);  // into buffers A, B and C together
     } else if constexpr (PART == NL_ADVECT) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) fw[0][q] = wv[q];
-        row_r2c_reg<R, H, 1>(fw, ra, BS, a.twR, a.twX, t);
+        step_r2c<R, H, 1>(a, fw, ra, BS, t);
     } else {
         // the penalization's y and x components into the buffers A and B (the whole kernel's
         // B and C)
 #pragma unroll
         for (int q = 0; q < 8; ++q) { fw[0][q] = pyv[q]; fw[1][q] = pxv[q]; }
-        row_r2c_reg<R, H, 2>(fw, ra, BS, a.twR, a.twX, t);
+        step_r2c<R, H, 2>(a, fw, ra, BS, t);
     }
     // the right-hand side only matters where the update keeps modes (kx < kcut):
     // A = X(w) + i kx X(pen_y), B = X(pen_x); the advection part writes X(w) and a zero B,
@@ -662,16 +695,24 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
         fab[0][q] = a.A[row + t + q * G];
         fab[1][q] = a.B[row + t + q * G];
     }
-    block_fft_reg_m<R, NY, false, 2>(fab, bufA, padded_len(NY), a.twY, t);  // A and B together
+    block_fft_reg_m<R, NY, false, 2>(fab, bufA, padded_len(NY), a.twY, t, a.enorm);  // A and B together
     if constexpr (kIsF32<R>) {
         cp_async_wait_f();
         __syncthreads();
+    }
+    // FP64 form: the row's state, loaded before it is needed
+    C2<R> wo[8], mo[8];
+    if constexpr (!kIsF32<R>) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) { wo[q] = a.W[row + t + q * G]; mo[q] = a.M[row + t + q * G]; }
     }
     const DevScalars* S = a.S;
     const double dt1 = S->dt1, b10 = S->b10, b11 = S->b11;
     const bool expl = S->explicit_step != 0;
     const double norm = g.inv_nxny;
     const int cut = a.dcut[kx];
+    double kx2 = 0.0, etx = 0.0;
+    if constexpr (!kIsF32<R>) { kx2 = __dmul_rn((double)(kx * kx), g.scalex); etx = a.etab[kx]; }
     C2<R> wn[8], ps[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -679,10 +720,10 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
         const int ks = signed_k(ky, NY);
         const int ka = ks < 0 ? -ks : ks;
         const bool nyq = (ky == NY / 2);
-        const R kys = (R)ks * (R)g.kys;
+        const R kys = ky_wave<R>(a, ky, ks);
         const C2<R> fa = fab[0][q], fb = fab[1][q];
         C2<R> N = csub<R>(fa, cimul<R>(fb, kys));
-        N = cscale<R>(N, (R)norm);
+        if constexpr (kIsF32<R>) N = cscale<R>(N, (R)norm);  // (FP64: scaled by the transform)
         if (nyq) N = mk<R>(0, 0);
         const bool keep = (g.idealis != 1) || (ka < cut);
         C2<R> Wn, Mn;
@@ -708,25 +749,26 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
             a.Wlo[row + ky] = mk<R>(l0, l1);
             Mn = cscale<R>(N, Eh);
         } else {
-            const R E1 = a.etab[kx] * a.etab[g.hx + ka];
-            const R D = keep ? (R)1 : (R)0;
-            const C2<R> Wo = a.W[row + ky];
+            const R E1 = etx * __ldg(&a.etab[g.hx + ka]);
+            const C2<R> Wo = wo[q];
             if (expl) {
-                Wn = mk<R>((Wo.x + (R)dt1 * N.x) * E1 * D, (Wo.y + (R)dt1 * N.y) * E1 * D);
+                Wn = mk<R>((Wo.x + (R)dt1 * N.x) * E1, (Wo.y + (R)dt1 * N.y) * E1);
             } else {
-                const C2<R> Mo = a.M[row + ky];
-                Wn = mk<R>(((Wo.x + (R)b10 * N.x) + (R)b11 * Mo.x) * E1 * D, ((Wo.y + (R)b10 * N.y) + (R)b11 * Mo.y) * E1 * D);
+                const C2<R> Mo = mo[q];
+                Wn = mk<R>(((Wo.x + (R)b10 * N.x) + (R)b11 * Mo.x) * E1, ((Wo.y + (R)b10 * N.y) + (R)b11 * Mo.y) * E1);
             }
-            if (nyq) Wn = mk<R>(0, 0);
+            if (!keep || nyq) Wn = mk<R>(0, 0);
             Mn = cscale<R>(N, E1);
         }
         a.W[row + ky] = Wn;
         a.M[row + ky] = Mn;
         wn[q] = Wn;
-        const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
-        if (kx == 0 && ky == 0) ps[q] = mk<R>(0, 0);
-        else if constexpr (kIsF32<R>) ps[q] = cscale<R>(Wn, (R)1 / k2);
-        else ps[q] = mk<R>(Wn.x / k2, Wn.y / k2);   // poisson.f90:159-162 divides
+        if constexpr (kIsF32<R>) {
+            const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
+            ps[q] = (kx == 0 && ky == 0) ? mk<R>(0, 0) : cscale<R>(Wn, (R)1 / k2);
+        } else {
+            ps[q] = (kx == 0 && ky == 0) ? mk<R>(0, 0) : over_k2(a, Wn, kx2, kx, ka);
+        }
     }
     // inverse-y outputs, NBO at a time: their transforms share the stages' synchronisations and
     // twiddle loads (NBO buffers of shared memory).  In the FP32 form the factor i kx, constant
@@ -740,7 +782,7 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
     constexpr int NBO = kIsF32<R> ? 5 : 2;
     static_assert(NBO <= nl_y_bufs<R>(), "one shared-memory row buffer per transform");
     constexpr int PLY = padded_len(NY);
-    const R kxs = (R)kx * (R)g.kxs;
+    const R kxs = kIsF32<R> ? (R)kx * (R)g.kxs : kx_wave<R>(a, kx);
     // spectra: 0 cofdy psi, 1 cofdx psi, 2 omega, 3 cofdy omega, 4 (kx^2 - ky^2) psi, and in
     // the FP64 form 5 cofdx omega, 6 d2psi/dxdy
     const int ntr = kIsF32<R> ? (a.viscous ? 5 : 4) : (a.viscous ? 7 : 5);
@@ -756,7 +798,7 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
             for (int q = 0; q < 8; ++q) {
                 const int ky = t + q * G;
                 const int ks = signed_k(ky, NY);
-                const R kys = (R)ks * (R)g.kys;
+                const R kys = ky_wave<R>(a, ky, ks);
                 C2<R> val;
                 // (FP64 without the stresses: spectra 0..3 and 5; sp 4 stands for 5 there)
                 const int spk = (!kIsF32<R> && !a.viscous && sp == 4) ? 5 : sp;
@@ -828,9 +870,9 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
     const double time = S->time, dt1 = S->dt1;
     const R U = (R)S->mean_u_next, V = (R)S->mean_v_next;
     const int ixmin = S->win[0], ixmax = S->win[1], iymin = S->win[2], iymax = S->win[3];
-    // FP32 form: time_avg_vort's weights time / (time + dt) and dt / (time + dt), once a block
-    __shared__ float vm_w[2];
-    if (kIsF32<R> && threadIdx.x == 0) { vm_w[0] = (float)(time / (time + dt1)); vm_w[1] = (float)(dt1 / (time + dt1)); }
+    // time_avg_vort's weights time / (time + dt) and dt / (time + dt), once a block
+    __shared__ R vm_w[2];
+    if (threadIdx.x == 0) { vm_w[0] = (R)(time / (time + dt1)); vm_w[1] = (R)(dt1 / (time + dt1)); }
 
     load_tileT<R, H, X::TR, X::PL>(bufA, a.Tu, ny, iy0, a.kcut);
     load_tileT<R, H, X::TR, X::PL>(bufB, a.Tv, ny, iy0, a.kcut);
@@ -840,7 +882,7 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
     // u, v and omega together, this thread's elements m = t + q G to registers (the row buffers
     // are free afterwards)
     C2<R> uvw[3][8];
-    row_c2r_reg<R, H, 3>(ra, BS, a.twR, a.twX, t, uvw);
+    step_c2r<R, H, 3>(a, ra, BS, t, uvw);
     C2<R> uv[8], vv[8], wv[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -924,46 +966,62 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
             cols[s * X::THREADS + threadIdx.x] = (s == RED_INFLOW_MEAN) ? spx : f[s];
         cols[RED_NSLOTS * X::THREADS + threadIdx.x] = spy;
     } else {
+    // FP64 form: thirteen FP64 instructions a cell outside the mask, where the penalization and its
+    // sums add nothing and are left out (a comparison or a conversion would take the FP64 pipe as
+    // long as an addition: the mask's test and the maximum are on the bits)
+    const R ca = vm_w[0], cb = vm_w[1];
+    long long um = 0;  // bits of the largest |u|^2; NaN is passed over, as fmax does
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int m = t + q * X::G;
-        const C2<R> uu = uv[q], vq = vv[q], w = wv[q];
+        const C2<R> ur = uvw[0][q], vr = uvw[1][q], uu = uv[q], vq = vv[q], w = wv[q];
         u2[m] = uu;
         v2[m] = vq;
-        const C2<R> kk = k2[m], mx = x2[m], my = y2[m];
+        const C2<R> kk = k2[m];
         const C2<R> vmo = vm2[m];
-        R px[2], py[2];
         const R uc[2] = {uu.x, uu.y}, vc[2] = {vq.x, vq.y}, wc[2] = {w.x, w.y};
-        const R kc[2] = {kk.x, kk.y}, xc[2] = {mx.x, mx.y}, yc[2] = {my.x, my.y}, vmc[2] = {vmo.x, vmo.y};
+        const R upc[2] = {ur.x, ur.y}, vpc[2] = {vr.x, vr.y};
+        R px[2] = {0, 0}, py[2] = {0, 0};
+        if (!(is_zero(kk.x) && is_zero(kk.y))) {
+            const C2<R> mx = x2[m], my = y2[m];
+            const R kc[2] = {kk.x, kk.y}, xc[2] = {mx.x, mx.y}, yc[2] = {my.x, my.y};
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int ix = 2 * m + e;
+                const R rx = uc[e] - xc[e], ry = vc[e] - yc[e];
+                const R penx = kc[e] * rx, peny = kc[e] * ry;
+                acc[RED_POROUS] += (double)(kc[e] * (rx * rx + ry * ry));
+                acc[RED_INFLOW_SOLID] += (double)(kc[e] * (xc[e] * rx + yc[e] * ry));
+                acc[RED_INFLOW_MEAN] += Ud * (double)penx + Vd * (double)peny;
+                if (in_rows && ix >= ixmin && ix <= ixmax) {
+                    acc[RED_DRAG_X] += (double)penx;
+                    acc[RED_DRAG_Y] += (double)peny;
+                    acc[RED_UNST_X] += (double)(xc[e] * kc[e]);
+                    acc[RED_UNST_Y] += (double)(yc[e] * kc[e]);
+                }
+                px[e] = penx;
+                py[e] = peny;
+            }
+        }
+        const R vmc[2] = {vmo.x, vmo.y};
         R vmn[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const int ix = 2 * m + e;
-            const R rx = uc[e] - xc[e], ry = vc[e] - yc[e];
-            const R penx = kc[e] * rx, peny = kc[e] * ry;
             acc[RED_OMEGA2] += (double)(wc[e] * wc[e]);
-            const double du = (double)uc[e] - Ud, dv = (double)vc[e] - Vd;
-            acc[RED_KIN] += du * du + dv * dv;
-            acc[RED_POROUS] += (double)(kc[e] * (rx * rx + ry * ry));
-            acc[RED_INFLOW_SOLID] += (double)(kc[e] * (xc[e] * rx + yc[e] * ry));
-            acc[RED_INFLOW_MEAN] += Ud * (double)penx + Vd * (double)peny;
+            acc[RED_KIN] += (double)(upc[e] * upc[e] + vpc[e] * vpc[e]);
             acc[RED_SUM_U] += (double)uc[e];
             acc[RED_SUM_V] += (double)vc[e];
-            acc[RED_UMAX2] = fmax(acc[RED_UMAX2], (double)(uc[e] * uc[e] + vc[e] * vc[e]));
-            if (in_rows && ix >= ixmin && ix <= ixmax) {
-                acc[RED_DRAG_X] += (double)penx;
-                acc[RED_DRAG_Y] += (double)peny;
-                acc[RED_UNST_X] += (double)(xc[e] * kc[e]);
-                acc[RED_UNST_Y] += (double)(yc[e] * kc[e]);
-            }
-            vmn[e] = (R)(((double)vmc[e] * time + dt1 * (double)wc[e]) / (time + dt1));
-            px[e] = penx - wc[e] * vc[e];
-            py[e] = peny + wc[e] * uc[e];
+            const long long ub = __double_as_longlong((double)(uc[e] * uc[e] + vc[e] * vc[e]));
+            if (ub > um && ub <= 0x7ff0000000000000LL) um = ub;
+            vmn[e] = vmc[e] * ca + wc[e] * cb;
+            px[e] = px[e] - wc[e] * vc[e];
+            py[e] = py[e] + wc[e] * uc[e];
         }
         vm2[m] = mk<R>(vmn[0], vmn[1]);
         pxy[0][q] = mk<R>(px[0], px[1]);
         pxy[1][q] = mk<R>(py[0], py[1]);
     }
+    acc[RED_UMAX2] = __longlong_as_double(um);
     }
     // block reduction in a fixed order: every thread's partials go to the spare row buffer as
     // columns; one warp per column sums it in FP64 (its lanes over the column, then a shuffle
@@ -1004,7 +1062,7 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
         if (blockIdx.x == 0 && s == 0) a.S->nred = (int)gridDim.x;
     }
     if (a.pressure_on) {
-        row_r2c_reg<R, H, 2>(pxy, ra, BS, a.twR, a.twX, t);  // x and y parts together
+        step_r2c<R, H, 2>(a, pxy, ra, BS, t);  // x and y parts together
         for (int i = threadIdx.x; i < H * X::TR; i += blockDim.x) {
             const int rr = i % X::TR, kx = i / X::TR;
             const R kxs = kx_wave<R>(a, kx);
@@ -1020,14 +1078,15 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
         load_tileT<R, H, X::TR, X::PL>(bufB, a.Tsb, ny, iy0, a.kcut);
         cp_async_wait_f();
         __syncthreads();
-        row_c2r_m<R, H, 2>(ra, BS, a.twR, a.twX, t);  // ra and rb together
+        C2<R> sv[2][8];
+        step_c2r<R, H, 2>(a, ra, BS, t, sv);
         C2<R>* sa2 = reinterpret_cast<C2<R>*>(a.sa) + roff;
         C2<R>* sb2 = reinterpret_cast<C2<R>*>(a.sb) + roff;
         const R c2 = (R)(2.0 * a.nu), c1 = (R)a.nu;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int m = t + q * X::G;
-            const C2<R> x = ra[pad8(m)], y = rb[pad8(m)];
+            const C2<R> x = sv[0][q], y = sv[1][q];
             sa2[m] = mk<R>(c2 * x.x, c2 * x.y);
             sb2[m] = mk<R>(c1 * y.x, c1 * y.y);
         }
@@ -1228,7 +1287,7 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k
     cp_async_wait_f();
     __syncthreads();
     C2<R> sv[2][8];
-    row_c2r_reg<R, H, 2>(ra, BS, a.twR, a.twX, t, sv);  // both together, to registers
+    step_c2r<R, H, 2>(a, ra, BS, t, sv);  // both together, to registers
     const size_t roff = (size_t)(iy0 + r) * H;
     C2<R>* sa2 = reinterpret_cast<C2<R>*>(a.sa) + roff;
     C2<R>* sb2 = reinterpret_cast<C2<R>*>(a.sb) + roff;
@@ -1312,20 +1371,26 @@ __global__ void __launch_bounds__(press_y_threads<R, NY, ENG>(), (kIsF32<R> && N
         fp[0][q] = a.P1[row + t + q * G];
         fp[1][q] = a.P2[row + t + q * G];
     }
-    block_fft_reg_m<R, NY, false, 2>(fp, bufA, padded_len(NY), a.twY, t);  // P1 and P2 together
+    block_fft_reg_m<R, NY, false, 2>(fp, bufA, padded_len(NY), a.twY, t, a.enorm);  // P1 and P2 together
     const R norm = (R)g.inv_nxny;
+    double kx2 = 0.0;
+    if constexpr (!kIsF32<R>) kx2 = __dmul_rn((double)(kx * kx), g.scalex);
     C2<R> qv[1][8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int ky = t + q * G;
         const int ks = signed_k(ky, NY);
-        const R kys = (R)ks * (R)g.kys;
-        C2<R> Q = cadd<R>(cscale<R>(fp[0][q], norm), cimul<R>(cscale<R>(fp[1][q], norm), kys));
-        const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
+        const R kys = ky_wave<R>(a, ky, ks);
         C2<R> qh;
+        if constexpr (kIsF32<R>) {
+            const C2<R> Q = cadd<R>(cscale<R>(fp[0][q], norm), cimul<R>(cscale<R>(fp[1][q], norm), kys));
+            const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
+            qh = cscale<R>(Q, (R)1 / k2);
+        } else {
+            const C2<R> Q = cadd<R>(fp[0][q], cimul<R>(fp[1][q], kys));  // scaled by the transform
+            qh = over_k2(a, Q, kx2, kx, ks < 0 ? -ks : ks);
+        }
         if (kx == 0 && ky == 0) qh = mk<R>(0, 0);
-        else if constexpr (kIsF32<R>) qh = cscale<R>(Q, (R)1 / k2);
-        else qh = mk<R>(Q.x / k2, Q.y / k2);
         if (ky == NY / 2) qh = mk<R>(0, 0);
         qv[0][q] = qh;
     }
@@ -1363,7 +1428,7 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k
     cp_async_wait_f();
     __syncthreads();
     C2<R> qv[1][8];
-    row_c2r_reg<R, H, 1>(rb, X::PL, a.twR, a.twX, t, qv);  // to registers
+    step_c2r<R, H, 1>(a, rb, X::PL, t, qv);  // to registers
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int m = t + q * X::G;
