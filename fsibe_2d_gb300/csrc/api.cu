@@ -632,34 +632,30 @@ template <> SizeKernels<float>& ky_of<float>(fsibe_ctx* c) { return c->kyf; }
 
 // launch helpers (count launches for the bench's gpu_launches)
 template <typename R>
-static void launch_x(fsibe_ctx* c, void (*k)(KArgs<R>), int smem, const KArgs<R>& a, const char* name = "x_pass",
-                     int nfields = 1) {
-    const SizeKernels<R>& K = kx_of<R>(c);
+static void launch_x(fsibe_ctx* c, const KLaunch<R>& k, const KArgs<R>& a, const char* name = "x_pass", int nfields = 1) {
     prof_begin(c, name);
-    k<<<dim3(c->g.ny / K.x_rows, nfields), K.x_threads, smem, c->stream>>>(a);
+    k.k<<<dim3(c->g.ny / kx_of<R>(c).x_rows, nfields), k.threads, k.smem, c->stream>>>(a);
     prof_end(c);
     c->launches++;
 }
 template <typename R>
 // pdl: a programmatic dependent launch (only for kernels that begin with pdl_wait)
-static void launch_y(fsibe_ctx* c, void (*k)(KArgs<R>), int smem, const KArgs<R>& a, const char* name = "y_pass",
-                     int nfields = 1, bool pdl = false, int threads = 0) {
-    const SizeKernels<R>& K = ky_of<R>(c);
+static void launch_y(fsibe_ctx* c, const KLaunch<R>& k, const KArgs<R>& a, const char* name = "y_pass", int nfields = 1,
+                     bool pdl = false) {
     prof_begin(c, name);
-    launch_k(k, dim3(c->g.hx, nfields), dim3(threads > 0 ? threads : K.y_threads), smem, c->stream, pdl && c->pdl, a);
+    launch_k(k.k, dim3(c->g.hx, nfields), dim3(k.threads), k.smem, c->stream, pdl && c->pdl, a);
     prof_end(c);
     c->launches++;
 }
 
-// a fused x kernel with one of its tile-height variants (nbuf row buffers of shared memory);
-// on the main stream a programmatic dependent launch (the fused x kernels begin with pdl_wait)
+// a fused x kernel of one of the tile-height variants (rows a block); on the main stream a
+// programmatic dependent launch (the fused x kernels begin with pdl_wait)
 template <typename R>
-static void launch_xv(fsibe_ctx* c, void (*k)(KArgs<R>), const typename SizeKernels<R>::XVariant& v, int nbuf,
-                      const KArgs<R>& a, const char* name, cudaStream_t st = nullptr, int grid = 0) {
+static void launch_xv(fsibe_ctx* c, const KLaunch<R>& k, int rows, const KArgs<R>& a, const char* name,
+                      cudaStream_t st = nullptr, int grid = 0) {
     if (!st) st = c->stream;
     prof_begin(c, name, st);
-    launch_k(k, dim3(grid > 0 ? grid : c->g.ny / v.rows), dim3(v.threads), nbuf == 3 ? v.smem3 : nbuf * v.smem1, st,
-             c->pdl && st == c->stream, a);
+    launch_k(k.k, dim3(grid > 0 ? grid : c->g.ny / rows), dim3(k.threads), k.smem, st, c->pdl && st == c->stream, a);
     prof_end(c, st);
     c->launches++;
 }
@@ -807,7 +803,7 @@ static void nl_advect_t(fsibe_ctx* c, int explicit_step) {
     // a run with the vorticity sponge takes the default tile, the one instantiated with it
     const auto& V = c->spg ? KX.xv[1] : KX.xv[c->xv_nl];
     const int tiles = c->g.ny / V.rows;
-    launch_xv<R>(c, c->spg ? V.nl_adv_spg : V.nl_adv, V, 2, a, "nl_adv", c->side2,
+    launch_xv<R>(c, c->spg ? V.nl_adv_spg : V.nl_adv, V.rows, a, "nl_adv", c->side2,
                  tiles <= 2 * c->nsm ? (tiles < c->nsm ? tiles : c->nsm) : tiles);
 }
 
@@ -845,17 +841,17 @@ static int fluid_step_t(fsibe_ctx* c, int explicit_step, bool adv_forked = false
         KArgs<R> p = a;
         // walls, sponges and the outflow sponge's integral: every row is penalized
         p.rect = (c->full_mask || c->s10) ? c->rect_full : c->rect;
-        if (c->s10) launch_xv<R>(c, KX.xv[1].nl_pen_s10, KX.xv[1], 2, p, "nl_pen");
-        else launch_xv<R>(c, KX.xv[c->xv_nl].nl_pen, KX.xv[c->xv_nl], 2, p, "nl_pen");
+        if (c->s10) launch_xv<R>(c, KX.xv[1].nl_pen_s10, KX.xv[1].rows, p, "nl_pen");
+        else launch_xv<R>(c, KX.xv[c->xv_nl].nl_pen, KX.xv[c->xv_nl].rows, p, "nl_pen");
     } else if (c->spg) {
-        launch_xv<R>(c, KX.xv[1].nl_x_spg, KX.xv[1], 3, a, "nl_x");  // the default tile carries the sponge
+        launch_xv<R>(c, KX.xv[1].nl_x_spg, KX.xv[1].rows, a, "nl_x");  // the default tile carries the sponge
     } else if (c->s10) {
-        launch_xv<R>(c, KX.xv[1].nl_x_s10, KX.xv[1], 3, a, "nl_x");
+        launch_xv<R>(c, KX.xv[1].nl_x_s10, KX.xv[1].rows, a, "nl_x");
     } else {
-        launch_xv<R>(c, KX.xv[c->xv_nl].nl_x, KX.xv[c->xv_nl], 3, a, "nl_x");
+        launch_xv<R>(c, KX.xv[c->xv_nl].nl_x, KX.xv[c->xv_nl].rows, a, "nl_x");
     }
     CK(c, cudaStreamWaitEvent(c->stream, c->ev_sb, 0));
-    launch_y<R>(c, KY.nl_y, KY.y_smem_nl, a, "nl_y", 1, true);
+    launch_y<R>(c, KY.nl_y, a, "nl_y", 1, true);
     if (a.viscous && c->stress_split) {
         // the viscous stresses, read only by GetForces, on the second side stream beside the
         // pressure kernels (joined with ev_ffj below)
@@ -864,14 +860,14 @@ static int fluid_step_t(fsibe_ctx* c, int explicit_step, bool adv_forked = false
         KArgs<R> s = a;
         s.srows = (stress_rows && c->P.iBeam > 0) ? 1 : 0;  // the row range k_step_begin formed
         const int vs = c->xv_px < 4 ? c->xv_px : 1;  // the paired press_x leaves the stresses to the default tile
-        launch_xv<R>(c, KX.xv[vs].stress_x, KX.xv[vs], 2, s, "stress_x", c->side2);
+        launch_xv<R>(c, KX.xv[vs].stress_x, KX.xv[vs].rows, s, "stress_x", c->side2);
         a.stress_split = 1;
     }
-    if (c->xv_px == 4 && KX.xp.press_x && (a.stress_split || !a.viscous))
-        launch_xv<R>(c, KX.xp.press_x, KX.xp, 3, a, "press_x");  // the paired FP32 kernel
+    if (c->xv_px == 4 && KX.xp.press_x.k && (a.stress_split || !a.viscous))
+        launch_xv<R>(c, KX.xp.press_x, KX.xp.rows, a, "press_x");  // the paired FP32 kernel
     else {
         const int vp = c->xv_px < 4 ? c->xv_px : 1;
-        launch_xv<R>(c, KX.xv[vp].press_x, KX.xv[vp], 3, a, "press_x");
+        launch_xv<R>(c, KX.xv[vp].press_x, KX.xv[vp].rows, a, "press_x");
     }
     // the energies, drag and unsteady forces from press_x's partial sums feed only scalars read
     // after the fluid step: a second side stream runs them beside the pressure transforms
@@ -890,13 +886,13 @@ static int fluid_step_t(fsibe_ctx* c, int explicit_step, bool adv_forked = false
         CK(c, cudaEventRecord(c->ev_adv, c->side2));
     }
     if (a.pressure_on) {
-        if (c->py_eng == 1 && KY.press_y1)  // the one-butterfly engine, where the autotuner found it faster
-            launch_y<R>(c, KY.press_y1, KY.press_y1_smem, a, "press_y", 1, true, KY.y_threads);
+        if (c->py_eng == 1 && KY.press_y1.k)  // the one-butterfly engine, where the autotuner found it faster
+            launch_y<R>(c, KY.press_y1, a, "press_y", 1, true);
         else
-            launch_y<R>(c, KY.press_y, KY.y_smem2, a, "press_y", 1, true, KY.press_y_threads);
+            launch_y<R>(c, KY.press_y, a, "press_y", 1, true);
         KArgs<R> f = a;
         f.srows = (stress_rows && c->P.iBeam > 0) ? 1 : 0;  // the forces' rows only (k_press_fin)
-        launch_xv<R>(c, KX.xv[c->xv_fin].press_fin, KX.xv[c->xv_fin], 1, f, "press_fin");
+        launch_xv<R>(c, KX.xv[c->xv_fin].press_fin, KX.xv[c->xv_fin].rows, f, "press_fin");
     } else {
         CK(c, cudaMemsetAsync(c->phys[PH_PRESS], 0, sizeof(R) * (size_t)c->g.nx * c->g.ny, c->stream));
     }
@@ -1100,7 +1096,7 @@ template <typename R>
 static int press_full_t(fsibe_ctx* c) {
     KArgs<R> a = kargs<R>(c);
     SizeKernels<R>& KX = kx_of<R>(c);
-    launch_xv<R>(c, KX.xv[c->xv_fin].press_fin, KX.xv[c->xv_fin], 1, a, "press_fin");
+    launch_xv<R>(c, KX.xv[c->xv_fin].press_fin, KX.xv[c->xv_fin].rows, a, "press_fin");
     CKL(c);
     return FSIBE_OK;
 }
@@ -1262,8 +1258,8 @@ template <typename R>
 static int fwd2d(fsibe_ctx* c, void* spec_out) {
     KArgs<R> a = kargs<R>(c);
     a.spec1 = reinterpret_cast<C2<R>*>(spec_out);
-    launch_x<R>(c, kx_of<R>(c).xfwd, kx_of<R>(c).x_smem1, a);
-    launch_y<R>(c, ky_of<R>(c).yfwd, ky_of<R>(c).y_smem1, a);
+    launch_x<R>(c, kx_of<R>(c).xfwd, a);
+    launch_y<R>(c, ky_of<R>(c).yfwd, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -1274,7 +1270,7 @@ static int inv_y(fsibe_ctx* c, const void* spec_in, void* t_out, int op) {
     a.spec1 = reinterpret_cast<C2<R>*>(const_cast<void*>(spec_in));
     a.spec0 = reinterpret_cast<C2<R>*>(t_out);
     a.op = op;
-    launch_y<R>(c, ky_of<R>(c).yinv, ky_of<R>(c).y_smem1, a);
+    launch_y<R>(c, ky_of<R>(c).yinv, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -1282,7 +1278,7 @@ static int inv_y(fsibe_ctx* c, const void* spec_in, void* t_out, int op) {
 template <typename R>
 static int inv_x(fsibe_ctx* c) {
     KArgs<R> a = kargs<R>(c);
-    launch_x<R>(c, kx_of<R>(c).xinv, kx_of<R>(c).x_smem1, a);
+    launch_x<R>(c, kx_of<R>(c).xinv, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -1298,7 +1294,7 @@ static int sponge10_term(fsibe_ctx* c) {
     KArgs<R> a = kargs<R>(c);
     a.spec0 = reinterpret_cast<C2<R>*>(c->spec[SP_0]);
     a.phys0 = reinterpret_cast<R*>(c->s10_dudx);
-    launch_x<R>(c, kx_of<R>(c).xinv, kx_of<R>(c).x_smem1, a);
+    launch_x<R>(c, kx_of<R>(c).xinv, a);
     k_sponge10<R><<<(c->g.ny + 127) / 128, 128, 0, c->stream>>>(reinterpret_cast<const R*>(c->s10_dudx),
                                                                reinterpret_cast<R*>(c->s10), c->g.nx, c->g.ny,
                                                                c->s10_ixmin, c->s10_ixmax, c->g.dx, 1.0 / c->P.eps_sponge);
@@ -1317,7 +1313,7 @@ static int init_velocity(fsibe_ctx* c) {
     if ((st = inv_y<R>(c, c->spec[SP_W], c->spec[SP_TDY], OP_DY))) return st;
     if ((st = inv_y<R>(c, c->spec[SP_W], c->spec[SP_TW], OP_ID))) return st;  // the sponge's vorticity
     KArgs<R> a = kargs<R>(c);
-    launch_x<R>(c, kx_of<R>(c).vel_x, kx_of<R>(c).x_smem2, a);
+    launch_x<R>(c, kx_of<R>(c).vel_x, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -1394,7 +1390,7 @@ static int pressure_snapshot_t(fsibe_ctx* c, double time, double* host_out) {
         KArgs<R> a = kargs<R>(c);
         a.spec0 = T;
         a.phys0 = out;
-        launch_x<R>(c, KX.xinv, KX.x_smem1, a);
+        launch_x<R>(c, KX.xinv, a);
         return FSIBE_OK;
     };
     auto to_spec = [&](R* in, C2<R>* out) {
@@ -1402,8 +1398,8 @@ static int pressure_snapshot_t(fsibe_ctx* c, double time, double* host_out) {
         a.phys0 = in;
         a.spec0 = T;
         a.spec1 = out;
-        launch_x<R>(c, KX.xfwd, KX.x_smem1, a);
-        launch_y<R>(c, KY.yfwd, KY.y_smem1, a);
+        launch_x<R>(c, KX.xfwd, a);
+        launch_y<R>(c, KY.yfwd, a);
     };
     int st;
     if ((st = to_phys(c->spec[SP_W], OP_U, pu))) return st;
@@ -1457,18 +1453,15 @@ const char* fsibe_last_error(const fsibe_ctx* ctx) { return ctx ? ctx->err.c_str
 // fastest per kernel.  The choice is cached per (precision, nx, ny) for the process, so an
 // ensemble of many runs of one size tunes once.  FSIBE_AUTOTUNE=0 keeps the default tiles.
 template <typename R>
-static float time_xv(fsibe_ctx* c, int kind, const typename SizeKernels<R>::XVariant& v) {
+static float time_kernel(fsibe_ctx* c, const KLaunch<R>& k, int grid) {
     KArgs<R> a = kargs<R>(c);
-    void (*k)(KArgs<R>) = kind == 0 ? v.nl_x : (kind == 1 ? v.press_x : v.press_fin);
-    const int smem = kind == 2 ? v.smem1 : v.smem3;
-    const dim3 grid(c->g.ny / v.rows);
-    for (int i = 0; i < 2; ++i) k<<<grid, v.threads, smem, c->stream>>>(a);
+    for (int i = 0; i < 2; ++i) k.k<<<grid, k.threads, k.smem, c->stream>>>(a);
     // the best of three rounds of five launches (one round's mean moved by up to 10% between
     // processes at 4096^2 and flipped the choice)
     float best = 1e30f;
     for (int round = 0; round < 3; ++round) {
         cudaEventRecord(c->ev0, c->stream);
-        for (int i = 0; i < 5; ++i) k<<<grid, v.threads, smem, c->stream>>>(a);
+        for (int i = 0; i < 5; ++i) k.k<<<grid, k.threads, k.smem, c->stream>>>(a);
         cudaEventRecord(c->ev1, c->stream);
         if (cudaEventSynchronize(c->ev1) != cudaSuccess) return 1e30f;
         float ms = 0.f;
@@ -1477,24 +1470,10 @@ static float time_xv(fsibe_ctx* c, int kind, const typename SizeKernels<R>::XVar
     }
     return best;
 }
-
-// One y-pass kernel over the kx rows, timed as time_xv times the x-pass candidates.
 template <typename R>
-static float time_y(fsibe_ctx* c, void (*k)(KArgs<R>), int smem, int threads) {
-    KArgs<R> a = kargs<R>(c);
-    const dim3 grid(c->g.hx);
-    for (int i = 0; i < 2; ++i) k<<<grid, threads, smem, c->stream>>>(a);
-    float best = 1e30f;
-    for (int round = 0; round < 3; ++round) {
-        cudaEventRecord(c->ev0, c->stream);
-        for (int i = 0; i < 5; ++i) k<<<grid, threads, smem, c->stream>>>(a);
-        cudaEventRecord(c->ev1, c->stream);
-        if (cudaEventSynchronize(c->ev1) != cudaSuccess) return 1e30f;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-        best = ms / 5.f < best ? ms / 5.f : best;
-    }
-    return best;
+static float time_xv(fsibe_ctx* c, int kind, const typename SizeKernels<R>::XVariant& v) {
+    const KLaunch<R>& k = kind == 0 ? v.nl_x : (kind == 1 ? v.press_x : v.press_fin);
+    return time_kernel<R>(c, k, c->g.ny / v.rows);
 }
 
 template <typename R>
@@ -1523,7 +1502,7 @@ static int autotune_x(fsibe_ctx* c) {
         }
         // FP32: the paired press_x (index 4), when its tile (128 threads: 128 / (H/16) rows)
         // divides the grid's rows
-        if (kind == 1 && K.xp.press_x && c->g.ny % K.xp.rows == 0) {
+        if (kind == 1 && K.xp.press_x.k && c->g.ny % K.xp.rows == 0) {
             const float t = time_xv<R>(c, kind, K.xp);
             if (t < 0.97f * tbest) { tbest = t; best = 4; }
         }
@@ -1533,9 +1512,9 @@ static int autotune_x(fsibe_ctx* c) {
     // it is faster by 3%
     int eng = 0;
     const SizeKernels<R>& KY = ky_of<R>(c);
-    if (KY.press_y1) {
-        const float t0 = time_y<R>(c, KY.press_y, KY.y_smem2, KY.press_y_threads);
-        const float t1 = time_y<R>(c, KY.press_y1, KY.press_y1_smem, KY.y_threads);
+    if (KY.press_y1.k) {
+        const float t0 = time_kernel<R>(c, KY.press_y, c->g.hx);
+        const float t1 = time_kernel<R>(c, KY.press_y1, c->g.hx);
         if (t1 < 0.97f * t0) eng = 1;
     }
     CKL(c);
@@ -2657,9 +2636,9 @@ static int adj_inv2d(fsibe_ctx* c, const void* spec, int nf, void* phys) {
     a.spec1 = reinterpret_cast<C2<double>*>(const_cast<void*>(spec));
     a.spec0 = reinterpret_cast<C2<double>*>(c->adj->spec[AS_T]);
     a.op = OP_ID;
-    launch_y<double>(c, ky_of<double>(c).yinv, ky_of<double>(c).y_smem1, a, "adj_yinv", nf);
+    launch_y<double>(c, ky_of<double>(c).yinv, a, "adj_yinv", nf);
     a.phys0 = reinterpret_cast<double*>(phys);
-    launch_x<double>(c, kx_of<double>(c).xinv, kx_of<double>(c).x_smem1, a, "adj_xinv", nf);
+    launch_x<double>(c, kx_of<double>(c).xinv, a, "adj_xinv", nf);
     CKL(c);
     return FSIBE_OK;
 }
@@ -2667,7 +2646,7 @@ static int adj_invx(fsibe_ctx* c, const void* T, void* phys) {
     KArgs<double> a = kargs<double>(c);
     a.spec0 = reinterpret_cast<C2<double>*>(const_cast<void*>(T));
     a.phys0 = reinterpret_cast<double*>(phys);
-    launch_x<double>(c, kx_of<double>(c).xinv, kx_of<double>(c).x_smem1, a, "adj_xinv");
+    launch_x<double>(c, kx_of<double>(c).xinv, a, "adj_xinv");
     CKL(c);
     return FSIBE_OK;
 }
@@ -2677,8 +2656,8 @@ static int adj_fwd2d(fsibe_ctx* c, const void* phys, int nf, void* spec) {
     a.phys0 = reinterpret_cast<double*>(const_cast<void*>(phys));
     a.spec0 = reinterpret_cast<C2<double>*>(c->adj->spec[AS_T]);
     a.spec1 = reinterpret_cast<C2<double>*>(spec);
-    launch_x<double>(c, kx_of<double>(c).xfwd, kx_of<double>(c).x_smem1, a, "adj_xfwd", nf);
-    launch_y<double>(c, ky_of<double>(c).yfwd, ky_of<double>(c).y_smem1, a, "adj_yfwd", nf);
+    launch_x<double>(c, kx_of<double>(c).xfwd, a, "adj_xfwd", nf);
+    launch_y<double>(c, ky_of<double>(c).yfwd, a, "adj_yfwd", nf);
     CKL(c);
     return FSIBE_OK;
 }
@@ -3287,8 +3266,8 @@ extern "C" int fsibe_coftxy_static(const double* f_dev, double* fk_dev, int32_t 
     a.spec0 = T;
     a.spec1 = Sx;
     a.twX = twX; a.twR = twR; a.twY = twY;
-    kx.xfwd<<<ny / kx.x_rows, kx.x_threads, kx.x_smem1, st>>>(a);
-    ky.yfwd<<<hx, ky.y_threads, ky.y_smem1, st>>>(a);
+    kx.xfwd.k<<<ny / kx.x_rows, kx.xfwd.threads, kx.xfwd.smem, st>>>(a);
+    ky.yfwd.k<<<hx, ky.yfwd.threads, ky.yfwd.smem, st>>>(a);
     k_pack<double><<<hx, 256, 0, st>>>(Sx, nullptr, fk_dev, nx, ny);
     e = cudaGetLastError();
     if (e != cudaSuccess) { g_err = std::string("fsibe_coftxy_static: ") + cudaGetErrorString(e); return FSIBE_ERR_CUDA; }

@@ -146,8 +146,12 @@ __device__ __forceinline__ void block_fft_reg_m(C2<R> (&v)[NBA][8], C2<R>* buf, 
                                                 const TwF<R>* __restrict__ tw, int t, int ex = 0) {
     static_assert(N >= 16 && (N & (N - 1)) == 0, "power-of-two length >= 16");
     static_assert(NB >= 1 && NB <= NBA, "NB of the NBA rows");
-    if constexpr (sizeof(R) == 8) fx_fft_reg<N, INV, NB>(v, buf, bstride, tw, t, ex);
-    else fft_reg_run<R, N, INV, NB, 1, NBA>(v, buf, bstride, tw, t);
+    if constexpr (sizeof(R) == 8) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) fx_fft<N, INV>(v[b], buf + b * bstride, tw, fx_block_group<N / 8>(t), ex);
+    } else {
+        fft_reg_run<R, N, INV, NB, 1, NBA>(v, buf, bstride, tw, t);
+    }
 }
 
 // ---- paired transforms (FP32): a thread owns two adjacent butterflies -----------------------

@@ -151,34 +151,48 @@ __device__ __forceinline__ double fx_to(long long q, int eb, unsigned nan) {
     return __hiloint2double((int)hi, m == 0 ? 0 : (int)(unsigned)b);
 }
 
-// ---- reductions over the threads of a row ----------------------------------------------------
-// A row's G threads are part of one warp (G <= 32; the rows of a warp then share one scale) or
-// whole warps.  The lanes' maxima (sums) of NB values, over the row's warps; with G > 32 the
-// partials go through slots (the caller synchronises before fx_row_read).
-template <int G> __device__ __forceinline__ unsigned fx_lanes() {
-    return blockDim.x >= 32 ? 0xffffffffu : (1u << blockDim.x) - 1u;
+// ---- the threads of one transform -----------------------------------------------------------
+// A transform of N points is the work of G = N/8 threads: part of a warp, or whole warps with a
+// named barrier of their own (id, from 1 on), so that the transforms of a block do not wait on one
+// another.  slot: G/32 words of shared memory of the group's own, twice (largest values, sums).
+struct FxGroup {
+    int t, id;        // thread of the group; its barrier
+    unsigned* slot;
+};
+// the group of the calling thread in a block whose groups are one row each (t: thread of the row)
+template <int G> __device__ __forceinline__ FxGroup fx_block_group(int t) {
+    __shared__ unsigned slots[64];  // 1024 threads' warps, twice
+    const int g = threadIdx.x / G;
+    return FxGroup{t, g + 1, slots + g * 2 * (G / 32)};
 }
-template <int G, int NB, bool SUM>
-__device__ __forceinline__ void fx_row_reduce(unsigned (&m)[NB], unsigned (*slot)[32]) {
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        m[b] = SUM ? __reduce_add_sync(fx_lanes<G>(), m[b]) : __reduce_max_sync(fx_lanes<G>(), m[b]);
-        if (G > 32 && (threadIdx.x & 31) == 0) slot[b][threadIdx.x >> 5] = m[b];
-    }
+template <int G> __device__ __forceinline__ unsigned fx_mask() {
+    return G >= 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
 }
-template <int G, int NB, bool SUM>
-__device__ __forceinline__ void fx_row_read(unsigned (&m)[NB], const unsigned (*slot)[32]) {
-    if constexpr (G > 32) {
-        constexpr int NW = G / 32;
-        const int w0 = (threadIdx.x >> 5) & ~(NW - 1);
+template <int G> __device__ __forceinline__ void fx_sync(const FxGroup& g) {
+    if constexpr (G > 32) asm volatile("bar.sync %0, %1;" ::"r"(g.id), "n"(G) : "memory");
+    else __syncwarp(fx_mask<G>());
+}
+// the group's largest value (sum) of m; with G > 32 the warps' go to slots, read after a fx_sync
+template <int G, bool SUM> __device__ __forceinline__ unsigned fx_reduce(unsigned m, unsigned* slot) {
+    if constexpr (G >= 32) {
+        m = SUM ? __reduce_add_sync(0xffffffffu, m) : __reduce_max_sync(0xffffffffu, m);
+        if (G > 32 && (threadIdx.x & 31) == 0) slot[(threadIdx.x >> 5) & (G / 32 - 1)] = m;
+    } else {
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            unsigned r = slot[b][w0];
-#pragma unroll
-            for (int w = 1; w < NW; ++w) r = SUM ? r + slot[b][w0 + w] : max(r, slot[b][w0 + w]);
-            m[b] = r;
+        for (int o = G / 2; o > 0; o >>= 1) {
+            const unsigned x = __shfl_xor_sync(fx_mask<G>(), m, o);
+            m = SUM ? m + x : max(m, x);
         }
     }
+    return m;
+}
+template <int G, bool SUM> __device__ __forceinline__ unsigned fx_read(unsigned m, const unsigned* slot) {
+    if constexpr (G > 32) {
+        m = slot[0];
+#pragma unroll
+        for (int w = 1; w < G / 32; ++w) m = SUM ? m + slot[w] : max(m, slot[w]);
+    }
+    return m;
 }
 // The scale of a row from its largest high word: the exponent field that fills its bits, and
 // the NaN bits of a row out of range.
@@ -198,87 +212,67 @@ __device__ __forceinline__ q2 fx_ldrow(const double2* b) { return *reinterpret_c
 __device__ __forceinline__ void fx_strow(double2* b, q2 v) { *reinterpret_cast<q2*>(b) = v; }
 
 // shift, twiddle and butterflies of one stage (radix P, 2^lg = the product of the radices already
-// applied) on v[b][q P + r] (input r of butterfly q)
-template <int N, int P, bool INV, bool TWID, int NB>
-__device__ __forceinline__ void fx_compute(q2 (&v)[NB][8], const int4* __restrict__ tw, int t, int lg, const int (&sh)[NB]) {
+// applied) on v[q P + r] (input r of butterfly q)
+template <int N, int P, bool INV, bool TWID>
+__device__ __forceinline__ void fx_compute(q2 (&v)[8], const int4* __restrict__ tw, int t, int lg, int sh) {
     constexpr int G = N / 8, PER = 8 / P;
+    if (sh > 0) {  // the same for the whole group
+        const int half = (1 << sh) >> 1;
 #pragma unroll
-    for (int b = 0; b < NB; ++b)
-        if (sh[b] > 0) {  // the same for the whole warp
-            const int half = (1 << sh[b]) >> 1;
-#pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                v[b][m].x = fx_shr(v[b][m].x, sh[b], half);
-                v[b][m].y = fx_shr(v[b][m].y, sh[b], half);
-            }
+        for (int m = 0; m < 8; ++m) {
+            v[m].x = fx_shr(v[m].x, sh, half);
+            v[m].y = fx_shr(v[m].y, sh, half);
         }
+    }
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
-        const int k = (t + q * G) & ((1 << lg) - 1);
+        if constexpr (TWID) {
+            const int k = (t + q * G) & ((1 << lg) - 1);
 #pragma unroll
-        for (int r = 1; r < P; ++r) {
-            if (!TWID) continue;
-            int4 w = __ldg(&tw[(r * k * (N / P)) >> lg]);
-            if (INV) { w.z = -w.z; w.w = -w.w; }
-#pragma unroll
-            for (int b = 0; b < NB; ++b) v[b][q * P + r] = fx_cmul(v[b][q * P + r], w);
+            for (int r = 1; r < P; ++r) {
+                int4 w = __ldg(&tw[(r * k * (N / P)) >> lg]);
+                if (INV) { w.z = -w.z; w.w = -w.w; }
+                v[q * P + r] = fx_cmul(v[q * P + r], w);
+            }
         }
-#pragma unroll
-        for (int b = 0; b < NB; ++b) fx_dftp<P, INV>(v[b] + q * P);
+        fx_dftp<P, INV>(v + q * P);
     }
 }
 
-// NB transforms of q values in registers, v[b][m] = element t + m G with moduli below 2^(B0 + 1/2)
-// (a component of B0 bits) and the
-// row's sum of moduli in lsum (fx_l1's units); LATE: the sums of a row of several warps are still
-// in their slots and are read after the first exchange's synchronisation.  Leaves the transformed
-// elements in place and adds the shifts to e[b].
-template <int N, bool INV, int NB, int B0, bool LATE>
-__device__ __forceinline__ void fx_stages(q2 (&v)[NB][8], double2* buf, int bstride, const int4* __restrict__ tw, int t,
-                                          unsigned (&lsum)[NB], const unsigned (*lslot)[32], int (&e)[NB]) {
+// The transform of q values in registers, v[m] = element t + m G with components of B0 bits (moduli
+// below 2^(B0 + 1/2)) and the group's sum of moduli in lsum (fx_l1's units); LATE: the sum of a group
+// of several warps is still in its slots and is read after the first exchange's synchronisation.
+// Leaves the transformed elements in place and returns the bits shifted down.
+template <int N, bool INV, int B0, bool LATE>
+__device__ __forceinline__ int fx_stages(q2 (&v)[8], double2* buf, const int4* __restrict__ tw, const FxGroup& gr,
+                                         unsigned lsum) {
     constexpr int G = N / 8;
     constexpr int LOGN = N == 16 ? 4 : N == 32 ? 5 : N == 64 ? 6 : N == 128 ? 7 : N == 256 ? 8 : N == 512 ? 9 : N == 1024 ? 10 : N == 2048 ? 11 : 12;
     static_assert((1 << LOGN) == N, "length");
+    static_assert(!LATE || B0 + 3 <= FX_LIM, "first stage without the sum");
     constexpr int LAST = LOGN % 3 == 0 ? 8 : (LOGN % 3 == 1 ? 2 : 4);
-    int lb[NB], sh[NB], down[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        if (LATE) sh[b] = 0;  // the first stage fits (B0 + 3 <= FX_LIM)
-        else { lb[b] = 44 + fx_bitlen(lsum[b]); sh[b] = fx_down(B0, 3, lb[b]); }
-        down[b] = sh[b];
-    }
-    static_assert(!LATE || B0 + 3 <= FX_LIM, "first stage without the sums");
-    fx_compute<N, 8, INV, false, NB>(v, tw, t, 0, sh);
+    const int t = gr.t;
+    int lb = 44 + fx_bitlen(lsum), down = LATE ? 0 : fx_down(B0, 3, lb);
+    fx_compute<N, 8, INV, false>(v, tw, t, 0, down);
     // the exchange after a radix-8 stage: outputs to their autosorted positions, then the next
     // stage's inputs (radix P2)
     auto exchange = [&](int ns, auto p2) {
         constexpr int P2 = decltype(p2)::value, PER2 = 8 / P2, B2 = N / P2;
         const int k = t & (ns - 1), base = (t - k) * 8 + k;
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
+        for (int r = 0; r < 8; ++r) fx_strow(&buf[pad8(base + r * ns)], v[r]);
+        fx_sync<G>(gr);
+        if (LATE && ns == 1) lb = 44 + fx_bitlen(fx_read<G, true>(lsum, gr.slot + G / 32));
 #pragma unroll
-            for (int r = 0; r < 8; ++r) fx_strow(&buf[b * bstride + pad8(base + r * ns)], v[b][r]);
-        __syncthreads();
-        if (LATE && ns == 1) {
-            fx_row_read<G, NB, true>(lsum, lslot);
+        for (int q = 0; q < PER2; ++q)
 #pragma unroll
-            for (int b = 0; b < NB; ++b) lb[b] = 44 + fx_bitlen(lsum[b]);
-        }
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int q = 0; q < PER2; ++q)
-#pragma unroll
-                for (int r = 0; r < P2; ++r) v[b][q * P2 + r] = fx_ldrow(&buf[b * bstride + pad8(t + q * G + r * B2)]);
-        __syncthreads();  // every thread has its inputs before the buffer is written again
+            for (int r = 0; r < P2; ++r) v[q * P2 + r] = fx_ldrow(&buf[pad8(t + q * G + r * B2)]);
+        fx_sync<G>(gr);  // every thread has its inputs before the row is written again
     };
-    auto shifts = [&](int g) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int d = fx_down(B0, g, lb[b]);
-            sh[b] = d - down[b];
-            down[b] = d;
-        }
+    auto shift = [&](int g) {
+        const int d = fx_down(B0, g, lb), sh = d - down;
+        down = d;
+        return sh;
     };
     int ns = 1, g = 3;
     if constexpr (N >= 64) {
@@ -287,118 +281,90 @@ __device__ __forceinline__ void fx_stages(q2 (&v)[NB][8], double2* buf, int bstr
 #pragma unroll 1
         for (; ns * 64 <= N; ns *= 8) {
             exchange(ns, std::integral_constant<int, 8>{});
-            shifts(g + 3);
-            fx_compute<N, 8, INV, true, NB>(v, tw, t, g, sh);
+            fx_compute<N, 8, INV, true>(v, tw, t, g, shift(g + 3));
             g += 3;
         }
     }
     if constexpr (LAST != 8) {
         exchange(ns, std::integral_constant<int, LAST>{});
-        shifts(LOGN);
-        fx_compute<N, LAST, INV, true, NB>(v, tw, t, g, sh);
+        fx_compute<N, LAST, INV, true>(v, tw, t, g, shift(LOGN));
         // the last stage's butterfly q, output r is element t + (q + PER r) G: element order
         constexpr int PER = 8 / LAST;
+        q2 o[8];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            q2 o[8];
+        for (int q = 0; q < PER; ++q)
 #pragma unroll
-            for (int q = 0; q < PER; ++q)
+            for (int r = 0; r < LAST; ++r) o[q + PER * r] = v[q * LAST + r];
 #pragma unroll
-                for (int r = 0; r < LAST; ++r) o[q + PER * r] = v[b][q * LAST + r];
-#pragma unroll
-            for (int m = 0; m < 8; ++m) v[b][m] = o[m];
-        }
+        for (int m = 0; m < 8; ++m) v[m] = o[m];
     }
-#pragma unroll
-    for (int b = 0; b < NB; ++b) e[b] += down[b];
+    return down;
 }
 
-// doubles in registers to fixed point: the row's scale (one synchronisation when a row spans
-// warps) and the partial sums of moduli
-template <int G, int BITS, int NB>
-__device__ __forceinline__ void fx_enter(const double2 (&v)[NB][8], q2 (&z)[NB][8], unsigned (*mslot)[32], unsigned (*lslot)[32],
-                                         unsigned (&lsum)[NB], unsigned (&nan)[NB], int (&e)[NB]) {
-    unsigned mx[NB];
+// doubles in registers to fixed point: the group's scale (one synchronisation when it spans
+// warps), the exponent and the partial sum of moduli (complete for a group within a warp)
+template <int G, int BITS>
+__device__ __forceinline__ int fx_enter(const double2 (&v)[8], q2 (&z)[8], const FxGroup& gr, unsigned& lsum, unsigned& nan) {
+    unsigned mx = 0;
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        mx[b] = 0;
+    for (int m = 0; m < 8; ++m) mx = max(mx, max(fx_mag(v[m].x), fx_mag(v[m].y)));
+    mx = fx_reduce<G, false>(mx, gr.slot);
+    if (G > 32) fx_sync<G>(gr);
+    mx = fx_read<G, false>(mx, gr.slot);
+    const unsigned em = fx_scale(mx, nan);
+    lsum = 0;
 #pragma unroll
-        for (int m = 0; m < 8; ++m) mx[b] = max(mx[b], max(fx_mag(v[b][m].x), fx_mag(v[b][m].y)));
+    for (int m = 0; m < 8; ++m) {
+        z[m].x = fx_from<BITS>(v[m].x, em);
+        z[m].y = fx_from<BITS>(v[m].y, em);
+        lsum += fx_l1(z[m].x) + fx_l1(z[m].y);
     }
-    fx_row_reduce<G, NB, false>(mx, mslot);
-    if (G > 32) __syncthreads();
-    fx_row_read<G, NB, false>(mx, mslot);
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        const unsigned em = fx_scale(mx[b], nan[b]);
-        e[b] = (int)em - 1022 - BITS;
-        lsum[b] = 0;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            z[b][m].x = fx_from<BITS>(v[b][m].x, em);
-            z[b][m].y = fx_from<BITS>(v[b][m].y, em);
-            lsum[b] += fx_l1(z[b][m].x) + fx_l1(z[b][m].y);
-        }
-    }
-    fx_row_reduce<G, NB, true>(lsum, lslot);
+    lsum = fx_reduce<G, true>(lsum, gr.slot + G / 32);
+    return (int)em - 1022 - BITS;
+}
+__device__ __forceinline__ double2 fx_leave(q2 z, int e, unsigned nan) {
+    return make_double2(fx_to(z.x, e + 63 + 1022, nan), fx_to(z.y, e + 63 + 1022, nan));
 }
 
-// NB transforms of doubles in registers (block_fft_reg_m's contract; all threads of the block
-// call it): v[b][m] = element t + m (N/8), the rows of buf free when called and on return.  The
-// result is scaled by 2^ex (the normalisation 1/(nx ny), a power of two, costs nothing here).
-template <int N, bool INV, int NB, int NBA>
-__device__ __forceinline__ void fx_fft_reg(double2 (&v)[NBA][8], double2* buf, int bstride, const int4* __restrict__ tw, int t,
-                                           int ex) {
-    constexpr int G = N / 8;
-    __shared__ unsigned mslot[NB][32], lslot[NB][32];
-    q2 z[NB][8];
-    unsigned lsum[NB], nan[NB];
-    int e[NB];
-    {
-        double2 w[NB][8];
+// The transform of doubles in registers by one group: v[m] = element t + m (N/8); buf is the group's
+// row, free when called and on return.  The result is scaled by 2^ex (the normalisation 1/(nx ny),
+// a power of two, costs nothing here).
+template <int N, bool INV>
+__device__ __forceinline__ void fx_fft(double2 (&v)[8], double2* buf, const int4* __restrict__ tw, const FxGroup& gr, int ex = 0) {
+    q2 z[8];
+    unsigned lsum, nan;
+    int e = fx_enter<N / 8, FX_BITS>(v, z, gr, lsum, nan);
+    e += ex + fx_stages<N, INV, FX_BITS, true>(z, buf, tw, gr, lsum);
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int m = 0; m < 8; ++m) w[b][m] = v[b][m];
-        fx_enter<G, FX_BITS>(w, z, mslot, lslot, lsum, nan, e);
-    }
-    fx_stages<N, INV, NB, FX_BITS, true>(z, buf, bstride, tw, t, lsum, lslot, e);
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            v[b][m].x = fx_to(z[b][m].x, e[b] + ex + 63 + 1022, nan[b]);
-            v[b][m].y = fx_to(z[b][m].y, e[b] + ex + 63 + 1022, nan[b]);
-        }
+    for (int m = 0; m < 8; ++m) v[m] = fx_leave(z[m], e, nan);
 }
 
 // ---- real rows of 2H values as H complex ones (see r2c_split_m and c2r_merge_m) ---------------
 // The pairs (k, H - k) of a thread: k = 1 + t + i G, i < 4; the last thread's last pair is
 // (H/2, H/2), which it takes as the pair (0, H/2) of the two special elements.
 
-// Half spectra of doubles in the row buffers to real rows in registers: v[b][m] = element
-// t + m (H/8) (its x and y two neighbouring real values).  The rows are free on return.
-template <int H, int NB, int NBA>
-__device__ __forceinline__ void fx_c2r_reg(double2* rb, int bstride, const int4* __restrict__ twR, const int4* __restrict__ twX,
-                                           int t, double2 (&v)[NBA][8]) {
+// A half spectrum of doubles in the group's row (the group synchronised after it was written) to a
+// real row in registers: v[m] = element t + m (H/8), its x and y two neighbouring real values.
+// The row is free on return.
+template <int H>
+__device__ __forceinline__ void fx_c2r(double2* rb, const int4* __restrict__ twR, const int4* __restrict__ twX,
+                                       const FxGroup& gr, double2 (&v)[8]) {
     constexpr int G = H / 8;
-    __shared__ unsigned mslot[NB][32], lslot[NB][32];
-    q2 z[NB][8];
-    unsigned lsum[NB], nan[NB];
-    int e[NB];
+    const int t = gr.t;
+    q2 z[8];
+    unsigned lsum, nan;
+    int e;
     {
-        double2 x[NB][8];
+        double2 x[8];
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int k = 1 + t + i * G;
-                const bool sp = k == H / 2;
-                x[b][2 * i] = rb[b * bstride + pad8(sp ? 0 : k)];
-                x[b][2 * i + 1] = rb[b * bstride + pad8(H - k)];
-                if (i == 3 && sp) x[b][2 * i].y = 0.0;  // the imaginary part of X[0] is ignored
-            }
-        fx_enter<G, FX_BITS_C>(x, z, mslot, lslot, lsum, nan, e);
+        for (int i = 0; i < 4; ++i) {
+            const int k = 1 + t + i * G;
+            const bool sp = k == H / 2;
+            x[2 * i] = rb[pad8(sp ? 0 : k)];
+            x[2 * i + 1] = rb[pad8(H - k)];
+            if (i == 3 && sp) x[2 * i].y = 0.0;  // the imaginary part of X[0] is ignored
+        }
+        e = fx_enter<G, FX_BITS_C>(x, z, gr, lsum, nan);
     }
     // Z[k] = (X[k] + conj X[H-k]) + i (X[k] - conj X[H-k]) conj(w^k), and Z[H-k] likewise
 #pragma unroll
@@ -406,104 +372,74 @@ __device__ __forceinline__ void fx_c2r_reg(double2* rb, int bstride, const int4*
         const int k = 1 + t + i * G;
         const bool sp = i == 3 && k == H / 2;
         const int4 wk = __ldg(&twR[k]);
-        const int4 wm = make_int4(wk.x, wk.y, -wk.z, -wk.w);  // conj
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const q2 a = z[b][2 * i], c = z[b][2 * i + 1];
-            q2 s, d;
-            s.x = a.x + c.x; s.y = a.y - c.y;
-            d.x = a.x - c.x; d.y = a.y + c.y;
-            const q2 o = fx_cmul(d, wm);
-            // w^(H-k) = -conj(w^k): Z[H-k] = conj(s - i o)
-            q2 zk, zm;
-            zk.x = s.x - o.y; zk.y = s.y + o.x;
-            zm.x = s.x + o.y; zm.y = o.x - s.y;
-            if (sp) {
-                zk.x = a.x; zk.y = a.x;             // Z[0] = X[0] (1 + i)
-                zm.x = 2 * c.x; zm.y = -2 * c.y;    // Z[H/2] = 2 conj X[H/2]
-            }
-            fx_strow(&rb[b * bstride + pad8(sp ? 0 : k)], zk);
-            fx_strow(&rb[b * bstride + pad8(H - k)], zm);
+        const q2 a = z[2 * i], c = z[2 * i + 1];
+        q2 s, d;
+        s.x = a.x + c.x; s.y = a.y - c.y;
+        d.x = a.x - c.x; d.y = a.y + c.y;
+        const q2 o = fx_cmul(d, make_int4(wk.x, wk.y, -wk.z, -wk.w));
+        // w^(H-k) = -conj(w^k): Z[H-k] = conj(s - i o)
+        q2 zk, zm;
+        zk.x = s.x - o.y; zk.y = s.y + o.x;
+        zm.x = s.x + o.y; zm.y = o.x - s.y;
+        if (sp) {
+            zk.x = a.x; zk.y = a.x;             // Z[0] = X[0] (1 + i)
+            zm.x = 2 * c.x; zm.y = -2 * c.y;    // Z[H/2] = 2 conj X[H/2]
         }
+        fx_strow(&rb[pad8(sp ? 0 : k)], zk);
+        fx_strow(&rb[pad8(H - k)], zm);
     }
+    fx_sync<G>(gr);
     // |Z[k]|^2 + |Z[H-k]|^2 = 4 (|X[k]|^2 + |X[H-k]|^2), so the sum of the moduli grows by at most
     // 2 sqrt 2
-    __syncthreads();
-    fx_row_read<G, NB, true>(lsum, lslot);
+    lsum = 3 * fx_read<G, true>(lsum, gr.slot + G / 32);
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        lsum[b] *= 3;
+    for (int m = 0; m < 8; ++m) z[m] = fx_ldrow(&rb[pad8(t + m * G)]);
+    fx_sync<G>(gr);
+    e += fx_stages<H, true, FX_BITS_C + 2, false>(z, rb, twX, gr, lsum);
 #pragma unroll
-        for (int m = 0; m < 8; ++m) z[b][m] = fx_ldrow(&rb[b * bstride + pad8(t + m * G)]);
-    }
-    __syncthreads();
-    fx_stages<H, true, NB, FX_BITS_C + 2, false>(z, rb, bstride, twX, t, lsum, lslot, e);
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            v[b][m].x = fx_to(z[b][m].x, e[b] + 63 + 1022, nan[b]);
-            v[b][m].y = fx_to(z[b][m].y, e[b] + 63 + 1022, nan[b]);
-        }
+    for (int m = 0; m < 8; ++m) v[m] = fx_leave(z[m], e, nan);
 }
 
-// Real rows in registers to half spectra of doubles in the row buffers (free when called; the
-// caller reads them after this returns, synchronised).
-template <int H, int NB, int NBA>
-__device__ __forceinline__ void fx_r2c_reg(double2 (&v)[NBA][8], double2* rb, int bstride, const int4* __restrict__ twR,
-                                           const int4* __restrict__ twX, int t) {
+// A real row in registers to the half spectrum of doubles in the group's row (free when called;
+// readers outside the group synchronise first).
+template <int H>
+__device__ __forceinline__ void fx_r2c(const double2 (&v)[8], double2* rb, const int4* __restrict__ twR,
+                                       const int4* __restrict__ twX, const FxGroup& gr) {
     constexpr int G = H / 8;
-    __shared__ unsigned mslot[NB][32], lslot[NB][32];
-    q2 z[NB][8];
-    unsigned lsum[NB], nan[NB];
-    int e[NB];
-    {
-        double2 w[NB][8];
+    const int t = gr.t;
+    q2 z[8];
+    unsigned lsum, nan;
+    int e = fx_enter<G, FX_BITS>(v, z, gr, lsum, nan);
+    e += fx_stages<H, false, FX_BITS, true>(z, rb, twX, gr, lsum);
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int m = 0; m < 8; ++m) w[b][m] = v[b][m];
-        fx_enter<G, FX_BITS>(w, z, mslot, lslot, lsum, nan, e);
+    for (int m = 0; m < 8; ++m) {
+        q2 h;  // halves, for the split's sums
+        h.x = fx_shr(z[m].x, 1, 1);
+        h.y = fx_shr(z[m].y, 1, 1);
+        fx_strow(&rb[pad8(t + m * G)], h);
     }
-    fx_stages<H, false, NB, FX_BITS, true>(z, rb, bstride, twX, t, lsum, lslot, e);
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            // halves, for the split's sums
-            q2 h;
-            h.x = fx_shr(z[b][m].x, 1, 1);
-            h.y = fx_shr(z[b][m].y, 1, 1);
-            fx_strow(&rb[b * bstride + pad8(t + m * G)], h);
-        }
-    __syncthreads();
+    fx_sync<G>(gr);
     // X[k] = (z[k] + conj z[H-k])/2 + w^k (z[k] - conj z[H-k])/(2i), and X[H-k] likewise
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int k = 1 + t + i * G;
         const bool sp = i == 3 && k == H / 2;
-        const int4 wk = __ldg(&twR[k]);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            double2* pk = &rb[b * bstride + pad8(sp ? 0 : k)];
-            double2* pm = &rb[b * bstride + pad8(H - k)];
-            const q2 a = fx_ldrow(pk), c = fx_ldrow(pm);
-            q2 s, d;
-            s.x = a.x + c.x; s.y = a.y - c.y;
-            d.x = a.y + c.y; d.y = c.x - a.x;       // (z[k] - conj z[H-k]) / i
-            const q2 o = fx_cmul(d, wk);
-            q2 xk = fx_add(s, o), xm;
-            xm.x = s.x - o.x; xm.y = o.y - s.y;     // conj(s - o): w^(H-k) = -conj(w^k)
-            if (sp) {
-                xk.x = 2 * (a.x + a.y); xk.y = 0;   // X[0] = Re z[0] + Im z[0]
-                xm.x = 2 * c.x; xm.y = -2 * c.y;    // X[H/2] = conj z[H/2]
-            }
-            const int eb = e[b] + 63 + 1022;
-            *pk = make_double2(fx_to(xk.x, eb, nan[b]), sp ? 0.0 : fx_to(xk.y, eb, nan[b]));
-            *pm = make_double2(fx_to(xm.x, eb, nan[b]), fx_to(xm.y, eb, nan[b]));
+        double2 *pk = &rb[pad8(sp ? 0 : k)], *pm = &rb[pad8(H - k)];
+        const q2 a = fx_ldrow(pk), c = fx_ldrow(pm);
+        q2 s, d;
+        s.x = a.x + c.x; s.y = a.y - c.y;
+        d.x = a.y + c.y; d.y = c.x - a.x;       // (z[k] - conj z[H-k]) / i
+        const q2 o = fx_cmul(d, __ldg(&twR[k]));
+        q2 xk = fx_add(s, o), xm;
+        xm.x = s.x - o.x; xm.y = o.y - s.y;     // conj(s - o): w^(H-k) = -conj(w^k)
+        if (sp) {
+            xk.x = 2 * (a.x + a.y); xk.y = 0;   // X[0] = Re z[0] + Im z[0]
+            xm.x = 2 * c.x; xm.y = -2 * c.y;    // X[H/2] = conj z[H/2]
         }
+        *pk = fx_leave(xk, e, nan);
+        if (sp) pk->y = 0.0;
+        *pm = fx_leave(xm, e, nan);
     }
-    __syncthreads();
 }
 
 }  // namespace fsibe

@@ -118,9 +118,9 @@ __device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
 // the penalization part then adds the mask's term on the rows of the mask's box alone
 // (outside it the mask and the penalization are zero).
 enum { NL_WHOLE = 0, NL_ADVECT = 1, NL_PENAL = 2 };
-// shared-memory row buffers of k_nl_y: in FP32 two for the forward transforms and three for the
-// prefetched state, then all five for the inverse transforms; two in FP64
-template <typename R> constexpr int nl_y_bufs() { return kIsF32<R> ? 5 : 2; }
+// shared-memory row buffers of k_nl_y: two for the forward transforms and three for the
+// prefetched state, then all five for the inverse transforms
+constexpr int NL_Y_BUFS = 5;
 
 // 16-byte asynchronous global -> shared copies (the copy engine fills shared memory while the
 // threads compute); completed by cp_async_wait before use
@@ -247,13 +247,20 @@ template <typename R, int H, int NB, int NBA>
 __device__ __forceinline__ void row_c2r_reg(C2<R>* rb, int bstride, const TwF<R>* __restrict__ twR,
                                             const TwF<R>* __restrict__ twX, int t, C2<R> (&v)[NBA][8]) {
     if constexpr (kIsF32<R>) row_c2r_fp<R, H, NB>(rb, bstride, twR, twX, t, v);
-    else fx_c2r_reg<H, NB>(rb, bstride, twR, twX, t, v);
+    else {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) fx_c2r<H>(rb + b * bstride, twR, twX, fx_block_group<H / 8>(t), v[b]);
+    }
 }
 template <typename R, int H, int NB, int NBA>
 __device__ __forceinline__ void row_r2c_reg(C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, const TwF<R>* __restrict__ twR,
                                             const TwF<R>* __restrict__ twX, int t) {
     if constexpr (kIsF32<R>) row_r2c_fp<R, H, NB>(v, rb, bstride, twR, twX, t);
-    else fx_r2c_reg<H, NB>(v, rb, bstride, twR, twX, t);
+    else {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) fx_r2c<H>(v[b], rb + b * bstride, twR, twX, fx_block_group<H / 8>(t));
+        __syncthreads();  // the rows are read by the whole block
+    }
 }
 // The same in the time step's fused kernels.  FP64 rows of 4096 real values (H = 2048) keep the
 // FP64 stages there.  Fixed point is the more exact at that length too (4096^2, three steps: the
@@ -647,17 +654,19 @@ __global__ void __launch_bounds__(128) k_sponge10(const R* __restrict__ dudx, R*
 // K3: forward-y of the right-hand side, AB2 / Euler integrating-factor update, and the
 // inverse-y transforms of everything the velocity/pressure/force kernels need.
 // ======================================================================================
-// Blocks per SM that k_nl_y's launch bounds ask for: in FP32 as many as 128 registers a thread
+// Blocks per SM that k_nl_y's launch bounds ask for: as many as 128 registers a thread
 // allow (four at NY = 1024, so that its 512 rows run in one wave; one at NY = 4096), never
 // fewer registers than that (fewer spill the transforms' state)
-template <typename R, int NY>
+template <int NY>
 constexpr int nl_y_minb() {
-    return !kIsF32<R> ? 1 : (65536 / ((NY / 8) * 128) >= 4 ? 4 : (65536 / ((NY / 8) * 128) >= 1 ? 65536 / ((NY / 8) * 128) : 1));
+    return (65536 / ((NY / 8) * 128) >= 4 ? 4 : (65536 / ((NY / 8) * 128) >= 1 ? 65536 / ((NY / 8) * 128) : 1));
 }
 
-template <typename R, int NY>
-__global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> a) {
+// FP32 (the FP64 form's is k_nl_y_d)
+template <int NY>
+__global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float> a) {
     pdl_wait();     // the previous kernel of the stream has completed
+    using R = float;
     constexpr int G = NY / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C2<R>* bufA = reinterpret_cast<C2<R>*>(smem_raw);
@@ -672,21 +681,19 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
         for (int q = 0; q < 8; ++q) {
             a.W[row + t + q * G] = mk<R>(0, 0);
             a.M[row + t + q * G] = mk<R>(0, 0);
-            if constexpr (kIsF32<R>) a.Wlo[row + t + q * G] = mk<R>(0, 0);
+            a.Wlo[row + t + q * G] = mk<R>(0, 0);
         }
         return;
     }
-    // FP32 form: the row's state (W, Wlo, M) flows into the spare buffers C, D, E while the
+    // the row's state (W, Wlo, M) flows into the spare buffers C, D, E while the
     // forward transforms run (unpadded rows of NY complex values)
     C2<R>* preW = bufA + 2 * padded_len(NY);
     C2<R>* preWl = bufA + 3 * padded_len(NY);
     C2<R>* preM = bufA + 4 * padded_len(NY);
-    if constexpr (kIsF32<R>) {
-        for (int e = t; e < NY / 2; e += G) {  // 16 bytes = two complex values per copy
-            cp_async16_f(preW + 2 * e, a.W + row + 2 * e);
-            cp_async16_f(preWl + 2 * e, a.Wlo + row + 2 * e);
-            cp_async16_f(preM + 2 * e, a.M + row + 2 * e);
-        }
+    for (int e = t; e < NY / 2; e += G) {  // 16 bytes = two complex values per copy
+        cp_async16_f(preW + 2 * e, a.W + row + 2 * e);
+        cp_async16_f(preWl + 2 * e, a.Wlo + row + 2 * e);
+        cp_async16_f(preM + 2 * e, a.M + row + 2 * e);
     }
     // forward-y of A and B from registers (this thread's elements ky = t + q G) to registers
     C2<R> fab[2][8];
@@ -695,24 +702,14 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
         fab[0][q] = a.A[row + t + q * G];
         fab[1][q] = a.B[row + t + q * G];
     }
-    block_fft_reg_m<R, NY, false, 2>(fab, bufA, padded_len(NY), a.twY, t, a.enorm);  // A and B together
-    if constexpr (kIsF32<R>) {
-        cp_async_wait_f();
-        __syncthreads();
-    }
-    // FP64 form: the row's state, loaded before it is needed
-    C2<R> wo[8], mo[8];
-    if constexpr (!kIsF32<R>) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) { wo[q] = a.W[row + t + q * G]; mo[q] = a.M[row + t + q * G]; }
-    }
+    block_fft_reg_m<R, NY, false, 2>(fab, bufA, padded_len(NY), a.twY, t);  // A and B together
+    cp_async_wait_f();
+    __syncthreads();
     const DevScalars* S = a.S;
     const double dt1 = S->dt1, b10 = S->b10, b11 = S->b11;
     const bool expl = S->explicit_step != 0;
     const double norm = g.inv_nxny;
     const int cut = a.dcut[kx];
-    double kx2 = 0.0, etx = 0.0;
-    if constexpr (!kIsF32<R>) { kx2 = __dmul_rn((double)(kx * kx), g.scalex); etx = a.etab[kx]; }
     C2<R> wn[8], ps[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -723,122 +720,72 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<R, NY>())) k_nl_y(KArgs<R> 
         const R kys = ky_wave<R>(a, ky, ks);
         const C2<R> fa = fab[0][q], fb = fab[1][q];
         C2<R> N = csub<R>(fa, cimul<R>(fb, kys));
-        if constexpr (kIsF32<R>) N = cscale<R>(N, (R)norm);  // (FP64: scaled by the transform)
+        N = cscale<R>(N, (R)norm);
         if (nyq) N = mk<R>(0, 0);
         const bool keep = (g.idealis != 1) || (ka < cut);
         C2<R> Wn, Mn;
-        if constexpr (kIsF32<R>) {
-            const float2 ex = a.etabf[kx], ey = a.etabf[g.hx + ka];
-            const float Eh = __fmul_rn(ex.x, ey.x);
-            const float El = __fadd_rn(__fmaf_rn(ex.x, ey.x, -Eh), __fmaf_rn(ex.x, ey.y, __fmul_rn(ex.y, ey.x)));
-            const C2<R> Wo = preW[ky], Wl = preWl[ky];
-            float dx_, dy_;
-            if (expl) {
-                dx_ = (float)dt1 * N.x;
-                dy_ = (float)dt1 * N.y;
-            } else {
-                const C2<R> Mo = preM[ky];
-                dx_ = fmaf((float)b10, N.x, (float)b11 * Mo.x);
-                dy_ = fmaf((float)b10, N.y, (float)b11 * Mo.y);
-            }
-            float h0, l0, h1, l1;
-            ff_update(Wo.x, Wl.x, dx_, Eh, El, h0, l0);
-            ff_update(Wo.y, Wl.y, dy_, Eh, El, h1, l1);
-            if (!keep || nyq) { h0 = l0 = h1 = l1 = 0.f; }
-            Wn = mk<R>(h0, h1);
-            a.Wlo[row + ky] = mk<R>(l0, l1);
-            Mn = cscale<R>(N, Eh);
+        const float2 ex = a.etabf[kx], ey = a.etabf[g.hx + ka];
+        const float Eh = __fmul_rn(ex.x, ey.x);
+        const float El = __fadd_rn(__fmaf_rn(ex.x, ey.x, -Eh), __fmaf_rn(ex.x, ey.y, __fmul_rn(ex.y, ey.x)));
+        const C2<R> Wo = preW[ky], Wl = preWl[ky];
+        float dx_, dy_;
+        if (expl) {
+            dx_ = (float)dt1 * N.x;
+            dy_ = (float)dt1 * N.y;
         } else {
-            const R E1 = etx * __ldg(&a.etab[g.hx + ka]);
-            const C2<R> Wo = wo[q];
-            if (expl) {
-                Wn = mk<R>((Wo.x + (R)dt1 * N.x) * E1, (Wo.y + (R)dt1 * N.y) * E1);
-            } else {
-                const C2<R> Mo = mo[q];
-                Wn = mk<R>(((Wo.x + (R)b10 * N.x) + (R)b11 * Mo.x) * E1, ((Wo.y + (R)b10 * N.y) + (R)b11 * Mo.y) * E1);
-            }
-            if (!keep || nyq) Wn = mk<R>(0, 0);
-            Mn = cscale<R>(N, E1);
+            const C2<R> Mo = preM[ky];
+            dx_ = fmaf((float)b10, N.x, (float)b11 * Mo.x);
+            dy_ = fmaf((float)b10, N.y, (float)b11 * Mo.y);
         }
+        float h0, l0, h1, l1;
+        ff_update(Wo.x, Wl.x, dx_, Eh, El, h0, l0);
+        ff_update(Wo.y, Wl.y, dy_, Eh, El, h1, l1);
+        if (!keep || nyq) { h0 = l0 = h1 = l1 = 0.f; }
+        Wn = mk<R>(h0, h1);
+        a.Wlo[row + ky] = mk<R>(l0, l1);
+        Mn = cscale<R>(N, Eh);
         a.W[row + ky] = Wn;
         a.M[row + ky] = Mn;
         wn[q] = Wn;
-        if constexpr (kIsF32<R>) {
-            const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
-            ps[q] = (kx == 0 && ky == 0) ? mk<R>(0, 0) : cscale<R>(Wn, (R)1 / k2);
-        } else {
-            ps[q] = (kx == 0 && ky == 0) ? mk<R>(0, 0) : over_k2(a, Wn, kx2, kx, ka);
-        }
+        const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
+        ps[q] = (kx == 0 && ky == 0) ? mk<R>(0, 0) : cscale<R>(Wn, (R)1 / k2);
     }
-    // inverse-y outputs, NBO at a time: their transforms share the stages' synchronisations and
-    // twiddle loads (NBO buffers of shared memory).  In the FP32 form the factor i kx, constant
+    // inverse-y outputs, all at once: their transforms share the stages' synchronisations and
+    // twiddle loads (the prefetched state in the row buffers is consumed).  The factor i kx, constant
     // along a kx row, is applied after the transform where that saves one: cofdx(omega) =
-    // i kx T(omega) and d2psi/dxdy = i kx T(cofdy psi), so five spectra are transformed (cofdy
-    // psi, cofdx psi, omega, cofdy omega, (kx^2 - ky^2) psi).  The FP64 form transforms all seven
+    // i kx T(omega) and d2psi/dxdy = i kx T(cofdy psi), so five spectra are transformed: 0 cofdy psi,
+    // 1 cofdx psi, 2 omega, 3 cofdy omega, 4 (kx^2 - ky^2) psi (the stresses').  Their readers form
+    // i kx Tw and i kx Tu as they load Tw and Tu (load_tileT_dx).  The FP64 form transforms all seven
     // in the reference's order (cofdx, then cofitxy), which keeps its roundings those of the
     // operators its adjoint transposes.
-    // transforms at a time: the five FP32 buffers (the prefetched state they held is consumed),
-    // so the FP32 form's five spectra take one round; two in FP64
-    constexpr int NBO = kIsF32<R> ? 5 : 2;
-    static_assert(NBO <= nl_y_bufs<R>(), "one shared-memory row buffer per transform");
     constexpr int PLY = padded_len(NY);
-    const R kxs = kIsF32<R> ? (R)kx * (R)g.kxs : kx_wave<R>(a, kx);
-    // spectra: 0 cofdy psi, 1 cofdx psi, 2 omega, 3 cofdy omega, 4 (kx^2 - ky^2) psi, and in
-    // the FP64 form 5 cofdx omega, 6 d2psi/dxdy
-    const int ntr = kIsF32<R> ? (a.viscous ? 5 : 4) : (a.viscous ? 7 : 5);
-    for (int s0 = 0; s0 < ntr; s0 += NBO) {
-        const int cnt = (ntr - s0 < NBO) ? ntr - s0 : NBO;
-        // the spectra in registers (this thread's ky = t + q G), transformed with the
-        // shared-memory rows as exchange buffers, stored from registers
-        C2<R> ov[NBO][8];
+    const R kxs = (R)kx * (R)g.kxs;
+    // the spectra in registers (this thread's ky = t + q G), transformed with the shared-memory
+    // rows as exchange buffers, stored from registers
+    C2<R> ov[NL_Y_BUFS][8];
 #pragma unroll
-        for (int b = 0; b < NBO; ++b) {
-            const int sp = s0 + b;
+    for (int q = 0; q < 8; ++q) {
+        const int ky = t + q * G;
+        const R kys = ky_wave<R>(a, ky, signed_k(ky, NY));
+        ov[0][q] = cimul<R>(ps[q], kys);                        // cofdy(psi)   -> u
+        ov[1][q] = cimul<R>(ps[q], kxs);                        // cofdx(psi)   -> -v
+        ov[2][q] = wn[q];                                       // omega
+        ov[3][q] = cimul<R>(wn[q], kys);                        // cofdy(omega)
+        ov[4][q] = cscale<R>(ps[q], kxs * kxs - kys * kys);     // du/dy + dv/dx
+        if (ky == NY / 2) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int ky = t + q * G;
-                const int ks = signed_k(ky, NY);
-                const R kys = ky_wave<R>(a, ky, ks);
-                C2<R> val;
-                // (FP64 without the stresses: spectra 0..3 and 5; sp 4 stands for 5 there)
-                const int spk = (!kIsF32<R> && !a.viscous && sp == 4) ? 5 : sp;
-                switch (spk) {
-                    case 0: val = cimul<R>(ps[q], kys); break;                 // cofdy(psi)   -> u
-                    case 1: val = cimul<R>(ps[q], kxs); break;                 // cofdx(psi)   -> -v
-                    case 2: val = wn[q]; break;                                // omega
-                    case 3: val = cimul<R>(wn[q], kys); break;                 // cofdy(omega)
-                    case 4: val = cscale<R>(ps[q], kxs * kxs - kys * kys); break;  // du/dy + dv/dx
-                    case 5: val = cimul<R>(wn[q], kxs); break;                 // cofdx(omega)
-                    default: val = cscale<R>(ps[q], -(kxs * kys)); break;      // d2psi/dxdy = du/dx
-                }
-                if (ky == NY / 2) val = mk<R>(0, 0);
-                ov[b][q] = val;
-            }
+            for (int b = 0; b < NL_Y_BUFS; ++b) ov[b][q] = mk<R>(0, 0);
         }
-        // the buffers are free: the state loop above read the prefetched rows (buffers C..E),
-        // and a previous round's transform ended synchronised
-        __syncthreads();
-        if (cnt == 5) {
-            if constexpr (NBO >= 5) block_fft_reg_m<R, NY, true, 5>(ov, bufA, PLY, a.twY, t);
-        } else if (cnt == 4) {
-            if constexpr (NBO >= 4) block_fft_reg_m<R, NY, true, 4>(ov, bufA, PLY, a.twY, t);
-        } else if (cnt == 3) {
-            if constexpr (NBO >= 3) block_fft_reg_m<R, NY, true, 3>(ov, bufA, PLY, a.twY, t);
-        } else if (cnt == 2) {
-            block_fft_reg_m<R, NY, true, 2>(ov, bufA, PLY, a.twY, t);
-        } else {
-            block_fft_reg_m<R, NY, true, 1>(ov, bufA, PLY, a.twY, t);
-        }
-        for (int b = 0; b < cnt; ++b) {
-            const int sp = s0 + b;
-            const int spk = (!kIsF32<R> && !a.viscous && sp == 4) ? 5 : sp;
-            C2<R>* dst = (spk == 0) ? a.Tu : (spk == 1) ? a.Tv : (spk == 2) ? a.Tw : (spk == 3) ? a.Tdy
-                       : (spk == 4) ? a.Tsb : (spk == 5) ? a.Tdx : a.Tsa;
-            // (FP32: cofdx(omega) = i kx Tw and du/dx = i kx Tu are formed by their readers as
-            // they load Tw and Tu, load_tileT_dx)
+    }
+    __syncthreads();  // the state loop above read the prefetched rows
+    if (a.viscous) block_fft_reg_m<R, NY, true, 5>(ov, bufA, PLY, a.twY, t);
+    else block_fft_reg_m<R, NY, true, 4>(ov, bufA, PLY, a.twY, t);
+    C2<R>* const dst[NL_Y_BUFS] = {a.Tu, a.Tv, a.Tw, a.Tdy, a.Tsb};
 #pragma unroll
-            for (int q = 0; q < 8; ++q) dst[row + t + q * G] = ov[b][q];
-        }
+    for (int b = 0; b < NL_Y_BUFS; ++b) {
+        if (b == 4 && !a.viscous) break;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) dst[b][row + t + q * G] = ov[b][q];
     }
 }
 
@@ -1301,10 +1248,9 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k
     }
 }
 
-// Threads of k_press_y: the paired FP32 engine (two butterflies a thread) or the one-butterfly
-// engine (FP64).
-// ENG = 1 forces the one-butterfly engine in FP32 (the autotuner's other candidate).
-template <typename R, int NY, int ENG = 0> constexpr int press_y_threads() { return (kIsF32<R> && ENG == 0) ? NY / 16 : NY / 8; }
+// Threads of k_press_y: ENG = 0 the paired FP32 engine (two butterflies a thread), 1 the
+// one-butterfly engine (the autotuner's other candidate).
+template <int NY, int ENG = 0> constexpr int press_y_threads() { return ENG == 0 ? NY / 16 : NY / 8; }
 
 // K5, FP32: the paired engine.  Thread u holds the row's elements 2u + h + m (NY/8) as v[2m + h];
 // the pairs are loaded from and stored to global memory as 16-byte accesses.  The arithmetic of
@@ -1349,11 +1295,13 @@ __device__ __forceinline__ void press_y_paired(const KArgs<float>& a) {
         tq[u + m * HG] = make_float4(qv[0][2 * m].x, qv[0][2 * m].y, qv[0][2 * m + 1].x, qv[0][2 * m + 1].y);
 }
 
-// K5: forward-y of the Poisson right-hand side, divergence, poisson, inverse-y -> Tq
-template <typename R, int NY, int ENG = 0>
-__global__ void __launch_bounds__(press_y_threads<R, NY, ENG>(), (kIsF32<R> && NY >= 4096) ? 2 : 1) k_press_y(KArgs<R> a) {
+// K5: forward-y of the Poisson right-hand side, divergence, poisson, inverse-y -> Tq (FP32; the FP64
+// form's is k_press_y_d)
+template <int NY, int ENG = 0>
+__global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 : 1) k_press_y(KArgs<float> a) {
+    using R = float;
     pdl_wait();     // the previous kernel of the stream has completed
-    if constexpr (kIsF32<R> && ENG == 0) {
+    if constexpr (ENG == 0) {
         press_y_paired<NY>(a);
         return;
     }
@@ -1371,26 +1319,17 @@ __global__ void __launch_bounds__(press_y_threads<R, NY, ENG>(), (kIsF32<R> && N
         fp[0][q] = a.P1[row + t + q * G];
         fp[1][q] = a.P2[row + t + q * G];
     }
-    block_fft_reg_m<R, NY, false, 2>(fp, bufA, padded_len(NY), a.twY, t, a.enorm);  // P1 and P2 together
+    block_fft_reg_m<R, NY, false, 2>(fp, bufA, padded_len(NY), a.twY, t);  // P1 and P2 together
     const R norm = (R)g.inv_nxny;
-    double kx2 = 0.0;
-    if constexpr (!kIsF32<R>) kx2 = __dmul_rn((double)(kx * kx), g.scalex);
     C2<R> qv[1][8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int ky = t + q * G;
         const int ks = signed_k(ky, NY);
         const R kys = ky_wave<R>(a, ky, ks);
-        C2<R> qh;
-        if constexpr (kIsF32<R>) {
-            const C2<R> Q = cadd<R>(cscale<R>(fp[0][q], norm), cimul<R>(cscale<R>(fp[1][q], norm), kys));
-            const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
-            qh = cscale<R>(Q, (R)1 / k2);
-        } else {
-            const C2<R> Q = cadd<R>(fp[0][q], cimul<R>(fp[1][q], kys));  // scaled by the transform
-            qh = over_k2(a, Q, kx2, kx, ks < 0 ? -ks : ks);
-        }
-        if (kx == 0 && ky == 0) qh = mk<R>(0, 0);
+        const C2<R> Q = cadd<R>(cscale<R>(fp[0][q], norm), cimul<R>(cscale<R>(fp[1][q], norm), kys));
+        const R k2 = (R)(kx * kx) * (R)g.scalex + (R)(ks * ks) * (R)g.scaley;
+        C2<R> qh = (kx == 0 && ky == 0) ? mk<R>(0, 0) : cscale<R>(Q, (R)1 / k2);
         if (ky == NY / 2) qh = mk<R>(0, 0);
         qv[0][q] = qh;
     }
@@ -1445,133 +1384,123 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k
     }
 }
 
+}  // namespace fsibe
+#include "fluid_fx.cuh"
+namespace fsibe {
+
 // ======================================================================================
 // Dispatch table: one entry per supported length, filled by the inst_*.cu units.
 // ======================================================================================
+// a kernel with its block size and dynamic shared memory
+template <typename R>
+struct KLaunch {
+    void (*k)(KArgs<R>) = nullptr;
+    int threads = 0, smem = 0;
+};
+template <typename R>
+inline KLaunch<R> klaunch(void (*k)(KArgs<R>), int threads, int smem) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return KLaunch<R>{k, threads, smem};
+}
+
 template <typename R>
 struct SizeKernels {
-    // x-pass kernels for H = nx/2
-    void (*xfwd)(KArgs<R>);
-    void (*xinv)(KArgs<R>);
-    void (*vel_x)(KArgs<R>);
-    void (*nl_x)(KArgs<R>);
-    void (*press_x)(KArgs<R>);
-    void (*press_fin)(KArgs<R>);
-    int x_threads, x_rows, x_smem1, x_smem2;
+    // x-pass kernels for H = nx/2 (x_rows rows a block)
+    KLaunch<R> xfwd, xinv, vel_x;
+    int x_rows;
     // tile-height candidates of the fused x kernels (index 1 is the default)
     struct XVariant {
-        int rows, threads, smem1, smem3;  // smem3: the three row buffers of nl_x / press_x
-        int minb;                         // blocks per SM asked of the launch bounds (0: default)
-        void (*nl_x)(KArgs<R>);
-        void (*nl_adv)(KArgs<R>);  // k_nl_x's advection and penalization parts (two buffers)
-        void (*nl_pen)(KArgs<R>);
-        void (*nl_x_spg)(KArgs<R>);   // nl_x and its advection part with the vorticity sponge,
-        void (*nl_adv_spg)(KArgs<R>); // nl_x and its penalization part with the sharp outflow
-        void (*nl_x_s10)(KArgs<R>);   // sponge's integral (the default tile only; null
-        void (*nl_pen_s10)(KArgs<R>); // elsewhere)
-        void (*stress_x)(KArgs<R>);  // two buffers
-        void (*press_x)(KArgs<R>);
-        void (*press_fin)(KArgs<R>);
+        int rows = 0;
+        int minb = 0;                          // blocks per SM asked of the launch bounds (0: default)
+        KLaunch<R> nl_x, nl_adv, nl_pen;       // k_nl_x whole, its advection and its penalization part
+        KLaunch<R> nl_x_spg, nl_adv_spg;       // with the vorticity sponge, and with the sharp outflow
+        KLaunch<R> nl_x_s10, nl_pen_s10;       // sponge's integral (the default tile only)
+        KLaunch<R> stress_x, press_x, press_fin;
     } xv[4];  // [0..2]: half, the default and twice the default tile height; [3]: the default, two blocks an SM
-    XVariant xp;  // FP32: k_press_x on paired rows (press_x only; null in the FP64 form)
+    XVariant xp;  // FP32: k_press_x on paired rows (press_x only; none in the FP64 form)
     // y-pass kernels for NY
-    void (*yfwd)(KArgs<R>);
-    void (*yinv)(KArgs<R>);
-    void (*nl_y)(KArgs<R>);
-    void (*press_y)(KArgs<R>);
-    int y_threads, y_smem1, y_smem2, y_smem_nl;
-    int press_y_threads;  // the paired FP32 engine runs NY/16 threads
-    void (*press_y1)(KArgs<R>);  // FP32: k_press_y on the one-butterfly engine (NY/8 threads), or null
-    int press_y1_smem;
+    KLaunch<R> yfwd, yinv, nl_y, press_y;
+    KLaunch<R> press_y1;  // FP32: k_press_y on the one-butterfly engine (NY/8 threads), or none
 };
 
 template <typename R, int H, int TR, int MB = 0, bool SPG = false>
 inline void fill_xvariant(typename SizeKernels<R>::XVariant& v) {
     using X = XRows<R, H, TR>;
+    constexpr int T = X::THREADS, S1 = (int)(TR * X::PL * sizeof(C2<R>));
     v.rows = TR;
     v.minb = MB;
-    v.threads = X::THREADS;
-    v.smem1 = (int)(TR * X::PL * sizeof(C2<R>));
-    v.smem3 = 3 * v.smem1;
-    v.nl_x = k_nl_x<R, H, TR, NL_WHOLE, MB>;
-    v.nl_adv = k_nl_x<R, H, TR, NL_ADVECT, MB>;
-    v.nl_pen = k_nl_x<R, H, TR, NL_PENAL, MB>;
-    v.nl_x_spg = v.nl_adv_spg = v.nl_x_s10 = v.nl_pen_s10 = nullptr;
-    if constexpr (SPG) {
-        v.nl_x_spg = k_nl_x<R, H, TR, NL_WHOLE, MB, 1>;
-        v.nl_adv_spg = k_nl_x<R, H, TR, NL_ADVECT, MB, 1>;
-        v.nl_x_s10 = k_nl_x<R, H, TR, NL_WHOLE, MB, 2>;
-        v.nl_pen_s10 = k_nl_x<R, H, TR, NL_PENAL, MB, 2>;
-        cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_WHOLE, MB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem3);
-        cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_ADVECT, MB, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * v.smem1);
-        cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_WHOLE, MB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem3);
-        cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_PENAL, MB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * v.smem1);
+    v.press_fin = klaunch<R>(k_press_fin<R, H, TR, MB>, T, S1);
+    if constexpr (step_fp<R, H>()) {
+        v.nl_x = klaunch<R>(k_nl_x<R, H, TR, NL_WHOLE, MB>, T, 3 * S1);
+        v.nl_adv = klaunch<R>(k_nl_x<R, H, TR, NL_ADVECT, MB>, T, 2 * S1);
+        v.nl_pen = klaunch<R>(k_nl_x<R, H, TR, NL_PENAL, MB>, T, 2 * S1);
+        if constexpr (SPG) {
+            v.nl_x_spg = klaunch<R>(k_nl_x<R, H, TR, NL_WHOLE, MB, 1>, T, 3 * S1);
+            v.nl_adv_spg = klaunch<R>(k_nl_x<R, H, TR, NL_ADVECT, MB, 1>, T, 2 * S1);
+            v.nl_x_s10 = klaunch<R>(k_nl_x<R, H, TR, NL_WHOLE, MB, 2>, T, 3 * S1);
+            v.nl_pen_s10 = klaunch<R>(k_nl_x<R, H, TR, NL_PENAL, MB, 2>, T, 2 * S1);
+        }
+        v.stress_x = klaunch<R>(k_stress_x<R, H, TR, MB>, T, 2 * S1);
+        v.press_x = klaunch<R>(k_press_x<R, H, TR, MB>, T, 3 * S1);
+    } else {
+        // the FP64 form's kernels with a group of threads a transform (fluid_fx.cuh)
+        using X2 = XGroups<H, TR, 2>;
+        using X3 = XGroups<H, TR, 3>;
+        v.nl_x = klaunch<R>(k_nl_x_d<H, TR, NL_WHOLE, 0>, X3::THREADS, X3::SMEM);
+        v.nl_adv = klaunch<R>(k_nl_x_d<H, TR, NL_ADVECT, 0>, X2::THREADS, X2::SMEM);
+        v.nl_pen = klaunch<R>(k_nl_x_d<H, TR, NL_PENAL, 0>, X2::THREADS, X2::SMEM);
+        if constexpr (SPG) {
+            v.nl_x_spg = klaunch<R>(k_nl_x_d<H, TR, NL_WHOLE, 1>, X3::THREADS, X3::SMEM);
+            v.nl_adv_spg = klaunch<R>(k_nl_x_d<H, TR, NL_ADVECT, 1>, X3::THREADS, X3::SMEM);
+            v.nl_x_s10 = klaunch<R>(k_nl_x_d<H, TR, NL_WHOLE, 2>, X3::THREADS, X3::SMEM);
+            v.nl_pen_s10 = klaunch<R>(k_nl_x_d<H, TR, NL_PENAL, 2>, X2::THREADS, X2::SMEM);
+        }
+        v.stress_x = klaunch<R>(k_stress_x_d<H, TR>, X2::THREADS, X2::SMEM);
+        v.press_x = klaunch<R>(k_press_x_d<H, TR>, X3::THREADS, press_x_smem_d<H, TR>());
     }
-    v.stress_x = k_stress_x<R, H, TR, MB>;
-    cudaFuncSetAttribute(k_stress_x<R, H, TR, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * v.smem1);
-    cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_ADVECT, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * v.smem1);
-    cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_PENAL, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * v.smem1);
-    v.press_x = k_press_x<R, H, TR, MB>;
-    v.press_fin = k_press_fin<R, H, TR, MB>;
-    cudaFuncSetAttribute(k_nl_x<R, H, TR, NL_WHOLE, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem3);
-    cudaFuncSetAttribute(k_press_x<R, H, TR, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem3);
-    cudaFuncSetAttribute(k_press_fin<R, H, TR, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem1);
 }
 
 template <typename R, int N>
 inline void fill_size_kernels(SizeKernels<R>& k) {
     constexpr int H = N / 2;
     using X = XRows<R, H>;
-    k.xfwd = k_xfwd<R, H>;
-    k.xinv = k_xinv<R, H>;
-    k.vel_x = k_vel_x<R, H>;
-    k.x_threads = X::THREADS;
+    constexpr int S1 = (int)(X::TR * X::PL * sizeof(C2<R>)), SY = (int)(padded_len(N) * sizeof(C2<R>)), TY = N / 8;
     k.x_rows = X::TR;
-    k.x_smem1 = (int)(X::TR * X::PL * sizeof(C2<R>));
-    k.x_smem2 = 2 * k.x_smem1;
-    cudaFuncSetAttribute(k_xfwd<R, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.x_smem1);
-    cudaFuncSetAttribute(k_xinv<R, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.x_smem1);
-    cudaFuncSetAttribute(k_vel_x<R, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.x_smem2);
-    constexpr int T0 = xrows_valid<R, H>(X::TRD / 2), T1 = X::TRD, T2 = xrows_valid<R, H>(X::TRD * 2);
-    fill_xvariant<R, H, T0>(k.xv[0]);
-    fill_xvariant<R, H, T1, 0, true>(k.xv[1]);
-    fill_xvariant<R, H, T2>(k.xv[2]);
-    // the default tile with the registers capped for two resident blocks (when two fit an SM)
-    constexpr int MB2 = (2 * XRows<R, H, T1>::THREADS <= 2048) ? 2 : 1;
-    fill_xvariant<R, H, T1, MB2>(k.xv[3]);
+    k.xfwd = klaunch<R>(k_xfwd<R, H>, X::THREADS, S1);
+    k.xinv = klaunch<R>(k_xinv<R, H>, X::THREADS, S1);
+    k.vel_x = klaunch<R>(k_vel_x<R, H>, X::THREADS, 2 * S1);
+    constexpr int T1 = X::TRD;
     k.xp = typename SizeKernels<R>::XVariant{};
+    if constexpr (step_fp<R, H>()) {
+        constexpr int T0 = xrows_valid<R, H>(T1 / 2), T2 = xrows_valid<R, H>(T1 * 2);
+        fill_xvariant<R, H, T0>(k.xv[0]);
+        fill_xvariant<R, H, T1, 0, true>(k.xv[1]);
+        fill_xvariant<R, H, T2>(k.xv[2]);
+        // the default tile with the registers capped for two resident blocks (when two fit an SM)
+        constexpr int MB2 = (2 * XRows<R, H, T1>::THREADS <= 2048) ? 2 : 1;
+        fill_xvariant<R, H, T1, MB2>(k.xv[3]);
+    } else {
+        constexpr int T0 = xgroups_valid<H>(T1 / 2, T1), T2 = xgroups_valid<H>(T1 * 2, T1);
+        fill_xvariant<R, H, T0>(k.xv[0]);
+        fill_xvariant<R, H, T1, 0, true>(k.xv[1]);
+        fill_xvariant<R, H, T2>(k.xv[2]);
+        k.xv[3] = k.xv[1];
+    }
+    k.yfwd = klaunch<R>(k_yfwd<R, N>, TY, SY);
+    k.yinv = klaunch<R>(k_yinv<R, N>, TY, SY);
     if constexpr (kIsF32<R>) {
         constexpr int TP = xpairs_rows<H>();
         k.xp.rows = TP;
-        k.xp.threads = XPairs<H, TP>::THREADS;
-        k.xp.smem3 = 3 * TP * pair_slots(H) * 16;
-        k.xp.smem1 = k.xp.smem3 / 3;
         k.xp.minb = 16;  // the marker of the paired kernel in fsibe_tile_config
-        k.xp.press_x = k_press_x2<H, TP>;
-        cudaFuncSetAttribute(k_press_x2<H, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.xp.smem3);
-    }
-    k.nl_x = k.xv[1].nl_x;
-    k.press_x = k.xv[1].press_x;
-    k.press_fin = k.xv[1].press_fin;
-    k.yfwd = k_yfwd<R, N>;
-    k.yinv = k_yinv<R, N>;
-    k.nl_y = k_nl_y<R, N>;
-    k.press_y = k_press_y<R, N>;
-    k.y_threads = N / 8;
-    k.y_smem1 = (int)(padded_len(N) * sizeof(C2<R>));
-    k.y_smem2 = 2 * k.y_smem1;
-    if (kIsF32<R>) k.y_smem2 = std::max(k.y_smem2, 2 * pair_slots(N) * 16);
-    k.press_y_threads = press_y_threads<R, N>();
-    k.y_smem_nl = nl_y_bufs<R>() * k.y_smem1;
-    cudaFuncSetAttribute(k_yfwd<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.y_smem1);
-    cudaFuncSetAttribute(k_yinv<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.y_smem1);
-    cudaFuncSetAttribute(k_nl_y<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.y_smem_nl);
-    cudaFuncSetAttribute(k_press_y<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.y_smem2);
-    k.press_y1 = nullptr;
-    k.press_y1_smem = 2 * k.y_smem1;
-    if constexpr (kIsF32<R>) {
-        k.press_y1 = k_press_y<R, N, 1>;
-        cudaFuncSetAttribute(k_press_y<R, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, k.press_y1_smem);
+        k.xp.press_x = klaunch<R>(k_press_x2<H, TP>, XPairs<H, TP>::THREADS, 3 * TP * pair_slots(H) * 16);
+        k.nl_y = klaunch<R>(k_nl_y<N>, TY, NL_Y_BUFS * SY);
+        k.press_y = klaunch<R>(k_press_y<N>, press_y_threads<N>(), std::max(2 * SY, 2 * pair_slots(N) * 16));
+        k.press_y1 = klaunch<R>(k_press_y<N, 1>, TY, 2 * SY);
+    } else {
+        constexpr int NG = nl_y_groups<N>(), PG = press_y_groups<N>();
+        k.nl_y = klaunch<R>(k_nl_y_d<N, NG>, NG * TY, nl_y_smem_d<N, NG>());
+        k.press_y = klaunch<R>(k_press_y_d<N, PG>, PG * TY, press_y_smem_d<N, PG>());
+        k.press_y1 = KLaunch<R>{};
     }
 }
 
