@@ -452,7 +452,7 @@ struct fsibe_ctx {
     double* oo = nullptr;
     double* ws = nullptr;
     Prim* prims = nullptr;
-    PrimG* primg = nullptr;       // the FP32 raster's per-primitive data (FP32 form)
+    PrimG* primg = nullptr;       // the raster's per-primitive FP32 data
     int *nprims = nullptr, *rect = nullptr;
     unsigned* counter = nullptr;
     double* fterm = nullptr;
@@ -475,7 +475,7 @@ struct fsibe_ctx {
     double gerf = 0.0;
     double U_mean_true = 1.0;
     // walls, cylinder and sponges: static fields, formed once (null when not used)
-    bool full_mask = false;       // every cell of the mask is drawn each step
+    bool full_mask = false;       // the mask has a background: walls, cylinder, velocity sponge or frame
     double* bg = nullptr;         // walls + cylinder, unscaled
     double* frame = nullptr;      // iSponge = 22
     void* spg = nullptr;          // vorticity sponge / eps_sponge (R)
@@ -918,7 +918,7 @@ static MaskArgs mask_args(fsibe_ctx* c) {
     m.t_beam = c->P.t_beam; m.N_smooth = c->P.N_smooth; m.eps = c->P.eps; m.pi = c->g.pi;
     m.angle_deg = c->P.angle_beam;
     m.x = c->beam[B_X]; m.y = c->beam[B_Y]; m.vx = c->beam[B_VX]; m.vy = c->beam[B_VY]; m.th = c->beam[B_TH];
-    m.prims = c->prims; m.primg = c->fp32 ? c->primg : nullptr; m.nprims = c->nprims; m.rect = c->rect; m.nsm = c->nsm;
+    m.prims = c->prims; m.primg = c->primg; m.f32 = c->fp32 ? 1 : 0; m.nprims = c->nprims; m.rect = c->rect; m.nsm = c->nsm;
     m.rdx = 1.0 / m.dx; m.rdy = 1.0 / m.dy; m.rpi = 1.0 / m.pi;
     m.inv_delta = 1.0 / ((m.N_smooth * std::fmax(m.dx, m.dy)) * c->gerf);
     m.inv_ds = 1.0 / m.ds;
@@ -926,6 +926,7 @@ static MaskArgs mask_args(fsibe_ctx* c) {
     m.mo = motion_args(c);
     m.mask = c->phys[PH_MASK]; m.mvx = c->phys[PH_MVX]; m.mvy = c->phys[PH_MVY];
     m.full = c->full_mask ? 1 : 0;
+    m.every = (c->P.iSponge == 4 || c->P.iSponge == 22) ? 1 : 0;
     m.bg = c->bg;
     m.frame = c->frame;
     m.frame_c = c->P.eps / std::max(1.0e-3, c->P.eps);
@@ -1672,12 +1673,15 @@ int fsibe_create(const fsibe_params* p, fsibe_ctx** out) {
 
     }
     ALLOC(c->prims, sizeof(Prim) * (size_t)(2 * ns + 8));
-    if (c->fp32) ALLOC(c->primg, sizeof(PrimG) * (size_t)(2 * ns + 8));
+    ALLOC(c->primg, sizeof(PrimG) * (size_t)(2 * ns + 8));
     ALLOC(c->nprims, 16);
     ALLOC(c->rect, 64);
     {
-        // previous box: none drawn yet (all cells zero); box accumulator: empty
-        const int r0[16] = {0, 0, 0, 0, 0, 0, 0, 0, p->nx, -1, p->ny, -1, 0, 0, 0, 0};
+        // previous box: none drawn yet (all cells zero), or with a background the grid, which the
+        // first draw then covers; box accumulator: empty
+        int r0[16] = {0, 0, 0, 0, 0, 0, 0, 0, p->nx, -1, p->ny, -1, 0, 0, 0, 0};
+        const bool bg = p->iWalls > 0 || p->iCylinder > 0 || p->iSponge == 4 || p->iSponge == 22;
+        if (bg) { r0[1] = p->nx - 1; r0[3] = p->ny - 1; }
         cudaMemcpy(c->rect, r0, sizeof(r0), cudaMemcpyHostToDevice);
     }
     ALLOC(c->counter, 16);

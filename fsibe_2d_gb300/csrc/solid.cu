@@ -52,13 +52,27 @@ __global__ void __launch_bounds__(128) k_mask_prep(MaskArgs a, double gerf) {
     const int total = nseg + nsharp + nh + ndot;
     const int i = blockIdx.x * 32 + lane;
     int bx0 = a.nx, bx1 = -1, by0 = a.ny, by1 = -1;
-    // the FP32 raster's per-primitive data (the raster's expressions for its constants)
+    // the raster's per-primitive data (the raster's expressions for its constants)
     const double rcut_g = t + 10.0 * (N * mx) * gerf;
     const float mg = 1.0e-5f * (float)fmax((double)a.nx * dx, (double)a.ny * dy);
     auto emit = [&](int q, Prim& P) {
         clip_box(P.box, a.nx, a.ny);
         a.prims[q] = P;
-        if (a.primg && P.type != PRIM_SHARP) {
+        if (!a.f32) {
+            // the FP64 raster's pre-test data: a cell that fails it is outside the primitive by more
+            // than the margin, so the exact FP64 test (the reference's arithmetic) is skipped
+            PrimG G;
+            if (P.type == PRIM_SEGMENT || P.type == PRIM_SHARP) {
+                G.a = make_float4((float)P.p[0], (float)P.p[1], (float)P.p[2] - mg, (float)P.p[4] + mg);
+                G.b = make_float4((float)(P.p[3] + t_star) + mg, (float)(P.p[5] - t_star) - mg, 0.f, 0.f);
+            } else {
+                const float lim = (float)((P.type == PRIM_HINGE) ? t_star : rcut_g) + mg;
+                G.a = make_float4((float)P.p[0], (float)P.p[1], lim * lim, 0.f);
+                G.b = make_float4((float)P.p[2], (float)P.p[3], 0.f, 0.f);  // a hinge's angles
+            }
+            G.c = make_float4(0.f, 0.f, 0.f, 0.f);
+            a.primg[q] = G;
+        } else if (P.type != PRIM_SHARP) {
             PrimG G;
             if (P.type == PRIM_SEGMENT) {
                 G.a = make_float4((float)P.p[0], (float)P.p[1], 0.f, 0.f);
@@ -106,12 +120,12 @@ __global__ void __launch_bounds__(128) k_mask_prep(MaskArgs a, double gerf) {
         // the hinge's two angles: FP32 in the FP32 form, whose raster tests its wedges in FP32
         if (hinge) {
             const double ddy = a.y[i] - a.y[i - 1], ddx = a.x[i] - a.x[i - 1];
-            a1 = a.primg ? (double)atan2f((float)ddy, (float)ddx) : atan2(ddy, ddx);
+            a1 = a.f32 ? (double)atan2f((float)ddy, (float)ddx) : atan2(ddy, ddx);
         }
     } else if (warp == 2) {
         if (hinge) {
             const double ddy = a.y[i + 1] - a.y[i], ddx = a.x[i + 1] - a.x[i];
-            ang2[lane] = a.primg ? (double)atan2f((float)ddy, (float)ddx) : atan2(ddy, ddx);
+            ang2[lane] = a.f32 ? (double)atan2f((float)ddy, (float)ddx) : atan2(ddy, ddx);
         }
     } else {
         if (hinge) {
@@ -169,7 +183,7 @@ __global__ void __launch_bounds__(128) k_mask_prep(MaskArgs a, double gerf) {
         P.type = PRIM_HINGE;
         P.box[0] = hbox[lane][0]; P.box[1] = hbox[lane][1]; P.box[2] = hbox[lane][2]; P.box[3] = hbox[lane][3];
         P.p[0] = px; P.p[1] = py;
-        if (a.primg) {  // degrees as the FP32 raster forms a cell's angle
+        if (a.f32) {  // degrees as the FP32 raster forms a cell's angle
             P.p[2] = (double)deg_f((float)a1);
             P.p[3] = (double)deg_f((float)a2);
         } else {
@@ -205,7 +219,7 @@ __global__ void __launch_bounds__(128) k_mask_prep(MaskArgs a, double gerf) {
             const int p0 = R[0], p1 = R[1], p2 = R[2], p3 = R[3];
             R[0] = n0; R[1] = n1; R[2] = n2; R[3] = n3;
             R[4] = min(n0, p0); R[5] = max(n1, p1); R[6] = min(n2, p2); R[7] = max(n3, p3);
-            if (a.full) { R[4] = 0; R[5] = a.nx - 1; R[6] = 0; R[7] = a.ny - 1; }  // walls, sponges: every cell
+            if (a.every) { R[4] = 0; R[5] = a.nx - 1; R[6] = 0; R[7] = a.ny - 1; }
             R[8] = a.nx; R[9] = -1; R[10] = a.ny; R[11] = -1;
             R[12] = 0;
             *a.nprims = total;
@@ -248,44 +262,32 @@ __device__ __forceinline__ bool hinge_inside(T gamma, T beta1, T beta2, T margin
     return in1 && in2;
 }
 
-// FP32 pre-test data of one primitive: a cell that fails the pre-test is outside the primitive
-// by more than the margin, so the exact FP64 test (the reference's arithmetic) is skipped.
-struct PrimF {
-    float4 a;  // segment/sharp: (cos, sin, x*_lo, x*_hi)   hinge/dot: (px, py, R^2 limit, 0)
-    float2 b;  // segment/sharp: (y*_hi, y*_lo)
-};
-
-// SmoothStep in FP32 from the FP64 distance: the FP32 form's value, and for the FP64 form an
-// estimate within 1e-6 of the FP64 value (the argument is rounded once, |erf'| <= 2/sqrt(pi),
-// erff is within 2 ulp).
+// SmoothStep in FP32 from the FP64 distance: the FP32 form's value of the sharp end, and for the FP64
+// form an estimate within 4e-6 of the FP64 value (the arguments are rounded once or twice, |erf'| <=
+// 2/sqrt(pi) where erf is not flat, erff is within 2 ulp).
 __device__ __forceinline__ float smooth_step_f(double x, double t, double inv_delta, int sharp) {
     if (sharp) return (x <= t) ? 1.f : 0.f;
     const float a1 = (float)((t - x) * inv_delta), a2 = (float)((x + t) * inv_delta);
     return 0.5f * (erff(a1) + erff(a2));
 }
 // The FP64 value as the reference evaluates it (SmoothStep, create_mask.f90:697-717).
-__device__ __forceinline__ double smooth_step_d(double x, double t, double inv_delta, int sharp) {
+__device__ __noinline__ double smooth_step_d(double x, double t, double inv_delta, int sharp) {
     if (sharp) return (x <= t) ? 1.0 : 0.0;
     return 0.5 * (erf((t - x) * inv_delta) + erf((x + t) * inv_delta));
 }
 
-// Per-cell fold state of one warp over its share of the primitives: the largest SmoothStep so
-// far, its velocity and primitive index (INT_MAX: none yet), and an FP32 lower bound of m.
-// T: double in the FP64 form, float in the FP32 form.
-template <typename T>
+// Per-cell fold state of one warp over its share of the primitives (FP32 form): the largest
+// SmoothStep so far, its velocity and primitive index (INT_MAX: none yet).
 struct MaskFold {
-    T m, vx, vy;
+    float m, vx, vy;
     int idx;
-    float mlow;
 };
 
 // Draw order keeps the first of equal values (strict >); over a subset taken in any order the
 // same winner is the largest value with the smallest index among its ties.
-template <typename T>
-__device__ __forceinline__ void fold_take(MaskFold<T>& f, T temp, T vx, T vy, int q) {
+__device__ __forceinline__ void fold_take(MaskFold& f, float temp, float vx, float vy, int q) {
     if (temp > f.m || (temp == f.m && f.idx != 0x7fffffff && q < f.idx)) {
         f.m = temp; f.vx = vx; f.vy = vy; f.idx = q;
-        if constexpr (sizeof(T) == 8) f.mlow = __double2float_rd(temp);
     }
 }
 
@@ -300,14 +302,14 @@ __device__ __forceinline__ float smooth_step_ff(float x, float t, float inv_delt
 // hinge's disc with the same value and velocity, the outer edges have SmoothStep ~ 0), so the
 // exact FP64 edge tests of the FP64 form are not needed for its tolerance.
 __device__ __forceinline__ void mask_prim_f(const MaskArgs& a, const Prim& Q, const PrimG& G, int q, int i, int j,
-                                            float cx, float cy, float tf, float tsf, float idf, MaskFold<float>& f) {
+                                            float cx, float cy, float tf, float tsf, float idf, MaskFold& f) {
     if (i < Q.box[0] || i > Q.box[1] || j < Q.box[2] || j > Q.box[3]) return;
     if (Q.type == PRIM_SEGMENT) {
         const float xr = cx - G.a.z, yr = cy - G.a.w;
         const float u = G.a.x * xr - G.a.y * yr, w = G.a.y * xr + G.a.x * yr;
         if (u < 0.f || u > G.b.x || w > tsf || w < G.b.y) return;
         const float temp = smooth_step_ff(fabsf(w), tf, idf, a.sharp);
-        if (temp >= f.m) fold_take<float>(f, temp, G.c.x + u * G.c.z, G.c.y + u * G.c.w, q);
+        if (temp >= f.m) fold_take(f, temp, G.c.x + u * G.c.z, G.c.y + u * G.c.w, q);
         return;
     }
     const float ddx = cx - G.a.x, ddy = cy - G.a.y, r2 = ddx * ddx + ddy * ddy;
@@ -316,39 +318,72 @@ __device__ __forceinline__ void mask_prim_f(const MaskArgs& a, const Prim& Q, co
         const float gf = deg_f(atan2f(ddy, ddx));
         if (!hinge_inside<float>(gf, G.b.x, G.b.y, 0.f, nullptr)) return;
         const float Rr = sqrtf(r2);
-        if (Rr <= tsf) fold_take<float>(f, smooth_step_ff(Rr, tf, idf, a.sharp), G.c.x, G.c.y, q);
+        if (Rr <= tsf) fold_take(f, smooth_step_ff(Rr, tf, idf, a.sharp), G.c.x, G.c.y, q);
         return;
     }
-    fold_take<float>(f, smooth_step_ff(sqrtf(r2), tf, idf, a.sharp), G.c.x, G.c.y, q);
+    fold_take(f, smooth_step_ff(sqrtf(r2), tf, idf, a.sharp), G.c.x, G.c.y, q);
 }
 
-// Segment, hinge or dot q for the lane's cell (i, j), FP32 pre-test first.  R = float: the FP32
-// form, SmoothStep in FP32.  R = double: SmoothStep in FP64, evaluated only when its FP32
-// estimate (within 1e-6) could exceed the cell's current value by the margin 1e-5 -- a
-// candidate that cannot win changes nothing under the draw-order rule.
-template <typename R>
-__device__ __forceinline__ void mask_prim(const MaskArgs& a, const Prim& Q, const PrimF& F, int q, int i, int j,
-                                          double xi, double yj, float xf, float yf, double t, double t_star,
-                                          double inv_delta, double inv_ds, MaskFold<double>& f) {
+// The FP64 form's fold: the winner so far by its distance.  SmoothStep falls with the distance, so a
+// winner is known from the FP32 estimates unless they are within MASK_NEAR of each other, and then
+// still from the distances when SmoothStep falls by more than 1e-14 between them: its FP64 values (two
+// erf within 2 ulp each) then differ by 15 times their errors.  What
+// remains -- distances equal but for the last bits, the plateau inside thick bodies, the far tail --
+// takes the FP64 values (some hundred FP64 instructions each).  q is INT_MAX while there is none; ex
+// holds the winner's FP64 value once it was needed.
+struct MaskNear {
+    double d, ex;
+    float est;
+    int q;
+    bool known;
+};
+constexpr float MASK_NEAR = 2.0e-5f;
+// A lower bound of SmoothStep's fall over the distance x delta from d outwards (up to 0.1 delta of it):
+// its slope in units of 1/delta rises to its largest value and falls, so over an interval it is at
+// least the smaller of its ends'.
+__device__ __forceinline__ float near_fall(const MaskArgs& a, double d, float x) {
+    const float c = 2.f * (float)a.t_beam * (float)a.inv_delta, u = (float)(a.t_beam - d) * (float)a.inv_delta;
+    auto slope = [&](float v) { return 0.564189584f * (__expf(-v * v) - __expf(-(c - v) * (c - v))); };
+    x = fminf(x, 0.1f);
+    return x * fminf(slope(u), slope(u - x));
+}
+__device__ __forceinline__ void near_take(const MaskArgs& a, MaskNear& f, double d, float est, int q) {
+    if (f.q != 0x7fffffff && !(est > f.est + MASK_NEAR)) {
+        if (est < f.est - MASK_NEAR) return;
+        if (__double_as_longlong(d) == __double_as_longlong(f.d)) {  // the same value: the first drawn
+            f.q = min(f.q, q);
+            return;
+        }
+        const float x = (float)(d - f.d) * (float)a.inv_delta;  // > 0: the new one is further
+        if (!a.sharp && near_fall(a, fmin(d, f.d), fabsf(x)) > 1.0e-14f) {
+            if (x < 0.f) { f.d = d; f.est = est; f.q = q; f.known = false; }
+            return;
+        }
+        if (!f.known) { f.ex = smooth_step_d(f.d, a.t_beam, a.inv_delta, a.sharp); f.known = true; }
+        const double ex = smooth_step_d(d, a.t_beam, a.inv_delta, a.sharp);
+        if (ex > f.ex || (ex == f.ex && q < f.q)) { f.d = d; f.est = est; f.q = q; f.ex = ex; }
+        return;
+    }
+    f.d = d; f.est = est; f.q = q; f.known = false;
+}
+__device__ __forceinline__ void near_take(const MaskArgs& a, MaskNear& f, double d, int q, float tf, float idf) {
+    if (a.sharp) { near_take(a, f, d, (d <= a.t_beam) ? 1.f : 0.f, q); return; }
+    const float u = (float)(a.t_beam - d);  // 2 tf - u = t + d
+    near_take(a, f, d, 0.5f * (erff(u * idf) + erff((2.f * tf - u) * idf)), q);
+}
+
+// Segment, hinge or dot q for the lane's cell (i, j), FP32 pre-test first (FP64 form).
+__device__ __forceinline__ void mask_prim_d(const MaskArgs& a, const Prim& Q, const PrimG& F, int q, int i, int j,
+                                            double xi, double yj, float xf, float yf, double t_star, float tf, float idf,
+                                            MaskNear& f) {
     if (i < Q.box[0] || i > Q.box[1] || j < Q.box[2] || j > Q.box[3]) return;
     if (Q.type == PRIM_SEGMENT) {
         const float xs_f = xf * F.a.x - yf * F.a.y, ys_f = xf * F.a.y + yf * F.a.x;
         if (xs_f < F.a.z || xs_f > F.a.w || ys_f > F.b.x || ys_f < F.b.y) return;
         const double ca = Q.p[0], sa = Q.p[1];
         const double xs = xi * ca - yj * sa, ys = xi * sa + yj * ca;
-        if (xs >= Q.p[2] && xs <= Q.p[4] && ys <= (Q.p[3] + t_star) && ys >= (Q.p[5] - t_star)) {
-            const double dist = fabs(ys - Q.p[3]);
-            const float tf = smooth_step_f(dist, t, inv_delta, a.sharp);
-            double temp;
-            if (sizeof(R) == 4) temp = tf;
-            else {
-                if (tf + 1e-5f <= f.mlow) return;
-                temp = smooth_step_d(dist, t, inv_delta, a.sharp);
-            }
-            if (temp >= f.m)
-                fold_take(f, temp, (Q.p[6] + (xs - Q.p[2]) * (Q.p[8] - Q.p[6]) * inv_ds),
-                          (Q.p[7] + (xs - Q.p[2]) * (Q.p[9] - Q.p[7]) * inv_ds), q);
-        }
+        if (xs >= Q.p[2] && xs <= Q.p[4] && ys <= (Q.p[3] + t_star) && ys >= (Q.p[5] - t_star))
+            near_take(a, f, fabs(ys - Q.p[3]), q, tf, idf);
         return;
     }
     const float ex = xf - F.a.x, ey = yf - F.a.y;
@@ -356,39 +391,21 @@ __device__ __forceinline__ void mask_prim(const MaskArgs& a, const Prim& Q, cons
     const double ddx = xi - Q.p[0], ddy = yj - Q.p[1];
     if (Q.type == PRIM_HINGE) {
         // angular wedge first: FP32 atan2 of the FP64 offsets, exact FP64 only near an end
-        const float beta1f = (float)Q.p[2], beta2f = (float)Q.p[3];
         float gf = atan2f((float)ddy, (float)ddx);
         if (gf < 0.f) gf = 6.28318530717958647692f + gf;
         gf = gf * 57.2957795130823208768f;
         bool near = (fabsf(gf) < 1e-3f) || (fabsf(gf - 360.f) < 1e-3f) || (ddx == 0.0 && ddy == 0.0);
-        bool inw = hinge_inside<float>(gf, beta1f, beta2f, 1e-3f, &near);
+        bool inw = hinge_inside<float>(gf, F.b.x, F.b.y, 1e-3f, &near);
         if (near) {
             const double gamma = convert_angle(atan2(ddy, ddx), a.pi) * 180.0 / a.pi;
             inw = hinge_inside<double>(gamma, Q.p[2], Q.p[3], 0.0, nullptr);
         }
         if (!inw) return;
         const double Rr = sqrt(ddx * ddx + ddy * ddy);
-        if (Rr <= t_star) {
-            const float tf = smooth_step_f(Rr, t, inv_delta, a.sharp);
-            double temp;
-            if (sizeof(R) == 4) temp = tf;
-            else {
-                if (tf + 1e-5f <= f.mlow) return;
-                temp = smooth_step_d(Rr, t, inv_delta, a.sharp);
-            }
-            fold_take(f, temp, Q.p[4], Q.p[5], q);
-        }
+        if (Rr <= t_star) near_take(a, f, Rr, q, tf, idf);
         return;
     }
-    const double Rr = sqrt(ddx * ddx + ddy * ddy);
-    const float tf = smooth_step_f(Rr, t, inv_delta, a.sharp);
-    double temp;
-    if (sizeof(R) == 4) temp = tf;
-    else {
-        if (tf + 1e-5f <= f.mlow) return;
-        temp = smooth_step_d(Rr, t, inv_delta, a.sharp);
-    }
-    fold_take(f, temp, Q.p[2], Q.p[3], q);
+    near_take(a, f, sqrt(ddx * ddx + ddy * ddy), q, tf, idf);
 }
 
 // SmoothStep (create_mask.f90:475-520) with the reference's divisions, for the static parts.
@@ -431,16 +448,14 @@ __device__ __forceinline__ void mask_finish(const MaskArgs& a, double gerf, int 
 // overwrites the value.  Each warp folds its share of a range of primitives; the block
 // combines the partial folds after the segments (then applies the sharp end) and after the
 // hinges and dots.
-template <typename R>
-__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, double gerf) {
+// The FP32 form's (the FP64 form's is k_mask_raster_d).
+__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_f(MaskArgs a, double gerf) {
     pdl_wait();     // the previous kernel of the stream has completed
     if (a.until_full && a.S->time >= a.T_fullspeed) return;
-    constexpr bool F32 = sizeof(R) == 4;
-    using T = R;  // the fold's arithmetic: FP32 in the FP32 form, FP64 in the FP64 form
+    using R = float;
     __shared__ Prim sp[MASK_WARPS][32];
-    __shared__ PrimF sf[MASK_WARPS][F32 ? 1 : 32];
-    __shared__ PrimG sg[MASK_WARPS][F32 ? 32 : 1];
-    __shared__ double cmv[MASK_WARPS][3][32];
+    __shared__ PrimG sg[MASK_WARPS][32];
+    __shared__ float cmv[MASK_WARPS][3][32];
     __shared__ int cidx[MASK_WARPS][32];
     R* mk_ = reinterpret_cast<R*>(a.mask);
     R* vx_ = reinterpret_cast<R*>(a.mvx);
@@ -452,17 +467,15 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, dou
     const int tx0 = u0 / MASK_TX, ty0 = u2 / MASK_TY;
     const int ntx = u1 / MASK_TX - tx0 + 1, nty = u3 / MASK_TY - ty0 + 1;
     const double dx = a.dx, dy = a.dy, mxd = fmax(dx, dy), t = a.t_beam, N = a.N_smooth;
-    const double t_star = t + 2.0 * N * mxd, h = N * mxd;
-    const double rcut = t + 10.0 * h * gerf;
-    const double inv_delta = a.inv_delta, inv_ds = a.inv_ds, inv_eps = a.inv_eps;  // FP64 quotients from the host
+    const double t_star = t + 2.0 * N * mxd;
+    const double inv_delta = a.inv_delta, inv_eps = a.inv_eps;  // FP64 quotients from the host
     const double two_mxd = 2.0 * mxd;
-    const float mg = 1.0e-5f * (float)fmax((double)a.nx * dx, (double)a.ny * dy);
     const int total = *a.nprims;
     // Mean_ux, Mean_uy of the time, for the velocity sponge and the frame
     const double Um = a.full ? mean_flow_x(a.iMeanVelocity, a.S->time, a.cos_ti, a.T_fullspeed, a.pi) : 0.0;
     const double Vm = a.full ? mean_flow_y(a.iMeanVelocity, a.S->time, a.sin_ti, a.T_fullspeed, a.pi) : 0.0;
     const int nseg = a.ns - 1, nsharp = (a.sharp_trailing == 1) ? 1 : 0;
-    // FP32 form: the cell's offset from its tile's origin and the SmoothStep constants
+    // the cell's offset from its tile's origin and the SmoothStep constants
     const float cx = (float)((double)(lane % MASK_TX) * dx), cy = (float)((double)(lane / MASK_TX) * dy);
     const float tf = (float)t, tsf = (float)t_star, idf = (float)inv_delta;
     for (int tile = blockIdx.x; tile < ntx * nty; tile += gridDim.x) {
@@ -483,15 +496,10 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, dou
             continue;
         }
         const double xi = (double)i * dx, yj = (double)j * dy;
-        const float xf = (float)xi, yf = (float)yj;
         const double x0 = (double)ix0 * dx, y0 = (double)iy0 * dy;
-        MaskFold<T> f;
-        f.m = (T)0; f.vx = (T)0; f.vy = (T)0; f.idx = 0x7fffffff; f.mlow = 0.f;
-        if (a.bg) {  // walls and cylinder come first in the draw order (velocity 0)
-            const double b0 = a.bg[cell];
-            f.m = (T)b0;
-            f.mlow = __double2float_rd(b0);
-        }
+        MaskFold f;
+        f.m = 0.f; f.vx = 0.f; f.vy = 0.f; f.idx = 0x7fffffff;
+        if (a.bg) f.m = (float)a.bg[cell];  // walls and cylinder come first in the draw order (velocity 0)
         // this warp's primitives of [q0, q1): q = q0 + MASK_WARPS (32 c + lane) + warp, staged
         // per round of 32 with their FP32 pre-test data
         auto fold_range = [&](int q0, int q1) {
@@ -508,37 +516,19 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, dou
                 if (hit) {
                     const int e = __popc(bal & ((1u << lane) - 1u));
                     sp[warp][e] = P;
-                    if constexpr (F32) {
-                        // k_mask_prep's data, with this tile's offsets (two FP64 subtractions)
-                        PrimG G = a.primg[q];
-                        const bool seg = P.type == PRIM_SEGMENT;
-                        const float ox = (float)((seg ? P.p[10] : P.p[0]) - x0), oy = (float)((seg ? P.p[11] : P.p[1]) - y0);
-                        if (seg) { G.a.z = ox; G.a.w = oy; }
-                        else { G.a.x = ox; G.a.y = oy; }
-                        sg[warp][e] = G;
-                    } else {
-                        PrimF F;
-                        if (P.type == PRIM_SEGMENT || P.type == PRIM_SHARP) {
-                            F.a = make_float4((float)P.p[0], (float)P.p[1], (float)P.p[2] - mg, (float)P.p[4] + mg);
-                            F.b = make_float2((float)(P.p[3] + t_star) + mg, (float)(P.p[5] - t_star) - mg);
-                        } else {
-                            const float lim = (float)((P.type == PRIM_HINGE) ? t_star : rcut) + mg;
-                            F.a = make_float4((float)P.p[0], (float)P.p[1], lim * lim, 0.f);
-                            F.b = make_float2(0.f, 0.f);
-                        }
-                        sf[warp][e] = F;
-                    }
+                    // k_mask_prep's data, with this tile's offsets (two FP64 subtractions)
+                    PrimG G = a.primg[q];
+                    const bool seg = P.type == PRIM_SEGMENT;
+                    const float ox = (float)((seg ? P.p[10] : P.p[0]) - x0), oy = (float)((seg ? P.p[11] : P.p[1]) - y0);
+                    if (seg) { G.a.z = ox; G.a.w = oy; }
+                    else { G.a.x = ox; G.a.y = oy; }
+                    sg[warp][e] = G;
                     cidx[warp][e] = q;
                 }
                 __syncwarp();
                 const int nl = __popc(bal);
-                for (int e = 0; e < nl; ++e) {
-                    if constexpr (F32)
-                        mask_prim_f(a, sp[warp][e], sg[warp][e], cidx[warp][e], i, j, cx, cy, tf, tsf, idf, f);
-                    else
-                        mask_prim<R>(a, sp[warp][e], sf[warp][e], cidx[warp][e], i, j, xi, yj, xf, yf, t, t_star,
-                                     inv_delta, inv_ds, f);
-                }
+                for (int e = 0; e < nl; ++e)
+                    mask_prim_f(a, sp[warp][e], sg[warp][e], cidx[warp][e], i, j, cx, cy, tf, tsf, idf, f);
                 __syncwarp();
             }
         };
@@ -550,13 +540,12 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, dou
             cidx[warp][lane] = my;
             __syncthreads();
             for (int w = 0; w < MASK_WARPS; ++w) {
-                const T mw = (T)cmv[w][0][lane];
+                const float mw = cmv[w][0][lane];
                 const int iw = cidx[w][lane];
                 if (mw > f.m || (mw == f.m && iw < f.idx)) {
-                    f.m = mw; f.vx = (T)cmv[w][1][lane]; f.vy = (T)cmv[w][2][lane]; f.idx = iw;
+                    f.m = mw; f.vx = cmv[w][1][lane]; f.vy = cmv[w][2][lane]; f.idx = iw;
                 }
             }
-            if constexpr (!F32) f.mlow = __double2float_rd(f.m);
             __syncthreads();
         };
         fold_range(0, nseg);
@@ -567,17 +556,10 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, dou
                 const double ca = Q.p[0], sa = Q.p[1];
                 const double xs = xi * ca + yj * sa, ys = -xi * sa + yj * ca;
                 if (xs >= Q.p[2] && xs <= Q.p[4] && ys <= (Q.p[3] + t_star) && ys >= (Q.p[5] - t_star)) {
-                    double tmp2, temp;
-                    if (sizeof(R) == 4) {
-                        tmp2 = smooth_step_f(xs - Q.p[2], two_mxd, inv_delta, a.sharp);
-                        temp = smooth_step_f(fabs(ys - Q.p[3]), t, inv_delta, a.sharp);
-                    } else {
-                        tmp2 = smooth_step_d(xs - Q.p[2], two_mxd, inv_delta, a.sharp);
-                        temp = smooth_step_d(fabs(ys - Q.p[3]), t, inv_delta, a.sharp);
-                    }
-                    f.m = (T)(temp * tmp2);
-                    f.mlow = __double2float_rd(temp * tmp2);
-                    if (xs - Q.p[2] >= two_mxd) { f.vx = (T)Q.p[6]; f.vy = (T)Q.p[7]; }
+                    const double tmp2 = smooth_step_f(xs - Q.p[2], two_mxd, inv_delta, a.sharp);
+                    const double temp = smooth_step_f(fabs(ys - Q.p[3]), t, inv_delta, a.sharp);
+                    f.m = (float)(temp * tmp2);
+                    if (xs - Q.p[2] >= two_mxd) { f.vx = (float)Q.p[6]; f.vy = (float)Q.p[7]; }
                 }
             }
         }
@@ -591,6 +573,133 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster(MaskArgs a, dou
             vx_[cell] = (R)vx;
             vy_[cell] = (R)vy;
         }
+    }
+}
+
+// The FP64 form's raster: k_mask_raster_f's tiles, with the reference's FP64 tests.  FP64 issue bounds
+// it (64 cycles a warp instruction, few tiles), so the warps keep the winning primitive by its
+// distance (MaskNear) and the block evaluates what is FP64 and per cell once, each part on its own
+// warp (SMSP): the two erf of SmoothStep and the two velocity components.
+// Measured (GB300; before, SmoothStep and the velocity for every primitive that beat the fold so far):
+// 256^2, ns = 64 36.6 -> 26.4 us (the step 165 -> 156); 64^2, ns = 16 31.0 -> 30.5; 512 x 256 with walls and
+// a cylinder, where every cell was drawn each step, 43.8 -> 24.5.
+__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_d(MaskArgs a, double gerf) {
+    pdl_wait();     // the previous kernel of the stream has completed
+    if (a.until_full && a.S->time >= a.T_fullspeed) return;
+    __shared__ Prim sp[MASK_WARPS][32];
+    __shared__ PrimG sg[MASK_WARPS][32];
+    __shared__ double cd[MASK_WARPS][32];
+    __shared__ float ce[MASK_WARPS][32];
+    __shared__ int cidx[MASK_WARPS][32];
+    double *mk_ = reinterpret_cast<double*>(a.mask), *vx_ = reinterpret_cast<double*>(a.mvx), *vy_ = reinterpret_cast<double*>(a.mvy);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = a.rect[0], r1 = a.rect[1], r2 = a.rect[2], r3 = a.rect[3];
+    const int u0 = a.rect[4], u1 = a.rect[5], u2 = a.rect[6], u3 = a.rect[7];
+    if (u1 < u0 || u3 < u2) return;
+    const int tx0 = u0 / MASK_TX, ty0 = u2 / MASK_TY;
+    const int ntx = u1 / MASK_TX - tx0 + 1, nty = u3 / MASK_TY - ty0 + 1;
+    const double dx = a.dx, dy = a.dy, mxd = fmax(dx, dy), t = a.t_beam;
+    const double t_star = t + 2.0 * a.N_smooth * mxd, inv_delta = a.inv_delta, two_mxd = 2.0 * mxd;
+    const float tf = (float)t, idf = (float)inv_delta;
+    const int total = *a.nprims, nseg = a.ns - 1, nsharp = (a.sharp_trailing == 1) ? 1 : 0;
+    // Mean_ux, Mean_uy of the time, for the velocity sponge and the frame
+    const double Um = a.full ? mean_flow_x(a.iMeanVelocity, a.S->time, a.cos_ti, a.T_fullspeed, a.pi) : 0.0;
+    const double Vm = a.full ? mean_flow_y(a.iMeanVelocity, a.S->time, a.sin_ti, a.T_fullspeed, a.pi) : 0.0;
+    for (int tile = blockIdx.x; tile < ntx * nty; tile += gridDim.x) {
+        const int ix0 = (tx0 + tile % ntx) * MASK_TX, iy0 = (ty0 + tile / ntx) * MASK_TY;
+        const int ix1 = ix0 + MASK_TX - 1, iy1 = iy0 + MASK_TY - 1;
+        const int i = ix0 + (lane % MASK_TX), j = iy0 + (lane / MASK_TX);
+        const size_t cell = (size_t)j * a.nx + i;
+        // the cell's value and velocity before the primitives (warp 0's are used): walls and
+        // cylinder come first in the draw order (velocity 0)
+        double m = a.bg ? a.bg[cell] : 0.0, vx = 0.0, vy = 0.0;
+        auto write = [&]() {
+            if (a.full) mask_finish(a, gerf, i, j, cell, Um, Vm, m, vx, vy);
+            mk_[cell] = m * a.inv_eps;
+            vx_[cell] = vx;
+            vy_[cell] = vy;
+        };
+        if (r1 < ix0 || r0 > ix1 || r3 < iy0 || r2 > iy1) {
+            if (warp == 0) write();
+            continue;
+        }
+        const double xi = (double)i * dx, yj = (double)j * dy;
+        const float xf = (float)xi, yf = (float)yj;
+        // the primitives [q0, q1): each warp folds its share (dealt as in k_mask_raster_f), the block
+        // combines, and the winner's value and velocity replace the cell's where the value is larger
+        auto draw = [&](int q0, int q1) {
+            MaskNear f;
+            f.q = 0x7fffffff; f.d = 0.0; f.ex = 0.0; f.est = 0.f; f.known = false;
+            for (int base = q0; base < q1; base += 32 * MASK_WARPS) {
+                const int q = base + MASK_WARPS * lane + warp;
+                bool hit = false;
+                if (q < q1) {
+                    const int* bx = a.prims[q].box;
+                    hit = !(bx[1] < ix0 || bx[0] > ix1 || bx[3] < iy0 || bx[2] > iy1) && bx[0] <= bx[1] && bx[2] <= bx[3];
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, hit);
+                if (hit) {
+                    const int e = __popc(bal & ((1u << lane) - 1u));
+                    sp[warp][e] = a.prims[q];
+                    sg[warp][e] = a.primg[q];
+                    cidx[warp][e] = q;
+                }
+                __syncwarp();
+                const int nl = __popc(bal);
+                for (int e = 0; e < nl; ++e)
+                    mask_prim_d(a, sp[warp][e], sg[warp][e], cidx[warp][e], i, j, xi, yj, xf, yf, t_star, tf, idf, f);
+                __syncwarp();
+            }
+            cd[warp][lane] = f.d;
+            ce[warp][lane] = f.est;
+            __syncthreads();
+            cidx[warp][lane] = f.q;
+            __syncthreads();
+            f.q = 0x7fffffff;
+            for (int w = 0; w < MASK_WARPS; ++w)
+                if (cidx[w][lane] != 0x7fffffff) near_take(a, f, cd[w][lane], ce[w][lane], cidx[w][lane]);
+            __syncthreads();
+            const bool any = f.q != 0x7fffffff;
+            if (any) {
+                const Prim& Q = a.prims[f.q];
+                if (warp == 0) cd[0][lane] = a.sharp ? 0.0 : erf((t - f.d) * inv_delta);
+                else if (warp == 1) cd[1][lane] = a.sharp ? 0.0 : erf((f.d + t) * inv_delta);
+                else {
+                    const int c = warp - 2;  // velocity component
+                    double v;
+                    if (Q.type == PRIM_SEGMENT) {
+                        const double xs = xi * Q.p[0] - yj * Q.p[1];
+                        v = Q.p[6 + c] + (xs - Q.p[2]) * (Q.p[8 + c] - Q.p[6 + c]) * a.inv_ds;
+                    } else {
+                        v = Q.type == PRIM_HINGE ? Q.p[4 + c] : Q.p[2 + c];
+                    }
+                    cd[warp][lane] = v;
+                }
+            }
+            __syncthreads();
+            if (warp == 0 && any) {
+                const double temp = a.sharp ? ((f.d <= t) ? 1.0 : 0.0) : 0.5 * (cd[0][lane] + cd[1][lane]);
+                if (temp > m) { m = temp; vx = cd[2][lane]; vy = cd[3][lane]; }
+            }
+            __syncthreads();  // the next range or tile writes the shared values
+        };
+        if (!nsharp) {
+            draw(0, total);
+        } else {
+            draw(0, nseg);
+            const Prim& Q = a.prims[nseg];  // the sharp end overwrites the segments' value
+            if (warp == 0 && !(i < Q.box[0] || i > Q.box[1] || j < Q.box[2] || j > Q.box[3])) {
+                const double ca = Q.p[0], sa = Q.p[1];
+                const double xs = xi * ca + yj * sa, ys = -xi * sa + yj * ca;
+                if (xs >= Q.p[2] && xs <= Q.p[4] && ys <= (Q.p[3] + t_star) && ys >= (Q.p[5] - t_star)) {
+                    const double tmp2 = smooth_step_d(xs - Q.p[2], two_mxd, inv_delta, a.sharp);
+                    m = smooth_step_d(fabs(ys - Q.p[3]), t, inv_delta, a.sharp) * tmp2;
+                    if (xs - Q.p[2] >= two_mxd) { vx = Q.p[6]; vy = Q.p[7]; }
+                }
+            }
+            draw(nseg + 1, total);
+        }
+        if (warp == 0) write();
     }
 }
 
@@ -885,8 +994,8 @@ void launch_sponge_mask(const StaticMaskArgs& a, double gerf, cudaStream_t st) {
 void launch_mask(const MaskArgs& a, double gerf, bool fp32, cudaStream_t st, bool pdl) {
     // four-warp blocks, two per SM: a tile's primitives over the four SMSPs of an SM
     const int blocks = 2 * a.nsm;
-    if (fp32) launch_k(k_mask_raster<float>, dim3(blocks), dim3(32 * MASK_WARPS), 0, st, pdl, a, gerf);
-    else launch_k(k_mask_raster<double>, dim3(blocks), dim3(32 * MASK_WARPS), 0, st, pdl, a, gerf);
+    if (fp32) launch_k(k_mask_raster_f, dim3(blocks), dim3(32 * MASK_WARPS), 0, st, pdl, a, gerf);
+    else launch_k(k_mask_raster_d, dim3(blocks), dim3(32 * MASK_WARPS), 0, st, pdl, a, gerf);
 }
 
 // BeamSurfaceIntegral (BeamForces.f90:306-509)

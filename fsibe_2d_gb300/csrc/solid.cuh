@@ -79,6 +79,9 @@ struct Prim {
 //            normal offset, -, -), c = (v1x, v1y, (v2x - v1x)/ds, (v2y - v1y)/ds)
 //   hinge / dot: a = (px - x0, py - y0, R^2 limit, -), b = (beta1, beta2, -, -), c = (vx, vy, -, -)
 // k_mask_prep forms everything but the tile-relative offsets (zero there) once per primitive.
+// The FP64 form keeps its pre-test data there, in the domain's coordinates:
+//   segment / sharp: a = (cos, sin, lower, upper bound along the axis), b = (upper, lower bound across)
+//   hinge / dot: a = (px, py, R^2 limit, -), b = (beta1, beta2 or the velocity, -, -)
 struct PrimG {
     float4 a, b, c;
 };
@@ -91,7 +94,8 @@ struct MaskArgs {
     double dx, dy, ds, t_beam, N_smooth, eps, pi, angle_deg;
     const double *x, *y, *vx, *vy, *th;
     Prim* prims;
-    PrimG* primg;  // the FP32 form's data of prims (k_mask_prep), or null
+    PrimG* primg;  // the raster's FP32 data of prims (k_mask_prep)
+    int f32;       // 1: the FP32 form
     int* nprims;
     int* rect;    // [0..3] union of this step's primitive boxes (x0, x1, y0, y1), [4..7] its union
                   // with the previous step's box (every cell outside [0..3] is zero), [8..11] the
@@ -101,9 +105,12 @@ struct MaskArgs {
     MotionArgs mo;         // the leading edge's motion (alpha of the time)
     int nsm;      // SMs of the device (raster grid size)
     void *mask, *mvx, *mvy;  // R*[ny][nx]
-    // the parts of the mask that are not the beam (create_mask.f90:21-68, 120-204); with `full`
-    // set every cell is drawn each step (the box is the grid)
-    int full;
+    // the parts of the mask that are not the beam (create_mask.f90:21-68, 120-204): with `full` set
+    // a cell without a primitive holds the finished background instead of zero.  Walls and the
+    // cylinder do not change, so after the first draw (the previous box starts as the grid) only the
+    // beam's boxes are drawn; with `every` set (the velocity sponge and the frame, which follow the
+    // mean flow) every cell is, each step
+    int full, every;
     const double* bg;        // walls and the leading-edge cylinder (unscaled, velocity 0), or null
     const double* frame;     // iSponge = 22: the smoothed frame around the domain, or null
     double frame_c;          // its weight eps / max(1e-3, eps)
