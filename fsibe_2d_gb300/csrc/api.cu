@@ -1651,11 +1651,11 @@ int fsibe_create(const fsibe_params* p, fsibe_ctx** out) {
     }
     c->beam_smem = beam_smem_setup(ns);
     {
-        // the beam's Newton step on a cluster of 16 (or 8) CTAs when the device places one;
-        // FSIBE_BEAM_CLUSTER = 0 / 8 / 16 caps the size (0: the single-CTA kernel)
+        // the beam's Newton step on a cluster of 16, 8 or 4 CTAs when the device places one;
+        // FSIBE_BEAM_CLUSTER = 0 / 4 / 8 / 16 caps the size (0: the single-CTA kernel)
         const char* e = std::getenv("FSIBE_BEAM_CLUSTER");
         const int want = e ? std::atoi(e) : 16;
-        c->beam_cl = (want >= 8) ? beam_cluster_setup(ns, want, &c->beam_cl_smem, &c->beam_cl_big) : 0;
+        c->beam_cl = (want >= 4) ? beam_cluster_setup(ns, want, &c->beam_cl_smem, &c->beam_cl_big) : 0;
         if (c->beam_cl) {
             ALLOC(c->minv, 4 * beam_cluster_minv_floats(ns, c->beam_cl));
             ALLOC(c->minv_rse, 4 * (size_t)(n + 16));

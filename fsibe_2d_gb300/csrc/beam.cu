@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(256) k_beam(BeamArgs b) {
     // integer arithmetic, checked step by step: running_sum.cuh)
     {
         __shared__ int rs_flags[4];
-        const int nser = running_sums4(w.cs, ns + 8, w.pre, ns + 8, ns, rs_flags, NoIdle());
+        const int nser = running_sums4<false>(w.cs, ns + 8, w.pre, ns + 8, ns, rs_flags, NoIdle());
         if (threadIdx.x == 0 && nser) S->phase[30] += nser;
     }
     // positions and velocities, and in the same pass each thread's terms of the emergency brake

@@ -1,6 +1,6 @@
 // beam_cluster.cu -- the Newton step of the beam (the work of k_beam: IBES_solver after the
 // step's loads are known, SolidSolver.f90:197-414, with integrate_position and SolidEnergies)
-// on one thread-block cluster of R CTAs (R = 16, or 8 where 16 cannot be placed).
+// on one thread-block cluster of R CTAs (16, 8 or 4: beam_cluster_setup).
 //
 // Why a cluster: FP64 issue limits the beam (one FP64 warp instruction per SMSP every ~64
 // cycles on this chip) and one CTA has four SMSPs.  Spreading F, the Jacobian rows and the
@@ -675,23 +675,25 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
         S->dt_old = dt;
     }
     // the four running sums in the reference's order (the positions decide grid-aligned boxes
-    // of the mask and the drag window, so their roundings must be the reference's): one lane a
-    // sum in integer arithmetic, checked step by step (running_sum.cuh), while the other warps
-    // copy.  The large-beam form first stages the terms into the shared memory of the solution
-    // vectors x and xdi (32 ns + 192 bytes, at least the 32 ns needed), which the Newton loop
-    // is done with.
+    // of the mask and the drag window, so their roundings must be the reference's;
+    // running_sum.cuh), a warp a sum, while the other warps copy.  The large-beam form first
+    // stages the terms into the shared memory of the solution vectors x and xdi (32 ns + 192
+    // bytes, at least the 32 ns needed), and the sums go to the node arrays oo5 .. taun_s: the
+    // Newton loop is done with both.
     const double* src0 = pcs;
+    double* pre = pcs + 4 * L;
     if (big) {
         double* st = x;  // x, then xdi: contiguous
         for (int i = tid; i < ns; i += nthr) {
             st[i] = pcs[i]; st[ns + i] = pcs[L + i]; st[2 * ns + i] = pcs[2 * L + i]; st[3 * ns + i] = pcs[3 * L + i];
         }
         src0 = st;
+        pre = oo5;
         __syncthreads();
     }
     {
         __shared__ int rs_flags[4];
-        const int nser = running_sums4(src0, big ? ns : L, pcs + 4 * L, L, ns, rs_flags, copies);
+        const int nser = running_sums4<true>(src0, big ? ns : L, pre, L, ns, rs_flags, copies);
         if (tid == 0 && nser) S->phase[30] += nser;
     }
     PH(8);
@@ -701,7 +703,6 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
     {
         __shared__ double ecol[6][256];
         static_assert(256 >= 32 * 6, "one warp a column");
-        const double* pre = pcs + 4 * L;
         const double ca = mo.ca, sa = mo.sa, alpha_t = mo.alpha_t, idt = 1.0 / dt;
         double sk = 0, sp = 0, se = 0, sax = 0, say = 0, mx = 0;
         for (int i = tid; i < ns; i += nthr) {
@@ -772,10 +773,13 @@ size_t beam_cluster_minv_floats(int ns, int R) {
     return (size_t)R * Y.rmax * Y.mld;
 }
 
-// The cluster size for a beam of ns nodes: 16 when the device places a 16-CTA cluster with
-// this kernel's shared memory and every CTA gets at least 8 rows, else 8 under the same
-// conditions, else 0 (the single-CTA kernel).  want caps it.  *big_out = 1 when only the
-// large-beam form (factor and M^-1 in global memory) fits.
+// The cluster size for a beam of ns nodes: 16 CTAs above 144 nodes, 8 up to there, 4 where 8 would
+// leave a CTA without a quad of rows (ns < 14); the next smaller where the device does not place one
+// with this kernel's shared memory, and 0 (the single-CTA kernel) where none fits.  A wider cluster
+// divides the rows' FP64 and the inverse products, a narrower one has the cheaper barriers (two a
+// pass).  Measured (GB300, 16 / 8 / 4 CTAs, the beam kernel in us): ns = 16 - / 61 / 60 (single CTA
+// 100), 64 63 / 58.5 / 57.5, 101 84 / 80 / 83.5, 127 78.5 / 74 / 84, 256 88 / 111 / 131.  want caps it.
+// *big_out = 1 when only the large-beam form (factor and M^-1 in global memory) fits.
 int beam_cluster_setup(int ns, int want, size_t* smem_out, int* big_out) {
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
@@ -785,8 +789,8 @@ int beam_cluster_setup(int ns, int want, size_t* smem_out, int* big_out) {
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, (const void*)k_beam_cl) != cudaSuccess) return 0;
     static size_t cur = 0;
-    for (int R = 16; R >= 8; R /= 2) {
-        if (R > want || 2 * ns + 4 < 8 * R) continue;  // at least 8 rows per CTA
+    for (int R = ns > 144 ? 16 : 8; R >= 4; R /= 2) {
+        if (R > want || 2 * ns + 4 < 4 * R) continue;  // at least one quad of rows per CTA
         for (int big = 0; big <= 1; ++big) {
             ClLayout Y;
             cl_layout(ns, R, Y, big != 0);
@@ -828,7 +832,7 @@ size_t beam_cluster_fact_floats(int ns, int R) { return (size_t)R * cl_fact_floa
 // the terms and sums in global memory.
 __global__ void __launch_bounds__(256, 1) k_running_sums(const double* src, double* dst, int n, int* nserial) {
     __shared__ int flags[4];
-    const int r = running_sums4(src, n, dst, n, n, flags, NoIdle());
+    const int r = running_sums4<false>(src, n, dst, n, n, flags, NoIdle());
     if (threadIdx.x == 0) *nserial = r;
 }
 cudaError_t launch_running_sums(const double* src, double* dst, int n, int* nserial, cudaStream_t st) {

@@ -1,18 +1,28 @@
 // The four running sums of integrate_position (integrate_position.f90:14-44), bit for bit the
-// sequential FP64 loop s_0 = +0, s_(k+1) = s_k + a_k (round to nearest even), mostly in integer
-// arithmetic.
+// sequential FP64 loop s_0 = +0, s_(k+1) = s_k + a_k (round to nearest even).
 //
 // A dependent FP64 addition costs about 75 cycles on this chip.  While s_k and s_(k+1) stay in
 // one binade [2^e, 2^(e+1)), the FP64 sum is an integer sum on that binade's grid 2^g
 // (g = e - 52): with s_k = m 2^g,
 //     s_(k+1) = (m + RN(a_k / 2^g)) 2^g,
-// where RN rounds to the nearest integer and a tie towards the even m + RN.  The result is in
-// the binade exactly when 2^52 < |m + RN| < 2^53 (at 2^52 the exact sum may lie below the
-// binade, where the grid is finer).  So a warp per sum takes 32 steps at a time as a prefix sum
-// of the rounded terms, up to the first step that leaves the binade, which is done by the FP64
-// addition; its result gives the next binade.  Afterwards every step is checked in parallel by
-// the FP64 addition, bits(s_k + a_k) == bits(s_(k+1)), and a sum with any mismatch is formed
-// again by the plain serial loop: the result is that loop's in every case.
+// where RN rounds to the nearest integer; only a tie depends on m.  So a warp a sum
+//   * sums the terms approximately in fixed point (each lane a run of consecutive terms, one scan),
+//     which tells every s_k's binade where the error bound leaves no doubt;
+//   * rounds the terms of steps within a binade to its grid in parallel: their increments and those
+//     increments' prefix sums do not depend on the running value.  What is left are the events:
+//     steps into another binade, ties, zeros, values near a power of two;
+//   * walks the events in order: the value before an event is the value after the last one plus a
+//     prefix difference (integers), the event itself an FP64 addition;
+//   * fills in every s_k in parallel.
+// Afterwards every step is checked in parallel by the FP64 addition, bits(s_k + a_k) ==
+// bits(s_(k+1)), and a sum with any mismatch is formed again by the serial loop: the result is that
+// loop's in every case.  A beam of 1024 nodes has 11 to 81 events a sum.  Up to RS_SERIAL terms the
+// serial loop itself is the shortest (78 cycles a step from shared memory): this code runs once a
+// launch, on one warp, and its integer chains are long.  Sums with many events, non-finite or very
+// small terms take the serial loop too.
+// Measured (GB300, cycles of the phase in k_beam_cl; batches of 32 integer steps from one binade change to
+// the next before): ns = 16 9.4 -> 3.1 k, 64 13.6 -> 6.7, 101 41 -> 10.1, 127 11.3 -> 11.8, 256 30.7 -> 22
+// (by events 27), 1024 79 -> 69 (serial 82).
 #pragma once
 #include "common.cuh"
 
@@ -38,103 +48,167 @@ __device__ __forceinline__ long long term_inc(double a, int g, bool& ok, bool& t
     return neg ? -r : r;
 }
 
-// One sum on one warp (all 32 lanes, the same arguments): dst[k] = s_k for k < n.  After an
-// FP64 step, batches of 32 integer steps on the grid of its result's binade: lane t rounds term
-// k + t (a tie by the parity of s_(k+t), from a scan of the steps' parity maps), a warp scan of
-// the increments gives every s_(k+t+1), and the first step whose result leaves the binade (or
-// whose term does not allow an integer step) ends the batch and is the next FP64 step.
-__device__ __forceinline__ void running_sum_warp(const double* __restrict__ src, double* __restrict__ dst, int n) {
-    const unsigned long long TWO52 = 1ull << 52, TWO53 = 1ull << 53, FRAC = TWO52 - 1ull;
-    const int lane = threadIdx.x & 31;
-    double cur = 0.0;  // s_k, the same in every lane
+constexpr int RS_SERIAL = 320, RS_MAX = 2016, RS_EVENTS = 96;  // RS_MAX: 63 terms a lane
+
+// The serial loop, by lane 0 of a warp: 78 cycles a step with the rows in shared memory (SH), 112
+// through generic addresses.
+template <bool SH>
+__device__ __forceinline__ void running_sum_serial(const double* __restrict__ src, double* __restrict__ dst, int n) {
+    if ((threadIdx.x & 31) != 0) return;
+    if (SH) { __builtin_assume(__isShared(src)); __builtin_assume(__isShared(dst)); }
+    double v = 0.0;
     int k = 0;
-    while (k < n) {
-        // the FP64 step k, then the binade of its result
-        if (lane == 0) dst[k] = cur;
-        cur = cur + src[k];
-        ++k;
-        const unsigned long long cb = (unsigned long long)__double_as_longlong(cur);
-        const int ex = (int)((cb >> 52) & 0x7FF);
-        if (ex == 0 || ex == 0x7FF) continue;  // zero, subnormal or non-finite: FP64 steps
-        const bool negs = (cb >> 63) != 0;
-        const long long mc = (long long)((cb & FRAC) | TWO52);
-        long long m = negs ? -mc : mc;  // s_k = m 2^g, 2^52 <= |m| < 2^53
-        const int g = ex - 1075;
-        const unsigned long long hi = cb & ~FRAC;
-        const long long blo = negs ? -(long long)TWO53 : (long long)TWO52;  // blo < s_(k+1) / 2^g < bhi
-        const long long bhi = negs ? -(long long)TWO52 : (long long)TWO53;
-        while (k < n) {
-            const int j = k + lane;
-            bool ok, tie;
-            long long inc = term_inc(j < n ? src[j] : 0.0, g, ok, tie);
-            // the parity of the running value before each step, by a scan of parity maps: a tie
-            // makes the value even (bit 1: reset), any other step flips it by inc's low bit (bit 0)
-            if (__any_sync(0xffffffffu, tie && ok)) {
-                unsigned f = tie ? 2u : (unsigned)(inc & 1);
+    for (; k + 8 <= n; k += 8) {
+        double t[8];
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned e = __shfl_up_sync(0xffffffffu, f, o);  // the earlier steps' map
-                    if (lane >= o) f = (f & 2u) ? f : ((e & 2u) | ((e ^ f) & 1u));
-                }
-                unsigned fe = __shfl_up_sync(0xffffffffu, f, 1);
-                if (lane == 0) fe = 0u;
-                const long long par = (fe & 2u) ? (long long)(fe & 1u) : ((m ^ (long long)fe) & 1);
-                if (tie) inc += (par ^ inc) & 1;  // the even of the two candidates
-            }
-            long long p = inc;  // inclusive scan of the increments
+        for (int i = 0; i < 8; ++i) t[i] = src[k + i];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long v = __shfl_up_sync(0xffffffffu, p, o);
-                if (lane >= o) p += v;
-            }
-            const long long m1 = m + p;  // s_(j+1) / 2^g while the steps before it hold
-            ok = ok && j < n && m1 > blo && m1 < bhi;
-            const unsigned bad = __ballot_sync(0xffffffffu, !ok);
-            const int nok = bad ? __ffs((int)bad) - 1 : 32;  // steps k .. k + nok - 1 hold
-            if (lane < nok) {
-                const long long mv = m + p - inc;  // s_j / 2^g
-                dst[j] = __longlong_as_double((long long)(hi | ((unsigned long long)(mv < 0 ? -mv : mv) & FRAC)));
-            }
-            if (nok > 0) {
-                m = __shfl_sync(0xffffffffu, m1, nok - 1);
-                cur = __longlong_as_double((long long)(hi | ((unsigned long long)(m < 0 ? -m : m) & FRAC)));
-            }
-            k += nok;
-            if (nok < 32) break;  // step k (if any) is an FP64 step
+        for (int i = 0; i < 8; ++i) { dst[k + i] = v; v = v + t[i]; }
+    }
+    for (; k < n; ++k) { dst[k] = v; v = v + src[k]; }
+}
+
+template <typename T> __device__ __forceinline__ T rs_scan(T v) {  // exclusive sum over the lanes
+    const int lane = threadIdx.x & 31;
+    T p = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T x = __shfl_up_sync(0xffffffffu, p, o);
+        if (lane >= o) p += x;
+    }
+    return p - v;
+}
+// the value d steps of cur's grid further, in its binade
+__device__ __forceinline__ double rs_advance(double cur, long long d) {
+    const unsigned long long TWO52 = 1ull << 52, FRAC = TWO52 - 1ull;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(cur);
+    const long long mc = (long long)((b & FRAC) | TWO52), m = ((long long)b < 0 ? -mc : mc) + d;
+    return d == 0 ? cur : __longlong_as_double((long long)((b & ~FRAC) | ((unsigned long long)(m < 0 ? -m : m) & FRAC)));
+}
+
+// One sum on one warp (all 32 lanes, the same arguments): dst[k] = s_k for k < n <= RS_MAX; start
+// and base have RS_EVENTS entries of shared memory.  False when the sum is left to the serial loop.
+template <bool SH>
+__device__ __noinline__ bool running_sum_warp(const double* __restrict__ src, double* __restrict__ dst, int n, double* start, long long* base) {
+    if (SH) { __builtin_assume(__isShared(src)); __builtin_assume(__isShared(dst)); }
+    // an odd run of terms a lane: the lanes' accesses fall in different banks
+    const int lane = threadIdx.x & 31, c = ((n + 31) / 32) | 1;
+    const int k0 = min(lane * c, n), k1 = min(k0 + c, n);
+    long long* pre = reinterpret_cast<long long*>(dst);  // prefix sums until the sums replace them
+    unsigned mx = 0;
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) mx = max(mx, (unsigned)__double2hiint(src[k]) & 0x7fffffffu);
+    const int em = (int)(__reduce_max_sync(0xffffffffu, mx) >> 20);
+    if (em == 0x7FF || em < 64) return false;
+    // a term in units of 2^(em - 1073), towards zero (below 2^51; n of them below 2^62)
+    auto fix = [&](double a) {
+        const int hi = __double2hiint(a), e = (hi >> 20) & 0x7FF;
+        const unsigned long long m = (((unsigned long long)(((unsigned)hi & 0xfffffu) | 0x100000u)) << 32) | (unsigned)__double2loint(a);
+        const long long v = (long long)(m >> min(em - e + 2, 63));
+        return hi < 0 ? -v : v;
+    };
+    long long tot = 0, mag = 0;
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+        const long long q = fix(src[k]);
+        tot += q;
+        mag += q < 0 ? -q : q;
+    }
+    long long s = rs_scan(tot);
+    mag = rs_scan(mag) + mag;
+    mag = __shfl_sync(0xffffffffu, mag, 31);
+    // error of s against the sequential sum: the truncations, and the n rounding errors, each at most
+    // 2^-53 of the sum of magnitudes
+    const long long err = 2 * n + (mag >> 41);
+    // s_k's binade: 1 + its exponent above the unit, with the sign; 0 in doubt
+    auto binade = [&](long long v) {
+        const long long a = v < 0 ? -v : v, lo = a - err, hi = a + err;
+        if (lo <= 0) return 0;
+        const int bl = 64 - __clzll(lo), bh = 64 - __clzll(hi);
+        return bl != bh ? 0 : (v < 0 ? -bl : bl);
+    };
+    unsigned long long events = 0;  // of the lane's steps
+    long long p = 0;                // prefix sum of its increments
+    int bin = lane == 0 ? 0 : binade(s);
+#pragma unroll 2
+    for (int k = k0; k < k1; ++k) {
+        const double a = src[k];
+        s += fix(a);
+        const int next = binade(s);
+        bool ok = false, tie = false;
+        long long inc = 0;
+        if (bin != 0 && bin == next) inc = term_inc(a, (bin < 0 ? -bin : bin) - 53 + (em - 1073), ok, tie);
+        pre[k] = p;
+        if (ok && !tie) p += inc;
+        else events |= 1ull << (k - k0);
+        bin = next;
+    }
+    const long long off = rs_scan(p);
+    const int nev = __popcll(events), ord = rs_scan(nev);
+    if (__shfl_sync(0xffffffffu, ord + nev, 31) > RS_EVENTS) return false;
+    __syncwarp();
+    // the events in order, every lane alike: step 0 is one (s_0 = 0)
+    double cur = 0.0;
+    long long at = 0;
+    int ne = 0;
+    for (int l = 0; l < 32; ++l) {
+        unsigned long long m = __shfl_sync(0xffffffffu, events, l);
+        const long long o = __shfl_sync(0xffffffffu, off, l);
+        while (m) {
+            const int k = l * c + __ffsll((long long)m) - 1;
+            m &= m - 1ull;
+            const long long pk = o + pre[k];
+            cur = rs_advance(cur, pk - at) + src[k];
+            at = pk;
+            if (lane == 0) { start[ne] = cur; base[ne] = pk; }
+            ++ne;
         }
     }
+    __syncwarp();
+    int j = ord;  // events before step k
+    for (int k = k0; k < k1; ++k) {
+        dst[k] = k == 0 ? 0.0 : rs_advance(start[j - 1], off + pre[k] - base[j - 1]);
+        if ((events >> (k - k0)) & 1ull) ++j;
+    }
+    return true;
 }
 
 // The four sums of rows src + q sld into dst + q dld (q < 4), each by warp q, then checked by
 // all threads of the (256-thread) block.  idle(i, m) runs on
 // warps 4..7 (i < m) meanwhile.  flags: 4 ints of shared memory.  Returns the number of sums the
 // check sent to the plain serial loop.  Ends with a barrier.
-template <typename Idle>
+// SH: src and dst are shared memory.
+template <bool SH, typename Idle>
 __device__ int running_sums4(const double* src, int sld, double* dst, int dld, int n, int* flags, Idle idle) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ double start[4][RS_EVENTS];
+    __shared__ long long base[4][RS_EVENTS];
     if (warp < 4) {
+        const double* s = src + (size_t)warp * sld;
+        double* d = dst + (size_t)warp * dld;
         if (lane == 0) flags[warp] = 0;
-        running_sum_warp(src + (size_t)warp * sld, dst + (size_t)warp * dld, n);
+        if (n <= RS_SERIAL || n > RS_MAX || !running_sum_warp<SH>(s, d, n, start[warp], base[warp])) {
+            __syncwarp();
+            running_sum_serial<SH>(s, d, n);
+        }
     } else {
         idle(tid - 128, blockDim.x - 128);
     }
     __syncthreads();
+    if (n <= RS_SERIAL) return 0;
     for (int j = tid; j < 4 * n; j += blockDim.x) {
         const int q = j / n, k = j - q * n;
         if (k + 1 < n) {
             const double* s = src + (size_t)q * sld;
             const double* d = dst + (size_t)q * dld;
-            if (__double_as_longlong(d[k] + s[k]) != __double_as_longlong(d[k + 1])) flags[q] = 1;
+            // (a NaN's bits differ from one operation to another: two NaNs agree)
+            const double v = d[k] + s[k], x = d[k + 1];
+            if (__double_as_longlong(v) != __double_as_longlong(x) && (v == v || x == x)) flags[q] = 1;
         }
     }
     __syncthreads();
     const int bad = (flags[0] != 0) + (flags[1] != 0) + (flags[2] != 0) + (flags[3] != 0);
-    if (lane == 0 && warp < 4 && flags[warp]) {
-        const double* s = src + (size_t)warp * sld;
-        double* d = dst + (size_t)warp * dld;
-        double v = 0.0;
-        for (int k = 0; k < n; ++k) { d[k] = v; v = v + s[k]; }
-    }
+    if (warp < 4 && flags[warp]) running_sum_serial<SH>(src + (size_t)warp * sld, dst + (size_t)warp * dld, n);
     __syncthreads();
     return bad;
 }

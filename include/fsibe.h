@@ -298,9 +298,9 @@ int fsibe_tile_config(fsibe_ctx* ctx, int32_t* out6);
  * faster; FSIBE_PY_ENG = 0 / 1 forces one. */
 int fsibe_press_y_engine(fsibe_ctx* ctx, int32_t* eng);
 
-/* CTAs of the thread-block cluster that runs the beam's Newton step (16 or 8; 0 when the
- * single-CTA kernel runs it).  Chosen at fsibe_create from what the device can place;
- * the environment variable FSIBE_BEAM_CLUSTER = 0, 8 or 16 caps it. */
+/* CTAs of the thread-block cluster that runs the beam's Newton step (16, 8 or 4; 0 when the
+ * single-CTA kernel runs it).  Chosen at fsibe_create from the number of nodes and what the
+ * device can place; the environment variable FSIBE_BEAM_CLUSTER = 0, 4, 8 or 16 caps it. */
 int fsibe_beam_cluster(fsibe_ctx* ctx, int32_t* ctas);
 /* Number of kernel launches one fsibe_step issues (for the bench's gpu_launches). */
 int fsibe_launches_per_step(fsibe_ctx* ctx, int* launches);
