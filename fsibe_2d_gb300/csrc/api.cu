@@ -800,8 +800,11 @@ static void nl_advect_t(fsibe_ctx* c, int explicit_step) {
     // mask raster launched after it finds room on every SM.  Beyond that the kernel is long
     // beside the raster, and a block a tile keeps more of it in flight (4096²: 281 µs against
     // 513 µs with one block a SM).
-    // a run with the vorticity sponge takes the default tile, the one instantiated with it
-    const auto& V = c->spg ? KX.xv[1] : KX.xv[c->xv_nl];
+    // a run with the vorticity sponge takes the default tile, the one instantiated with it, and so does
+    // the pipelined part, which runs beside the beam: a tile with more blocks an SM is faster by
+    // itself and holds the beam back more (4096²: 258 µs instead of 268, the beam 399 instead of 339,
+    // the step 1272 instead of 1208)
+    const auto& V = (c->spg || c->adv_pipe) ? KX.xv[1] : KX.xv[c->xv_nl];
     const int tiles = c->g.ny / V.rows;
     launch_xv<R>(c, c->spg ? V.nl_adv_spg : V.nl_adv, V.rows, a, "nl_adv", c->side2,
                  tiles <= 2 * c->nsm ? (tiles < c->nsm ? tiles : c->nsm) : tiles);
@@ -1456,6 +1459,7 @@ const char* fsibe_last_error(const fsibe_ctx* ctx) { return ctx ? ctx->err.c_str
 template <typename R>
 static float time_kernel(fsibe_ctx* c, const KLaunch<R>& k, int grid) {
     KArgs<R> a = kargs<R>(c);
+    a.stress_split = c->stress_split ? 1 : 0;  // press_x as the step launches it
     for (int i = 0; i < 2; ++i) k.k<<<grid, k.threads, k.smem, c->stream>>>(a);
     // the best of three rounds of five launches (one round's mean moved by up to 10% between
     // processes at 4096^2 and flipped the choice)

@@ -63,10 +63,26 @@ template <typename R> __device__ __forceinline__ C2<R> cscale(C2<R> a, R s) { re
 // (i * s) * a
 template <typename R> __device__ __forceinline__ C2<R> cimul(C2<R> a, R s) { return mk<R>(-a.y * s, a.x * s); }
 
-// Shared-memory index padding: one slot every 8 complex values keeps the strided
-// Stockham writes free of bank conflicts for both float2 and double2.
-__host__ __device__ __forceinline__ int pad8(int i) { return i + (i >> 3); }
+// The place of element i of a shared-memory row of complex values, free of bank conflicts for the
+// Stockham exchanges.
+//   FP64, 16 bytes (eight lanes a wavefront): one slot of padding every 8 values.
+//   FP32, 8 bytes (sixteen lanes a wavefront): the low four bits XORed with bits of the rest.  Sixteen
+//   neighbours from a multiple of 16 on, i = 8 t + r, and i = 64 a + 8 r + b (b < 8) then fall in
+//   sixteen different bank pairs; with the padding, sixteen neighbours span seventeen slots, and every
+//   linear access took a wavefront more a half warp (4096^2 k_nl_x: 21 of its 49 million shared-memory
+//   wavefronts, the load/store pipe 64% busy).  Measured, padding -> XOR: 4096^2 k_nl_x's advection part
+//   295 -> 268 us, k_nl_y 253 -> 201, k_press_x 465 -> 413; 2048^2 k_nl_x 99 -> 89, k_nl_y 55 -> 47,
+//   k_press_x 131 -> 99; 1024^2 k_nl_y 19.3 -> 17.2, k_press_x 30.9 -> 23.9.
+__host__ __device__ constexpr int pad8(int i) { return i + (i >> 3); }
 __host__ __device__ constexpr int padded_len(int n) { return n + (n >> 3); }
+template <typename R> __host__ __device__ constexpr int pad(int i) {
+    return sizeof(R) == 4 ? i ^ (((i >> 4) & 7) | ((i >> 3) & 8)) : pad8(i);
+}
+template <typename R> __host__ __device__ constexpr int plen(int n) { return sizeof(R) == 4 ? n : padded_len(n); }
+// row stride of a tile of tr rows: tr rows side by side fall in different banks
+template <typename R> __host__ __device__ constexpr int row_stride(int n, int tr) {
+    return sizeof(R) == 4 ? n + (tr >= 16 ? 1 : 16 / tr) : padded_len(n) + 1;
+}
 
 // Scalars shared by all kernels of a step; lives in device memory so that a whole step can
 // run (and be captured in a CUDA graph) without host round trips.

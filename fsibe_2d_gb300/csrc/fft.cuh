@@ -5,7 +5,7 @@
 // A length-N complex sequence is transformed by a group of G = N/8 threads that hold it in
 // registers.  Each stage is a radix-8 Stockham pass (radix 4 or 2 for the last stage when log2 N
 // is not a multiple of 3); between stages the outputs go to their autosorted positions in a
-// shared-memory row (padded with pad8).  Twiddles come from a table W_N^m = exp(-2 pi i m/N)
+// shared-memory row (placed by pad).  Twiddles come from a table W_N^m = exp(-2 pi i m/N)
 // computed on the host in long double and rounded once to the storage type.
 //
 // Forward = exp(-i..), inverse = exp(+i..), both unnormalised (like FFTW).
@@ -69,6 +69,16 @@ __device__ __forceinline__ void dftp(C2<R>* v) {
 // registers needs shared memory only between stages: stages - 1 exchanges instead of a load and
 // a store per stage plus the staging in and out.
 
+// What a transform's threads synchronise with: the block, or one group of it (FxGroup).
+struct BlockSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+template <int G>
+struct GroupSync {
+    const FxGroup& g;
+    __device__ __forceinline__ void operator()() const { fx_sync<G>(g); }
+};
+
 // The butterflies of one stage on v[b][q P + r] (input r of butterfly q, j = t + q G), b < NB
 // of the NBA rows of v.
 template <typename R, int N, int P, int NS, bool INV, int NB, int NBA>
@@ -92,9 +102,9 @@ __device__ __forceinline__ void fft_reg_compute(C2<R> (&v)[NBA][8], const C2<R>*
     }
 }
 
-template <typename R, int N, bool INV, int NB, int NS, int NBA>
+template <typename R, int N, bool INV, int NB, int NS, int NBA, typename Sync = BlockSync>
 __device__ __forceinline__ void fft_reg_run(C2<R> (&v)[NBA][8], C2<R>* buf, int bstride, const C2<R>* __restrict__ tw,
-                                            int t) {
+                                            int t, const Sync& sync = Sync()) {
     constexpr int G = N / 8;
     constexpr int P = (NS * 8 <= N) ? 8 : ((NS * 4 == N) ? 4 : 2), PER = 8 / P;
     fft_reg_compute<R, N, P, NS, INV, NB, NBA>(v, tw, t);
@@ -108,9 +118,9 @@ __device__ __forceinline__ void fft_reg_run(C2<R> (&v)[NBA][8], C2<R>* buf, int 
 #pragma unroll
             for (int b = 0; b < NB; ++b)
 #pragma unroll
-                for (int r = 0; r < P; ++r) buf[b * bstride + pad8(base + r * NS)] = v[b][q * P + r];
+                for (int r = 0; r < P; ++r) buf[b * bstride + pad<R>(base + r * NS)] = v[b][q * P + r];
         }
-        __syncthreads();
+        sync();
         constexpr int NS2 = NS * P;
         constexpr int P2 = (NS2 * 8 <= N) ? 8 : ((NS2 * 4 == N) ? 4 : 2), PER2 = 8 / P2, B2 = N / P2;
 #pragma unroll
@@ -118,9 +128,9 @@ __device__ __forceinline__ void fft_reg_run(C2<R> (&v)[NBA][8], C2<R>* buf, int 
 #pragma unroll
             for (int q = 0; q < PER2; ++q)
 #pragma unroll
-                for (int r = 0; r < P2; ++r) v[b][q * P2 + r] = buf[b * bstride + pad8(t + q * G + r * B2)];
-        __syncthreads();  // every thread has its inputs before the buffer is written again
-        fft_reg_run<R, N, INV, NB, NS2, NBA>(v, buf, bstride, tw, t);
+                for (int r = 0; r < P2; ++r) v[b][q * P2 + r] = buf[b * bstride + pad<R>(t + q * G + r * B2)];
+        sync();  // every thread has its inputs before the buffer is written again
+        fft_reg_run<R, N, INV, NB, NS2, NBA>(v, buf, bstride, tw, t, sync);
     } else if constexpr (PER > 1) {
         // the last stage's butterfly q, output r is element t + (q + PER r) G: element order
 #pragma unroll
@@ -288,7 +298,7 @@ __device__ __forceinline__ void r2c_split_m(C2<R>* buf, int bstride, const C2<R>
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             C2<R>* bb = buf + b * bstride;
-            const C2<R> zk = bb[pad8(k)], zm = bb[pad8(H - k)];
+            const C2<R> zk = bb[pad<R>(k)], zm = bb[pad<R>(H - k)];
             C2<R> e = mk<R>((R)0.5 * (zk.x + zm.x), (R)0.5 * (zk.y - zm.y));
             C2<R> d = mk<R>(zk.x - zm.x, zk.y + zm.y);
             C2<R> o = mk<R>((R)0.5 * d.y, (R)-0.5 * d.x);
@@ -297,18 +307,18 @@ __device__ __forceinline__ void r2c_split_m(C2<R>* buf, int bstride, const C2<R>
             C2<R> d2 = mk<R>(zm.x - zk.x, zm.y + zk.y);
             C2<R> o2 = mk<R>((R)0.5 * d2.y, (R)-0.5 * d2.x);
             C2<R> Xm = cadd<R>(e2, cmul<R>(wm, o2));
-            bb[pad8(k)] = Xk;
-            bb[pad8(H - k)] = Xm;
+            bb[pad<R>(k)] = Xk;
+            bb[pad<R>(H - k)] = Xm;
         }
     }
     if (t == 0) {
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             C2<R>* bb = buf + b * bstride;
-            C2<R> z0 = bb[pad8(0)];
-            bb[pad8(0)] = mk<R>(z0.x + z0.y, (R)0);
-            C2<R> zh = bb[pad8(H / 2)];
-            bb[pad8(H / 2)] = mk<R>(zh.x, -zh.y);
+            C2<R> z0 = bb[pad<R>(0)];
+            bb[pad<R>(0)] = mk<R>(z0.x + z0.y, (R)0);
+            C2<R> zh = bb[pad<R>(H / 2)];
+            bb[pad<R>(H / 2)] = mk<R>(zh.x, -zh.y);
         }
     }
     __syncthreads();
@@ -322,28 +332,99 @@ __device__ __forceinline__ void c2r_merge_m(C2<R>* buf, int bstride, const C2<R>
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             C2<R>* bb = buf + b * bstride;
-            const C2<R> xk = bb[pad8(k)], xm = bb[pad8(H - k)];
+            const C2<R> xk = bb[pad<R>(k)], xm = bb[pad<R>(H - k)];
             C2<R> e = mk<R>(xk.x + xm.x, xk.y - xm.y);
             C2<R> o = cmul<R>(mk<R>(xk.x - xm.x, xk.y + xm.y), mk<R>(wk.x, -wk.y));
             C2<R> Zk = mk<R>(e.x - o.y, e.y + o.x);
             C2<R> e2 = mk<R>(xm.x + xk.x, xm.y - xk.y);
             C2<R> o2 = cmul<R>(mk<R>(xm.x - xk.x, xm.y + xk.y), mk<R>(wm.x, -wm.y));
             C2<R> Zm = mk<R>(e2.x - o2.y, e2.y + o2.x);
-            bb[pad8(k)] = Zk;
-            bb[pad8(H - k)] = Zm;
+            bb[pad<R>(k)] = Zk;
+            bb[pad<R>(H - k)] = Zm;
         }
     }
     if (t == 0) {
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             C2<R>* bb = buf + b * bstride;
-            C2<R> x0 = bb[pad8(0)];
-            bb[pad8(0)] = mk<R>(x0.x, x0.x);
-            C2<R> xh = bb[pad8(H / 2)];
-            bb[pad8(H / 2)] = mk<R>((R)2 * xh.x, (R)-2 * xh.y);
+            C2<R> x0 = bb[pad<R>(0)];
+            bb[pad<R>(0)] = mk<R>(x0.x, x0.x);
+            C2<R> xh = bb[pad<R>(H / 2)];
+            bb[pad<R>(H / 2)] = mk<R>((R)2 * xh.x, (R)-2 * xh.y);
         }
     }
     __syncthreads();
+}
+
+// ---- FP32 rows by one group of threads (fx_c2r's and fx_r2c's contracts) ------------------------
+// The arithmetic is that of c2r_merge_m, r2c_split_m and fft_reg_run.  DX: the row holds X and the
+// transform is of i kx X (kx's wavenumber kx kxs as k_nl_y forms it).
+template <int H, bool DX = false>
+__device__ __forceinline__ void f32_c2r(float2* rb, const float2* __restrict__ twR, const float2* __restrict__ twX,
+                                        const FxGroup& gr, float2 (&v)[8], float kxs = 0.f) {
+    constexpr int G = H / 8;
+    const int t = gr.t;
+    const GroupSync<G> sync{gr};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = 1 + t + i * G;
+        if (i == 3 && k == H / 2) {  // the last thread's last pair: the elements 0 and H/2
+            float2 x0 = rb[pad<float>(0)], xh = rb[pad<float>(H / 2)];
+            if (DX) { x0 = cimul<float>(x0, 0.f * kxs); xh = cimul<float>(xh, (float)(H / 2) * kxs); }
+            rb[pad<float>(0)] = mk<float>(x0.x, x0.x);
+            rb[pad<float>(H / 2)] = mk<float>(2.f * xh.x, -2.f * xh.y);
+            continue;
+        }
+        float2 xk = rb[pad<float>(k)], xm = rb[pad<float>(H - k)];
+        if (DX) { xk = cimul<float>(xk, (float)k * kxs); xm = cimul<float>(xm, (float)(H - k) * kxs); }
+        const float2 wk = __ldg(&twR[k]), wm = __ldg(&twR[H - k]);
+        const float2 e = mk<float>(xk.x + xm.x, xk.y - xm.y);
+        const float2 o = cmul<float>(mk<float>(xk.x - xm.x, xk.y + xm.y), mk<float>(wk.x, -wk.y));
+        const float2 e2 = mk<float>(xm.x + xk.x, xm.y - xk.y);
+        const float2 o2 = cmul<float>(mk<float>(xm.x - xk.x, xm.y + xk.y), mk<float>(wm.x, -wm.y));
+        rb[pad<float>(k)] = mk<float>(e.x - o.y, e.y + o.x);
+        rb[pad<float>(H - k)] = mk<float>(e2.x - o2.y, e2.y + o2.x);
+    }
+    sync();
+    float2 z[1][8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) z[0][q] = rb[pad<float>(t + q * G)];
+    sync();
+    fft_reg_run<float, H, true, 1, 1>(z, rb, 0, twX, t, sync);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = z[0][q];
+}
+template <int H>
+__device__ __forceinline__ void f32_r2c(const float2 (&v)[8], float2* rb, const float2* __restrict__ twR,
+                                        const float2* __restrict__ twX, const FxGroup& gr) {
+    constexpr int G = H / 8;
+    const int t = gr.t;
+    const GroupSync<G> sync{gr};
+    float2 z[1][8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) z[0][q] = v[q];
+    fft_reg_run<float, H, false, 1, 1>(z, rb, 0, twX, t, sync);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) rb[pad<float>(t + q * G)] = z[0][q];
+    sync();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = 1 + t + i * G;
+        if (i == 3 && k == H / 2) {
+            const float2 z0 = rb[pad<float>(0)], zh = rb[pad<float>(H / 2)];
+            rb[pad<float>(0)] = mk<float>(z0.x + z0.y, 0.f);
+            rb[pad<float>(H / 2)] = mk<float>(zh.x, -zh.y);
+            continue;
+        }
+        const float2 zk = rb[pad<float>(k)], zm = rb[pad<float>(H - k)];
+        const float2 wk = __ldg(&twR[k]), wm = __ldg(&twR[H - k]);
+        const float2 e = mk<float>(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+        const float2 d = mk<float>(zk.x - zm.x, zk.y + zm.y);
+        const float2 e2 = mk<float>(0.5f * (zm.x + zk.x), 0.5f * (zm.y - zk.y));
+        const float2 d2 = mk<float>(zm.x - zk.x, zm.y + zk.y);
+        rb[pad<float>(k)] = cadd<float>(e, cmul<float>(wk, mk<float>(0.5f * d.y, -0.5f * d.x)));
+        rb[pad<float>(H - k)] = cadd<float>(e2, cmul<float>(wm, mk<float>(0.5f * d2.y, -0.5f * d2.x)));
+    }
 }
 
 // ---- the x direction's split steps on paired rows (FP32) -----------------------------------

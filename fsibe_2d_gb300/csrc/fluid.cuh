@@ -175,7 +175,7 @@ struct XRows {
     static constexpr int TRD = (G * TR0 >= 32) ? TR0 : 32 / G;
     // TRV > 0: an explicit tile height (the autotuner's candidates)
     static constexpr int TR = TRV > 0 ? TRV : TRD;
-    static constexpr int PL = padded_len(H) + 1;  // row stride (complex) in shared memory
+    static constexpr int PL = row_stride<R>(H, TR);  // row stride (complex) in shared memory
     static constexpr int THREADS = G * TR;
     // blocks per SM that keep a thread at <= 128 registers
     static constexpr int MINB128 = (65536 / (THREADS * 128)) > 0 ? 65536 / (THREADS * 128) : 1;
@@ -197,8 +197,8 @@ template <typename R, int H, int TR, int PL>
 __device__ __forceinline__ void load_tileT(C2<R>* buf, const C2<R>* __restrict__ T, int ny, int iy0, int kmax = H) {
     for (int i = threadIdx.x; i < H * TR; i += blockDim.x) {
         const int r = i % TR, kx = i / TR;
-        if (kx < kmax) cp_async_el<R>(&buf[r * PL + pad8(kx)], &T[(size_t)kx * ny + iy0 + r]);
-        else buf[r * PL + pad8(kx)] = mk<R>(0, 0);
+        if (kx < kmax) cp_async_el<R>(&buf[r * PL + pad<R>(kx)], &T[(size_t)kx * ny + iy0 + r]);
+        else buf[r * PL + pad<R>(kx)] = mk<R>(0, 0);
     }
 }
 
@@ -209,7 +209,7 @@ __device__ __forceinline__ void load_tileT_dx(C2<R>* buf, const C2<R>* __restric
                                               double kxs0) {
     for (int i = threadIdx.x; i < H * TR; i += blockDim.x) {
         const int r = i % TR, kx = i / TR;
-        buf[r * PL + pad8(kx)] = (kx < kmax) ? cimul<R>(T[(size_t)kx * ny + iy0 + r], (R)kx * (R)kxs0) : mk<R>(0, 0);
+        buf[r * PL + pad<R>(kx)] = (kx < kmax) ? cimul<R>(T[(size_t)kx * ny + iy0 + r], (R)kx * (R)kxs0) : mk<R>(0, 0);
     }
 }
 
@@ -224,7 +224,7 @@ __device__ __forceinline__ void row_c2r_fp(C2<R>* rb, int bstride, const C2<R>* 
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[b][q] = rb[b * bstride + pad8(t + q * G)];
+        for (int q = 0; q < 8; ++q) v[b][q] = rb[b * bstride + pad<R>(t + q * G)];
     __syncthreads();
     fft_reg_run<R, H, true, NB, 1>(v, rb, bstride, twX, t);
 }
@@ -238,7 +238,7 @@ __device__ __forceinline__ void row_r2c_fp(C2<R> (&v)[NBA][8], C2<R>* rb, int bs
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) rb[b * bstride + pad8(t + q * G)] = v[b][q];
+        for (int q = 0; q < 8; ++q) rb[b * bstride + pad<R>(t + q * G)] = v[b][q];
     __syncthreads();
     r2c_split_m<R, H, NB>(rb, bstride, twR, t);
 }
@@ -267,15 +267,22 @@ __device__ __forceinline__ void row_r2c_reg(C2<R> (&v)[NBA][8], C2<R>* rb, int b
 // pressure within 3.7e-16 of the CPU's, 4.0e-16 with the FP64 stages), but at 4096^2 the pressure
 // jump at the beam's free end is what is left of two values 2 10^7 times as large, one or two units
 // of their last place, and the comparison on record at that size holds that last place.
-template <typename R, int H> constexpr bool step_fp() { return kIsF32<R> || H == 2048; }
+template <typename R, int H> constexpr bool step_fp() { return !kIsF32<R> && H == 2048; }
+// The step's x kernels with a group of threads a transform (fluid_fx.cuh): the FP64 form up to 2048,
+// where the integer chains want the warps; the FP32 form up to 512, where one block's latency is the
+// time (512^2: k_press_x 17.8 -> 14.4 us).  From 1024 on the FP32 rows' extra trips through shared
+// memory cost more than the warps gain (both with padded rows: 1024^2 k_press_x 30.9 us with the
+// transforms in one thread's registers against 32.0 with groups, 4096^2 465 against 558, k_nl_x's
+// advection part 295 against 455): there a thread keeps two or three transforms in registers.
+template <typename R, int H> constexpr bool step_groups() { return kIsF32<R> ? H <= 256 : !step_fp<R, H>(); }
 template <typename R, int H, int NB, int NBA>
 __device__ __forceinline__ void step_c2r(const KArgs<R>& a, C2<R>* rb, int bstride, int t, C2<R> (&v)[NBA][8]) {
-    if constexpr (sizeof(R) == 8 && step_fp<R, H>()) row_c2r_fp<R, H, NB>(rb, bstride, a.twR64, a.twX64, t, v);
+    if constexpr (step_fp<R, H>()) row_c2r_fp<R, H, NB>(rb, bstride, a.twR64, a.twX64, t, v);
     else row_c2r_reg<R, H, NB>(rb, bstride, a.twR, a.twX, t, v);
 }
 template <typename R, int H, int NB, int NBA>
 __device__ __forceinline__ void step_r2c(const KArgs<R>& a, C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, int t) {
-    if constexpr (sizeof(R) == 8 && step_fp<R, H>()) row_r2c_fp<R, H, NB>(v, rb, bstride, a.twR64, a.twX64, t);
+    if constexpr (step_fp<R, H>()) row_r2c_fp<R, H, NB>(v, rb, bstride, a.twR64, a.twX64, t);
     else row_r2c_reg<R, H, NB>(v, rb, bstride, a.twR, a.twX, t);
 }
 
@@ -313,7 +320,7 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xfwd(KArgs<R> a) {
     C2<R>* T = a.spec0 + boff;
     for (int i = threadIdx.x; i < H * X::TR; i += blockDim.x) {
         const int rr = i % X::TR, kx = i / X::TR;
-        T[(size_t)kx * ny + iy0 + rr] = buf[rr * X::PL + pad8(kx)];
+        T[(size_t)kx * ny + iy0 + rr] = buf[rr * X::PL + pad<R>(kx)];
     }
 }
 
@@ -585,19 +592,19 @@ __device__ __forceinline__ void nl_x_tile(const KArgs<R>& a, const int iy0) {
                 const int rr = i % X::TR, kx = i / X::TR;
                 const size_t o = (size_t)kx * ny + iy0 + rr;
                 const R kxs = kx_wave<R>(a, kx);
-                a.A[o] = cadd<R>(av[u], cimul<R>(bufA[rr * X::PL + pad8(kx)], kxs));
-                a.B[o] = bufB[rr * X::PL + pad8(kx)];
+                a.A[o] = cadd<R>(av[u], cimul<R>(bufA[rr * X::PL + pad<R>(kx)], kxs));
+                a.B[o] = bufB[rr * X::PL + pad<R>(kx)];
             }
         }
     } else {
         for (int i = threadIdx.x; i < nout; i += blockDim.x) {
             const int rr = i % X::TR, kx = i / X::TR;
             const size_t o = (size_t)kx * ny + iy0 + rr;
-            const C2<R> xa = bufA[rr * X::PL + pad8(kx)];
+            const C2<R> xa = bufA[rr * X::PL + pad<R>(kx)];
             if constexpr (PART == NL_WHOLE) {
                 const R kxs = kx_wave<R>(a, kx);
-                a.A[o] = cadd<R>(xa, cimul<R>(bufB[rr * X::PL + pad8(kx)], kxs));
-                a.B[o] = bufC[rr * X::PL + pad8(kx)];
+                a.A[o] = cadd<R>(xa, cimul<R>(bufB[rr * X::PL + pad<R>(kx)], kxs));
+                a.B[o] = bufC[rr * X::PL + pad<R>(kx)];
             } else {
                 a.A[o] = xa;
                 a.B[o] = mk<R>(0, 0);
@@ -670,7 +677,7 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float>
     constexpr int G = NY / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C2<R>* bufA = reinterpret_cast<C2<R>*>(smem_raw);
-    C2<R>* bufB = bufA + padded_len(NY);
+    C2<R>* bufB = bufA + plen<R>(NY);
     const int kx = blockIdx.x, t = threadIdx.x;
     const Geometry& g = a.g;
     const size_t row = (size_t)kx * NY;
@@ -687,9 +694,9 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float>
     }
     // the row's state (W, Wlo, M) flows into the spare buffers C, D, E while the
     // forward transforms run (unpadded rows of NY complex values)
-    C2<R>* preW = bufA + 2 * padded_len(NY);
-    C2<R>* preWl = bufA + 3 * padded_len(NY);
-    C2<R>* preM = bufA + 4 * padded_len(NY);
+    C2<R>* preW = bufA + 2 * plen<R>(NY);
+    C2<R>* preWl = bufA + 3 * plen<R>(NY);
+    C2<R>* preM = bufA + 4 * plen<R>(NY);
     for (int e = t; e < NY / 2; e += G) {  // 16 bytes = two complex values per copy
         cp_async16_f(preW + 2 * e, a.W + row + 2 * e);
         cp_async16_f(preWl + 2 * e, a.Wlo + row + 2 * e);
@@ -702,7 +709,7 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float>
         fab[0][q] = a.A[row + t + q * G];
         fab[1][q] = a.B[row + t + q * G];
     }
-    block_fft_reg_m<R, NY, false, 2>(fab, bufA, padded_len(NY), a.twY, t);  // A and B together
+    block_fft_reg_m<R, NY, false, 2>(fab, bufA, plen<R>(NY), a.twY, t);  // A and B together
     cp_async_wait_f();
     __syncthreads();
     const DevScalars* S = a.S;
@@ -758,7 +765,7 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float>
     // i kx Tw and i kx Tu as they load Tw and Tu (load_tileT_dx).  The FP64 form transforms all seven
     // in the reference's order (cofdx, then cofitxy), which keeps its roundings those of the
     // operators its adjoint transposes.
-    constexpr int PLY = padded_len(NY);
+    constexpr int PLY = plen<R>(NY);
     const R kxs = (R)kx * (R)g.kxs;
     // the spectra in registers (this thread's ky = t + q G), transformed with the shared-memory
     // rows as exchange buffers, stored from registers
@@ -1014,8 +1021,8 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
             const int rr = i % X::TR, kx = i / X::TR;
             const R kxs = kx_wave<R>(a, kx);
             const size_t o = (size_t)kx * ny + iy0 + rr;
-            a.P1[o] = cimul<R>(bufA[rr * X::PL + pad8(kx)], kxs);
-            a.P2[o] = bufB[rr * X::PL + pad8(kx)];
+            a.P1[o] = cimul<R>(bufA[rr * X::PL + pad<R>(kx)], kxs);
+            a.P2[o] = bufB[rr * X::PL + pad<R>(kx)];
         }
     }
     if (a.viscous && !a.stress_split) {
@@ -1308,7 +1315,7 @@ __global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 :
     constexpr int G = NY / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C2<R>* bufA = reinterpret_cast<C2<R>*>(smem_raw);
-    C2<R>* bufB = bufA + padded_len(NY);
+    C2<R>* bufB = bufA + plen<R>(NY);
     const int kx = blockIdx.x, t = threadIdx.x;
     const Geometry& g = a.g;
     const size_t row = (size_t)kx * NY;
@@ -1319,7 +1326,7 @@ __global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 :
         fp[0][q] = a.P1[row + t + q * G];
         fp[1][q] = a.P2[row + t + q * G];
     }
-    block_fft_reg_m<R, NY, false, 2>(fp, bufA, padded_len(NY), a.twY, t);  // P1 and P2 together
+    block_fft_reg_m<R, NY, false, 2>(fp, bufA, plen<R>(NY), a.twY, t);  // P1 and P2 together
     const R norm = (R)g.inv_nxny;
     C2<R> qv[1][8];
 #pragma unroll
@@ -1334,7 +1341,7 @@ __global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 :
         qv[0][q] = qh;
     }
     // inverse-y of q from registers to registers (the forward transform left bufA free)
-    block_fft_reg_m<R, NY, true, 1>(qv, bufA, padded_len(NY), a.twY, t);
+    block_fft_reg_m<R, NY, true, 1>(qv, bufA, plen<R>(NY), a.twY, t);
 #pragma unroll
     for (int q = 0; q < 8; ++q) a.Tq[row + t + q * G] = qv[0][q];
 }
@@ -1423,6 +1430,26 @@ struct SizeKernels {
     KLaunch<R> press_y1;  // FP32: k_press_y on the one-butterfly engine (NY/8 threads), or none
 };
 
+// the kernels with a group of threads a transform (fluid_fx.cuh), TR rows a block
+template <typename R, int H, int TR, bool SPG>
+inline void fill_xgroups(typename SizeKernels<R>::XVariant& v) {
+    constexpr int RG = xgroups_rg<H>(TR);
+    using X2 = XGroups<R, H, TR, RG, 2>;
+    using X3 = XGroups<R, H, TR, RG, 3>;
+    v.rows = TR;
+    v.nl_x = klaunch<R>(k_nl_x_g<R, H, TR, NL_WHOLE, 0>, X3::THREADS, X3::SMEM);
+    v.nl_adv = klaunch<R>(k_nl_x_g<R, H, TR, NL_ADVECT, 0>, X2::THREADS, X2::SMEM);
+    v.nl_pen = klaunch<R>(k_nl_x_g<R, H, TR, NL_PENAL, 0>, X2::THREADS, X2::SMEM);
+    if constexpr (SPG) {
+        v.nl_x_spg = klaunch<R>(k_nl_x_g<R, H, TR, NL_WHOLE, 1>, X3::THREADS, X3::SMEM);
+        v.nl_adv_spg = klaunch<R>(k_nl_x_g<R, H, TR, NL_ADVECT, 1>, X3::THREADS, X3::SMEM);
+        v.nl_x_s10 = klaunch<R>(k_nl_x_g<R, H, TR, NL_WHOLE, 2>, X3::THREADS, X3::SMEM);
+        v.nl_pen_s10 = klaunch<R>(k_nl_x_g<R, H, TR, NL_PENAL, 2>, X2::THREADS, X2::SMEM);
+    }
+    v.stress_x = klaunch<R>(k_stress_x_g<R, H, TR>, X2::THREADS, X2::SMEM);
+    v.press_x = klaunch<R>(k_press_x_g<R, H, TR>, X3::THREADS, press_x_smem_g<R, H, TR>());
+}
+
 template <typename R, int H, int TR, int MB = 0, bool SPG = false>
 inline void fill_xvariant(typename SizeKernels<R>::XVariant& v) {
     using X = XRows<R, H, TR>;
@@ -1430,7 +1457,7 @@ inline void fill_xvariant(typename SizeKernels<R>::XVariant& v) {
     v.rows = TR;
     v.minb = MB;
     v.press_fin = klaunch<R>(k_press_fin<R, H, TR, MB>, T, S1);
-    if constexpr (step_fp<R, H>()) {
+    if constexpr (!step_groups<R, H>()) {
         v.nl_x = klaunch<R>(k_nl_x<R, H, TR, NL_WHOLE, MB>, T, 3 * S1);
         v.nl_adv = klaunch<R>(k_nl_x<R, H, TR, NL_ADVECT, MB>, T, 2 * S1);
         v.nl_pen = klaunch<R>(k_nl_x<R, H, TR, NL_PENAL, MB>, T, 2 * S1);
@@ -1443,20 +1470,7 @@ inline void fill_xvariant(typename SizeKernels<R>::XVariant& v) {
         v.stress_x = klaunch<R>(k_stress_x<R, H, TR, MB>, T, 2 * S1);
         v.press_x = klaunch<R>(k_press_x<R, H, TR, MB>, T, 3 * S1);
     } else {
-        // the FP64 form's kernels with a group of threads a transform (fluid_fx.cuh)
-        using X2 = XGroups<H, TR, 2>;
-        using X3 = XGroups<H, TR, 3>;
-        v.nl_x = klaunch<R>(k_nl_x_d<H, TR, NL_WHOLE, 0>, X3::THREADS, X3::SMEM);
-        v.nl_adv = klaunch<R>(k_nl_x_d<H, TR, NL_ADVECT, 0>, X2::THREADS, X2::SMEM);
-        v.nl_pen = klaunch<R>(k_nl_x_d<H, TR, NL_PENAL, 0>, X2::THREADS, X2::SMEM);
-        if constexpr (SPG) {
-            v.nl_x_spg = klaunch<R>(k_nl_x_d<H, TR, NL_WHOLE, 1>, X3::THREADS, X3::SMEM);
-            v.nl_adv_spg = klaunch<R>(k_nl_x_d<H, TR, NL_ADVECT, 1>, X3::THREADS, X3::SMEM);
-            v.nl_x_s10 = klaunch<R>(k_nl_x_d<H, TR, NL_WHOLE, 2>, X3::THREADS, X3::SMEM);
-            v.nl_pen_s10 = klaunch<R>(k_nl_x_d<H, TR, NL_PENAL, 2>, X2::THREADS, X2::SMEM);
-        }
-        v.stress_x = klaunch<R>(k_stress_x_d<H, TR>, X2::THREADS, X2::SMEM);
-        v.press_x = klaunch<R>(k_press_x_d<H, TR>, X3::THREADS, press_x_smem_d<H, TR>());
+        fill_xgroups<R, H, TR, SPG>(v);
     }
 }
 
@@ -1464,14 +1478,14 @@ template <typename R, int N>
 inline void fill_size_kernels(SizeKernels<R>& k) {
     constexpr int H = N / 2;
     using X = XRows<R, H>;
-    constexpr int S1 = (int)(X::TR * X::PL * sizeof(C2<R>)), SY = (int)(padded_len(N) * sizeof(C2<R>)), TY = N / 8;
+    constexpr int S1 = (int)(X::TR * X::PL * sizeof(C2<R>)), SY = (int)(plen<R>(N) * sizeof(C2<R>)), TY = N / 8;
     k.x_rows = X::TR;
     k.xfwd = klaunch<R>(k_xfwd<R, H>, X::THREADS, S1);
     k.xinv = klaunch<R>(k_xinv<R, H>, X::THREADS, S1);
     k.vel_x = klaunch<R>(k_vel_x<R, H>, X::THREADS, 2 * S1);
     constexpr int T1 = X::TRD;
     k.xp = typename SizeKernels<R>::XVariant{};
-    if constexpr (step_fp<R, H>()) {
+    if constexpr (!step_groups<R, H>()) {
         constexpr int T0 = xrows_valid<R, H>(T1 / 2), T2 = xrows_valid<R, H>(T1 * 2);
         fill_xvariant<R, H, T0>(k.xv[0]);
         fill_xvariant<R, H, T1, 0, true>(k.xv[1]);
@@ -1480,7 +1494,7 @@ inline void fill_size_kernels(SizeKernels<R>& k) {
         constexpr int MB2 = (2 * XRows<R, H, T1>::THREADS <= 2048) ? 2 : 1;
         fill_xvariant<R, H, T1, MB2>(k.xv[3]);
     } else {
-        constexpr int T0 = xgroups_valid<H>(T1 / 2, T1), T2 = xgroups_valid<H>(T1 * 2, T1);
+        constexpr int T0 = xgroups_valid<R, H>(T1 / 2, T1), T2 = xgroups_valid<R, H>(T1 * 2, T1);
         fill_xvariant<R, H, T0>(k.xv[0]);
         fill_xvariant<R, H, T1, 0, true>(k.xv[1]);
         fill_xvariant<R, H, T2>(k.xv[2]);

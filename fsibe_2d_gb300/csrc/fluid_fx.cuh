@@ -1,4 +1,5 @@
-// fluid_fx.cuh -- the FP64 form's fused kernels (the map onto the reference is fluid.cuh's).
+// fluid_fx.cuh -- fused kernels with a group of threads a transform (the map onto the reference is
+// fluid.cuh's): the FP64 form's y and x passes, and the FP32 form's x pass.
 //
 // Each transform of a block belongs to its own group of threads (fft_fx.cuh), with a row of shared
 // memory for its exchanges; the pointwise work between transforms goes over all threads of the
@@ -148,67 +149,88 @@ __global__ void __launch_bounds__(NG * NY / 8) k_press_y_d(KArgs<double> a) {
     for (int m = 0; m < 8; ++m) a.Tq[row + gr.t + m * G] = v[m];
 }
 
-// ---- x pass ----------------------------------------------------------------------------------
-// A block of TR rows and NF fields: group f TR + r transforms row r of field f.
-template <int H, int TR, int NF>
+// ---- x pass (both forms) -----------------------------------------------------------------------
+// A block of TR rows and NF fields, RG rows of every field at a time: group f RG + q transforms the
+// rows q, q + RG, ... of field f.
+template <typename R, int H, int TR, int RG, int NF>
 struct XGroups {
-    static constexpr int G = H / 8, PL = padded_len(H) + 1, BS = TR * PL, THREADS = NF * TR * G;
-    static constexpr int SMEM = NF * BS * 16;
+    static constexpr int G = H / 8, PL = row_stride<R>(H, TR), BS = TR * PL, THREADS = NF * RG * G;
+    static constexpr int SMEM = NF * BS * (int)sizeof(C2<R>);
+    static_assert(TR % RG == 0, "whole rounds of rows");
 };
 // fields of k_nl_x's parts: the derivatives (and, with the vorticity sponge, the vorticity), and
 // what is transformed forward
 template <int PART, int SPG> constexpr int nl_x_fields() { return (PART == NL_WHOLE || SPG == 1) ? 3 : 2; }
-// A tile height for the FP64 kernels: tr when its block of three fields has a full warp and at most
-// 1024 threads (with G > 32, then, at most 15 groups: the named barriers), else the default.
-template <int H>
+// Rows at a time for a tile of tr: as many as give three fields at most 768 threads (with G > 32,
+// then, at most 15 groups: the named barriers).
+template <int H> constexpr int xgroups_rg(int tr) {
+    int rg = tr;
+    while (rg > 1 && 3 * (H / 8) * rg > 768) rg /= 2;
+    return rg;
+}
+// A tile height of the group kernels: tr when its block has whole warps and three fields' rows fit
+// shared memory, else the default.
+template <typename R, int H>
 constexpr int xgroups_valid(int tr, int def) {
-    return (tr >= 1 && (H / 8) * tr >= 32 && 3 * (H / 8) * tr <= 1024 && 3 * tr * (padded_len(H) + 1) * 16 <= 128 * 1024) ? tr : def;
+    return (tr >= 1 && (H / 8) * xgroups_rg<H>(tr) >= 32 &&
+            3 * tr * row_stride<R>(H, tr) * (int)sizeof(C2<R>) <= 128 * 1024) ? tr : def;
 }
 
-template <int H, int TR, int NF>
+template <typename R, int H, int TR, int RG, int NF>
 struct XBlock {
-    using X = XGroups<H, TR, NF>;
-    double2* rows;
+    using X = XGroups<R, H, TR, RG, NF>;
+    C2<R>* rows;
     FxGroup gr;
-    int f, r;      // the group's field and row
+    int f, r0;      // the group's field and first row
     __device__ __forceinline__ XBlock(unsigned char* smem, unsigned* slots) {
         const int gi = threadIdx.x / X::G;
-        rows = reinterpret_cast<double2*>(smem);
+        rows = reinterpret_cast<C2<R>*>(smem);
         gr = FxGroup{(int)threadIdx.x % X::G, gi + 1, slots + gi * fx_slots<X::G>()};
-        f = gi / TR;
-        r = gi % TR;
+        f = gi / RG;
+        r0 = gi % RG;
     }
-    __device__ __forceinline__ double2* own() const { return rows + f * X::BS + r * X::PL; }
-    // the group's half spectrum to a real row of pairs, in place
-    __device__ __forceinline__ void to_real(const KArgs<double>& a) const {
-        double2 v[8];
-        fx_c2r<H>(own(), a.twR, a.twX, gr, v);
-#pragma unroll
-        for (int m = 0; m < 8; ++m) own()[pad8(gr.t + m * X::G)] = v[m];
+    __device__ __forceinline__ C2<R>* row(int r) const { return rows + f * X::BS + r * X::PL; }
+    // a half spectrum of the group's to its real row of pairs in registers (DX: FP32, of i kx times it)
+    template <bool DX = false>
+    __device__ __forceinline__ void c2r(const KArgs<R>& a, int r, C2<R> (&v)[8]) const {
+        if constexpr (kIsF32<R>) f32_c2r<H, DX>(row(r), a.twR, a.twX, gr, v, (float)a.g.kxs);
+        else fx_c2r<H>(row(r), a.twR, a.twX, gr, v);
     }
-    __device__ __forceinline__ void to_half(const KArgs<double>& a) const {
-        double2 v[8];
+    template <bool DX = false>
+    __device__ __forceinline__ void to_real(const KArgs<R>& a) const {  // in place, every row
+        C2<R> v[8];
+        for (int r = r0; r < TR; r += RG) {
+            c2r<DX>(a, r, v);
 #pragma unroll
-        for (int m = 0; m < 8; ++m) v[m] = own()[pad8(gr.t + m * X::G)];
-        fx_sync<X::G>(gr);
-        fx_r2c<H>(v, own(), a.twR, a.twX, gr);
+            for (int m = 0; m < 8; ++m) row(r)[pad<R>(gr.t + m * X::G)] = v[m];
+        }
+    }
+    __device__ __forceinline__ void to_half(const KArgs<R>& a) const {
+        C2<R> v[8];
+        for (int r = r0; r < TR; r += RG) {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[m] = row(r)[pad<R>(gr.t + m * X::G)];
+            fx_sync<X::G>(gr);
+            if constexpr (kIsF32<R>) f32_r2c<H>(v, row(r), a.twR, a.twX, gr);
+            else fx_r2c<H>(v, row(r), a.twR, a.twX, gr);
+        }
     }
 };
 
 // cal_nlk's physical-space part (nl_x_tile)
-template <int H, int TR, int PART, int SPG>
-__device__ __forceinline__ void nl_x_tile_d(const KArgs<double>& a, const int iy0, unsigned* slots) {
+template <typename R, int H, int TR, int RG, int PART, int SPG>
+__device__ __forceinline__ void nl_x_tile_g(const KArgs<R>& a, const int iy0, unsigned* slots) {
     constexpr int NF = nl_x_fields<PART, SPG>();
-    using X = XGroups<H, TR, NF>;
+    using X = XGroups<R, H, TR, RG, NF>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int ny = a.g.ny;
     if (PART == NL_PENAL && (iy0 + TR - 1 < a.rect[2] || iy0 > a.rect[3])) return;
-    const XBlock<H, TR, NF> B(smem_raw, slots);
-    double2 *bufA = B.rows, *bufB = bufA + X::BS, *bufC = bufB + X::BS;
+    const XBlock<R, H, TR, RG, NF> B(smem_raw, slots);
+    C2<R> *bufA = B.rows, *bufB = bufA + X::BS, *bufC = bufB + X::BS;
     // the penalization part adds to the advection part's A, loaded first
-    constexpr int NLA = H * TR / X::THREADS;
+    constexpr int NLA = (H * TR + X::THREADS - 1) / X::THREADS;
     const int nout = a.kcut * TR;
-    double2 av[NLA];
+    C2<R> av[NLA];
     if (PART == NL_PENAL) {
 #pragma unroll
         for (int u = 0; u < NLA; ++u) {
@@ -217,44 +239,50 @@ __device__ __forceinline__ void nl_x_tile_d(const KArgs<double>& a, const int iy
         }
     } else {
         const int kin = a.explicit_step ? H : a.kcut;
-        load_tileT<double, H, TR, X::PL>(bufA, a.Tdx, ny, iy0, kin);
-        load_tileT<double, H, TR, X::PL>(bufB, a.Tdy, ny, iy0, kin);
-        if (SPG == 1) load_tileT<double, H, TR, X::PL>(bufC, a.Tw, ny, iy0, kin);
+        load_tileT<R, H, TR, X::PL>(bufA, kIsF32<R> ? a.Tw : a.Tdx, ny, iy0, kin);
+        load_tileT<R, H, TR, X::PL>(bufB, a.Tdy, ny, iy0, kin);
+        if (SPG == 1) load_tileT<R, H, TR, X::PL>(bufC, a.Tw, ny, iy0, kin);
         cp_async_wait_f();
         __syncthreads();
-        if (B.f < (SPG == 1 ? 3 : 2)) B.to_real(a);
+        if (kIsF32<R> && B.f == 0) B.template to_real<kIsF32<R>>(a);
+        else if (B.f < (SPG == 1 ? 3 : 2)) B.to_real(a);
         __syncthreads();
     }
     const size_t roff = (size_t)iy0 * H;
-    const double2 *u2 = reinterpret_cast<const double2*>(a.u) + roff, *v2 = reinterpret_cast<const double2*>(a.v) + roff;
-    const double2 *k2 = reinterpret_cast<const double2*>(a.mask) + roff;
-    const double2 *x2 = reinterpret_cast<const double2*>(a.mvx) + roff, *y2 = reinterpret_cast<const double2*>(a.mvy) + roff;
+    const C2<R> *u2 = reinterpret_cast<const C2<R>*>(a.u) + roff, *v2 = reinterpret_cast<const C2<R>*>(a.v) + roff;
+    const C2<R> *k2 = reinterpret_cast<const C2<R>*>(a.mask) + roff;
+    const C2<R> *x2 = reinterpret_cast<const C2<R>*>(a.mvx) + roff, *y2 = reinterpret_cast<const C2<R>*>(a.mvy) + roff;
     const bool pen = PART != NL_ADVECT && a.penalize;
+    const R Uc = kIsF32<R> ? (R)a.S->mean_u_cur : (R)0, Vc = kIsF32<R> ? (R)a.S->mean_v_cur : (R)0;
     for (int i = threadIdx.x; i < TR * H; i += X::THREADS) {
-        const int o = (i / H) * X::PL + pad8(i % H);
-        const double2 uu = u2[i], vv = v2[i];
-        double2 px = make_double2(0.0, 0.0), py = px;
+        const int o = (i / H) * X::PL + pad<R>(i % H);
+        C2<R> uu = u2[i], vv = v2[i];
+        if (kIsF32<R>) {  // the stored velocity is the perturbation
+            uu = mk<R>(uu.x + Uc, uu.y + Uc);
+            vv = mk<R>(vv.x + Vc, vv.y + Vc);
+        }
+        C2<R> px = mk<R>(0, 0), py = px;
         if (pen) {
-            const double2 kk = k2[i];
+            const C2<R> kk = k2[i];
             if (!(is_zero(kk.x) && is_zero(kk.y))) {
-                const double2 mx = x2[i], my = y2[i];
-                px = make_double2(-kk.x * (uu.x - mx.x), -kk.y * (uu.y - mx.y));
-                py = make_double2(-kk.x * (vv.x - my.x), -kk.y * (vv.y - my.y));
+                const C2<R> mx = x2[i], my = y2[i];
+                px = mk<R>(-kk.x * (uu.x - mx.x), -kk.y * (uu.y - mx.y));
+                py = mk<R>(-kk.x * (vv.x - my.x), -kk.y * (vv.y - my.y));
             }
             if (SPG == 2) {
-                const double2 si = reinterpret_cast<const double2*>(a.s10)[roff + i];
-                px = make_double2(px.x + si.x, px.y + si.y);
+                const C2<R> si = reinterpret_cast<const C2<R>*>(a.s10)[roff + i];
+                px = mk<R>(px.x + si.x, px.y + si.y);
             }
         }
         if (PART == NL_PENAL) {
             bufA[o] = py;
             bufB[o] = px;
         } else {
-            const double2 dx = bufA[o], dy = bufB[o];
-            double2 w = make_double2(-uu.x * dx.x - vv.x * dy.x, -uu.y * dx.y - vv.y * dy.y);
+            const C2<R> dx = bufA[o], dy = bufB[o];
+            C2<R> w = mk<R>(-uu.x * dx.x - vv.x * dy.x, -uu.y * dx.y - vv.y * dy.y);
             if (SPG == 1) {
-                const double2 sg = reinterpret_cast<const double2*>(a.spg)[roff + i], om = bufC[o];
-                w = make_double2(w.x - sg.x * om.x, w.y - sg.y * om.y);
+                const C2<R> sg = reinterpret_cast<const C2<R>*>(a.spg)[roff + i], om = bufC[o];
+                w = mk<R>(w.x - sg.x * om.x, w.y - sg.y * om.y);
             }
             bufA[o] = w;
             if (PART == NL_WHOLE) { bufB[o] = py; bufC[o] = px; }
@@ -263,209 +291,258 @@ __device__ __forceinline__ void nl_x_tile_d(const KArgs<double>& a, const int iy
     __syncthreads();
     if (B.f < (PART == NL_WHOLE ? 3 : (PART == NL_PENAL ? 2 : 1))) B.to_half(a);
     __syncthreads();
-    // A = X(w) + i kx X(pen_y), B = X(pen_x) on the modes the update keeps (see nl_x_tile)
+    // the right-hand side only matters where the update keeps modes (kx < kcut): A = X(w) +
+    // i kx X(pen_y), B = X(pen_x); the advection part writes X(w) and a zero B, the penalization part
+    // adds its terms to that
     if constexpr (PART == NL_PENAL) {
 #pragma unroll
         for (int u = 0; u < NLA; ++u) {
             const int i = threadIdx.x + u * X::THREADS;
             if (i >= nout) break;
-            const int s = (i % TR) * X::PL + pad8(i / TR);
+            const int s = (i % TR) * X::PL + pad<R>(i / TR);
             const size_t o = (size_t)(i / TR) * ny + iy0 + i % TR;
-            a.A[o] = cadd<double>(av[u], cimul<double>(bufA[s], __ldg(&a.kxd[i / TR])));
+            a.A[o] = cadd<R>(av[u], cimul<R>(bufA[s], kx_wave<R>(a, i / TR)));
             a.B[o] = bufB[s];
         }
     } else {
         for (int i = threadIdx.x; i < nout; i += X::THREADS) {
-            const int s = (i % TR) * X::PL + pad8(i / TR);
+            const int s = (i % TR) * X::PL + pad<R>(i / TR);
             const size_t o = (size_t)(i / TR) * ny + iy0 + i % TR;
             if (PART == NL_WHOLE) {
-                a.A[o] = cadd<double>(bufA[s], cimul<double>(bufB[s], __ldg(&a.kxd[i / TR])));
+                a.A[o] = cadd<R>(bufA[s], cimul<R>(bufB[s], kx_wave<R>(a, i / TR)));
                 a.B[o] = bufC[s];
             } else {
                 a.A[o] = bufA[s];
-                a.B[o] = make_double2(0.0, 0.0);
+                a.B[o] = mk<R>(0, 0);
             }
         }
     }
 }
 
-template <int H, int TR, int PART, int SPG>
-__global__ void __launch_bounds__(XGroups<H, TR, nl_x_fields<PART, SPG>()>::THREADS) k_nl_x_d(KArgs<double> a) {
+template <typename R, int H, int TR, int PART, int SPG>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), nl_x_fields<PART, SPG>()>::THREADS) k_nl_x_g(KArgs<R> a) {
     pdl_wait();     // the previous kernel of the stream has completed
-    constexpr int NF = nl_x_fields<PART, SPG>();
-    __shared__ unsigned slots[NF * TR * fx_slots<H / 8>()];
+    constexpr int NF = nl_x_fields<PART, SPG>(), RG = xgroups_rg<H>(TR);
+    __shared__ unsigned slots[NF * RG * fx_slots<H / 8>()];
     if constexpr (PART == NL_ADVECT) {
-        for (int tile = blockIdx.x; tile < a.g.ny / TR; tile += gridDim.x) {  // (see k_nl_x)
-            nl_x_tile_d<H, TR, PART, SPG>(a, tile * TR, slots);
+        // the advection part runs beside the mask kernels on fewer blocks than tiles (the
+        // launch gives one a SM), each taking tiles in turn, so that the raster launched after
+        // it still finds room on every SM
+        for (int tile = blockIdx.x; tile < a.g.ny / TR; tile += gridDim.x) {
+            nl_x_tile_g<R, H, TR, RG, PART, SPG>(a, tile * TR, slots);
             __syncthreads();  // the next tile reuses the rows
         }
     } else {
-        nl_x_tile_d<H, TR, PART, SPG>(a, blockIdx.x * TR, slots);
+        nl_x_tile_g<R, H, TR, RG, PART, SPG>(a, blockIdx.x * TR, slots);
     }
 }
 
-// the viscous stresses (k_stress_x)
-template <int H, int TR>
-__device__ __forceinline__ void stress_tile_d(const KArgs<double>& a, const int iy0, unsigned* slots) {
-    using X = XGroups<H, TR, 2>;
+// The viscous stresses (NavierStokes.f90:354-370: 2 nu d2psi/dxdy, nu (d2psi/dy2 - d2psi/dx2))
+// to physical space, beside k_press_x on another stream: only GetForces reads them.  With
+// a.srows set, a block whose rows no stencil of the forces reaches (rows j - 4 .. j + 4 of the
+// stress points' cells j, BeamForces.f90:105-124, which lie within the stress points' offset
+// of the beam's y range; k_step_begin forms the range into S->srow) leaves them.
+template <typename R, int H, int TR, int RG>
+__device__ __forceinline__ void stress_tile_g(const KArgs<R>& a, const int iy0, unsigned* slots) {
+    using X = XGroups<R, H, TR, RG, 2>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const XBlock<H, TR, 2> B(smem_raw, slots);
-    load_tileT<double, H, TR, X::PL>(B.rows, a.Tsa, a.g.ny, iy0, a.kcut);
-    load_tileT<double, H, TR, X::PL>(B.rows + X::BS, a.Tsb, a.g.ny, iy0, a.kcut);
+    const XBlock<R, H, TR, RG, 2> B(smem_raw, slots);
+    load_tileT<R, H, TR, X::PL>(B.rows, kIsF32<R> ? a.Tu : a.Tsa, a.g.ny, iy0, a.kcut);  // FP32: du/dx = i kx Tu
+    load_tileT<R, H, TR, X::PL>(B.rows + X::BS, a.Tsb, a.g.ny, iy0, a.kcut);
     cp_async_wait_f();
     __syncthreads();
     if (B.f > 1) return;
-    double2 v[8];
-    fx_c2r<H>(B.own(), a.twR, a.twX, B.gr, v);
-    double2* out = reinterpret_cast<double2*>(B.f == 0 ? a.sa : a.sb) + (size_t)(iy0 + B.r) * H;
-    const double c = B.f == 0 ? 2.0 * a.nu : a.nu;
+    const R c = B.f == 0 ? (R)(2.0 * a.nu) : (R)a.nu;
+    C2<R> v[8];
+    for (int r = B.r0; r < TR; r += RG) {
+        if (kIsF32<R> && B.f == 0) B.template c2r<kIsF32<R>>(a, r, v);
+        else B.c2r(a, r, v);
+        C2<R>* out = reinterpret_cast<C2<R>*>(B.f == 0 ? a.sa : a.sb) + (size_t)(iy0 + r) * H;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) out[B.gr.t + m * X::G] = make_double2(c * v[m].x, c * v[m].y);
+        for (int m = 0; m < 8; ++m) out[B.gr.t + m * X::G] = mk<R>(c * v[m].x, c * v[m].y);
+    }
 }
-template <int H, int TR>
-__global__ void __launch_bounds__(XGroups<H, TR, 2>::THREADS) k_stress_x_d(KArgs<double> a) {
-    __shared__ unsigned slots[2 * TR * fx_slots<H / 8>()];
+template <typename R, int H, int TR>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), 2>::THREADS) k_stress_x_g(KArgs<R> a) {
+    constexpr int RG = xgroups_rg<H>(TR);
+    __shared__ unsigned slots[2 * RG * fx_slots<H / 8>()];
     const int iy0 = blockIdx.x * TR;
     if (a.srows) {
         const int j0 = a.S->srow[0], j1 = a.S->srow[1];
         if (iy0 + TR - 1 < j0 || iy0 > j1) return;
     }
-    stress_tile_d<H, TR>(a, iy0, slots);
+    stress_tile_g<R, H, TR, RG>(a, iy0, slots);
 }
 
-// shared memory of k_press_x_d: the rows of three fields and the reduction's columns
-template <int H, int TR> constexpr int press_x_smem_d() { return XGroups<H, TR, 3>::SMEM + RED_NSLOTS * XGroups<H, TR, 3>::THREADS * 8; }
+// k_press_x_g's sums: the columns every cell adds to, and those of the penalization (INFLOW_MEAN as
+// the sums of chi (u - u_s) and chi (v - v_s) in the FP32 form)
+constexpr int PXC_ALL = 5, PXC_PEN = 8;
+enum { PX_OMEGA2 = 0, PX_KIN, PX_SUM_U, PX_SUM_V, PX_UMAX2, PX_POROUS, PX_INFLOW, PX_PENX, PX_PENY, PX_DRAGX, PX_DRAGY, PX_UNSTX, PX_UNSTY };
+// shared memory: the rows of three fields, and the threads' columns (one thread's are never
+// reduced before another's are written: they have their own place)
+template <typename R, int H, int TR> constexpr int press_x_smem_g() {
+    using X = XGroups<R, H, TR, xgroups_rg<H>(TR), 3>;
+    return X::SMEM + (PXC_ALL + PXC_PEN) * X::THREADS * (int)sizeof(R);
+}
 
 // k_press_x: u, v and omega, the penalization, the sums, vor_mean, the pressure's right-hand side
-template <int H, int TR>
-__global__ void __launch_bounds__(XGroups<H, TR, 3>::THREADS) k_press_x_d(KArgs<double> a) {
+template <typename R, int H, int TR>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), 3>::THREADS) k_press_x_g(KArgs<R> a) {
     pdl_wait();     // the previous kernel of the stream has completed
-    using X = XGroups<H, TR, 3>;
-    constexpr int T = X::THREADS, NW = TR * X::G / 32;
+    constexpr int RG = xgroups_rg<H>(TR);
+    using X = XGroups<R, H, TR, RG, 3>;
+    constexpr int T = X::THREADS, NW = RG * X::G / 32;
+    constexpr bool F32 = kIsF32<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ unsigned slots[3 * TR * fx_slots<X::G>()];
-    __shared__ double vm_w[2];
-    const XBlock<H, TR, 3> B(smem_raw, slots);
-    double2 *bufU = B.rows, *bufV = bufU + X::BS, *bufW = bufV + X::BS;
-    double* cols = reinterpret_cast<double*>(smem_raw + X::SMEM);
+    __shared__ unsigned slots[3 * RG * fx_slots<X::G>()];
+    __shared__ R vm_w[2];
+    __shared__ double red_s[PXC_ALL + PXC_PEN];
+    const XBlock<R, H, TR, RG, 3> B(smem_raw, slots);
+    C2<R> *bufU = B.rows, *bufV = bufU + X::BS, *bufW = bufV + X::BS;
+    R* cols = reinterpret_cast<R*>(smem_raw + X::SMEM);
     const int iy0 = blockIdx.x * TR, ny = a.g.ny;
     const DevScalars* S = a.S;
     if (threadIdx.x == 0) {  // time_avg_vort's weights
         const double time = S->time, dt1 = S->dt1;
-        vm_w[0] = time / (time + dt1);
-        vm_w[1] = dt1 / (time + dt1);
+        vm_w[0] = (R)(time / (time + dt1));
+        vm_w[1] = (R)(dt1 / (time + dt1));
     }
-    load_tileT<double, H, TR, X::PL>(bufU, a.Tu, ny, iy0, a.kcut);
-    load_tileT<double, H, TR, X::PL>(bufV, a.Tv, ny, iy0, a.kcut);
-    load_tileT<double, H, TR, X::PL>(bufW, a.Tw, ny, iy0, a.kcut);
+    load_tileT<R, H, TR, X::PL>(bufU, a.Tu, ny, iy0, a.kcut);
+    load_tileT<R, H, TR, X::PL>(bufV, a.Tv, ny, iy0, a.kcut);
+    load_tileT<R, H, TR, X::PL>(bufW, a.Tw, ny, iy0, a.kcut);
     cp_async_wait_f();
     __syncthreads();
     B.to_real(a);
     __syncthreads();
     const size_t roff = (size_t)iy0 * H;
-    double2 *u2 = reinterpret_cast<double2*>(a.u) + roff, *v2 = reinterpret_cast<double2*>(a.v) + roff;
-    double2* vm2 = reinterpret_cast<double2*>(a.vor_mean) + roff;
-    const double2 *k2 = reinterpret_cast<const double2*>(a.mask) + roff;
-    const double2 *x2 = reinterpret_cast<const double2*>(a.mvx) + roff, *y2 = reinterpret_cast<const double2*>(a.mvy) + roff;
-    const double U = S->mean_u_next, V = S->mean_v_next, ca = vm_w[0], cb = vm_w[1];
+    C2<R> *u2 = reinterpret_cast<C2<R>*>(a.u) + roff, *v2 = reinterpret_cast<C2<R>*>(a.v) + roff;
+    C2<R>* vm2 = reinterpret_cast<C2<R>*>(a.vor_mean) + roff;
+    const C2<R> *k2 = reinterpret_cast<const C2<R>*>(a.mask) + roff;
+    const C2<R> *x2 = reinterpret_cast<const C2<R>*>(a.mvx) + roff, *y2 = reinterpret_cast<const C2<R>*>(a.mvy) + roff;
+    const double Ud = S->mean_u_next, Vd = S->mean_v_next;
+    const R U = (R)Ud, V = (R)Vd, ca = vm_w[0], cb = vm_w[1];
     const int ixmin = S->win[0], ixmax = S->win[1], iymin = S->win[2], iymax = S->win[3];
-    double acc[RED_NSLOTS];
+    R acc[PXC_ALL + PXC_PEN];
 #pragma unroll
-    for (int s = 0; s < RED_NSLOTS; ++s) acc[s] = 0.0;
-    long long um = 0;  // bits of the largest |u|^2; NaN is passed over, as fmax does
+    for (int s = 0; s < PXC_ALL + PXC_PEN; ++s) acc[s] = (R)0;
+    long long um = 0;  // FP64: bits of the largest |u|^2; NaN is passed over, as fmax does
     bool masked = false;
-    // thirteen FP64 instructions a cell outside the mask, where the penalization and its sums add
-    // nothing and are left out (a comparison or a conversion would take the FP64 pipe as long as an
-    // addition: the mask's test and the maximum are on the bits)
+    // Outside the mask the penalization and its sums add nothing and are left out.  In FP64 that leaves
+    // thirteen FP64 instructions a cell (a comparison or a conversion would take the FP64 pipe as long
+    // as an addition: the mask's test and the maximum are on the bits).
     for (int i = threadIdx.x; i < TR * H; i += T) {
-        const int rr = i / H, m = i % H, o = rr * X::PL + pad8(m), iy = iy0 + rr;
-        const double2 kk = k2[i], vmo = vm2[i];
-        const double2 ur = bufU[o], vr = bufV[o], w = bufW[o];
-        const double2 uu = make_double2(ur.x + U, ur.y + U), vv = make_double2(-vr.x + V, -vr.y + V);
-        u2[i] = uu;
-        v2[i] = vv;
-        const double uc[2] = {uu.x, uu.y}, vc[2] = {vv.x, vv.y}, wc[2] = {w.x, w.y};
-        const double upc[2] = {ur.x, ur.y}, vpc[2] = {vr.x, vr.y};
-        double px[2] = {0.0, 0.0}, py[2] = {0.0, 0.0};
+        const int rr = i / H, m = i % H, o = rr * X::PL + pad<R>(m), iy = iy0 + rr;
+        const C2<R> kk = k2[i], vmo = vm2[i];
+        const C2<R> ur = bufU[o], vr = bufV[o], w = bufW[o];
+        const C2<R> uu = mk<R>(ur.x + U, ur.y + U), vv = mk<R>(-vr.x + V, -vr.y + V);
+        // the FP32 form stores the perturbation (the mean flow stays in FP64 scalars)
+        u2[i] = F32 ? ur : uu;
+        v2[i] = F32 ? mk<R>(-vr.x, -vr.y) : vv;
+        const R uc[2] = {uu.x, uu.y}, vc[2] = {vv.x, vv.y}, wc[2] = {w.x, w.y};
+        const R upc[2] = {ur.x, ur.y}, vpc[2] = {vr.x, vr.y};
+        R px[2] = {0, 0}, py[2] = {0, 0};
         if (!(is_zero(kk.x) && is_zero(kk.y))) {
             masked = true;
-            const double2 mx = x2[i], my = y2[i];
-            const double kc[2] = {kk.x, kk.y}, xc[2] = {mx.x, mx.y}, yc[2] = {my.x, my.y};
+            const C2<R> mx = x2[i], my = y2[i];
+            const R kc[2] = {kk.x, kk.y}, xc[2] = {mx.x, mx.y}, yc[2] = {my.x, my.y};
             const bool in_rows = (iy >= iymin && iy <= iymax);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int ix = 2 * m + e;
-                const double rx = uc[e] - xc[e], ry = vc[e] - yc[e];
-                const double penx = kc[e] * rx, peny = kc[e] * ry;
-                acc[RED_POROUS] += kc[e] * (rx * rx + ry * ry);
-                acc[RED_INFLOW_SOLID] += kc[e] * (xc[e] * rx + yc[e] * ry);
-                acc[RED_INFLOW_MEAN] += U * penx + V * peny;
+                const R rx = uc[e] - xc[e], ry = vc[e] - yc[e];
+                const R penx = kc[e] * rx, peny = kc[e] * ry;
+                acc[PX_POROUS] += kc[e] * (rx * rx + ry * ry);
+                acc[PX_INFLOW] += kc[e] * (xc[e] * rx + yc[e] * ry);
+                acc[PX_PENX] += penx;
+                acc[PX_PENY] += peny;
                 if (in_rows && ix >= ixmin && ix <= ixmax) {
-                    acc[RED_DRAG_X] += penx;
-                    acc[RED_DRAG_Y] += peny;
-                    acc[RED_UNST_X] += xc[e] * kc[e];
-                    acc[RED_UNST_Y] += yc[e] * kc[e];
+                    acc[PX_DRAGX] += penx;
+                    acc[PX_DRAGY] += peny;
+                    acc[PX_UNSTX] += xc[e] * kc[e];
+                    acc[PX_UNSTY] += yc[e] * kc[e];
                 }
                 px[e] = penx;
                 py[e] = peny;
             }
         }
-        const double vmc[2] = {vmo.x, vmo.y};
-        double vmn[2];
+        const R vmc[2] = {vmo.x, vmo.y};
+        R vmn[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            acc[RED_OMEGA2] += wc[e] * wc[e];
-            acc[RED_KIN] += upc[e] * upc[e] + vpc[e] * vpc[e];
-            acc[RED_SUM_U] += uc[e];
-            acc[RED_SUM_V] += vc[e];
-            const long long ub = __double_as_longlong(uc[e] * uc[e] + vc[e] * vc[e]);
-            if (ub > um && ub <= 0x7ff0000000000000LL) um = ub;
+            acc[PX_OMEGA2] += wc[e] * wc[e];
+            acc[PX_KIN] += upc[e] * upc[e] + vpc[e] * vpc[e];
+            acc[PX_SUM_U] += uc[e];
+            acc[PX_SUM_V] += vc[e];
+            const R q2 = uc[e] * uc[e] + vc[e] * vc[e];
+            if constexpr (F32) {
+                acc[PX_UMAX2] = fmaxf(acc[PX_UMAX2], q2);
+            } else {
+                const long long ub = __double_as_longlong(q2);
+                if (ub > um && ub <= 0x7ff0000000000000LL) um = ub;
+            }
             vmn[e] = vmc[e] * ca + wc[e] * cb;
             px[e] = px[e] - wc[e] * vc[e];
             py[e] = py[e] + wc[e] * uc[e];
         }
-        vm2[i] = make_double2(vmn[0], vmn[1]);
-        bufU[o] = make_double2(px[0], px[1]);
-        bufV[o] = make_double2(py[0], py[1]);
+        vm2[i] = mk<R>(vmn[0], vmn[1]);
+        bufU[o] = mk<R>(px[0], px[1]);
+        bufV[o] = mk<R>(py[0], py[1]);
     }
-    acc[RED_UMAX2] = __longlong_as_double(um);
-#pragma unroll
-    for (int s = 0; s < RED_NSLOTS; ++s) cols[s * T + threadIdx.x] = acc[s];
+    if constexpr (!F32) acc[PX_UMAX2] = __longlong_as_double(um);
     // a block without mask has zeros in the penalization's columns: they are not summed
     const bool any = __syncthreads_or(masked) != 0;
+    const int ncol = any ? PXC_ALL + PXC_PEN : PXC_ALL;
+#pragma unroll
+    for (int s = 0; s < PXC_ALL + PXC_PEN; ++s)
+        if (s < ncol) cols[s * T + threadIdx.x] = acc[s];
+    __syncthreads();
     if (B.f < 2) {
         if (a.pressure_on) B.to_half(a);  // the right-hand side's x and y parts
     } else {
         // the block's sums in a fixed order, one warp of the third field's groups a column
-        const int w = (threadIdx.x - 2 * TR * X::G) >> 5, l = threadIdx.x & 31;
-        for (int s = w; s < RED_NSLOTS; s += NW) {
+        const int w = (threadIdx.x - 2 * RG * X::G) >> 5, l = threadIdx.x & 31;
+        for (int s = w; s < PXC_ALL + PXC_PEN; s += NW) {
             double v = 0.0;
-            if (s == RED_UMAX2) {
-                long long b = 0;
-                for (int i = l; i < T; i += 32) b = max(b, __double_as_longlong(cols[s * T + i]));
+            if (s < ncol) {
+                if constexpr (F32) {
+                    v = col_reduce_ff(cols + s * T, T, s == PX_UMAX2);
+                } else if (s == PX_UMAX2) {
+                    long long b = 0;
+                    for (int i = l; i < T; i += 32) b = max(b, __double_as_longlong(cols[s * T + i]));
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-                v = __longlong_as_double(b);
-            } else if (any || s == RED_OMEGA2 || s == RED_KIN || s == RED_SUM_U || s == RED_SUM_V) {
-                for (int i = l; i < T; i += 32) v += cols[s * T + i];
-                v = warp_sum<double>(v);
+                    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+                    v = __longlong_as_double(b);
+                } else {
+                    for (int i = l; i < T; i += 32) v += cols[s * T + i];
+                    v = warp_sum<double>(v);
+                }
             }
-            if (l == 0) a.red[(size_t)blockIdx.x * RED_NSLOTS + s] = v;
+            if (l == 0) red_s[s] = v;
         }
-        if (blockIdx.x == 0 && w == 0 && l == 0) a.S->nred = (int)gridDim.x;
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        double* out = a.red + (size_t)blockIdx.x * RED_NSLOTS;
+        out[RED_OMEGA2] = red_s[PX_OMEGA2]; out[RED_KIN] = red_s[PX_KIN];
+        out[RED_POROUS] = red_s[PX_POROUS]; out[RED_INFLOW_SOLID] = red_s[PX_INFLOW];
+        out[RED_INFLOW_MEAN] = any ? Ud * red_s[PX_PENX] + Vd * red_s[PX_PENY] : 0.0;
+        out[RED_SUM_U] = red_s[PX_SUM_U]; out[RED_SUM_V] = red_s[PX_SUM_V];
+        out[RED_DRAG_X] = red_s[PX_DRAGX]; out[RED_DRAG_Y] = red_s[PX_DRAGY];
+        out[RED_UNST_X] = red_s[PX_UNSTX]; out[RED_UNST_Y] = red_s[PX_UNSTY];
+        out[RED_UMAX2] = red_s[PX_UMAX2];
+        if (blockIdx.x == 0) a.S->nred = (int)gridDim.x;
+    }
     if (a.pressure_on) {
         for (int i = threadIdx.x; i < H * TR; i += T) {
-            const int kx = i / TR, s = (i % TR) * X::PL + pad8(kx);
+            const int kx = i / TR, s = (i % TR) * X::PL + pad<R>(kx);
             const size_t o = (size_t)kx * ny + iy0 + i % TR;
-            a.P1[o] = cimul<double>(bufU[s], __ldg(&a.kxd[kx]));
+            a.P1[o] = cimul<R>(bufU[s], kx_wave<R>(a, kx));
             a.P2[o] = bufV[s];
         }
     }
     if (a.viscous && !a.stress_split) {
         __syncthreads();
-        stress_tile_d<H, TR>(a, iy0, slots);
+        stress_tile_g<R, H, TR, RG>(a, iy0, slots);
     }
 }
 
