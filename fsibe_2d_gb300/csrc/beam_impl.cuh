@@ -109,7 +109,7 @@ __host__ __device__ inline size_t beam_lu_floats(int ns) { return (size_t)(2 * n
 // the rest of the factor: row exponents and the chunk-boundary responses E, F
 __host__ __device__ inline size_t beam_fact_floats(int ns) {
     const int n = 2 * ns + 4, C = beam_chunks(n);
-    return r4((size_t)(n + 16) + (size_t)C * (64 + 224));
+    return r4(n + 16) + (size_t)C * (64 + 224);
 }
 __host__ __device__ inline size_t beam_scr_floats(int ns) {
     const int n = 2 * ns + 4, C = beam_chunks(n);
@@ -180,7 +180,7 @@ __device__ BeamWS carve(const BeamParts& P, int ns) {
     w.Uf = P.lu;
     w.Lf = P.lu + (size_t)(n + 16) * 16;
     float* f = P.fact;
-    w.rse = reinterpret_cast<int*>(f); f += n + 16;
+    w.rse = reinterpret_cast<int*>(f); f += r4(n + 16);  // E is read in 16-byte pieces (n + 16 = 2 mod 4 for odd ns)
     w.Ec = f; f += (size_t)C * 64;
     w.Fc = f;
     f = P.scr;
