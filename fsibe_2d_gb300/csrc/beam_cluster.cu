@@ -7,7 +7,7 @@
 // residuals over R SMs divides that work by R; the cluster's hardware barrier and distributed
 // shared memory (DSMEM) keep every exchange between the SMs on chip.
 //
-// Layout: CTA r owns the interleaved rows [r n / R, (r+1) n / R) of the Newton system
+// Layout: CTA r owns a run of the interleaved rows (cl_rows) of the Newton system
 // (n = 2 ns + 4): their F values, their FP64 Jacobian band rows, and the same rows of M^-1,
 // the inverse of the row-scaled FP32 LU factor that preconditions the FP64 iterative
 // refinement.  Every CTA keeps a full copy of the iterate x and of the refinement solution.
@@ -21,6 +21,11 @@
 // memory under the single-CTA kernel's reuse rule (kept while <= 5 passes per Newton step).
 // The iterate update, the norms and the stopping test run redundantly in every CTA on
 // identical data, so they need no exchange.
+// What bounds it: chains of dependent FP64 (an addition is some 70 cycles) and the barriers, two a
+// pass.  A warp evaluates one of the two node equations (they alternate by row, and a warp of both ran
+// the two codes one after the other), and the passes end when their corrections no longer change the
+// iterate (newton_pass).  Measured (us, before -> after both, and rows of the band on different banks):
+// ns = 64 55 -> 46, 128 (heaving) 74 -> 59, 256 84 -> 62, 1024 333 -> 250.
 // Large beams (ns >= 512: M^-1's rows and the factor exceed a CTA's shared memory) run the
 // same algorithm with both in global memory, where they stay L2-resident: each CTA reads its
 // rows of M^-1 from its slice of the persistent copy, and factors its own copy of the band
@@ -71,12 +76,47 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Row stride of M^-1: >= n, 16-byte rows, = 4 (mod 32) words.
 __host__ __device__ inline int cl_mld(int n) { return ((n + 27) / 32) * 32 + 4; }
 __host__ __device__ inline size_t al16(size_t v) { return (v + 15) & ~(size_t)15; }
+// doubles a band row: one more than its 16 entries, so that the rows of a warp's lanes fall in different
+// banks (at 16 every access of a Jacobian warp was a 32-way conflict)
+constexpr int CL_BAND = 17;
 constexpr int CL_NODE = 9;  // per-node FP64 arrays: tdn, bo3, bo4, bo5, bo6, oo5, oo6, old_rhs, taun_s
 
 struct ClLayout {
     int n, L, R, rmax, mld;
     size_t x, xdi, node, bvec, band, part, slots, yf, fact, minv, total;  // byte offsets
 };
+
+// The rows [lo, hi) of CTA r: quads of rows, so that every CTA's slice of the FP32 right-hand side (and
+// of the FP64 solution) starts on a 16-byte boundary.  With R >= 8 and n <= 640 the first and the last
+// CTA hold the four boundary equations alone (and one node, when ns is odd) and the others share the
+// rest evenly: a warp of generic rows takes its time whether one row or 32, and the boundary
+// equations' beside it on the same SMSPs made those two CTAs the slowest (F and J of an iteration
+// 4.6k cycles with them, 3.1k without).  Above, where rows and M^-1's size count, all share evenly.
+__host__ __device__ inline bool cl_ends_alone(int n, int R) {
+    const int nq = (n + 3) / 4, last = nq - (n - 4) / 4;
+    return R >= 8 && n <= 640 && nq - 1 - last >= R - 2;
+}
+__host__ __device__ inline void cl_rows(int n, int R, int r, int& lo, int& hi) {
+    const int nq = (n + 3) / 4;
+    if (cl_ends_alone(n, R)) {
+        const int mid = (n - 4) / 4 - 1;  // quads of the CTAs between
+        lo = (r == 0) ? 0 : 1 + (r - 1) * mid / (R - 2);
+        hi = (r == R - 1) ? nq : 1 + r * mid / (R - 2);
+        lo *= 4;
+        hi *= 4;
+    } else {
+        lo = 4 * (int)(((long long)r * nq) / R);
+        hi = 4 * (int)(((long long)(r + 1) * nq) / R);
+    }
+    lo = lo < n ? lo : n;
+    hi = hi < n ? hi : n;
+}
+__host__ __device__ inline int cl_rmax(int n, int R) {
+    const int nq = (n + 3) / 4;
+    if (!cl_ends_alone(n, R)) return 4 * ((nq + R - 1) / R);
+    const int mid = ((n - 4) / 4 - 1 + R - 3) / (R - 2), last = nq - (n - 4) / 4;
+    return 4 * (mid > last ? mid : last);
+}
 
 // Floats of one CTA's global copy of the factor area in the large-beam form (the factor, or
 // after the Newton loop the position sums, as in shared memory), a multiple of 4.
@@ -91,16 +131,16 @@ __host__ __device__ inline void cl_layout(int ns, int R, ClLayout& Y, bool big =
     Y.n = 2 * ns + 4;
     Y.L = ns + 8;
     Y.R = R;
-    Y.rmax = 4 * (((Y.n + 3) / 4 + R - 1) / R);  // rows are dealt in quads (cl_rows)
+    Y.rmax = cl_rmax(Y.n, R);
     Y.mld = cl_mld(Y.n);
     size_t o = 0;
     Y.x = o;     o = al16(o + 8 * (size_t)(Y.n + 8));
     Y.xdi = o;   o = al16(o + 8 * (size_t)(Y.n + 8));
     Y.node = o;  o = al16(o + 8 * (size_t)CL_NODE * Y.L);
     Y.bvec = o;  o = al16(o + 8 * (size_t)Y.rmax);
-    Y.band = o;  o = al16(o + 8 * 16 * (size_t)Y.rmax);
+    Y.band = o;  o = al16(o + 8 * CL_BAND * (size_t)Y.rmax);
     Y.part = o;  o = al16(o + 8 * 4 * (size_t)Y.rmax);
-    Y.slots = o; o = al16(o + 8 * 4 * (size_t)R);
+    Y.slots = o; o = al16(o + 8 * 3 * (size_t)R);
     Y.yf = o;    o = al16(o + 4 * (size_t)(Y.mld + 16));
     if (big) { Y.fact = Y.minv = Y.total = o; return; }
     Y.fact = o;
@@ -110,16 +150,6 @@ __host__ __device__ inline void cl_layout(int ns, int R, ClLayout& Y, bool big =
     o = al16(o + (fact > post ? fact : post));
     Y.minv = o;  o = al16(o + 4 * (size_t)Y.rmax * Y.mld);
     Y.total = o;
-}
-
-// The rows [lo, hi) of CTA r: quads of rows dealt evenly, so that every CTA's slice of the FP32
-// right-hand side (and of the FP64 solution) starts on a 16-byte boundary.
-__host__ __device__ inline void cl_rows(int n, int R, int r, int& lo, int& hi) {
-    const int nq = (n + 3) / 4;
-    lo = 4 * (int)(((long long)r * nq) / R);
-    hi = 4 * (int)(((long long)(r + 1) * nq) / R);
-    lo = lo < n ? lo : n;
-    hi = hi < n ? hi : n;
 }
 
 // Fortran equation (1-based) of interleaved row r: the inverse of row_of.
@@ -185,6 +215,65 @@ __device__ void inv_row(const float* __restrict__ U, const float* __restrict__ L
     for (int k = n; k < mld; ++k) out[k] = 0.f;
 }
 
+// The value of a double whose high word (sign cleared) is h, rounded down to its 20 bits, in FP32 (zero
+// and infinity outside FP32's normal range).
+__device__ __forceinline__ float hi_to_float(unsigned h) {
+    const int e = (int)(h >> 20) - 1023;
+    if (e < -126) return 0.f;
+    if (e > 127) return __int_as_float(0x7f800000);
+    return __uint_as_float((unsigned)(e + 127) << 23 | (h & 0xfffffu) << 3);
+}
+
+// The decision after a pass of the iterative refinement of Newton's linear system: 1 done, 0 another
+// pass, -1 a new factor.  Of [0] the angles and [1] the tensions, cm is the pass's largest correction,
+// cp the previous pass's (at pass 0 the last one of the iteration before), c0 the first pass's, i.e. the
+// size of dx, and xmax the iterate's largest entry.
+//
+// The first two iterations are always followed by another, whose residual sees what they leave:
+//   iter 0  dx to 2^-30, by the size of the last correction, or of the one that would follow it;
+//   iter 1  the correction that would follow small beside the stopping tolerance (by sqrt(n) 16), so
+//           that the stopping test at iter 2 sees what it would after an exact solve;
+//   iter 2 on  either unknown to 2^-30 of its dx or 2^-58 of its iterate, whichever is larger, judged
+//           by the correction that would follow; at pass 0 the contraction is that since the
+//           iteration before.  The norms of the angles and of the tensions are kept apart: the
+//           tensions' rounding is often larger than every angle.  Both are taken to contract as
+//           the slower does.
+// An FP64 solve's error is at 2^-53 of the iterate at best.  2^-30 of every dx, in every iteration, took
+// 7 to 10 passes a step, the last three or four of them on corrections below the iterate's last place;
+// this takes 5 or 6.  The positions' and the loads' errors against the oracle are the same.
+// A first contraction above 2^-6 asks for a new factor in the next iteration (slow).  Corrections that
+// stop shrinking end the passes: with a good first contraction they are at the residual's rounding and
+// dx stands if it is known to 2^-30, else a factor kept from an earlier step is replaced.
+__device__ __forceinline__ int newton_pass(int iter, int pass, const float* cm, const float* cp, const float* c0,
+                                           const float* xmax, float rn, float tol, bool is_new, bool& slow) {
+    const float cn = fmaxf(cm[0], cm[1]), c0n = fmaxf(c0[0], c0[1]), xn = fmaxf(xmax[0], xmax[1]);
+    const bool exact = !(cn > 0x1p-30f * c0n);  // also NaN, which the update flags
+    const float most = is_new ? 0.5f : 0.125f;
+    bool conv, stall = false;
+    const float q0 = cm[0] > 0.f ? cm[0] / cp[0] : 0.f, q1 = cm[1] > 0.f ? cm[1] / cp[1] : 0.f;
+    const float ratio = fmaxf(q0, q1);
+    if (iter < 2) {
+        const float cpn = fmaxf(cp[0], cp[1]);
+        const bool next = (iter == 0) ? cn * (cn / cpn) <= 0x1p-30f * c0n : 16.f * rn * (cn * ratio) <= tol * fmaxf(1.f, xn);
+        conv = exact || (pass >= 1 && next);
+        stall = pass >= 2 && cn > most * cpn;
+        slow |= pass == 1 && !conv && cn > 0x1p-6f * cpn;
+    } else {
+        conv = true;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const float t = fmaxf(fmaxf(0x1p-30f * c0[q], 0x1p-58f * xmax[q]), 0x1p-86f * xn);
+            const bool cv = !(cm[q] > t) || cm[q] * ratio <= t;
+            conv = conv && cv;
+            stall |= pass >= 2 && !cv && cm[q] > most * cp[q];
+            slow |= pass == 1 && !cv && cm[q] > 0x1p-6f * cp[q];
+        }
+    }
+    if (conv) return 1;
+    if (!stall && pass < 9) return 0;
+    return (exact && (is_new || !slow)) ? 1 : -1;
+}
+
 }  // namespace
 
 #define PH(k) do { const long long t_ = clock64(); ph[k] += t_ - ph_t; ph_t = t_; } while (0)
@@ -216,9 +305,9 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
     double* bvec = reinterpret_cast<double*>(cl_smem + Y.bvec);
     double* band = reinterpret_cast<double*>(cl_smem + Y.band);
     double* part = reinterpret_cast<double*>(cl_smem + Y.part);
-    // exchange words, written by every CTA into every CTA: [0, R) the passes' max |c| (FP32
-    // bits), [R, 2R) max |x| (FP64 bits), [2R, 3R) the flags sent with the right-hand side,
-    // [3R, 4R) the flags sent with the factor rows
+    // exchange words, written by every CTA into every CTA: [0, R) the passes' max |c| of the angles
+    // and, in the high word, of the tensions (FP32 bits), [R, 2R) the flags sent with the right-hand
+    // side, [2R, 3R) the flags sent with the factor rows
     unsigned long long* slots = reinterpret_cast<unsigned long long*>(cl_smem + Y.slots);
     float* yf = reinterpret_cast<float*>(cl_smem + Y.yf);
     float* Uf = big ? b.clws + (size_t)rank * fstride : reinterpret_cast<float*>(cl_smem + Y.fact);
@@ -228,9 +317,9 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
     __shared__ D1DTab dtab;
     __shared__ NewtonCtx cs;
     __shared__ double red[2][8];
-    __shared__ unsigned long long redu[2][8];
-    __shared__ int flag_s, stop_s, info_s, dec_s;
-    __shared__ float cprev_s;
+    __shared__ unsigned redu[2][8];
+    __shared__ __align__(16) unsigned xhi[2][8];
+    __shared__ int flag_s, stop_s, info_s;
 
     BeamWS w;
     memset(&w, 0, sizeof(w));
@@ -267,6 +356,32 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
         }
         for (int i = tid; i < n; i += nthr)
             if (i != xi_th(-1) && i != xi_T(ns, -1)) x[i] = b.pred[i];
+        for (int i = tid; i < ns; i += nthr) old_rhs[i] = b.pred[n + i];
+        // the Newton constants (divisions done by the predictor)
+        if (tid == 32) {
+            cs.time = time; cs.dt = dt; cs.dt_old = S->dt_old; cs.alpha_t = mo.alpha_t; cs.alpha_tt = mo.alpha_tt; cs.grav = grav;
+            newton_consts_pre(cs, b, b.pred + pred_consts(ns));
+        }
+        __syncthreads();
+        for (int i = tid; i < ns; i += nthr) tdn[i] = cs.D * (x[xi_th(i)] - cs.C3 * bo5[i] - cs.C4 * oo5[i]) - cs.C2 * bo6[i];
+    }
+    // the loads' share of the initial ghost values (SolidSolver.f90:175-187, 197-202) is added below
+    const double* K = b.pred + pred_consts(ns);
+    const double* g5 = b.pred + n + ns;
+    const double* T = g5 + ns;
+    double gh0 = 0.0, gh1 = 0.0, gh2 = 0.0, gh3 = 0.0;
+    if (released && tid == 0) {
+        gh0 = mue * (mo.le[5] * mo.ca - mo.le[4] * mo.sa + grav * mo.ca);
+        gh1 = T[0] * g5[1];
+        gh2 = (eta / (ds * ds)) * (10.0 * g5[0] - 12.0 * g5[1] + 6.0 * g5[2] - g5[3]);
+    }
+    if (released && tid == 64) {
+        gh0 = mue * (mo.le[4] * mo.ca + mo.le[5] * mo.sa + grav * mo.sa);
+        const double th_ss0 = (2.0 * g5[0] - 5.0 * g5[1] + 4.0 * g5[2] - 1.0 * g5[3]) * b.k.ids2;
+        const double th_s0 = (-1.5 * g5[0] + 2.0 * g5[1] - 0.5 * g5[2]) * b.k.ids;
+        gh1 = -eta * th_ss0;
+        gh2 = th_s0;
+        gh3 = T[1];
     }
     pdl_wait();     // k_forces has completed: its loads and any status it raised are visible
     if (S->status != 0) {  // the same value in every CTA: they all return here
@@ -274,76 +389,69 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
         return;
     }
     if (released) {
-        const double* K = b.pred + pred_consts(ns);
-        for (int i = tid; i < ns; i += nthr) {
-            old_rhs[i] = b.pred[n + i];
-            taun_s[i] = d1d(&dtab, b.tau_new, ns, 1, i);
-        }
-        // initial guess ghost values from the new loads (SolidSolver.f90:175-187, 197-202)
-        // on warp 0, the Newton constants (divisions done by the predictor) on warp 1
+        for (int i = tid; i < ns; i += nthr) taun_s[i] = d1d(&dtab, b.tau_new, ns, 1, i);
+        // initial guess ghost values from the new loads (SolidSolver.f90:175-187, 197-202), on two warps
         if (tid == 0) {
-            const double* g5 = b.pred + n + ns;
-            const double* T = g5 + ns;
-            const double ds2 = ds * ds;
-            const double K2 = b.p_new[0] + mue * (mo.le[5] * mo.ca - mo.le[4] * mo.sa + grav * mo.ca);
-            const double C2v = 2.0 * ds * K2 - T[0] * g5[1] + (eta / ds2) * (10.0 * g5[0] - 12.0 * g5[1] + 6.0 * g5[2] - g5[3]);
+            const double K2 = b.p_new[0] + gh0;
+            cs.K2 = K2;
+            const double C2v = 2.0 * ds * K2 - gh1 + gh2;
             x[xi_th(-1)] = div_cr(C2v, K[8], K[9]);  // C2v / (3 eta/ds^2 - T_0), correctly rounded
-            const double K1 = mue * (mo.le[4] * mo.ca + mo.le[5] * mo.sa + grav * mo.sa) - b.tau_new[0];
-            const double th_ss0 = (2.0 * g5[0] - 5.0 * g5[1] + 4.0 * g5[2] - 1.0 * g5[3]) * b.k.ids2;
-            const double th_s0 = (-1.5 * g5[0] + 2.0 * g5[1] - 0.5 * g5[2]) * b.k.ids;
-            const double T_s0 = -eta * th_ss0 * th_s0 + K1;
-            x[xi_T(ns, -1)] = T[1] - 2.0 * ds * T_s0;
         }
-        if (tid == 32) {
-            cs.time = time; cs.dt = dt; cs.dt_old = S->dt_old; cs.alpha_t = mo.alpha_t; cs.alpha_tt = mo.alpha_tt; cs.grav = grav;
-            newton_consts_pre(cs, b, K);
-            cs.K1 = mue * (mo.le[4] * mo.ca + mo.le[5] * mo.sa + grav * mo.sa) - b.tau_new[0];
-            cs.K2 = b.p_new[0] + mue * (mo.le[5] * mo.ca - mo.le[4] * mo.sa + grav * mo.ca);
+        if (tid == 64) {
+            const double K1 = gh0 - b.tau_new[0];
+            cs.K1 = K1;
+            const double T_s0 = gh1 * gh2 + K1;
+            x[xi_T(ns, -1)] = gh3 - 2.0 * ds * T_s0;
         }
         __syncthreads();
         const NewtonCtx& c = cs;
         bool inv_pending = have_inv && !big;  // the stored inverse rows are still arriving (cp.async)
         bool need_factor = !have_inv, factored = false;
         // own rows: generic ones [glo, ghi); the boundary equations (rows 0..3: k = 1, 2, 3, 7;
-        // rows 2ns..2ns+3: k = 8, 6, 5, 4) sit in the first and last CTA and take warps 4..7,
-        // one F or J evaluation per lane, so that their separate code paths do not serialise
-        // a warp of generic rows
+        // rows 2ns..2ns+3: k = 8, 6, 5, 4) sit in the first and last CTA and take warps 4..7, so that
+        // their separate code paths do not serialise a warp of generic rows
         const int glo = lo > 4 ? lo : 4, ghi = hi < 2 * ns ? hi : 2 * ns;
         const int ngen = ghi > glo ? ghi - glo : 0;
         const bool has_sp = (lo < 4) || (hi > 2 * ns);
-        const int npairs = has_sp ? 2 : (nwarp >> 1);
+        // generic rows alternate between the two node equations, whose code differs: a warp takes one
+        // of them, for F or for J (warp & 3: the four SMSPs), 32 rows at a time
+        const int neq = ngen / 2, nseg = has_sp ? 1 : 2;
+        const int ja = lo / 2 - 1 > 0 ? lo / 2 - 1 : 0, jb = hi / 2 < ns ? hi / 2 : ns;  // nodes of the own rows
+        // the refinement's state, the same in every thread: the first, the previous and the last
+        // correction's maxima of the angles and of the tensions, and the iterate's
+        float c0[2] = {0.f, 0.f}, cp[2] = {0.f, 0.f}, xmax[2] = {0.f, 0.f};
+        const float rn = sqrtf((float)n), tolf = (float)b.tol;
         PH(22);
         for (;;) {
-            for (int i = tid; i < ns; i += nthr)
-                tdn[i] = c.D * (x[xi_th(i)] - c.C3 * bo5[i] - c.C4 * oo5[i]) - c.C2 * bo6[i];
-            __syncthreads();
-            // F (even warps) and the Jacobian rows (odd warps: another SMSP), 32 rows a pair
-            if ((warp >> 1) < npairs) {
-                for (int g = warp >> 1; g * 32 < ngen; g += npairs) {
-                    const int r = glo + g * 32 + lane;
-                    if (r < ghi) {
-                        const int k = k_of_row(ns, r);
+            if ((warp >> 2) < nseg) {
+                const int odd = (warp >> 1) & 1;
+                for (int g = warp >> 2; g * 32 < neq; g += nseg) {
+                    const int q = g * 32 + lane;
+                    if (q < neq) {
+                        const int r = glo + 2 * q + odd;
+                        const int k = odd ? 8 + (ns - 2) + ((r - 1) / 2 - 1) : 8 + (r / 2 - 1);
                         if ((warp & 1) == 0) {
                             const double f = f_eq(b, w, c, k);
                             if (isnan(f)) flag_s = FSIBE_ERR_NAN;
                             bvec[r - lo] = -1.0 * f;
-                        } else if (jac_row(b, w, c, k, band + (size_t)(r - lo) * 16)) {
+                        } else if (jac_row(b, w, c, k, band + (size_t)(r - lo) * CL_BAND)) {
                             flag_s = FSIBE_ERR_NAN;
                         }
                     }
                 }
             } else if (has_sp && warp >= 4) {
-                // special s (0..3 in row order) -> F on warp 4 + 2 (s & 1), J on warp 5 + 2 (s & 1)
-                const int s = 2 * lane + ((warp >> 1) & 1);
-                const int base = (lo < 4) ? 0 : 2 * ns;
+                // the boundary equations: the long one's (k = 7 or 8) F and J on warps 4 and 5, one a lane
+                // of the other three on warps 6 and 7
+                const int base = (lo < 4) ? 0 : 2 * ns, heavy = (lo < 4) ? 3 : 0;
+                const int s = (warp < 6) ? heavy : (lane < heavy ? lane : lane + 1);
                 const int r = base + s;
-                if (lane < 2 && r >= lo && r < hi) {
+                if (lane < (warp < 6 ? 1 : 3) && r >= lo && r < hi) {
                     const int k = k_of_row(ns, r);
                     if ((warp & 1) == 0) {
                         const double f = f_eq(b, w, c, k);
                         if (isnan(f)) flag_s = FSIBE_ERR_NAN;
                         bvec[r - lo] = -1.0 * f;
-                    } else if (jac_row(b, w, c, k, band + (size_t)(r - lo) * 16)) {
+                    } else if (jac_row(b, w, c, k, band + (size_t)(r - lo) * CL_BAND)) {
                         flag_s = FSIBE_ERR_NAN;
                     }
                 }
@@ -356,12 +464,14 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
             }
             if (!cl_up) { cl_sync(); cl_up = true; }
             int solves = 0;
+            bool slow = false;  // a contraction of more than 2^-6
+            float dxb = 0.f;    // the corrections' maxima summed: no entry of dx is larger
             for (int attempt = 0; attempt < 2; ++attempt) {
                 const bool fresh = need_factor;
                 if (need_factor) {
                     // the scaled FP32 rows: own copy first, then every other CTA's
                     for (int r = lo + tid; r < hi; r += nthr)
-                        scale_band_row(band + (size_t)(r - lo) * 16, Uf + (size_t)r * 16, rse + r);
+                        scale_band_row(band + (size_t)(r - lo) * CL_BAND, Uf + (size_t)r * 16, rse + r);
                     __syncthreads();
                     for (int e = tid; e < nr * 5 * ((int)R - 1); e += nthr) {
                         const unsigned dst = (rank + 1 + (unsigned)(e / (nr * 5))) % R;
@@ -376,10 +486,10 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                             else *cl_map(rse + r, dst) = rse[r];
                         }
                     }
-                    if (tid < (int)R) *cl_map(slots + 3 * R + rank, (unsigned)tid) = (unsigned long long)flag_s;
+                    if (tid < (int)R) *cl_map(slots + 2 * R + rank, (unsigned)tid) = (unsigned long long)flag_s;
                     cl_sync();
                     int fl = 0;
-                    for (unsigned q = 0; q < R; ++q) fl = fl ? fl : (int)slots[3 * R + q];
+                    for (unsigned q = 0; q < R; ++q) fl = fl ? fl : (int)slots[2 * R + q];
                     if (fl) { if (rank == 0 && tid == 0) set_status(S, fl); return; }
                     if (warp == 0) {
                         const int info = band_factor_f32(w, n);
@@ -403,7 +513,7 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                             const int t = g * 32 + lane;
                             if (t < nr) {
                                 const int k = lo + t;
-                                const double* Bk = band + (size_t)t * 16;
+                                const double* Bk = band + (size_t)t * CL_BAND;
                                 double acc = 0.0;
 #pragma unroll
                                 for (int u = 0; u < 4; ++u) {
@@ -432,7 +542,7 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                             *cl_map(p4, dst) = *p4;
                         }
                     }
-                    if (tid < (int)R) *cl_map(slots + 2 * R + rank, (unsigned)tid) = (unsigned long long)flag_s;
+                    if (tid < (int)R) *cl_map(slots + R + rank, (unsigned)tid) = (unsigned long long)flag_s;
                     PH(20);
                     cl_sync();
                     PH(16);
@@ -440,15 +550,14 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                         int fl = 0;
 #pragma unroll
                         for (int q = 0; q < 16; ++q)
-                            if (q < (int)R) fl = fl ? fl : (int)slots[2 * R + q];
+                            if (q < (int)R) fl = fl ? fl : (int)slots[R + q];
                         if (fl) { if (rank == 0 && tid == 0) set_status(S, fl); return; }
                     }
                     // own rows of M^-1 y, eight rows per warp: lanes split the columns (float4),
                     // a transposing butterfly leaves the sum of row
                     // 4 ((l >> 4) & 1) + 2 ((l >> 3) & 1) + ((l >> 2) & 1) in lanes l = 0 (mod 4);
                     // those lanes update the FP64 solution rows
-                    unsigned cm = 0;
-                    unsigned long long xm = 0;
+                    unsigned cmt = 0, cmT = 0;  // max |c| of the angles and of the tensions (FP32 bits)
                     const float4* y4 = reinterpret_cast<const float4*>(yf);
                     for (int g = warp; g * 8 < nr; g += nwarp) {
                         const int t0 = g * 8;
@@ -498,29 +607,19 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                             const double xn = (pass == 0) ? (double)s : xdi[k] + (double)s;
                             xdi[k] = xn;
                             const unsigned a = __float_as_uint(s) & 0x7fffffffu;
-                            const unsigned long long ax = (unsigned long long)__double_as_longlong(xn) & 0x7fffffffffffffffull;
-                            cm = (a > cm) ? a : cm;
-                            xm = (ax > xm) ? ax : xm;
+                            if ((k & 1) && k < 2 * ns + 2) cmT = (a > cmT) ? a : cmT;
+                            else cmt = (a > cmt) ? a : cmt;
                         }
                     }
-#pragma unroll
-                    for (int o = 16; o >= 4; o >>= 1) {
-                        const unsigned c2 = __shfl_xor_sync(0xffffffffu, cm, o);
-                        const unsigned long long x2 = __shfl_xor_sync(0xffffffffu, xm, o);
-                        cm = (c2 > cm) ? c2 : cm;
-                        xm = (x2 > xm) ? x2 : xm;
-                    }
-                    if (lane == 0) { redu[0][warp] = cm; redu[1][warp] = xm; }
+                    cmt = __reduce_max_sync(0xffffffffu, cmt);
+                    cmT = __reduce_max_sync(0xffffffffu, cmT);
+                    if (lane == 0) { redu[0][warp] = cmt; redu[1][warp] = cmT; }
                     __syncthreads();
                     PH(17);
-                    if (tid < (int)R) {
-                        unsigned long long c2 = 0, x2 = 0;
-                        for (int q = 0; q < nwarp; ++q) {
-                            c2 = (redu[0][q] > c2) ? redu[0][q] : c2;
-                            x2 = (redu[1][q] > x2) ? redu[1][q] : x2;
-                        }
-                        *cl_map(slots + rank, (unsigned)tid) = c2;
-                        *cl_map(slots + R + rank, (unsigned)tid) = x2;
+                    if (warp == 0) {
+                        const unsigned mt = __reduce_max_sync(0xffffffffu, lane < nwarp ? redu[0][lane] : 0u);
+                        const unsigned mT = __reduce_max_sync(0xffffffffu, lane < nwarp ? redu[1][lane] : 0u);
+                        if (lane < (int)R) *cl_map(slots + rank, (unsigned)lane) = ((unsigned long long)mT << 32) | mt;
                     }
                     // the own solution rows to every other CTA, 16 bytes a store
                     {
@@ -535,51 +634,53 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                     cl_sync();
                     PH(18);
                     ++solves;
-                    // the convergence decision of refine_step from the cluster's maxima, on one
-                    // thread (FP64 issue is per warp)
-                    if (tid == 0) {
-                        unsigned long long c2 = 0, x2 = 0;
-                        for (int q = 0; q < (int)R; ++q) {
-                            c2 = (slots[q] > c2) ? slots[q] : c2;
-                            x2 = (slots[R + q] > x2) ? slots[R + q] : x2;
-                        }
-                        const float cpf = (pass == 0) ? 0.f : cprev_s;
-                        const double cmd = (double)__uint_as_float((unsigned)c2), cpd = (double)cpf;
-                        const double xmd = __longlong_as_double((long long)x2);
-                        // 2^-30 of the correction (refine_step says why that suffices)
-                        const double tol = 0x1p-30 * xmd;
-                        const bool conv = !(cmd > tol) || (pass >= 1 && cmd * cmd <= tol * cpd);
-                        const bool stall = pass >= 2 && cmd > 0.5 * cpd;
-                        cprev_s = __uint_as_float((unsigned)c2);
-                        dec_s = (conv || (stall && cmd <= 0x1p-30 * xmd)) ? 1 : ((stall || pass >= 9) ? -1 : 0);
-                    }
-                    __syncthreads();
-                    const int dec = dec_s;
+                    // the decision, from the cluster's maxima, by every warp (newton_pass)
+                    const unsigned long long sl = (lane < (int)R) ? slots[lane] : 0ull;
+                    const float cm[2] = {__uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)sl)),
+                                         __uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)(sl >> 32)))};
+                    if (pass == 0) { c0[0] = cm[0]; c0[1] = cm[1]; dxb = 0.f; }
+                    dxb += fmaxf(cm[0], cm[1]);
+                    const int dec = newton_pass(iter, pass, cm, cp, c0, xmax, rn, tolf, fresh || factored, slow);
+                    cp[0] = cm[0];
+                    cp[1] = cm[1];
                     if (dec > 0) { ok = true; break; }
                     if (dec < 0) break;
                 }
                 if (ok || fresh) break;
                 need_factor = true;
             }
-            if (solves > 5) need_factor = true;
+            if (solves > 5 || (slow && !factored)) need_factor = true;
             if (tid == 0) ph[10] += solves;
             PH(6);
             // x += dx in Fortran order, the norms and the stopping test: the same data in every
             // CTA, so the same decisions without an exchange
-            // the stopping test needs iter > 2: before that the norms are not formed
+            // the stopping test needs iter > 2: before that the norms are not formed, nor where the bound
+            // sqrt(n) max |dx| on the update's norm (and max |x| below the iterate's) decides: its
+            // margin of 2^-6 covers the FP32 arithmetic
             const bool test = iter + 1 > 2;
+            const float xlow = fmaxf(xmax[0], xmax[1]) - dxb;
+            const bool below = test && 1.015625f * rn * dxb < tolf * fmaxf(1.f, xlow);
+            const bool norms = test && !below;
             double sd = 0.0, sx = 0.0;
+            unsigned xt = 0, xT = 0;
             for (int l = tid; l < n; l += nthr) {
                 const double d = xdi[col_of(ns, l + 1)];
-                if (isnan(d)) flag_s = FSIBE_ERR_NAN;
+                if ((__double2hiint(d) & 0x7ff00000) == 0x7ff00000 && isnan(d)) flag_s = FSIBE_ERR_NAN;
                 const double xn = x[l] + d;
                 x[l] = xn;
-                if (test) {
+                const unsigned h = (unsigned)__double2hiint(xn) & 0x7fffffffu;
+                if (l < ns + 3) xt = h > xt ? h : xt;
+                else xT = h > xT ? h : xT;
+                if (l > ja && l <= jb) tdn[l - 1] = c.D * (xn - c.C3 * bo5[l - 1] - c.C4 * oo5[l - 1]) - c.C2 * bo6[l - 1];
+                if (norms) {
                     sd += d * d;
                     sx += xn * xn;
                 }
             }
-            if (test) {
+            xt = __reduce_max_sync(0xffffffffu, xt);
+            xT = __reduce_max_sync(0xffffffffu, xT);
+            if (lane == 0) { xhi[0][warp] = xt; xhi[1][warp] = xT; }
+            if (norms) {
                 for (int o = 16; o > 0; o >>= 1) {
                     sd += __shfl_xor_sync(0xffffffffu, sd, o);
                     sx += __shfl_xor_sync(0xffffffffu, sx, o);
@@ -589,7 +690,7 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
             __syncthreads();
             if (flag_s) { if (rank == 0 && tid == 0) set_status(S, flag_s); return; }
             iter = iter + 1;
-            if (test) {
+            if (norms) {
                 if (tid < 32) {
                     double tsd = (lane < nwarp) ? red[0][lane] : 0.0, tsx = (lane < nwarp) ? red[1][lane] : 0.0;
                     for (int o = 4; o > 0; o >>= 1) {
@@ -599,12 +700,15 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
                     if (lane == 0) stop_s = newton_stop(tsd, tsx, b.tol);
                 }
                 __syncthreads();
-            } else if (tid == 0) {
-                stop_s = 0;
             }
-            __syncthreads();
+            // the iterate's maxima, rounded down to 20 bits
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const unsigned m = __reduce_max_sync(0xffffffffu, xhi[q][lane & 7]);
+                xmax[q] = hi_to_float(m);
+            }
             PH(23);
-            const bool stop = stop_s != 0;
+            const bool stop = below || (norms && stop_s != 0);
             if (iter > b.maxit - 1) {
                 if (rank == 0 && tid == 0) set_status(S, FSIBE_ERR_NEWTON_MAXIT);
                 return;
