@@ -29,12 +29,12 @@ void fill_sizes_1024(SizeKernels<double>&, SizeKernels<float>&);
 void fill_sizes_2048(SizeKernels<double>&, SizeKernels<float>&);
 void fill_sizes_4096(SizeKernels<double>&, SizeKernels<float>&);
 size_t beam_ws_doubles(int ns);
-void launch_mask_prep(const MaskArgs& a, double gerf, cudaStream_t st, bool pdl);
-void launch_mask(const MaskArgs& a, double gerf, bool fp32, cudaStream_t st, bool pdl);
-void launch_forces(const ForceArgs& a, double dxi, double dyi, cudaStream_t st, bool pdl);
+void launch_mask_prep(const MaskArgs& a, cudaStream_t st, bool pdl);
+void launch_mask(const MaskArgs& a, bool fp32, cudaStream_t st, bool pdl);
+void launch_forces(const ForceArgs& a, cudaStream_t st, bool pdl);
 void launch_static_masks(const StaticMaskArgs& a, double gerf, cudaStream_t st);
 void launch_sponge_mask(const StaticMaskArgs& a, double gerf, cudaStream_t st);
-void launch_forces_geo(const ForceArgs& a, double dxi, double dyi, cudaStream_t st);
+void launch_forces_geo(const ForceArgs& a, cudaStream_t st);
 void launch_surface_integral(const ForceArgs& a, const SurfArgs& s, double dxi, double dyi, double time, cudaStream_t st);
 void launch_beam(const BeamArgs& b, cudaStream_t st);
 void launch_beam_pre(const BeamArgs& b, cudaStream_t st);
@@ -118,7 +118,7 @@ __device__ double mean_uy(int mode, double time, double sin_ti, double Tf, doubl
 // Start of a fluid step: the CFL/penalization/fixed dt of cal_nlk (NavierStokes.f90:59-78)
 // from the velocity statistics of the previous step, the AB2 weights (:488-489), the mean
 // flow at time+dt1 and the drag window of cal_drag (:539-564).
-__global__ void __launch_bounds__(256) k_step_begin(StepArgs a) {
+__device__ __forceinline__ void step_begin_run(const StepArgs& a) {
     // one warp per statistic (FP64 adds and compares are slow here: each warp reduces its own
     // quantity with shuffles): 0 max |u|^2, 1 sum u, 2 sum v, 3 min x, 4 max x, 5 min y, 6 max y
     __shared__ double q[8];
@@ -240,10 +240,12 @@ __global__ void __launch_bounds__(256) k_step_begin(StepArgs a) {
     __syncthreads();
     if (threadIdx.x == 0) { S->etab_cx = coefx; S->etab_cy = coefy; S->etab_valid = 1; }
 }
+__global__ void __launch_bounds__(256) k_step_begin(const __grid_constant__ StepArgs a) { step_begin_run(a); }
+__global__ void __launch_bounds__(256) k_step_begin_b(const __grid_constant__ Batch<StepArgs> a) { step_begin_run(a.a[blockIdx.z]); }
 
 // End of the fluid part: cal_energy (NavierStokes.f90:222-263) and cal_drag (:566-589)
 // from the per-block partial sums, summed in a fixed order.
-__global__ void __launch_bounds__(256) k_fluid_finish(StepArgs a) {
+__device__ __forceinline__ void fluid_finish_run(const StepArgs& a) {
     // one warp per slot group: warp w reduces slots w and w + 8 with shuffles
     __shared__ double sm[RED_NSLOTS][1];
     const int lane = threadIdx.x & 31;
@@ -285,9 +287,12 @@ __global__ void __launch_bounds__(256) k_fluid_finish(StepArgs a) {
     __syncthreads();
     if (threadIdx.x == 0 && a.iBeam > 0) S->unst_ready = 1;
 }
+__global__ void __launch_bounds__(256) k_fluid_finish(const __grid_constant__ StepArgs a) { fluid_finish_run(a); }
+__global__ void __launch_bounds__(256) k_fluid_finish_b(const __grid_constant__ Batch<StepArgs> a) { fluid_finish_run(a.a[blockIdx.z]); }
 
 // time_step.f90:152-161 / :222-236 (advance_state in solid.cuh) as its own kernel.
-__global__ void __launch_bounds__(256) k_advance(AdvArgs a) { advance_state(a); }
+__global__ void __launch_bounds__(256) k_advance(const __grid_constant__ AdvArgs a) { advance_state(a); }
+__global__ void __launch_bounds__(256) k_advance_b(const __grid_constant__ Batch<AdvArgs> a) { advance_state(a.a[blockIdx.z]); }
 
 // 1 / |k|^2 per mode, correctly rounded (0 at k = 0), from the rounded squares the kernels add
 __global__ void k_recip_k2(double* rk2, const double* ky2, double scalex, int hx, int nyh) {
@@ -643,7 +648,7 @@ template <typename R>
 static void launch_y(fsibe_ctx* c, const KLaunch<R>& k, const KArgs<R>& a, const char* name = "y_pass", int nfields = 1,
                      bool pdl = false) {
     prof_begin(c, name);
-    launch_k(k.k, dim3(c->g.hx, nfields), dim3(k.threads), k.smem, c->stream, pdl && c->pdl, a);
+    launch_b(k.k, k.kb, dim3(c->g.hx, nfields), dim3(k.threads), k.smem, c->stream, pdl && c->pdl, a);
     prof_end(c);
     c->launches++;
 }
@@ -655,7 +660,7 @@ static void launch_xv(fsibe_ctx* c, const KLaunch<R>& k, int rows, const KArgs<R
                       cudaStream_t st = nullptr, int grid = 0) {
     if (!st) st = c->stream;
     prof_begin(c, name, st);
-    launch_k(k.k, dim3(grid > 0 ? grid : c->g.ny / rows), dim3(k.threads), k.smem, st, c->pdl && st == c->stream, a);
+    launch_b(k.k, k.kb, dim3(grid > 0 ? grid : c->g.ny / rows), dim3(k.threads), k.smem, st, c->pdl && st == c->stream, a);
     prof_end(c, st);
     c->launches++;
 }
@@ -831,7 +836,7 @@ static int fluid_step_t(fsibe_ctx* c, int explicit_step, bool adv_forked = false
     CK(c, cudaEventRecord(c->ev_sb0, c->stream));
     CK(c, cudaStreamWaitEvent(c->side, c->ev_sb0, 0));
     prof_begin(c, "step_begin", c->side);
-    k_step_begin<<<1, 256, 0, c->side>>>(sa);
+    launch_b(k_step_begin, k_step_begin_b, dim3(1), dim3(256), 0, c->side, false, sa);
     prof_end(c, c->side);
     CK(c, cudaEventRecord(c->ev_sb, c->side));
     c->launches++;
@@ -877,7 +882,7 @@ static int fluid_step_t(fsibe_ctx* c, int explicit_step, bool adv_forked = false
     CK(c, cudaEventRecord(c->ev_ff, c->stream));
     CK(c, cudaStreamWaitEvent(c->side2, c->ev_ff, 0));
     prof_begin(c, "fluid_finish", c->side2);
-    k_fluid_finish<<<1, 256, 0, c->side2>>>(sa);
+    launch_b(k_fluid_finish, k_fluid_finish_b, dim3(1), dim3(256), 0, c->side2, false, sa);
     prof_end(c, c->side2);
     CK(c, cudaEventRecord(c->ev_ffj, c->side2));
     c->launches++;
@@ -925,6 +930,7 @@ static MaskArgs mask_args(fsibe_ctx* c) {
     m.rdx = 1.0 / m.dx; m.rdy = 1.0 / m.dy; m.rpi = 1.0 / m.pi;
     m.inv_delta = 1.0 / ((m.N_smooth * std::fmax(m.dx, m.dy)) * c->gerf);
     m.inv_ds = 1.0 / m.ds;
+    m.gerf = c->gerf;
     m.inv_eps = 1.0 / m.eps;
     m.mo = motion_args(c);
     m.mask = c->phys[PH_MASK]; m.mvx = c->phys[PH_MVX]; m.mvy = c->phys[PH_MVY];
@@ -986,10 +992,10 @@ static int create_mask(fsibe_ctx* c, bool until_full = false) {
     MaskArgs m = mask_args(c);
     m.until_full = until_full ? 1 : 0;
     prof_begin(c, "mask_prep");
-    launch_mask_prep(m, c->gerf, c->stream, c->pdl);
+    launch_mask_prep(m, c->stream, c->pdl);
     prof_end(c);
     prof_begin(c, "mask");
-    launch_mask(m, c->gerf, c->fp32, c->stream, c->pdl);
+    launch_mask(m, c->fp32, c->stream, c->pdl);
     prof_end(c);
     c->launches += 2;
     CKL(c);
@@ -1015,6 +1021,7 @@ static ForceArgs force_args(fsibe_ctx* c, double& dxi, double& dyi) {
     f.geo = c->fgeo;
     f.gij = c->fgij;
     f.mo = motion_args(c);
+    f.dxi = dxi; f.dyi = dyi;
     f.rdxi = 1.0 / dxi;
     f.rdyi = 1.0 / dyi;
     return f;
@@ -1025,7 +1032,7 @@ static void forces_geo(fsibe_ctx* c, cudaStream_t st) {
     double dxi, dyi;
     const ForceArgs f = force_args(c, dxi, dyi);
     prof_begin(c, "forces_geo", st);
-    launch_forces_geo(f, dxi, dyi, st);
+    launch_forces_geo(f, st);
     prof_end(c, st);
     c->launches++;
 }
@@ -1037,7 +1044,7 @@ static int get_forces(fsibe_ctx* c, bool geo_done = false) {
     if (geo_done) CK(c, cudaStreamWaitEvent(c->stream, c->ev_geo, 0));
     else forces_geo(c, c->stream);
     prof_begin(c, "forces");
-    launch_forces(f, dxi, dyi, c->stream, c->pdl);
+    launch_forces(f, c->stream, c->pdl);
     prof_end(c);
     c->launches++;
     CKL(c);
@@ -1083,7 +1090,7 @@ static int solid_step(fsibe_ctx* c, bool end_step = false, bool* advanced = null
 static int advance(fsibe_ctx* c) {
     const AdvArgs a = adv_args(c);
     prof_begin(c, "advance");
-    k_advance<<<1, 256, 0, c->stream>>>(a);
+    launch_b(k_advance, k_advance_b, dim3(1), dim3(256), 0, c->stream, false, a);
     prof_end(c);
     c->launches++;
     CKL(c);
@@ -2959,11 +2966,15 @@ int fsibe_drag_gradient(fsibe_ctx* c, const double* vort0, double nu, int nsteps
 // =====================================================================================
 // Ensembles: independent runs advanced together, one graph launch per step
 // =====================================================================================
-// Every run keeps its own context (fields, streams, beam workspace).  One step of the
-// ensemble is captured once as a CUDA graph: a fork from the ensemble's stream, each run's
-// whole step on its own stream (with its own predictor fork), and a join.  The runs' kernels
-// of different grid sizes then share the GPU in one launch; the single-CTA beam kernels of
-// many runs fill separate SMs at the same time.
+// Every run keeps its own context (fields, streams, beam workspace).  One step of the ensemble is
+// captured once as a CUDA graph: a fork from the ensemble's stream, each batch's step on its first run's
+// streams, and a join.  A batch is up to kBatch runs whose steps are the same launches, each of them made
+// once for all (Batch, ens_groups); the other runs' steps stay their own.  The GPU starts a graph's
+// kernels at one in 1.3 us however small they are, so that 48 runs of 256^2, 14 kernels each, took
+// 876 us a step where their work is 400; batched they take 399, and the 64-run batch (48 x 256^2,
+// 12 x 512^2, 4 x 1024^2) 1024 instead of 1569.  One batch a shape: smaller ones, which would
+// overlap more, measured no better (64-run batch with at most 0.25 / 1 / 2 million cells a batch 1248 /
+// 1192 / 1181 us, without that limit 1149).
 struct fsibe_ensemble {
     std::vector<fsibe_ctx*> runs;
     cudaStream_t master = nullptr;
@@ -3012,6 +3023,40 @@ static int ens_join_runs(fsibe_ensemble* e, bool runs_first) {
     return FSIBE_OK;
 }
 
+// The batches of a step: lead[i] is the run whose streams carry run i's launches.  Runs whose steps are
+// the same launches (kernels, grids, blocks, shared memory) share one, up to kBatch; a run whose step has
+// a launch without a batched form, or a copy, is its own leader.  Each run's step is recorded by running
+// step_body with the launches held back.  From 8 runs on, as the ensemble's other choices: the compiler
+// may fuse other multiply-add pairs in a kernel's batched form, so that a batched run's last places can
+// differ from the run's alone, which fewer runs keep.
+static int ens_groups(fsibe_ensemble* e, std::vector<BatchRec>& rec, std::vector<size_t>& lead) {
+    const size_t n = e->runs.size();
+    rec.assign(n, BatchRec());
+    lead.resize(n);
+    std::vector<size_t> count(n, 0);
+    for (size_t i = 0; i < n; ++i) {
+        fsibe_ctx* c = e->runs[i];
+        lead[i] = i;
+        count[i] = 1;
+        if (n < 8 || c->P.iBeam <= 0 || c->P.iFLUSI != 1 || c->spg || c->s10 || c->profiling) continue;
+        const int before = c->launches;
+        const bool ready = c->adv_ready;
+        g_batch = &rec[i];
+        const int st = step_body(c, 0);
+        g_batch = nullptr;
+        c->launches = before;
+        c->adv_ready = ready;
+        if (st) { e->err = c->err; g_err = e->err; return st; }
+        for (size_t k = 0; k < i; ++k)
+            if (lead[k] == k && count[k] < (size_t)kBatch && rec[k].like(rec[i])) {
+                lead[i] = k;
+                ++count[k];
+                break;
+            }
+    }
+    return FSIBE_OK;
+}
+
 static int ens_step(fsibe_ensemble* e) {
     bool started = true;
     for (fsibe_ctx* c : e->runs) {
@@ -3032,14 +3077,24 @@ static int ens_step(fsibe_ensemble* e) {
         return ens_join_runs(e, true);
     }
     if (!e->gexec) {
+        std::vector<BatchRec> rec;
+        std::vector<size_t> lead;
+        int st = ens_groups(e, rec, lead);
+        if (st) return st;
         CKE(e, cudaStreamBeginCapture(e->master, cudaStreamCaptureModeThreadLocal));
         CKE(e, cudaEventRecord(e->fork, e->master));
-        int st = FSIBE_OK;
         for (size_t i = 0; i < e->runs.size() && !st; ++i) {
             fsibe_ctx* c = e->runs[i];
+            if (lead[i] != i) continue;  // its launches are in its leader's batch
             if (cudaStreamWaitEvent(c->stream, e->fork, 0) != cudaSuccess) { st = FSIBE_ERR_CUDA; break; }
             const int before = c->launches;
+            std::vector<BatchRec> group;
+            for (size_t k = i; k < e->runs.size(); ++k) if (lead[k] == i) group.push_back(rec[k]);
+            BatchRec emit;
+            emit.group = &group;
+            if (group.size() > 1) g_batch = &emit;
             st = step_body(c, 0);
+            g_batch = nullptr;
             c->launches = before;
             if (st) { e->err = c->err; break; }
             if (cudaEventRecord(e->done[i], c->stream) != cudaSuccess ||
@@ -3071,15 +3126,18 @@ int fsibe_ensemble_create(const fsibe_params* params, int nruns, fsibe_ensemble*
         if (st) { ens_free(e); return st; }
         e->runs.push_back(c);
     }
-    // Many concurrent runs fill the GPU by themselves: the single-CTA beam kernel then gives
-    // more throughput than 16-SM clusters, which wait for whole free GPCs (measured with the
-    // 64-run batch: 6276 against 4854 Mcell-steps/s).  FSIBE_BEAM_CLUSTER, when set, decides.
-    if (nruns >= 8 && !std::getenv("FSIBE_BEAM_CLUSTER"))
+    // The beams of many runs fill the GPU by themselves: above two cluster CTAs an SM the single-CTA beam
+    // kernel gives as much (us a step with clusters / single CTAs: 48 runs of 256^2, 384 CTAs, 470 / 425,
+    // 32, 256 CTAs, 333 / 331; the 64-run batch, 544 CTAs, 1072 / 1065), below it the clusters do, whose
+    // beams end sooner (24 of 256^2 253 / 289, 8 of 512^2 244 / 339, 8 + 4 + 2 of 256^2, 512^2 and 1024^2
+    // 384 / 504).  FSIBE_BEAM_CLUSTER, when set, decides.
+    int ctas = 0;
+    for (fsibe_ctx* c : e->runs) ctas += c->beam_cl;
+    if (ctas > 2 * e->runs[0]->nsm && !std::getenv("FSIBE_BEAM_CLUSTER"))
         for (fsibe_ctx* c : e->runs) c->beam_cl = 0;
-    // For the same reason the launches that take work off one run's critical path (the split
-    // nonlinear term, the stresses beside k_press_x) only add graph nodes here (64-run batch:
-    // 6350 against 6220 Mcell-steps/s without them).  FSIBE_NL_SPLIT / FSIBE_STRESS_SPLIT decide
-    // when set.
+    // In a batch of many runs the launches that take work off one run's critical path (the split
+    // nonlinear term, the stresses beside k_press_x) only add launches (64-run batch: 1587 us
+    // a step with them, 1024 without).  FSIBE_NL_SPLIT / FSIBE_STRESS_SPLIT decide when set.
     if (nruns >= 8) {
         for (fsibe_ctx* c : e->runs) {
             if (!std::getenv("FSIBE_NL_SPLIT")) c->nl_split = false;

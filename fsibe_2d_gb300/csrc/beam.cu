@@ -76,7 +76,7 @@ __device__ double gravity_impulse(const BeamArgs& b, double time, double grav) {
 // EE1 predictor (RHS_beameqn with the tension solve), the initial guess except its two
 // ghost values that use the new loads, and the Crank-Nicolson right-hand side.  It runs on a
 // side stream while the fluid step of the same time step runs; its output goes to b.pred.
-__global__ void __launch_bounds__(256) k_beam_pre(BeamArgs b) {
+__device__ __forceinline__ void beam_pre_run(const BeamArgs& b) {
     extern __shared__ __align__(16) double smem_ws[];
     DevScalars* S = b.S;
     if (S->status != 0) return;
@@ -153,11 +153,13 @@ __global__ void __launch_bounds__(256) k_beam_pre(BeamArgs b) {
     if (threadIdx.x == 0)
         for (int k = 0; k < 4; ++k) S->phase[k] += ph[k];
 }
+__global__ void __launch_bounds__(256) k_beam_pre(const __grid_constant__ BeamArgs b) { beam_pre_run(b); }
+__global__ void __launch_bounds__(256) k_beam_pre_b(const __grid_constant__ Batch<BeamArgs> b) { beam_pre_run(b.a[blockIdx.z]); }
 
 // IBES_solver / SolidSolverWrapper / SolidEnergies after the loads of the step are known:
 // Newton with the banded Jacobian, positions, energies; one CTA.  k_beam_pre of the same
 // step ran before it.
-__global__ void __launch_bounds__(256) k_beam(BeamArgs b) {
+__device__ __forceinline__ void beam_run(const BeamArgs& b) {
     extern __shared__ __align__(16) double smem_ws[];
     DevScalars* S = b.S;
     if (S->status != 0) return;
@@ -459,6 +461,8 @@ __global__ void __launch_bounds__(256) k_beam(BeamArgs b) {
     if (threadIdx.x == 0)
         for (int k = 4; k < 24; ++k) S->phase[k] += ph[k];
 }
+__global__ void __launch_bounds__(256) k_beam(const __grid_constant__ BeamArgs b) { beam_run(b); }
+__global__ void __launch_bounds__(256) k_beam_b(const __grid_constant__ Batch<BeamArgs> b) { beam_run(b.a[blockIdx.z]); }
 
 // integrate_position (integrate_position.f90:14-44) by one thread: the four running sums in the
 // reference's order and the positions and velocities of the motion mo.
@@ -515,18 +519,19 @@ static size_t beam_smem_bytes(int ns, int mask) {
     return bytes;
 }
 void launch_beam(const BeamArgs& b, cudaStream_t st) {
-    k_beam<<<1, 256, beam_smem_bytes(b.ns, b.use_smem), st>>>(b);
+    launch_b(k_beam, k_beam_b, dim3(1), dim3(256), beam_smem_bytes(b.ns, b.use_smem), st, false, b);
 }
 void launch_beam_pre(const BeamArgs& b, cudaStream_t st) {
-    k_beam_pre<<<1, 256, beam_smem_bytes(b.ns, b.use_smem), st>>>(b);
+    launch_b(k_beam_pre, k_beam_pre_b, dim3(1), dim3(256), beam_smem_bytes(b.ns, b.use_smem), st, false, b);
 }
 // The dynamic shared-memory limit of a kernel is one setting per function, shared by every
 // context of the process: it is only ever raised, to the largest size any context needs.
-static bool raise_smem_limit(const void* fn, size_t bytes, size_t* current) {
+static bool raise_smem_limit(const void* fn, const void* fn_b, size_t bytes, size_t* current) {
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
     if (bytes <= *current) return true;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    for (const void* f : {fn, fn_b})
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
     *current = bytes;
     return true;
 }
@@ -536,7 +541,7 @@ static size_t g_pre_smem = 0, g_beam_smem = 0;
 int beam_pre_smem_setup(int ns) {
     const size_t bytes = beam_part_bytes(ns, 2);
     if (bytes > 216 * 1024) return 0;
-    return raise_smem_limit((const void*)k_beam_pre, bytes, &g_pre_smem) ? 4 : 0;
+    return raise_smem_limit((const void*)k_beam_pre, (const void*)k_beam_pre_b, bytes, &g_pre_smem) ? 4 : 0;
 }
 // Shared-memory placement of the beam workspace: parts taken in beam_part_at order (scratch,
 // LU factor, rest of the factor, FP64 vectors, band), each one kept when it still fits beside
@@ -558,7 +563,7 @@ int beam_smem_setup(int ns) {
         const size_t pb = beam_part_bytes(ns, part);
         if (bytes + pb <= budget) { mask |= 1 << part; bytes += pb; }
     }
-    if (mask && !raise_smem_limit((const void*)k_beam, bytes, &g_beam_smem)) mask = 0;
+    if (mask && !raise_smem_limit((const void*)k_beam, (const void*)k_beam_b, bytes, &g_beam_smem)) mask = 0;
     return mask;
 }
 void launch_init_beam(const BeamArgs& b, cudaStream_t st) { k_init_beam<<<1, 256, 0, st>>>(b); }

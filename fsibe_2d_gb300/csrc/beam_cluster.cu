@@ -283,7 +283,7 @@ __device__ __forceinline__ int newton_pass(int iter, int pass, const float* cm, 
 // k_forces lets it start early (pdl_trigger): the set-up that reads only what earlier kernels
 // wrote (the beam state, the predictor's output, the stored inverse rows) runs before its
 // pdl_wait, which precedes every read of the forces' loads and of the status.
-__global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
+__device__ __forceinline__ void beam_cl_run(const BeamArgs& b) {
     extern __shared__ __align__(16) unsigned char cl_smem[];
     DevScalars* S = b.S;
     const unsigned rank = cl_rank(), R = cl_nrank();
@@ -868,6 +868,8 @@ __global__ void __launch_bounds__(256, 1) k_beam_cl(BeamArgs b) {
     if (tid == 0)
         for (int k = 4; k < 28; ++k) S->phase[k] += ph[k];
 }
+__global__ void __launch_bounds__(256, 1) k_beam_cl(const __grid_constant__ BeamArgs b) { beam_cl_run(b); }
+__global__ void __launch_bounds__(256, 1) k_beam_cl_b(const __grid_constant__ Batch<BeamArgs> b) { beam_cl_run(b.a[blockIdx.z]); }
 
 // ---- host side ------------------------------------------------------------------------
 // Floats of the global copy of M^-1 (R slices of rmax rows) and ints of its row exponents.
@@ -900,10 +902,12 @@ int beam_cluster_setup(int ns, int want, size_t* smem_out, int* big_out) {
             cl_layout(ns, R, Y, big != 0);
             if (Y.total + fa.sharedSizeBytes > (size_t)optin) continue;
             if (Y.total > cur) {
-                if (cudaFuncSetAttribute((const void*)k_beam_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Y.total) != cudaSuccess) continue;
+                if (cudaFuncSetAttribute((const void*)k_beam_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Y.total) != cudaSuccess ||
+                    cudaFuncSetAttribute((const void*)k_beam_cl_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Y.total) != cudaSuccess) continue;
                 cur = Y.total;
             }
-            if (R > 8 && cudaFuncSetAttribute((const void*)k_beam_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) continue;
+            if (R > 8 && (cudaFuncSetAttribute((const void*)k_beam_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+                          cudaFuncSetAttribute((const void*)k_beam_cl_b, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) continue;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(R);
             cfg.blockDim = dim3(256);
@@ -959,7 +963,11 @@ void launch_beam_cluster(const BeamArgs& b, int R, size_t smem, cudaStream_t st,
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, k_beam_cl, b);
+    if (!g_batch) { cudaLaunchKernelEx(&cfg, k_beam_cl, b); return; }
+    launch_batched<BeamArgs>((const void*)k_beam_cl, k_beam_cl_b, dim3(R), dim3(256), smem, pdl, b, [&](dim3 gz, const Batch<BeamArgs>& ba) {
+        cfg.gridDim = gz;
+        return cudaLaunchKernelEx(&cfg, k_beam_cl_b, ba);
+    });
 }
 
 }  // namespace fsibe

@@ -11,7 +11,9 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <cstring>
 #include <type_traits>
+#include <vector>
 
 #include "../../include/fsibe.h"
 
@@ -40,6 +42,52 @@ inline cudaError_t launch_k(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaSt
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, k, static_cast<A&&>(args)...);
+}
+
+// Runs of one shape advanced together (ensembles): one launch of a kernel for up to kBatch of them, the
+// z-th layer of its grid with the z-th run's arguments.  A kernel NAME(A) has the form NAME_b(Batch<A>);
+// the arguments stay in the launch's parameters, whose constant bank a layer's index addresses as a
+// single run's are.
+constexpr int kBatch = 16;
+template <typename A> struct Batch { A a[kBatch]; };
+// While g_batch is set, this thread's launches of a step are recorded instead of made, or, once group
+// names the records of several runs, made for all of them at the recording run's places in its streams.
+struct BatchRec {
+    struct Item { const void* k; bool batched; unsigned g[3], b[3]; size_t smem; bool pdl; std::vector<unsigned char> args; };
+    std::vector<Item> items;
+    const std::vector<BatchRec>* group = nullptr;
+    size_t next = 0;
+    bool like(const BatchRec& o) const {
+        if (items.size() != o.items.size()) return false;
+        for (size_t i = 0; i < items.size(); ++i) {
+            const Item &p = items[i], &q = o.items[i];
+            if (p.k != q.k || !p.batched || p.smem != q.smem || p.pdl != q.pdl || p.args.size() != q.args.size()) return false;
+            for (int d = 0; d < 3; ++d) if (p.g[d] != q.g[d] || p.b[d] != q.b[d]) return false;
+        }
+        return true;
+    }
+};
+inline thread_local BatchRec* g_batch = nullptr;
+template <typename A, typename L>
+inline cudaError_t launch_batched(const void* k, void (*kb)(Batch<A>), dim3 g, dim3 b, size_t smem, bool pdl, const A& a, L&& launch) {
+    BatchRec& r = *g_batch;
+    if (!r.group) {
+        const unsigned char* p = reinterpret_cast<const unsigned char*>(&a);
+        r.items.push_back({k, kb != nullptr, {g.x, g.y, g.z}, {b.x, b.y, b.z}, smem, pdl, {p, p + sizeof(A)}});
+        return cudaSuccess;
+    }
+    Batch<A> ba;
+    std::memset((void*)&ba, 0, sizeof(ba));
+    for (size_t i = 0; i < r.group->size(); ++i) std::memcpy((void*)&ba.a[i], (*r.group)[i].items[r.next].args.data(), sizeof(A));
+    ++r.next;
+    g.z = (unsigned)r.group->size();
+    return launch(g, ba);
+}
+template <typename A>
+inline cudaError_t launch_b(void (*k)(A), void (*kb)(Batch<A>), dim3 g, dim3 b, size_t smem, cudaStream_t st, bool pdl, const A& a) {
+    if (!g_batch) return launch_k(k, g, b, smem, st, pdl, a);
+    return launch_batched<A>((const void*)k, kb, g, b, smem, pdl, a,
+                             [&](dim3 gz, const Batch<A>& ba) { return launch_k(kb, gz, b, smem, st, pdl, ba); });
 }
 
 template <typename R> struct C2T;

@@ -619,7 +619,7 @@ template <int MB, int DEF>
 constexpr int xminb() { return MB > 0 ? MB : DEF; }
 
 template <typename R, int H, int TRV, int PART = NL_WHOLE, int MB = 0, int SPG = 0>
-__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k_nl_x(KArgs<R> a) {
+__device__ __forceinline__ void nl_x_run(const KArgs<R>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     using X = XRows<R, H, TRV>;
     if constexpr (PART == NL_ADVECT) {
@@ -635,6 +635,10 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k
         nl_x_tile<R, H, TRV, PART, SPG>(a, blockIdx.x * X::TR);
     }
 }
+template <typename R, int H, int TRV, int PART = NL_WHOLE, int MB = 0, int SPG = 0>
+__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k_nl_x(const __grid_constant__ KArgs<R> a) { nl_x_run<R, H, TRV, PART, MB, SPG>(a); }
+template <typename R, int H, int TRV, int PART = NL_WHOLE, int MB = 0, int SPG = 0>
+__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k_nl_x_b(const __grid_constant__ Batch<KArgs<R>> a) { nl_x_run<R, H, TRV, PART, MB, SPG>(a.a[blockIdx.z]); }
 
 // The sharp outflow sponge (iSponge = 10, NavierStokes.f90:103-122): per row iy, the term added
 // to the x penalization at ix in [ixmin, ixmax] is the trapezoid integral from ixmin to ix of
@@ -671,7 +675,7 @@ constexpr int nl_y_minb() {
 
 // FP32 (the FP64 form's is k_nl_y_d)
 template <int NY>
-__global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float> a) {
+__device__ __forceinline__ void nl_y_run(const KArgs<float>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     using R = float;
     constexpr int G = NY / 8;
@@ -795,16 +799,19 @@ __global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(KArgs<float>
         for (int q = 0; q < 8; ++q) dst[b][row + t + q * G] = ov[b][q];
     }
 }
+template <int NY>
+__global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y(const __grid_constant__ KArgs<float> a) { nl_y_run<NY>(a); }
+template <int NY>
+__global__ void __launch_bounds__(NY / 8, (nl_y_minb<NY>())) k_nl_y_b(const __grid_constant__ Batch<KArgs<float>> a) { nl_y_run<NY>(a.a[blockIdx.z]); }
 
 // ======================================================================================
 // K4: velocity at n+1, penalty, drag/energy reductions, vor_mean, Poisson RHS (forward-x),
 // stresses to physical space.
 // ======================================================================================
-template <typename R, int H, int TRV, int MB = 0>
 // (FP32: at most 128 registers a thread, so that two 256-thread blocks share an SM and the
 // 1024^2 grid runs in one wave; FP64 is bound by its arithmetic and keeps its registers)
-__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
-                                  (xminb<MB, (sizeof(R) == 4) ? XRows<R, H, TRV>::MINB128 : 1>())) k_press_x(KArgs<R> a) {
+template <typename R, int H, int TRV, int MB = 0>
+__device__ __forceinline__ void press_x_run(const KArgs<R>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     using X = XRows<R, H, TRV>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1046,6 +1053,12 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
         }
     }
 }
+template <typename R, int H, int TRV, int MB = 0>
+__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
+                                  (xminb<MB, (sizeof(R) == 4) ? XRows<R, H, TRV>::MINB128 : 1>())) k_press_x(const __grid_constant__ KArgs<R> a) { press_x_run<R, H, TRV, MB>(a); }
+template <typename R, int H, int TRV, int MB = 0>
+__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS,
+                                  (xminb<MB, (sizeof(R) == 4) ? XRows<R, H, TRV>::MINB128 : 1>())) k_press_x_b(const __grid_constant__ Batch<KArgs<R>> a) { press_x_run<R, H, TRV, MB>(a.a[blockIdx.z]); }
 
 // ---- k_press_x on paired rows (FP32) ---------------------------------------------------------
 // The same work as k_press_x's FP32 form (the stresses in their own kernel), with the row
@@ -1305,7 +1318,7 @@ __device__ __forceinline__ void press_y_paired(const KArgs<float>& a) {
 // K5: forward-y of the Poisson right-hand side, divergence, poisson, inverse-y -> Tq (FP32; the FP64
 // form's is k_press_y_d)
 template <int NY, int ENG = 0>
-__global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 : 1) k_press_y(KArgs<float> a) {
+__device__ __forceinline__ void press_y_run(const KArgs<float>& a) {
     using R = float;
     pdl_wait();     // the previous kernel of the stream has completed
     if constexpr (ENG == 0) {
@@ -1345,10 +1358,14 @@ __global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 :
 #pragma unroll
     for (int q = 0; q < 8; ++q) a.Tq[row + t + q * G] = qv[0][q];
 }
+template <int NY, int ENG = 0>
+__global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 : 1) k_press_y(const __grid_constant__ KArgs<float> a) { press_y_run<NY, ENG>(a); }
+template <int NY, int ENG = 0>
+__global__ void __launch_bounds__((press_y_threads<NY, ENG>()), NY >= 4096 ? 2 : 1) k_press_y_b(const __grid_constant__ Batch<KArgs<float>> a) { press_y_run<NY, ENG>(a.a[blockIdx.z]); }
 
 // K6: inverse-x of q, p = q - |u|^2/2
 template <typename R, int H, int TRV, int MB = 0>
-__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k_press_fin(KArgs<R> a) {
+__device__ __forceinline__ void press_fin_run(const KArgs<R>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     using X = XRows<R, H, TRV>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1390,6 +1407,10 @@ __global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k
         p2[m] = mk<R>(qq.x - (R)0.5 * (uu.x * uu.x + vq.x * vq.x), qq.y - (R)0.5 * (uu.y * uu.y + vq.y * vq.y));
     }
 }
+template <typename R, int H, int TRV, int MB = 0>
+__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k_press_fin(const __grid_constant__ KArgs<R> a) { press_fin_run<R, H, TRV, MB>(a); }
+template <typename R, int H, int TRV, int MB = 0>
+__global__ void __launch_bounds__(XRows<R, H, TRV>::THREADS, (xminb<MB, 1>())) k_press_fin_b(const __grid_constant__ Batch<KArgs<R>> a) { press_fin_run<R, H, TRV, MB>(a.a[blockIdx.z]); }
 
 }  // namespace fsibe
 #include "fluid_fx.cuh"
@@ -1403,12 +1424,18 @@ template <typename R>
 struct KLaunch {
     void (*k)(KArgs<R>) = nullptr;
     int threads = 0, smem = 0;
+    void (*kb)(Batch<KArgs<R>>) = nullptr;  // its form for a batch of runs, where there is one
 };
 template <typename R>
-inline KLaunch<R> klaunch(void (*k)(KArgs<R>), int threads, int smem) {
+inline KLaunch<R> klaunch(void (*k)(KArgs<R>), int threads, int smem, void (*kb)(Batch<KArgs<R>>) = nullptr) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return KLaunch<R>{k, threads, smem};
+    if (kb) cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return KLaunch<R>{k, threads, smem, kb};
 }
+// The lengths whose kernels have a form for a batch of runs: up to 1024, above which one run's launch
+// fills the GPU and the launches are not what bounds an ensemble.
+template <int N> constexpr bool batched() { return N <= 1024; }
+#define FSIBE_KB(N, ...) [] { if constexpr (batched<N>()) return &__VA_ARGS__; else return (void (*)(Batch<KArgs<R>>))nullptr; }()
 
 template <typename R>
 struct SizeKernels {
@@ -1437,7 +1464,7 @@ inline void fill_xgroups(typename SizeKernels<R>::XVariant& v) {
     using X2 = XGroups<R, H, TR, RG, 2>;
     using X3 = XGroups<R, H, TR, RG, 3>;
     v.rows = TR;
-    v.nl_x = klaunch<R>(k_nl_x_g<R, H, TR, NL_WHOLE, 0>, X3::THREADS, X3::SMEM);
+    v.nl_x = klaunch<R>(k_nl_x_g<R, H, TR, NL_WHOLE, 0>, X3::THREADS, X3::SMEM, FSIBE_KB(2 * H, k_nl_x_g_b<R, H, TR, NL_WHOLE, 0>));
     v.nl_adv = klaunch<R>(k_nl_x_g<R, H, TR, NL_ADVECT, 0>, X2::THREADS, X2::SMEM);
     v.nl_pen = klaunch<R>(k_nl_x_g<R, H, TR, NL_PENAL, 0>, X2::THREADS, X2::SMEM);
     if constexpr (SPG) {
@@ -1447,7 +1474,7 @@ inline void fill_xgroups(typename SizeKernels<R>::XVariant& v) {
         v.nl_pen_s10 = klaunch<R>(k_nl_x_g<R, H, TR, NL_PENAL, 2>, X2::THREADS, X2::SMEM);
     }
     v.stress_x = klaunch<R>(k_stress_x_g<R, H, TR>, X2::THREADS, X2::SMEM);
-    v.press_x = klaunch<R>(k_press_x_g<R, H, TR>, X3::THREADS, press_x_smem_g<R, H, TR>());
+    v.press_x = klaunch<R>(k_press_x_g<R, H, TR>, X3::THREADS, press_x_smem_g<R, H, TR>(), FSIBE_KB(2 * H, k_press_x_g_b<R, H, TR>));
 }
 
 template <typename R, int H, int TR, int MB = 0, bool SPG = false>
@@ -1456,9 +1483,9 @@ inline void fill_xvariant(typename SizeKernels<R>::XVariant& v) {
     constexpr int T = X::THREADS, S1 = (int)(TR * X::PL * sizeof(C2<R>));
     v.rows = TR;
     v.minb = MB;
-    v.press_fin = klaunch<R>(k_press_fin<R, H, TR, MB>, T, S1);
+    v.press_fin = klaunch<R>(k_press_fin<R, H, TR, MB>, T, S1, FSIBE_KB(2 * H, k_press_fin_b<R, H, TR, MB>));
     if constexpr (!step_groups<R, H>()) {
-        v.nl_x = klaunch<R>(k_nl_x<R, H, TR, NL_WHOLE, MB>, T, 3 * S1);
+        v.nl_x = klaunch<R>(k_nl_x<R, H, TR, NL_WHOLE, MB>, T, 3 * S1, FSIBE_KB(2 * H, k_nl_x_b<R, H, TR, NL_WHOLE, MB>));
         v.nl_adv = klaunch<R>(k_nl_x<R, H, TR, NL_ADVECT, MB>, T, 2 * S1);
         v.nl_pen = klaunch<R>(k_nl_x<R, H, TR, NL_PENAL, MB>, T, 2 * S1);
         if constexpr (SPG) {
@@ -1468,7 +1495,7 @@ inline void fill_xvariant(typename SizeKernels<R>::XVariant& v) {
             v.nl_pen_s10 = klaunch<R>(k_nl_x<R, H, TR, NL_PENAL, MB, 2>, T, 2 * S1);
         }
         v.stress_x = klaunch<R>(k_stress_x<R, H, TR, MB>, T, 2 * S1);
-        v.press_x = klaunch<R>(k_press_x<R, H, TR, MB>, T, 3 * S1);
+        v.press_x = klaunch<R>(k_press_x<R, H, TR, MB>, T, 3 * S1, FSIBE_KB(2 * H, k_press_x_b<R, H, TR, MB>));
     } else {
         fill_xgroups<R, H, TR, SPG>(v);
     }
@@ -1507,13 +1534,13 @@ inline void fill_size_kernels(SizeKernels<R>& k) {
         k.xp.rows = TP;
         k.xp.minb = 16;  // the marker of the paired kernel in fsibe_tile_config
         k.xp.press_x = klaunch<R>(k_press_x2<H, TP>, XPairs<H, TP>::THREADS, 3 * TP * pair_slots(H) * 16);
-        k.nl_y = klaunch<R>(k_nl_y<N>, TY, NL_Y_BUFS * SY);
-        k.press_y = klaunch<R>(k_press_y<N>, press_y_threads<N>(), std::max(2 * SY, 2 * pair_slots(N) * 16));
-        k.press_y1 = klaunch<R>(k_press_y<N, 1>, TY, 2 * SY);
+        k.nl_y = klaunch<R>(k_nl_y<N>, TY, NL_Y_BUFS * SY, FSIBE_KB(N, k_nl_y_b<N>));
+        k.press_y = klaunch<R>(k_press_y<N>, press_y_threads<N>(), std::max(2 * SY, 2 * pair_slots(N) * 16), FSIBE_KB(N, k_press_y_b<N>));
+        k.press_y1 = klaunch<R>(k_press_y<N, 1>, TY, 2 * SY, FSIBE_KB(N, k_press_y_b<N, 1>));
     } else {
         constexpr int NG = nl_y_groups<N>(), PG = press_y_groups<N>();
-        k.nl_y = klaunch<R>(k_nl_y_d<N, NG>, NG * TY, nl_y_smem_d<N, NG>());
-        k.press_y = klaunch<R>(k_press_y_d<N, PG>, PG * TY, press_y_smem_d<N, PG>());
+        k.nl_y = klaunch<R>(k_nl_y_d<N, NG>, NG * TY, nl_y_smem_d<N, NG>(), FSIBE_KB(N, k_nl_y_d_b<N, NG>));
+        k.press_y = klaunch<R>(k_press_y_d<N, PG>, PG * TY, press_y_smem_d<N, PG>(), FSIBE_KB(N, k_press_y_d_b<N, PG>));
         k.press_y1 = KLaunch<R>{};
     }
 }

@@ -29,7 +29,7 @@ template <int NY, int NG> constexpr int press_y_smem_d() { return 2 * padded_len
 
 // k_nl_y: forward y of A and B, the AB2 / Euler update, the inverse-y outputs
 template <int NY, int NG>
-__global__ void __launch_bounds__(NG * NY / 8) k_nl_y_d(KArgs<double> a) {
+__device__ __forceinline__ void nl_y_d_run(const KArgs<double>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     constexpr int G = NY / 8, T = NG * G, PLY = padded_len(NY), EPT = (NY + T - 1) / T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -111,10 +111,14 @@ __global__ void __launch_bounds__(NG * NY / 8) k_nl_y_d(KArgs<double> a) {
         for (int m = 0; m < 8; ++m) dst[gr.t + m * G] = v[m];
     }
 }
+template <int NY, int NG>
+__global__ void __launch_bounds__(NG * NY / 8) k_nl_y_d(const __grid_constant__ KArgs<double> a) { nl_y_d_run<NY, NG>(a); }
+template <int NY, int NG>
+__global__ void __launch_bounds__(NG * NY / 8) k_nl_y_d_b(const __grid_constant__ Batch<KArgs<double>> a) { nl_y_d_run<NY, NG>(a.a[blockIdx.z]); }
 
 // k_press_y: forward y of P1 and P2, divergence, Poisson divide, inverse y
 template <int NY, int NG>
-__global__ void __launch_bounds__(NG * NY / 8) k_press_y_d(KArgs<double> a) {
+__device__ __forceinline__ void press_y_d_run(const KArgs<double>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     constexpr int G = NY / 8, T = NG * G, PLY = padded_len(NY);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -148,6 +152,10 @@ __global__ void __launch_bounds__(NG * NY / 8) k_press_y_d(KArgs<double> a) {
 #pragma unroll
     for (int m = 0; m < 8; ++m) a.Tq[row + gr.t + m * G] = v[m];
 }
+template <int NY, int NG>
+__global__ void __launch_bounds__(NG * NY / 8) k_press_y_d(const __grid_constant__ KArgs<double> a) { press_y_d_run<NY, NG>(a); }
+template <int NY, int NG>
+__global__ void __launch_bounds__(NG * NY / 8) k_press_y_d_b(const __grid_constant__ Batch<KArgs<double>> a) { press_y_d_run<NY, NG>(a.a[blockIdx.z]); }
 
 // ---- x pass (both forms) -----------------------------------------------------------------------
 // A block of TR rows and NF fields, RG rows of every field at a time: group f RG + q transforms the
@@ -320,7 +328,7 @@ __device__ __forceinline__ void nl_x_tile_g(const KArgs<R>& a, const int iy0, un
 }
 
 template <typename R, int H, int TR, int PART, int SPG>
-__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), nl_x_fields<PART, SPG>()>::THREADS) k_nl_x_g(KArgs<R> a) {
+__device__ __forceinline__ void nl_x_g_run(const KArgs<R>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     constexpr int NF = nl_x_fields<PART, SPG>(), RG = xgroups_rg<H>(TR);
     __shared__ unsigned slots[NF * RG * fx_slots<H / 8>()];
@@ -336,6 +344,10 @@ __global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), nl_x_fiel
         nl_x_tile_g<R, H, TR, RG, PART, SPG>(a, blockIdx.x * TR, slots);
     }
 }
+template <typename R, int H, int TR, int PART, int SPG>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), nl_x_fields<PART, SPG>()>::THREADS) k_nl_x_g(const __grid_constant__ KArgs<R> a) { nl_x_g_run<R, H, TR, PART, SPG>(a); }
+template <typename R, int H, int TR, int PART, int SPG>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), nl_x_fields<PART, SPG>()>::THREADS) k_nl_x_g_b(const __grid_constant__ Batch<KArgs<R>> a) { nl_x_g_run<R, H, TR, PART, SPG>(a.a[blockIdx.z]); }
 
 // The viscous stresses (NavierStokes.f90:354-370: 2 nu d2psi/dxdy, nu (d2psi/dy2 - d2psi/dx2))
 // to physical space, beside k_press_x on another stream: only GetForces reads them.  With
@@ -387,7 +399,7 @@ template <typename R, int H, int TR> constexpr int press_x_smem_g() {
 
 // k_press_x: u, v and omega, the penalization, the sums, vor_mean, the pressure's right-hand side
 template <typename R, int H, int TR>
-__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), 3>::THREADS) k_press_x_g(KArgs<R> a) {
+__device__ __forceinline__ void press_x_g_run(const KArgs<R>& a) {
     pdl_wait();     // the previous kernel of the stream has completed
     constexpr int RG = xgroups_rg<H>(TR);
     using X = XGroups<R, H, TR, RG, 3>;
@@ -545,5 +557,9 @@ __global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), 3>::THREA
         stress_tile_g<R, H, TR, RG>(a, iy0, slots);
     }
 }
+template <typename R, int H, int TR>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), 3>::THREADS) k_press_x_g(const __grid_constant__ KArgs<R> a) { press_x_g_run<R, H, TR>(a); }
+template <typename R, int H, int TR>
+__global__ void __launch_bounds__(XGroups<R, H, TR, xgroups_rg<H>(TR), 3>::THREADS) k_press_x_g_b(const __grid_constant__ Batch<KArgs<R>> a) { press_x_g_run<R, H, TR>(a.a[blockIdx.z]); }
 
 }  // namespace fsibe

@@ -4,6 +4,7 @@
 //     interpolation (Interpolation.f90:6-101).
 // Built with -fmad=false so the geometric tests of the mask see the same roundings as the
 // reference's separate multiply/add.
+#include <algorithm>
 #include <math.h>
 
 #include "solid.cuh"
@@ -37,7 +38,8 @@ __device__ __forceinline__ void clip_box(int* bx, int nx, int ny) {
 // hinge's box, then the sharp end and the dots.  After one barrier warp 1 finishes the hinge.
 // The bounding box of all primitives is reduced with atomics; the last block publishes it with
 // its union with the previous step's box and resets the accumulator.
-__global__ void __launch_bounds__(128) k_mask_prep(MaskArgs a, double gerf) {
+__device__ __forceinline__ void mask_prep_run(const MaskArgs& a) {
+    const double gerf = a.gerf;
     pdl_wait();     // the previous kernel of the stream has completed
     if (a.until_full && a.S->time >= a.T_fullspeed) return;
     __shared__ double ang2[32];
@@ -226,6 +228,8 @@ __global__ void __launch_bounds__(128) k_mask_prep(MaskArgs a, double gerf) {
         }
     }
 }
+__global__ void __launch_bounds__(128) k_mask_prep(const __grid_constant__ MaskArgs a) { mask_prep_run(a); }
+__global__ void __launch_bounds__(128) k_mask_prep_b(const __grid_constant__ Batch<MaskArgs> a) { mask_prep_run(a.a[blockIdx.z]); }
 
 // Raster tiles: 8 x 4 cells, one block of MASK_WARPS warps each; blocks stride over the tiles
 // of the union of this step's and the previous step's primitive box, so every other cell keeps
@@ -449,7 +453,8 @@ __device__ __forceinline__ void mask_finish(const MaskArgs& a, double gerf, int 
 // combines the partial folds after the segments (then applies the sharp end) and after the
 // hinges and dots.
 // The FP32 form's (the FP64 form's is k_mask_raster_d).
-__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_f(MaskArgs a, double gerf) {
+__device__ __forceinline__ void mask_raster_f_run(const MaskArgs& a) {
+    const double gerf = a.gerf;
     pdl_wait();     // the previous kernel of the stream has completed
     if (a.until_full && a.S->time >= a.T_fullspeed) return;
     using R = float;
@@ -575,6 +580,8 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_f(MaskArgs a, d
         }
     }
 }
+__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_f(const __grid_constant__ MaskArgs a) { mask_raster_f_run(a); }
+__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_f_b(const __grid_constant__ Batch<MaskArgs> a) { mask_raster_f_run(a.a[blockIdx.z]); }
 
 // The FP64 form's raster: k_mask_raster_f's tiles, with the reference's FP64 tests.  FP64 issue bounds
 // it (64 cycles a warp instruction, few tiles), so the warps keep the winning primitive by its
@@ -583,7 +590,8 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_f(MaskArgs a, d
 // Measured (GB300; before, SmoothStep and the velocity for every primitive that beat the fold so far):
 // 256^2, ns = 64 36.6 -> 26.4 us (the step 165 -> 156); 64^2, ns = 16 31.0 -> 30.5; 512 x 256 with walls and
 // a cylinder, where every cell was drawn each step, 43.8 -> 24.5.
-__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_d(MaskArgs a, double gerf) {
+__device__ __forceinline__ void mask_raster_d_run(const MaskArgs& a) {
+    const double gerf = a.gerf;
     pdl_wait();     // the previous kernel of the stream has completed
     if (a.until_full && a.S->time >= a.T_fullspeed) return;
     __shared__ Prim sp[MASK_WARPS][32];
@@ -702,6 +710,8 @@ __global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_d(MaskArgs a, d
         if (warp == 0) write();
     }
 }
+__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_d(const __grid_constant__ MaskArgs a) { mask_raster_d_run(a); }
+__global__ void __launch_bounds__(32 * MASK_WARPS) k_mask_raster_d_b(const __grid_constant__ Batch<MaskArgs> a) { mask_raster_d_run(a.a[blockIdx.z]); }
 
 // ===================================================================================
 // Forces: phi4* delta interpolation of p and the viscous stresses at the beam surface
@@ -724,43 +734,52 @@ __device__ __forceinline__ double fld(const void* f, int fp32, size_t k) {
     return fp32 ? (double)reinterpret_cast<const float*>(f)[k] : reinterpret_cast<const double*>(f)[k];
 }
 
-// One block per beam node.  The trigonometric values are evaluated once per block; the six
-// 9 x 9 interpolation sums run as 54 nine-term partial sums; the force integral of all nodes
-// is a block reduction in the last block.  Summation orders differ from the reference's
-// sequential loops (relative differences of a few ulps).
-// The geometry of the interpolation at node n (BeamForces.f90:105-124): the trigonometric
-// values, the four surface points' cells and their phi4* weights.  It depends only on the beam
-// state, so the step computes it beside the fluid kernels; k_forces then reads it.
+// The geometry of the interpolation at a node (BeamForces.f90:105-124): the trigonometric values, the
+// four surface points' cells and their phi4* weights.  It depends only on the beam state, so the step
+// computes it beside the fluid kernels; k_forces then reads it.
 // Per node in a.geo: trig[4], dl[4][18]; in a.gij: ij[4][2].
-__global__ void __launch_bounds__(128) k_forces_geo(ForceArgs a, double dxi, double dyi) {
-    const int n = blockIdx.x;
-    __shared__ double dl[4][18];
-    __shared__ int ij[4][2];
-    __shared__ double trig[4];  // sin, cos of theta + alpha and of twice it
-    __shared__ double px[4], py[4];
+//
+// A block takes NODES nodes, and each offset of a weight from its point's cell, nine in x and in y, for
+// all of the block's points is 8 NODES lanes: the FP64 pipe is what bounds this kernel (an instruction
+// holds it 64 cycles whatever its lanes do), the weights of one offset lie on the same branches of phi4*,
+// and three of the nine are zero.  One run takes a node a block, for the latency (two warps of weights on
+// two SMSPs); a batch four, a warp an offset: 1024 nodes (16 runs of 64) in 19 us, a node a block 31.
+constexpr int GEO_BATCH = 4;
+template <int NODES> constexpr int geo_threads() { return (72 * NODES + 31) / 32 * 32; }
+template <int NODES>
+__device__ __forceinline__ void forces_geo_run(const ForceArgs& a) {
+    constexpr int GEO_PTS = 4 * NODES, T = geo_threads<NODES>();
+    const double dxi = a.dxi, dyi = a.dyi;
+    const int n0 = blockIdx.x * NODES, nn = min(NODES, a.ns - n0);
+    __shared__ double dl[GEO_PTS][18];
+    __shared__ int ij[GEO_PTS][2];
+    __shared__ double trig[NODES][4];  // sin, cos of theta + alpha and of twice it
+    __shared__ double px[GEO_PTS], py[GEO_PTS];
     // the two sincos on two warps (SMSPs)
-    if (threadIdx.x == 0 || threadIdx.x == 32) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 2 && lane < nn) {
+        const int n = n0 + lane;
         const double thn = a.th[n] + motion_at(a.mo, a.S->time).alpha;  // mouvement(time)
         double sv, cv;
-        if (threadIdx.x == 0) {
+        if (warp == 0) {
             sincos(thn, &sv, &cv);
-            trig[0] = sv; trig[1] = cv;
+            trig[lane][0] = sv; trig[lane][1] = cv;
             const double mx = fmax(a.dy, a.dx);
             const double off = a.t_beam + a.N_smooth * mx;
             const double off1 = a.t_beam - 0.0 * a.N_smooth * mx;
             const double x = a.x[n], y = a.y[n];
-            px[0] = x - off1 * sv; py[0] = y + off1 * cv;
-            px[1] = x + off1 * sv; py[1] = y - off1 * cv;
-            px[2] = x - off * sv; py[2] = y + off * cv;
-            px[3] = x + off * sv; py[3] = y - off * cv;
+            px[4 * lane + 0] = x - off1 * sv; py[4 * lane + 0] = y + off1 * cv;
+            px[4 * lane + 1] = x + off1 * sv; py[4 * lane + 1] = y - off1 * cv;
+            px[4 * lane + 2] = x - off * sv; py[4 * lane + 2] = y + off * cv;
+            px[4 * lane + 3] = x + off * sv; py[4 * lane + 3] = y - off * cv;
         } else {
             sincos(2.0 * thn, &sv, &cv);
-            trig[2] = sv; trig[3] = cv;
+            trig[lane][2] = sv; trig[lane][3] = cv;
         }
     }
     __syncthreads();
     const double x2 = a.xl - a.dx, y2 = a.yl - a.dy;
-    if (threadIdx.x < 4) {
+    if (threadIdx.x < 4 * nn) {
         const int p = threadIdx.x;
         const double xt = px[p], yt = py[p];
         const int i = (int)div_cr((xt - 0.0), dxi, a.rdxi), j = (int)div_cr((yt - 0.0), dyi, a.rdyi);
@@ -769,24 +788,36 @@ __global__ void __launch_bounds__(128) k_forces_geo(ForceArgs a, double dxi, dou
             set_status(a.S, FSIBE_ERR_INTERP_OOB);
     }
     __syncthreads();
-    if (threadIdx.x < 72) {
-        const int p = threadIdx.x / 18, d = threadIdx.x % 18;
-        if (d < 9) {
-            const double xl_ = (double)(ij[p][0] - 4 + d) * dxi + 0.0;
-            dl[p][d] = delta_phi4star(fabs(xl_ - px[p]), dxi, a.rdxi, a.pi);
-        } else {
-            const double yl_ = (double)(ij[p][1] - 4 + d - 9) * dyi + 0.0;
-            dl[p][d] = delta_phi4star(fabs(yl_ - py[p]), dyi, a.rdyi, a.pi);
+    {
+        const int d = threadIdx.x / (2 * GEO_PTS), q = threadIdx.x % (2 * GEO_PTS), p = q % GEO_PTS;
+        if (d < 9 && p < 4 * nn) {
+            if (q < GEO_PTS) {
+                const double xl_ = (double)(ij[p][0] - 4 + d) * dxi + 0.0;
+                dl[p][d] = delta_phi4star(fabs(xl_ - px[p]), dxi, a.rdxi, a.pi);
+            } else {
+                const double yl_ = (double)(ij[p][1] - 4 + d) * dyi + 0.0;
+                dl[p][9 + d] = delta_phi4star(fabs(yl_ - py[p]), dyi, a.rdyi, a.pi);
+            }
         }
     }
     __syncthreads();
-    double* g = a.geo + (size_t)n * 76;
-    if (threadIdx.x < 4) g[threadIdx.x] = trig[threadIdx.x];
-    if (threadIdx.x < 72) g[4 + threadIdx.x] = dl[threadIdx.x / 18][threadIdx.x % 18];
-    if (threadIdx.x < 8) a.gij[(size_t)n * 8 + threadIdx.x] = ij[threadIdx.x / 2][threadIdx.x % 2];
+    double* g = a.geo + (size_t)n0 * 76;
+    for (int e = threadIdx.x; e < 76 * nn; e += T) {
+        const int q = e / 76, r = e % 76;
+        g[e] = r < 4 ? trig[q][r] : dl[4 * q + (r - 4) / 18][(r - 4) % 18];
+    }
+    for (int e = threadIdx.x; e < 8 * nn; e += T) a.gij[(size_t)n0 * 8 + e] = ij[e / 2][e % 2];
+}
+__global__ void __launch_bounds__(geo_threads<1>()) k_forces_geo(const __grid_constant__ ForceArgs a) { forces_geo_run<1>(a); }
+__global__ void __launch_bounds__(geo_threads<GEO_BATCH>()) k_forces_geo_b(const __grid_constant__ Batch<ForceArgs> a) {
+    forces_geo_run<GEO_BATCH>(a.a[blockIdx.z]);
 }
 
-__global__ void __launch_bounds__(128) k_forces(ForceArgs a, double dxi, double dyi) {
+// One block per beam node.  The six 9 x 9 interpolation sums run as 54 nine-term partial sums; the force
+// integral of all nodes is a block reduction in the last block.  Summation orders differ from the
+// reference's sequential loops (relative differences of a few ulps).
+__device__ __forceinline__ void forces_run(const ForceArgs& a) {
+    const double dxi = a.dxi, dyi = a.dyi;
     pdl_wait();     // the previous kernel of the stream has completed
     pdl_trigger();  // the beam kernel may start its set-up (it waits for this kernel's results)
     const int n = blockIdx.x;
@@ -883,12 +914,14 @@ __global__ void __launch_bounds__(128) k_forces(ForceArgs a, double dxi, double 
         }
     }
 }
+__global__ void __launch_bounds__(128) k_forces(const __grid_constant__ ForceArgs a) { forces_run(a); }
+__global__ void __launch_bounds__(128) k_forces_b(const __grid_constant__ Batch<ForceArgs> a) { forces_run(a.a[blockIdx.z]); }
 
 // ===================================================================================
 // Host launchers
 // ===================================================================================
-void launch_mask_prep(const MaskArgs& a, double gerf, cudaStream_t st, bool pdl) {
-    launch_k(k_mask_prep, dim3((a.ns + 3 + 31) / 32), dim3(128), 0, st, pdl, a, gerf);
+void launch_mask_prep(const MaskArgs& a, cudaStream_t st, bool pdl) {
+    launch_b(k_mask_prep, k_mask_prep_b, dim3((a.ns + 3 + 31) / 32), dim3(128), 0, st, pdl, a);
 }
 // The walls (create_mask.f90:30-54: each wall row assigned its SmoothStep) and the leading-edge
 // cylinder (:66-68, DrawADot with the strict > rule), and the frame of iSponge = 22
@@ -991,11 +1024,19 @@ void launch_sponge_mask(const StaticMaskArgs& a, double gerf, cudaStream_t st) {
     else k_sponge_mask<double><<<1024, 256, 0, st>>>(a, gerf);
 }
 
-void launch_mask(const MaskArgs& a, double gerf, bool fp32, cudaStream_t st, bool pdl) {
-    // four-warp blocks, two per SM: a tile's primitives over the four SMSPs of an SM
-    const int blocks = 2 * a.nsm;
-    if (fp32) launch_k(k_mask_raster_f, dim3(blocks), dim3(32 * MASK_WARPS), 0, st, pdl, a, gerf);
-    else launch_k(k_mask_raster_d, dim3(blocks), dim3(32 * MASK_WARPS), 0, st, pdl, a, gerf);
+void launch_mask(const MaskArgs& a, bool fp32, cudaStream_t st, bool pdl) {
+    // four-warp blocks, two per SM: a tile's primitives over the four SMSPs of an SM.  A batch of n runs
+    // takes eight blocks an SM over all of them: more only start and leave (16 runs of 256^2, 304 blocks
+    // each: 28 us, so 22).
+    const unsigned blocks = 2 * a.nsm;
+    const dim3 th(32 * MASK_WARPS);
+    auto k = fp32 ? k_mask_raster_f : k_mask_raster_d;
+    auto kb = fp32 ? k_mask_raster_f_b : k_mask_raster_d_b;
+    if (!g_batch) { launch_k(k, dim3(blocks), th, 0, st, pdl, a); return; }
+    launch_batched<MaskArgs>((const void*)k, kb, dim3(blocks), th, 0, pdl, a, [&](dim3 g, const Batch<MaskArgs>& ba) {
+        g.x = std::min(blocks, 4 * blocks / g.z);
+        return launch_k(kb, g, th, 0, st, pdl, ba);
+    });
 }
 
 // BeamSurfaceIntegral (BeamForces.f90:306-509)
@@ -1124,11 +1165,14 @@ void launch_surface_integral(const ForceArgs& a, const SurfArgs& s, double dxi, 
     k_surface_integral<<<1, 256, 0, st>>>(a, s, dxi, dyi, time);
 }
 
-void launch_forces_geo(const ForceArgs& a, double dxi, double dyi, cudaStream_t st) {
-    k_forces_geo<<<a.ns, 128, 0, st>>>(a, dxi, dyi);
+void launch_forces_geo(const ForceArgs& a, cudaStream_t st) {
+    if (!g_batch) { launch_k(k_forces_geo, dim3(a.ns), dim3(geo_threads<1>()), 0, st, false, a); return; }
+    const dim3 th(geo_threads<GEO_BATCH>());
+    launch_batched<ForceArgs>((const void*)k_forces_geo, k_forces_geo_b, dim3((a.ns + GEO_BATCH - 1) / GEO_BATCH), th, 0, false, a,
+                              [&](dim3 g, const Batch<ForceArgs>& ba) { return launch_k(k_forces_geo_b, g, th, 0, st, false, ba); });
 }
-void launch_forces(const ForceArgs& a, double dxi, double dyi, cudaStream_t st, bool pdl) {
-    launch_k(k_forces, dim3(a.ns), dim3(128), 0, st, pdl, a, dxi, dyi);
+void launch_forces(const ForceArgs& a, cudaStream_t st, bool pdl) {
+    launch_b(k_forces, k_forces_b, dim3(a.ns), dim3(128), 0, st, pdl, a);
 }
 
 }  // namespace fsibe

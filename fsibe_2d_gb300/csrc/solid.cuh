@@ -92,6 +92,7 @@ struct MaskArgs {
                      // redraw for the velocity sponge and the frame, time_step.f90:187)
     int nx, ny, ns, sharp_trailing, sharp;
     double dx, dy, ds, t_beam, N_smooth, eps, pi, angle_deg;
+    double gerf;   // the smoothing step's constant
     const double *x, *y, *vx, *vy, *th;
     Prim* prims;
     PrimG* primg;  // the raster's FP32 data of prims (k_mask_prep)
@@ -156,6 +157,7 @@ struct ForceArgs {
     DevScalars* S;
     int nx, ny, ns, viscous;
     double xl, yl, dx, dy, ds, t_beam, N_smooth, pi, angle_deg, t_release, tau;
+    double dxi, dyi;    // the interpolation's spacings
     double rdxi, rdyi;  // RN(1/dxi), RN(1/dyi) (host)
     MotionArgs mo;      // the leading edge's motion (alpha of the time)
     double* geo;     // per node: trig[4], phi4* weights dl[4][18] (k_forces_geo)
