@@ -25,7 +25,8 @@
 // pass.  A warp evaluates one of the two node equations (they alternate by row, and a warp of both ran
 // the two codes one after the other), and the passes end when their corrections no longer change the
 // iterate (newton_pass).  Measured (us, before -> after both, and rows of the band on different banks):
-// ns = 64 55 -> 46, 128 (heaving) 74 -> 59, 256 84 -> 62, 1024 333 -> 250.
+// ns = 64 55 -> 46, 128 (heaving) 74 -> 59, 256 84 -> 62, 1024 333 -> 250 (and 212 with more loads in
+// flight in the product).
 // Large beams (ns >= 512: M^-1's rows and the factor exceed a CTA's shared memory) run the
 // same algorithm with both in global memory, where they stay L2-resident: each CTA reads its
 // rows of M^-1 from its slice of the persistent copy, and factors its own copy of the band
@@ -570,16 +571,33 @@ __device__ __forceinline__ void beam_cl_run(const BeamArgs& b) {
                         float acc[8];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-                        for (int q = lane; q < (mld >> 2); q += 32) {
-                            const float4 v = y4[q];
+                        auto add = [&](const float4& v, const float4 (&m)[8]) {
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                const float4 m = mr[j][q];
-                                acc[j] = __fmaf_rn(m.x, v.x, acc[j]);
-                                acc[j] = __fmaf_rn(m.y, v.y, acc[j]);
-                                acc[j] = __fmaf_rn(m.z, v.z, acc[j]);
-                                acc[j] = __fmaf_rn(m.w, v.w, acc[j]);
+                                acc[j] = __fmaf_rn(m[j].x, v.x, acc[j]);
+                                acc[j] = __fmaf_rn(m[j].y, v.y, acc[j]);
+                                acc[j] = __fmaf_rn(m[j].z, v.z, acc[j]);
+                                acc[j] = __fmaf_rn(m[j].w, v.w, acc[j]);
                             }
+                        };
+                        const int nq = mld >> 2;
+                        int q = lane;
+                        if (big) {
+                            // rows in L2: what bounds the product is how many loads are in flight, so
+                            // twice eight a lane (ns = 1024: 30k cycles a pass with eight, 20k with sixteen)
+                            for (; q + 32 < nq; q += 64) {
+                                float4 m0[8], m1[8];
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) { m0[j] = __ldcg(mr[j] + q); m1[j] = __ldcg(mr[j] + q + 32); }
+                                add(y4[q], m0);
+                                add(y4[q + 32], m1);
+                            }
+                        }
+                        for (; q < nq; q += 32) {
+                            float4 m0[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) m0[j] = mr[j][q];
+                            add(y4[q], m0);
                         }
                         {
                             const bool up = (lane & 16) != 0;
