@@ -13,7 +13,12 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "adjoint.cuh"
 #include "fluid.cuh"
@@ -1223,13 +1228,54 @@ static void free_graph(fsibe_ctx* c) {
 }
 
 // ---- transfers ----------------------------------------------------------------------
+// A copy to host memory that the caller may just have allocated.  From 32 MB on a C library's malloc maps
+// each allocation anew, and the first touch of its pages, by the copy, costs as much as the copy or
+// several times that (three fields of 2048^2, 100 MB, took 9 or 37 ms, from one call to the next): so the
+// pages of such a destination are made present first, by several threads and beside what the stream
+// still runs (9 to 10 ms in every call; a 4096^2 field 6.5 -> 5.3).  Smaller destinations are mostly
+// memory used before, where asking for the pages only costs (4 MB: 223 -> 233 us a pair of
+// transforms).  MADV_POPULATE_WRITE leaves the contents alone and reports what it cannot populate (memory
+// that is not pageable or not the caller's, a kernel without it); the copy then finds the pages as they
+// are.
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+static void populate_pages(void* dst, size_t bytes) {
+    constexpr size_t kLeast = (size_t)32 << 20, kSlice = (size_t)2 << 20;
+    if (bytes < kLeast) return;
+    const uintptr_t pg = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = ((uintptr_t)dst + pg - 1) / pg * pg, hi = ((uintptr_t)dst + bytes) / pg * pg;
+    if (hi <= lo) return;
+    size_t n = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), (hi - lo) / kSlice});
+    n = std::max<size_t>(n, 1);
+    const uintptr_t pages = (hi - lo) / pg;
+    auto part = [=](size_t k) {
+        const uintptr_t a = lo + pages * k / n * pg, b = lo + pages * (k + 1) / n * pg;
+        if (b > a) (void)madvise((void*)a, b - a, MADV_POPULATE_WRITE);
+    };
+    std::thread th[8];
+    size_t started = 0;
+    try {
+        for (; started + 1 < n; ++started) th[started] = std::thread(part, started);
+    } catch (const std::system_error&) {
+        // no more threads: the rest of the pages here
+    }
+    for (size_t k = started; k < n; ++k) part(k);
+    for (size_t k = 0; k < started; ++k) th[k].join();
+}
+
+static cudaError_t copy_out(fsibe_ctx* c, void* host, const void* dev, size_t bytes) {
+    populate_pages(host, bytes);
+    return cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream);
+}
+
 static int to_host(fsibe_ctx* c, const void* dev, size_t n, double* host, const double* offset = nullptr) {
     if (c->fp32) {
         k_convert<float><<<256, 256, 0, c->stream>>>(reinterpret_cast<const float*>(dev), c->dscratch, n, offset);
         CKL(c);
-        CK(c, cudaMemcpyAsync(host, c->dscratch, n * 8, cudaMemcpyDeviceToHost, c->stream));
+        CK(c, copy_out(c, host, c->dscratch, n * 8));
     } else {
-        CK(c, cudaMemcpyAsync(host, dev, n * 8, cudaMemcpyDeviceToHost, c->stream));
+        CK(c, copy_out(c, host, dev, n * 8));
     }
     CK(c, cudaStreamSynchronize(c->stream));
     return FSIBE_OK;
@@ -1251,7 +1297,7 @@ static int spec_to_packed(fsibe_ctx* c, const void* H, double* host_fk, const vo
     if (c->fp32) k_pack<float><<<c->g.hx, 256, 0, c->stream>>>(reinterpret_cast<const float2*>(H), reinterpret_cast<const float2*>(Hlo), c->dscratch, c->g.nx, c->g.ny);
     else k_pack<double><<<c->g.hx, 256, 0, c->stream>>>(reinterpret_cast<const double2*>(H), nullptr, c->dscratch, c->g.nx, c->g.ny);
     CKL(c);
-    CK(c, cudaMemcpyAsync(host_fk, c->dscratch, 8 * (size_t)c->g.nx * c->g.ny, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, copy_out(c, host_fk, c->dscratch, 8 * (size_t)c->g.nx * c->g.ny));
     CK(c, cudaStreamSynchronize(c->stream));
     return FSIBE_OK;
 }
@@ -1428,7 +1474,7 @@ static int pressure_snapshot_t(fsibe_ctx* c, double time, double* host_out) {
     double* out = c->dscratch;  // nx ny doubles
     k_snap_fin<R><<<grid, 256, 0, c->stream>>>(pw, pu, pv, out, NN);
     CKL(c);
-    CK(c, cudaMemcpyAsync(host_out, out, 8 * NN, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, copy_out(c, host_out, out, 8 * NN));
     CK(c, cudaStreamSynchronize(c->stream));
     return FSIBE_OK;
 }
@@ -1899,7 +1945,7 @@ static int packed_op(fsibe_ctx* c, const double* in, double* out, int op, double
     k_packed_op<<<512, 256, 0, c->stream>>>(c->dscratch, c->dscratch2, op, c->g.nx, c->g.ny, c->P.xl, c->P.yl, c->g.pi,
                                             c->g.scalex, c->g.scaley, c->P.nu, dt, c->P.idealis);
     CKL(c);
-    CK(c, cudaMemcpyAsync(out, c->dscratch2, 8 * NN, cudaMemcpyDeviceToHost, c->stream));
+    CK(c, copy_out(c, out, c->dscratch2, 8 * NN));
     CK(c, cudaStreamSynchronize(c->stream));
     return FSIBE_OK;
 }
