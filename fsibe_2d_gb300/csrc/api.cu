@@ -13,7 +13,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -1257,8 +1256,8 @@ static void populate_pages(void* dst, size_t bytes) {
     size_t started = 0;
     try {
         for (; started + 1 < n; ++started) th[started] = std::thread(part, started);
-    } catch (const std::system_error&) {
-        // no more threads: the rest of the pages here
+    } catch (...) {
+        // no more threads or memory for one: the rest of the pages here
     }
     for (size_t k = started; k < n; ++k) part(k);
     for (size_t k = 0; k < started; ++k) th[k].join();

@@ -18,7 +18,7 @@
 // A new factor: each CTA scales its band rows and all-gathers them; every CTA runs the same
 // FP32 band LU (the routine of the single-CTA kernel, so every copy is bitwise identical) and
 // computes its own rows of M^-1 by transposed solves.  M^-1 persists between steps in global
-// memory under the single-CTA kernel's reuse rule (kept while <= 5 passes per Newton step).
+// memory (kept while it contracts: newton_pass).
 // The iterate update, the norms and the stopping test run redundantly in every CTA on
 // identical data, so they need no exchange.
 // What bounds it: chains of dependent FP64 (an addition is some 70 cycles) and the barriers, two a
@@ -901,8 +901,8 @@ size_t beam_cluster_minv_floats(int ns, int R) {
 // leave a CTA without a quad of rows (ns < 14); the next smaller where the device does not place one
 // with this kernel's shared memory, and 0 (the single-CTA kernel) where none fits.  A wider cluster
 // divides the rows' FP64 and the inverse products, a narrower one has the cheaper barriers (two a
-// pass).  Measured (GB300, 16 / 8 / 4 CTAs, the beam kernel in us): ns = 16 - / 61 / 60 (single CTA
-// 100), 64 63 / 58.5 / 57.5, 101 84 / 80 / 83.5, 127 78.5 / 74 / 84, 256 88 / 111 / 131.  want caps it.
+// pass).  Measured (GB300, 16 / 8 / 4 CTAs, the beam kernel in us): ns = 16 - / 47 / 47 (single CTA
+// 100), 64 - / 49 / 51, 101 - / 52 / 53, 127 - / 59 / 63, 256 66 / 83 / 93.  want caps it.
 // *big_out = 1 when only the large-beam form (factor and M^-1 in global memory) fits.
 int beam_cluster_setup(int ns, int want, size_t* smem_out, int* big_out) {
     static std::mutex mu;

@@ -344,14 +344,14 @@ int fsibe_force_gradient(fsibe_ctx* ctx, int component, const double* vort0, dou
  * one after another).  The runs may differ in grid size, beam size, parameters and precision.
  * Each run is an ordinary context (fsibe_ensemble_get), initialised and read with the
  * functions above.  fsibe_ensemble_step advances every run by nsteps; after the first step
- * (every run's Euler start-up step) one step of all runs is one CUDA graph launch, with each
- * run's step on its own stream.  Work issued on a run's context directly is ordered before
- * and after the ensemble's steps.  Ensembles of 8 runs or more run each beam on one CTA
- * (fsibe_beam_cluster reports 0) unless FSIBE_BEAM_CLUSTER is set: many runs fill the GPU by
- * themselves, and the single-CTA kernel then gives the higher throughput.  For the same reason
- * their steps form the nonlinear term and the stresses in the fused kernels (the split launches
- * of a single run, see fsibe_step, would only add graph nodes) unless FSIBE_NL_SPLIT or
- * FSIBE_STRESS_SPLIT is set. */
+ * (every run's Euler start-up step) one step of all runs is one CUDA graph launch.  Work issued
+ * on a run's context directly is ordered before and after the ensemble's steps.
+ * From 8 runs on, runs whose steps are the same launches (equal grids, nodes, options and precision;
+ * up to 1024 columns and rows, no sponge) share each of them, up to 16 runs a launch, and their steps
+ * form the nonlinear term and the stresses in the fused kernels (the split launches of a single run,
+ * see fsibe_step, would only add launches) unless FSIBE_NL_SPLIT or FSIBE_STRESS_SPLIT is set.
+ * Where the beams' clusters would have more than two CTAs an SM in all, each beam runs on one CTA
+ * (fsibe_beam_cluster reports 0) unless FSIBE_BEAM_CLUSTER is set. */
 typedef struct fsibe_ensemble fsibe_ensemble;
 int fsibe_ensemble_create(const fsibe_params* params, int nruns, fsibe_ensemble** out);
 int fsibe_ensemble_destroy(fsibe_ensemble* ens);
