@@ -145,12 +145,21 @@ __global__ void __launch_bounds__(256) k_adj_nu(AdjArgs a) {
     }
 }
 
-// acc[slot] += scale * sum(part[0 .. nparts)), in a fixed order
-__global__ void k_adj_reduce(const double* part, int nparts, double scale, double* acc) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double t = 0.0;
-        for (int i = 0; i < nparts; ++i) t += part[i];
-        *acc += scale * t;
+// acc[slot] += scale * sum(part[0 .. nparts)), in a fixed order: a thread's terms, its warp's tree, the
+// warps' tree.  One block of 256 (one thread's chain of dependent FP64 additions and loads took 22 us a
+// reverse step for 304 parts, so 4).
+__global__ void __launch_bounds__(256) k_adj_reduce(const double* part, int nparts, double scale, double* acc) {
+    __shared__ double ws[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double t = 0.0;
+    for (int i = threadIdx.x; i < nparts; i += 256) t += part[i];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) ws[warp] = t;
+    __syncthreads();
+    if (warp == 0) {
+        t = lane < 8 ? ws[lane] : 0.0;
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) *acc += scale * t;
     }
 }
 

@@ -2791,7 +2791,7 @@ static int adj_step(fsibe_ctx* c, int k) {
     int st;
     // viscosity term of step k: d W'/d nu = -dt |k|^2 W', d M'/d nu = -dt |k|^2 M'
     k_adj_nu<<<w->nparts, 256, 0, c->stream>>>(a);
-    k_adj_reduce<<<1, 32, 0, c->stream>>>(w->part, w->nparts, -w->dt, w->acc + 1);
+    k_adj_reduce<<<1, 256, 0, c->stream>>>(w->part, w->nparts, -w->dt, w->acc + 1);
     // linearisation point of step k: u, v and omega_x, omega_y exactly as k_nl_x forms them
     // (the x inverse of the state's Tdx, Tdy)
     if ((st = adj_invx(c, c->spec[SP_TDX], w->phys[AP_WX]))) return st;
