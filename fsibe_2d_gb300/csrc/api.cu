@@ -1314,8 +1314,8 @@ template <typename R>
 static int fwd2d(fsibe_ctx* c, void* spec_out) {
     KArgs<R> a = kargs<R>(c);
     a.spec1 = reinterpret_cast<C2<R>*>(spec_out);
-    launch_x<R>(c, kx_of<R>(c).xfwd, a);
-    launch_y<R>(c, ky_of<R>(c).yfwd, a);
+    launch_x<R>(c, kx_of<R>(c).xfwd_w, a);
+    launch_y<R>(c, ky_of<R>(c).yfwd_w, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -1326,7 +1326,7 @@ static int inv_y(fsibe_ctx* c, const void* spec_in, void* t_out, int op) {
     a.spec1 = reinterpret_cast<C2<R>*>(const_cast<void*>(spec_in));
     a.spec0 = reinterpret_cast<C2<R>*>(t_out);
     a.op = op;
-    launch_y<R>(c, ky_of<R>(c).yinv, a);
+    launch_y<R>(c, ky_of<R>(c).yinv_w, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -1334,7 +1334,7 @@ static int inv_y(fsibe_ctx* c, const void* spec_in, void* t_out, int op) {
 template <typename R>
 static int inv_x(fsibe_ctx* c) {
     KArgs<R> a = kargs<R>(c);
-    launch_x<R>(c, kx_of<R>(c).xinv, a);
+    launch_x<R>(c, kx_of<R>(c).xinv_w, a);
     CKL(c);
     return FSIBE_OK;
 }
@@ -3377,8 +3377,8 @@ extern "C" int fsibe_coftxy_static(const double* f_dev, double* fk_dev, int32_t 
     a.spec0 = T;
     a.spec1 = Sx;
     a.twX = twX; a.twR = twR; a.twY = twY;
-    kx.xfwd.k<<<ny / kx.x_rows, kx.xfwd.threads, kx.xfwd.smem, st>>>(a);
-    ky.yfwd.k<<<hx, ky.yfwd.threads, ky.yfwd.smem, st>>>(a);
+    kx.xfwd_w.k<<<ny / kx.x_rows, kx.xfwd_w.threads, kx.xfwd_w.smem, st>>>(a);
+    ky.yfwd_w.k<<<hx, ky.yfwd_w.threads, ky.yfwd_w.smem, st>>>(a);
     k_pack<double><<<hx, 256, 0, st>>>(Sx, nullptr, fk_dev, nx, ny);
     e = cudaGetLastError();
     if (e != cudaSuccess) { g_err = std::string("fsibe_coftxy_static: ") + cudaGetErrorString(e); return FSIBE_ERR_CUDA; }

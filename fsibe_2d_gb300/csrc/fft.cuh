@@ -151,14 +151,14 @@ __device__ __forceinline__ void fft_reg_run(C2<R> (&v)[NBA][8], C2<R>* buf, int 
 // called (the caller synchronises after their last use); they are free again on return.  All
 // threads of the block call it.  FP64: the result is scaled by 2^ex (fft_fx.cuh); FP32 leaves the
 // scale to the caller (ex is not used).
-template <typename R, int N, bool INV, int NB, int NBA>
+template <typename R, int N, bool INV, int NB, bool WIDE = false, int NBA>
 __device__ __forceinline__ void block_fft_reg_m(C2<R> (&v)[NBA][8], C2<R>* buf, int bstride,
                                                 const TwF<R>* __restrict__ tw, int t, int ex = 0) {
     static_assert(N >= 16 && (N & (N - 1)) == 0, "power-of-two length >= 16");
     static_assert(NB >= 1 && NB <= NBA, "NB of the NBA rows");
     if constexpr (sizeof(R) == 8) {
 #pragma unroll
-        for (int b = 0; b < NB; ++b) fx_fft<N, INV>(v[b], buf + b * bstride, tw, fx_block_group<N / 8>(t), ex);
+        for (int b = 0; b < NB; ++b) fx_fft<N, INV, WIDE>(v[b], buf + b * bstride, tw, fx_block_group<N / 8>(t), ex);
     } else {
         fft_reg_run<R, N, INV, NB, 1, NBA>(v, buf, bstride, tw, t);
     }

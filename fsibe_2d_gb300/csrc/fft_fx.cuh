@@ -6,7 +6,7 @@
 // instructions (5400 cycles) or about 650 cycles of integer instructions, so the transforms take
 // each row's values as 64-bit integers q on one exponent, value = q 2^e:
 //   * the exponent comes from the row's largest component (a maximum over the row's threads), so
-//     that it fills 59 bits; a double's 53 bits are kept whole down to 2^-5 of the row's largest
+//     that it fills 59 bits; a double's 53 bits are kept whole down to 2^-6 of the row's largest
 //     value, and below that to 2^-59 of it;
 //   * a twiddle is a 62-bit fraction in two balanced 32-bit halves; a complex product is twelve
 //     32 x 32 -> 64 multiply-adds (the low x low parts, below the last bit, are left out) and is
@@ -21,8 +21,13 @@
 // Measured (GB300, 1024^2, ns = 256, the coupled FP64 step): k_nl_y 325 -> 181 us, k_press_x 334 -> 153,
 // k_press_y 145 -> 70, k_nl_x's advection part 148 -> 62, the step 1142 -> 601; at 256^2 the step
 // 323 -> 256 us.
-// A row whose largest value is not finite or above 2^1006 comes out as NaN; values below 2^-980
-// lose digits and those below 2^-989 count as zero.
+// Range.  The transforms that take or give a caller's arrays (WIDE) take every finite row: one whose largest
+// value is below 2^-927 is scaled up by a power of two as it enters, and results near the ends of the
+// exponent range are scaled as they leave (to zero, a denormal or infinity, rounded as any FP64 result).
+// The time step's and the adjoint's kernels leave both out (with them the 256^2 step took 1% longer, the
+// 512^2 gradient 2%): of a row below 2^-927 they hold no digits below 2^-985, and one above
+// 2^1006, whose square no double holds, comes out as NaN, as does any row with a value that is not
+// finite.
 #pragma once
 #include "common.cuh"
 
@@ -35,7 +40,10 @@ static_assert(sizeof(q2) == sizeof(double2), "a fixed-point value takes its doub
 // (FX_BITS_C; the merge adds two bits of modulus, and the sums are known before the first stage)
 constexpr int FX_BITS = 59, FX_BITS_C = 60;
 constexpr int FX_LIM = 62;    // the moduli stay below 2^62.5, so that sums of two components fit
+// Exponent fields: the scales of a row whose elements and results are formed without the powers of two of
+// WIDE, and the range in which fx_to forms every result itself.
 constexpr unsigned FX_EMIN = 96, FX_EMAX = 1023 + 1006;
+constexpr int FX_EB_MIN = 64, FX_EB_MAX = 2045;
 
 __device__ __forceinline__ long long fx_wide(int a, int b, long long c) {
     long long r;
@@ -138,8 +146,8 @@ template <int BITS> __device__ __forceinline__ long long fx_from(double d, unsig
     const long long g = (long long)(hi >> 31);
     return (v ^ g) - g;
 }
-// q 2^e as a double (rounded to nearest), eb = e + 63 + 1022 (above zero for every scale); a row
-// that was not finite has nan = the exponent and quiet bits
+// q 2^e as a double (rounded to nearest), eb = e + 63 + 1022 in [FX_EB_MIN, FX_EB_MAX]; a row that was
+// not finite has nan = the exponent and quiet bits
 __device__ __forceinline__ double fx_to(long long q, int eb, unsigned nan) {
     const long long g = q >> 63;
     const unsigned long long m = (unsigned long long)((q ^ g) - g);
@@ -196,10 +204,10 @@ template <int G, bool SUM> __device__ __forceinline__ unsigned fx_read(unsigned 
 }
 // The scale of a row from its largest high word: the exponent field that fills its bits, and
 // the NaN bits of a row out of range.
-__device__ __forceinline__ unsigned fx_scale(unsigned hi, unsigned& nan) {
+template <bool WIDE> __device__ __forceinline__ unsigned fx_scale(unsigned hi, unsigned& nan) {
     const unsigned e = hi >> 20;
-    nan = e > FX_EMAX ? 0x7ff80000u : 0u;
-    return min(max(e, FX_EMIN), 2046u);
+    nan = e > (WIDE ? 2046u : FX_EMAX) ? 0x7ff80000u : 0u;
+    return min(max(e, WIDE ? 1u : FX_EMIN), 2046u);
 }
 // |a| in units of 2^44, rounded up
 __device__ __forceinline__ unsigned fx_l1(long long a) { return (unsigned)abs((int)(a >> 44)) + 1u; }
@@ -303,7 +311,7 @@ __device__ __forceinline__ int fx_stages(q2 (&v)[8], double2* buf, const int4* _
 
 // doubles in registers to fixed point: the group's scale (one synchronisation when it spans
 // warps), the exponent and the partial sum of moduli (complete for a group within a warp)
-template <int G, int BITS>
+template <int G, int BITS, bool WIDE>
 __device__ __forceinline__ int fx_enter(const double2 (&v)[8], q2 (&z)[8], const FxGroup& gr, unsigned& lsum, unsigned& nan) {
     unsigned mx = 0;
 #pragma unroll
@@ -311,32 +319,76 @@ __device__ __forceinline__ int fx_enter(const double2 (&v)[8], q2 (&z)[8], const
     mx = fx_reduce<G, false>(mx, gr.slot);
     if (G > 32) fx_sync<G>(gr);
     mx = fx_read<G, false>(mx, gr.slot);
-    const unsigned em = fx_scale(mx, nan);
+    const unsigned em = fx_scale<WIDE>(mx, nan);
+    if (!WIDE || em >= FX_EMIN) {  // the same for the whole group
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            z[m].x = fx_from<BITS>(v[m].x, em);
+            z[m].y = fx_from<BITS>(v[m].y, em);
+        }
+    } else {
+        // a row of zeros, or of the smallest scales
+        unsigned any = 0;
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            any |= fx_mag(v[m].x) | fx_mag(v[m].y) | (unsigned)__double2loint(v[m].x) | (unsigned)__double2loint(v[m].y);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) z[m].x = z[m].y = 0;
+        if (any != 0) {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                z[m].x = fx_from<BITS>(v[m].x * 0x1p128, em + 128);
+                z[m].y = fx_from<BITS>(v[m].y * 0x1p128, em + 128);
+            }
+        }
+    }
     lsum = 0;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        z[m].x = fx_from<BITS>(v[m].x, em);
-        z[m].y = fx_from<BITS>(v[m].y, em);
-        lsum += fx_l1(z[m].x) + fx_l1(z[m].y);
-    }
+    for (int m = 0; m < 8; ++m) lsum += fx_l1(z[m].x) + fx_l1(z[m].y);
     lsum = fx_reduce<G, true>(lsum, gr.slot + G / 32);
     return (int)em - 1022 - BITS;
 }
-__device__ __forceinline__ double2 fx_leave(q2 z, int e, unsigned nan) {
-    return make_double2(fx_to(z.x, e + 63 + 1022, nan), fx_to(z.y, e + 63 + 1022, nan));
+// fixed point to doubles on the exponent e: fx_to's on one in its range, and with WIDE the power of two
+// between (scale: 0 for none)
+template <bool WIDE>
+struct FxOut {
+    int eb, scale = 0;
+    unsigned nan;
+    __device__ __forceinline__ FxOut(int e, unsigned nan_) : eb(e + 63 + 1022), nan(nan_) {
+        if (WIDE) {
+            const int b = eb;
+            eb = min(max(b, FX_EB_MIN), FX_EB_MAX);
+            scale = b - eb;
+        }
+    }
+    __device__ __forceinline__ double2 operator()(q2 z) const { return make_double2(fx_to(z.x, eb, nan), fx_to(z.y, eb, nan)); }
+    __device__ __forceinline__ double2 scaled(double2 v) const {  // (zeros stay out of the FP64 pipe)
+        const double s = __hiloint2double((1023 + scale) << 20, 0);
+        if (fx_mag(v.x) | fx_mag(v.y)) { v.x *= s; v.y *= s; }
+        return v;
+    }
+};
+template <bool WIDE>
+__device__ __forceinline__ void fx_leave(const q2 (&z)[8], int e, unsigned nan, double2 (&v)[8]) {
+    const FxOut<WIDE> out(e, nan);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) v[m] = out(z[m]);
+    if (WIDE && out.scale != 0) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) v[m] = out.scaled(v[m]);
+    }
 }
 
 // The transform of doubles in registers by one group: v[m] = element t + m (N/8); buf is the group's
 // row, free when called and on return.  The result is scaled by 2^ex (the normalisation 1/(nx ny),
 // a power of two, costs nothing here).
-template <int N, bool INV>
+template <int N, bool INV, bool WIDE = false>
 __device__ __forceinline__ void fx_fft(double2 (&v)[8], double2* buf, const int4* __restrict__ tw, const FxGroup& gr, int ex = 0) {
     q2 z[8];
     unsigned lsum, nan;
-    int e = fx_enter<N / 8, FX_BITS>(v, z, gr, lsum, nan);
+    int e = fx_enter<N / 8, FX_BITS, WIDE>(v, z, gr, lsum, nan);
     e += ex + fx_stages<N, INV, FX_BITS, true>(z, buf, tw, gr, lsum);
-#pragma unroll
-    for (int m = 0; m < 8; ++m) v[m] = fx_leave(z[m], e, nan);
+    fx_leave<WIDE>(z, e, nan, v);
 }
 
 // ---- real rows of 2H values as H complex ones (see r2c_split_m and c2r_merge_m) ---------------
@@ -346,7 +398,7 @@ __device__ __forceinline__ void fx_fft(double2 (&v)[8], double2* buf, const int4
 // A half spectrum of doubles in the group's row (the group synchronised after it was written) to a
 // real row in registers: v[m] = element t + m (H/8), its x and y two neighbouring real values.
 // The row is free on return.
-template <int H>
+template <int H, bool WIDE = false>
 __device__ __forceinline__ void fx_c2r(double2* rb, const int4* __restrict__ twR, const int4* __restrict__ twX,
                                        const FxGroup& gr, double2 (&v)[8]) {
     constexpr int G = H / 8;
@@ -364,7 +416,7 @@ __device__ __forceinline__ void fx_c2r(double2* rb, const int4* __restrict__ twR
             x[2 * i + 1] = rb[pad8(H - k)];
             if (i == 3 && sp) x[2 * i].y = 0.0;  // the imaginary part of X[0] is ignored
         }
-        e = fx_enter<G, FX_BITS_C>(x, z, gr, lsum, nan);
+        e = fx_enter<G, FX_BITS_C, WIDE>(x, z, gr, lsum, nan);
     }
     // Z[k] = (X[k] + conj X[H-k]) + i (X[k] - conj X[H-k]) conj(w^k), and Z[H-k] likewise
 #pragma unroll
@@ -396,20 +448,19 @@ __device__ __forceinline__ void fx_c2r(double2* rb, const int4* __restrict__ twR
     for (int m = 0; m < 8; ++m) z[m] = fx_ldrow(&rb[pad8(t + m * G)]);
     fx_sync<G>(gr);
     e += fx_stages<H, true, FX_BITS_C + 2, false>(z, rb, twX, gr, lsum);
-#pragma unroll
-    for (int m = 0; m < 8; ++m) v[m] = fx_leave(z[m], e, nan);
+    fx_leave<WIDE>(z, e, nan, v);
 }
 
 // A real row in registers to the half spectrum of doubles in the group's row (free when called;
 // readers outside the group synchronise first).
-template <int H>
+template <int H, bool WIDE = false>
 __device__ __forceinline__ void fx_r2c(const double2 (&v)[8], double2* rb, const int4* __restrict__ twR,
                                        const int4* __restrict__ twX, const FxGroup& gr) {
     constexpr int G = H / 8;
     const int t = gr.t;
     q2 z[8];
     unsigned lsum, nan;
-    int e = fx_enter<G, FX_BITS>(v, z, gr, lsum, nan);
+    int e = fx_enter<G, FX_BITS, WIDE>(v, z, gr, lsum, nan);
     e += fx_stages<H, false, FX_BITS, true>(z, rb, twX, gr, lsum);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -419,6 +470,7 @@ __device__ __forceinline__ void fx_r2c(const double2 (&v)[8], double2* rb, const
         fx_strow(&rb[pad8(t + m * G)], h);
     }
     fx_sync<G>(gr);
+    const FxOut<WIDE> out(e, nan);
     // X[k] = (z[k] + conj z[H-k])/2 + w^k (z[k] - conj z[H-k])/(2i), and X[H-k] likewise
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -436,9 +488,18 @@ __device__ __forceinline__ void fx_r2c(const double2 (&v)[8], double2* rb, const
             xk.x = 2 * (a.x + a.y); xk.y = 0;   // X[0] = Re z[0] + Im z[0]
             xm.x = 2 * c.x; xm.y = -2 * c.y;    // X[H/2] = conj z[H/2]
         }
-        *pk = fx_leave(xk, e, nan);
+        *pk = out(xk);
         if (sp) pk->y = 0.0;
-        *pm = fx_leave(xm, e, nan);
+        *pm = out(xm);
+    }
+    if (WIDE && out.scale != 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // the thread's own elements
+            const int k = 1 + t + i * G;
+            double2 *pk = &rb[pad8(i == 3 && k == H / 2 ? 0 : k)], *pm = &rb[pad8(H - k)];
+            *pk = out.scaled(*pk);
+            *pm = out.scaled(*pm);
+        }
     }
 }
 

@@ -242,23 +242,24 @@ __device__ __forceinline__ void row_r2c_fp(C2<R> (&v)[NBA][8], C2<R>* rb, int bs
     __syncthreads();
     r2c_split_m<R, H, NB>(rb, bstride, twR, t);
 }
-// The two in the precision form's engine: the floating-point stages in FP32, fixed point in FP64.
-template <typename R, int H, int NB, int NBA>
+// The two in the precision form's engine: the floating-point stages in FP32, fixed point in FP64
+// (WIDE: over all of the exponent range, fft_fx.cuh).
+template <typename R, int H, int NB, bool WIDE = false, int NBA>
 __device__ __forceinline__ void row_c2r_reg(C2<R>* rb, int bstride, const TwF<R>* __restrict__ twR,
                                             const TwF<R>* __restrict__ twX, int t, C2<R> (&v)[NBA][8]) {
     if constexpr (kIsF32<R>) row_c2r_fp<R, H, NB>(rb, bstride, twR, twX, t, v);
     else {
 #pragma unroll
-        for (int b = 0; b < NB; ++b) fx_c2r<H>(rb + b * bstride, twR, twX, fx_block_group<H / 8>(t), v[b]);
+        for (int b = 0; b < NB; ++b) fx_c2r<H, WIDE>(rb + b * bstride, twR, twX, fx_block_group<H / 8>(t), v[b]);
     }
 }
-template <typename R, int H, int NB, int NBA>
+template <typename R, int H, int NB, bool WIDE = false, int NBA>
 __device__ __forceinline__ void row_r2c_reg(C2<R> (&v)[NBA][8], C2<R>* rb, int bstride, const TwF<R>* __restrict__ twR,
                                             const TwF<R>* __restrict__ twX, int t) {
     if constexpr (kIsF32<R>) row_r2c_fp<R, H, NB>(v, rb, bstride, twR, twX, t);
     else {
 #pragma unroll
-        for (int b = 0; b < NB; ++b) fx_r2c<H>(v[b], rb + b * bstride, twR, twX, fx_block_group<H / 8>(t));
+        for (int b = 0; b < NB; ++b) fx_r2c<H, WIDE>(v[b], rb + b * bstride, twR, twX, fx_block_group<H / 8>(t));
         __syncthreads();  // the rows are read by the whole block
     }
 }
@@ -303,7 +304,7 @@ __device__ __forceinline__ double warp_max(double v) {
 // ======================================================================================
 
 // real field (phys0) -> T (spec0): forward x
-template <typename R, int H>
+template <typename R, int H, bool WIDE>
 __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xfwd(KArgs<R> a) {
     using X = XRows<R, H>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xfwd(KArgs<R> a) {
     C2<R> f[1][8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) f[0][q] = f2[t + q * X::G];
-    row_r2c_reg<R, H, 1>(f, rb, 0, a.twR, a.twX, t);
+    row_r2c_reg<R, H, 1, WIDE>(f, rb, 0, a.twR, a.twX, t);
     C2<R>* T = a.spec0 + boff;
     for (int i = threadIdx.x; i < H * X::TR; i += blockDim.x) {
         const int rr = i % X::TR, kx = i / X::TR;
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xfwd(KArgs<R> a) {
 }
 
 // T (spec0) -> real field (phys0): inverse x (unnormalised)
-template <typename R, int H>
+template <typename R, int H, bool WIDE>
 __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xinv(KArgs<R> a) {
     using X = XRows<R, H>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -338,14 +339,14 @@ __global__ void __launch_bounds__(XRows<R, H>::THREADS) k_xinv(KArgs<R> a) {
     cp_async_wait_f();
     __syncthreads();
     C2<R> f[1][8];
-    row_c2r_reg<R, H, 1>(rb, 0, a.twR, a.twX, t, f);
+    row_c2r_reg<R, H, 1, WIDE>(rb, 0, a.twR, a.twX, t, f);
     C2<R>* f2 = reinterpret_cast<C2<R>*>(a.phys0) + boff + (size_t)(iy0 + r) * H;
 #pragma unroll
     for (int q = 0; q < 8; ++q) f2[t + q * X::G] = f[0][q];
 }
 
 // forward y of spec0 (T) -> spec1 (S), scaled by 1/(nx ny), ky = ny/2 zeroed
-template <typename R, int NY>
+template <typename R, int NY, bool WIDE>
 __global__ void __launch_bounds__(NY / 8) k_yfwd(KArgs<R> a) {
     constexpr int G = NY / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(NY / 8) k_yfwd(KArgs<R> a) {
     C2<R> f[1][8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) f[0][q] = in[t + q * G];
-    block_fft_reg_m<R, NY, false, 1>(f, buf, 0, a.twY, t, a.enorm);
+    block_fft_reg_m<R, NY, false, 1, WIDE>(f, buf, 0, a.twY, t, a.enorm);
     const R norm = kIsF32<R> ? (R)a.g.inv_nxny : (R)1;  // (FP64: scaled by the transform)
     C2<R>* out = a.spec1 + boff + (size_t)kx * NY;
 #pragma unroll
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(NY / 8) k_yfwd(KArgs<R> a) {
 }
 
 // inverse y of op(spec1) -> spec0 (T)
-template <typename R, int NY>
+template <typename R, int NY, bool WIDE>
 __global__ void __launch_bounds__(NY / 8) k_yinv(KArgs<R> a) {
     constexpr int G = NY / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(NY / 8) k_yinv(KArgs<R> a) {
         if (ky == NY / 2) o = mk<R>(0, 0);
         f[0][q] = o;
     }
-    block_fft_reg_m<R, NY, true, 1>(f, buf, 0, a.twY, t);
+    block_fft_reg_m<R, NY, true, 1, WIDE>(f, buf, 0, a.twY, t);
     C2<R>* out = a.spec0 + boff + (size_t)kx * NY;
 #pragma unroll
     for (int q = 0; q < 8; ++q) out[t + q * G] = f[0][q];
@@ -1441,6 +1442,7 @@ template <typename R>
 struct SizeKernels {
     // x-pass kernels for H = nx/2 (x_rows rows a block)
     KLaunch<R> xfwd, xinv, vel_x;
+    KLaunch<R> xfwd_w, xinv_w;  // on a caller's arrays: the whole exponent range (WIDE, fft_fx.cuh; FP32: the same)
     int x_rows;
     // tile-height candidates of the fused x kernels (index 1 is the default)
     struct XVariant {
@@ -1454,6 +1456,7 @@ struct SizeKernels {
     XVariant xp;  // FP32: k_press_x on paired rows (press_x only; none in the FP64 form)
     // y-pass kernels for NY
     KLaunch<R> yfwd, yinv, nl_y, press_y;
+    KLaunch<R> yfwd_w, yinv_w;
     KLaunch<R> press_y1;  // FP32: k_press_y on the one-butterfly engine (NY/8 threads), or none
 };
 
@@ -1507,8 +1510,11 @@ inline void fill_size_kernels(SizeKernels<R>& k) {
     using X = XRows<R, H>;
     constexpr int S1 = (int)(X::TR * X::PL * sizeof(C2<R>)), SY = (int)(plen<R>(N) * sizeof(C2<R>)), TY = N / 8;
     k.x_rows = X::TR;
-    k.xfwd = klaunch<R>(k_xfwd<R, H>, X::THREADS, S1);
-    k.xinv = klaunch<R>(k_xinv<R, H>, X::THREADS, S1);
+    constexpr bool W = !kIsF32<R>;
+    k.xfwd = klaunch<R>(k_xfwd<R, H, false>, X::THREADS, S1);
+    k.xinv = klaunch<R>(k_xinv<R, H, false>, X::THREADS, S1);
+    k.xfwd_w = klaunch<R>(k_xfwd<R, H, W>, X::THREADS, S1);
+    k.xinv_w = klaunch<R>(k_xinv<R, H, W>, X::THREADS, S1);
     k.vel_x = klaunch<R>(k_vel_x<R, H>, X::THREADS, 2 * S1);
     constexpr int T1 = X::TRD;
     k.xp = typename SizeKernels<R>::XVariant{};
@@ -1527,8 +1533,10 @@ inline void fill_size_kernels(SizeKernels<R>& k) {
         fill_xvariant<R, H, T2>(k.xv[2]);
         k.xv[3] = k.xv[1];
     }
-    k.yfwd = klaunch<R>(k_yfwd<R, N>, TY, SY);
-    k.yinv = klaunch<R>(k_yinv<R, N>, TY, SY);
+    k.yfwd = klaunch<R>(k_yfwd<R, N, false>, TY, SY);
+    k.yinv = klaunch<R>(k_yinv<R, N, false>, TY, SY);
+    k.yfwd_w = klaunch<R>(k_yfwd<R, N, W>, TY, SY);
+    k.yinv_w = klaunch<R>(k_yinv<R, N, W>, TY, SY);
     if constexpr (kIsF32<R>) {
         constexpr int TP = xpairs_rows<H>();
         k.xp.rows = TP;
