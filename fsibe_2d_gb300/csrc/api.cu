@@ -5,7 +5,6 @@
 // window, status) live in a device struct, so a step needs no host round trip and can be
 // captured once in a CUDA graph and replayed.
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstddef>
 #include <cstdlib>
@@ -1507,7 +1506,13 @@ const char* fsibe_last_error(const fsibe_ctx* ctx) { return ctx ? ctx->err.c_str
 // grid per block).  A new context times each candidate on its own freshly allocated buffers
 // (no state exists yet; fsibe_init_fields overwrites everything they touch) and keeps the
 // fastest per kernel.  The choice is cached per (precision, nx, ny) for the process, so an
-// ensemble of many runs of one size tunes once.  FSIBE_AUTOTUNE=0 keeps the default tiles.
+// ensemble of many runs of one size tunes once; k_press_x's also by whether it forms the stresses.
+// A tile's height changes no bit of the fields; the paired press_x and press_y's engines round
+// differently.  FSIBE_AUTOTUNE=0 keeps the default tiles.
+
+// k_press_x forms the viscous stresses itself (they are not in their own launch): another body, with
+// its own best tile, and none of the paired kernel's.
+static bool stress_inside(const fsibe_ctx* c) { return c->P.iViscous == 1 && !c->stress_split; }
 template <typename R>
 static float time_kernel(fsibe_ctx* c, const KLaunch<R>& k, int grid) {
     KArgs<R> a = kargs<R>(c);
@@ -1533,51 +1538,79 @@ static float time_xv(fsibe_ctx* c, int kind, const typename SizeKernels<R>::XVar
     return time_kernel<R>(c, k, c->g.ny / v.rows);
 }
 
+// kind 0 k_nl_x, 1 k_press_x, 2 k_press_fin; the default first, a candidate must be faster by 3% to replace it
+template <typename R>
+static int best_tile(fsibe_ctx* c, int kind) {
+    const SizeKernels<R>& K = kx_of<R>(c);
+    int best = 1;
+    float tbest = time_xv<R>(c, kind, K.xv[1]);
+    for (int v : {0, 2, 3}) {
+        if (K.xv[v].rows == K.xv[1].rows && K.xv[v].minb == K.xv[1].minb) continue;
+        const float t = time_xv<R>(c, kind, K.xv[v]);
+        if (t < 0.97f * tbest) { tbest = t; best = v; }
+    }
+    // FP32: the paired press_x (index 4), when its tile (128 threads: 128 / (H/16) rows)
+    // divides the grid's rows
+    if (kind == 1 && !stress_inside(c) && K.xp.press_x.k && c->g.ny % K.xp.rows == 0) {
+        const float t = time_xv<R>(c, kind, K.xp);
+        if (t < 0.97f * tbest) { tbest = t; best = 4; }
+    }
+    return best;
+}
+
 template <typename R>
 static int autotune_x(fsibe_ctx* c) {
+    struct Choice { int f32, nx, ny, nl, px[2], fin, eng; };  // px: the stresses apart, inside; -1: not timed
     static std::mutex mu;
-    static std::vector<std::array<int, 7>> cache;  // fp32, nx, ny, nl, px, fin, press_y engine
+    static std::vector<Choice> cache;
     const char* env = std::getenv("FSIBE_AUTOTUNE");
     if (env && env[0] == '0') return FSIBE_OK;
     std::lock_guard<std::mutex> lock(mu);
-    const int f32 = c->fp32 ? 1 : 0;
-    for (const auto& e : cache)
-        if (e[0] == f32 && e[1] == c->g.nx && e[2] == c->g.ny) {
-            c->xv_nl = e[3]; c->xv_px = e[4]; c->xv_fin = e[5]; c->py_eng = e[6];
-            return FSIBE_OK;
+    const int f32 = c->fp32 ? 1 : 0, inside = stress_inside(c) ? 1 : 0;
+    Choice n{f32, c->g.nx, c->g.ny, -1, {-1, -1}, 1, 0};
+    Choice* e = nullptr;
+    for (Choice& k : cache)
+        if (k.f32 == f32 && k.nx == n.nx && k.ny == n.ny) e = &k;
+    if (e) n = *e;
+    const bool first = n.nl < 0, timed = first || n.px[inside] < 0;
+    if (first) n.nl = best_tile<R>(c, 0);
+    if (n.px[inside] < 0) n.px[inside] = best_tile<R>(c, 1);
+    if (first) {
+        n.fin = best_tile<R>(c, 2);
+        // k_press_y's transform engine (FP32): the paired one by default, the one-butterfly one when
+        // it is faster by 3%
+        const SizeKernels<R>& KY = ky_of<R>(c);
+        if (KY.press_y1.k) {
+            const float t0 = time_kernel<R>(c, KY.press_y, c->g.hx);
+            const float t1 = time_kernel<R>(c, KY.press_y1, c->g.hx);
+            if (t1 < 0.97f * t0) n.eng = 1;
         }
-    const SizeKernels<R>& K = kx_of<R>(c);
-    int choice[3];
-    for (int kind = 0; kind < 3; ++kind) {
-        // the default first; a candidate must be faster by 3% to replace it
-        int best = 1;
-        float tbest = time_xv<R>(c, kind, K.xv[1]);
-        for (int v : {0, 2, 3}) {
-            if (K.xv[v].rows == K.xv[1].rows && K.xv[v].minb == K.xv[1].minb) continue;
-            const float t = time_xv<R>(c, kind, K.xv[v]);
-            if (t < 0.97f * tbest) { tbest = t; best = v; }
-        }
-        // FP32: the paired press_x (index 4), when its tile (128 threads: 128 / (H/16) rows)
-        // divides the grid's rows
-        if (kind == 1 && K.xp.press_x.k && c->g.ny % K.xp.rows == 0) {
-            const float t = time_xv<R>(c, kind, K.xp);
-            if (t < 0.97f * tbest) { tbest = t; best = 4; }
-        }
-        choice[kind] = best;
     }
-    // k_press_y's transform engine (FP32): the paired one by default, the one-butterfly one when
-    // it is faster by 3%
-    int eng = 0;
-    const SizeKernels<R>& KY = ky_of<R>(c);
-    if (KY.press_y1.k) {
-        const float t0 = time_kernel<R>(c, KY.press_y, c->g.hx);
-        const float t1 = time_kernel<R>(c, KY.press_y1, c->g.hx);
-        if (t1 < 0.97f * t0) eng = 1;
+    if (timed) {
+        CKL(c);
+        CK(c, cudaStreamSynchronize(c->stream));
+        if (e) *e = n;
+        else cache.push_back(n);
     }
-    CKL(c);
-    CK(c, cudaStreamSynchronize(c->stream));
-    c->xv_nl = choice[0]; c->xv_px = choice[1]; c->xv_fin = choice[2]; c->py_eng = eng;
-    cache.push_back({f32, c->g.nx, c->g.ny, choice[0], choice[1], choice[2], eng});
+    c->xv_nl = n.nl; c->xv_px = n.px[inside]; c->xv_fin = n.fin; c->py_eng = n.eng;
+    return FSIBE_OK;
+}
+
+// The tiles and engines of a context's steps, by its flags; the context holds no state yet.
+static int choose_tiles(fsibe_ctx* c) {
+    c->xv_nl = c->xv_px = c->xv_fin = 1;
+    c->py_eng = 0;
+    const int st = c->fp32 ? autotune_x<float>(c) : autotune_x<double>(c);
+    if (st) return st;
+    // FSIBE_PX_PAIRED = 1 / 0 forces / forbids the paired FP32 press_x (tests of both forms)
+    const char* pe = std::getenv("FSIBE_PX_PAIRED");
+    if (pe && c->fp32) {
+        if (pe[0] == '1' && !stress_inside(c) && c->g.ny % c->kxf.xp.rows == 0) c->xv_px = 4;
+        else if (pe[0] == '0' && c->xv_px == 4) c->xv_px = 1;
+    }
+    // FSIBE_PY_ENG = 0 / 1 forces k_press_y's paired / one-butterfly engine (FP32)
+    const char* ye = std::getenv("FSIBE_PY_ENG");
+    if (ye && c->fp32) c->py_eng = (ye[0] == '1') ? 1 : 0;
     return FSIBE_OK;
 }
 
@@ -1879,17 +1912,8 @@ int fsibe_create(const fsibe_params* p, fsibe_ctx** out) {
     cudaEventCreateWithFlags(&c->ev_ny, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&c->ev_sb, cudaEventDisableTiming);
     {
-        const int st = c->fp32 ? autotune_x<float>(c) : autotune_x<double>(c);
+        const int st = choose_tiles(c);
         if (st) { g_err = c->err; fsibe_destroy(c); return st; }
-        // FSIBE_PX_PAIRED = 1 / 0 forces / forbids the paired FP32 press_x (tests of both forms)
-        const char* pe = std::getenv("FSIBE_PX_PAIRED");
-        if (pe && c->fp32) {
-            if (pe[0] == '1' && c->g.ny % c->kxf.xp.rows == 0) c->xv_px = 4;
-            else if (pe[0] == '0' && c->xv_px == 4) c->xv_px = 1;
-        }
-        // FSIBE_PY_ENG = 0 / 1 forces k_press_y's paired / one-butterfly engine (FP32)
-        const char* ye = std::getenv("FSIBE_PY_ENG");
-        if (ye && c->fp32) c->py_eng = (ye[0] == '1') ? 1 : 0;
     }
     e = cudaDeviceSynchronize();
     if (e != cudaSuccess) { g_err = std::string("create: ") + cudaGetErrorString(e); fsibe_destroy(c); return FSIBE_ERR_CUDA; }
@@ -3187,6 +3211,8 @@ int fsibe_ensemble_create(const fsibe_params* params, int nruns, fsibe_ensemble*
         for (fsibe_ctx* c : e->runs) {
             if (!std::getenv("FSIBE_NL_SPLIT")) c->nl_split = false;
             if (!std::getenv("FSIBE_STRESS_SPLIT")) c->stress_split = false;
+            const int st = choose_tiles(c);  // fsibe_create chose them with the stresses apart
+            if (st) { g_err = c->err; ens_free(e); return st; }
         }
     }
     cudaError_t ce = cudaStreamCreateWithFlags(&e->master, cudaStreamNonBlocking);
