@@ -88,14 +88,17 @@ struct ClLayout {
 };
 
 // The rows [lo, hi) of CTA r: quads of rows, so that every CTA's slice of the FP32 right-hand side (and
-// of the FP64 solution) starts on a 16-byte boundary.  With R >= 8 and n <= 640 the first and the last
+// of the FP64 solution) starts on a 16-byte boundary.  With R >= 8 and n <= 600 the first and the last
 // CTA hold the four boundary equations alone (and one node, when ns is odd) and the others share the
 // rest evenly: a warp of generic rows takes its time whether one row or 32, and the boundary
 // equations' beside it on the same SMSPs made those two CTAs the slowest (F and J of an iteration
-// 4.6k cycles with them, 3.1k without).  Above, where rows and M^-1's size count, all share evenly.
+// 4.6k cycles with them, 3.1k without).  The others' slices of M^-1 are larger for it: from ns = 302 on they
+// no longer fit 16 CTAs' shared memory, where an even split does up to 318.  The kernel in us, alone / even,
+// both in shared memory: ns = 144 55 / 57, 256 65 / 67.5, 296 70 / 73; alone in global memory: 312 78-82 /
+// 72-74, 318 77-84 / 74-75 (one process to another differs by up to 3).  Above, all share evenly.
 __host__ __device__ inline bool cl_ends_alone(int n, int R) {
     const int nq = (n + 3) / 4, last = nq - (n - 4) / 4;
-    return R >= 8 && n <= 640 && nq - 1 - last >= R - 2;
+    return R >= 8 && n <= 600 && nq - 1 - last >= R - 2;
 }
 __host__ __device__ inline void cl_rows(int n, int R, int r, int& lo, int& hi) {
     const int nq = (n + 3) / 4;
@@ -902,7 +905,9 @@ size_t beam_cluster_minv_floats(int ns, int R) {
 // with this kernel's shared memory, and 0 (the single-CTA kernel) where none fits.  A wider cluster
 // divides the rows' FP64 and the inverse products, a narrower one has the cheaper barriers (two a
 // pass).  Measured (GB300, 16 / 8 / 4 CTAs, the beam kernel in us): ns = 16 - / 47 / 47 (single CTA
-// 100), 64 - / 49 / 51, 101 - / 52 / 53, 127 - / 59 / 63, 256 66 / 83 / 93.  want caps it.
+// 100), 64 - / 49 / 51, 101 - / 52 / 53, 127 - / 59 / 63, 256 66 / 83 / 93; 16 / 8 with the sums by events, some
+// 4 us, 144 61.3 / 60.4, 160 61.3 / 61.3, 192 64.1 / 63.0, 224 64.2 / 76.6: from 145 nodes on the two are within 2%
+// until, from 215, the rows of M^-1 of 8 CTAs do not fit shared memory.  want caps it.
 // *big_out = 1 when only the large-beam form (factor and M^-1 in global memory) fits.
 int beam_cluster_setup(int ns, int want, size_t* smem_out, int* big_out) {
     static std::mutex mu;

@@ -16,13 +16,14 @@
 //   * fills in every s_k in parallel.
 // Afterwards every step is checked in parallel by the FP64 addition, bits(s_k + a_k) ==
 // bits(s_(k+1)), and a sum with any mismatch is formed again by the serial loop: the result is that
-// loop's in every case.  A beam of 1024 nodes has 11 to 81 events a sum.  Up to RS_SERIAL terms the
+// loop's in every case.  A beam of 1024 nodes has 11 to 81 events a sum.  Up to rs_serial terms the
 // serial loop itself is the shortest (78 cycles a step from shared memory): this code runs once a
 // launch, on one warp, and its integer chains are long.  Sums with many events, non-finite or very
 // small terms take the serial loop too.
-// Measured (GB300, cycles of the phase in k_beam_cl; batches of 32 integer steps from one binade change to
-// the next before): ns = 16 9.4 -> 3.1 k, 64 13.6 -> 6.7, 101 41 -> 10.1, 127 11.3 -> 11.8, 256 30.7 -> 22
-// (by events 27), 1024 79 -> 69 (serial 82).
+// Measured (GB300, k cycles of the phase in k_beam_cl, serial / by events; a straight beam and, after
+// the semicolon, a heaving one, which has fewer events): ns = 256 22 / 27, 384 33 / 38; 34 / 28, 512 43 / 58-70; 43 / 59,
+// 576 52 / 57; 52 / 46, 768 67 / 63; 67 / 51, 1024 87 / 73; 87 / 60.  The kernel, us: 512 103 / 120; 110 / 120,
+// 576 147 / 151; 154 / 151, 640 152 / 154; 157 / 155, 832 173 / 171; 180 / 171 (one process to another differs by 3).
 #pragma once
 #include "common.cuh"
 
@@ -48,7 +49,9 @@ __device__ __forceinline__ long long term_inc(double a, int g, bool& ok, bool& t
     return neg ? -r : r;
 }
 
-constexpr int RS_SERIAL = 320, RS_MAX = 2016, RS_EVENTS = 96;  // RS_MAX: 63 terms a lane
+constexpr int RS_MAX = 2016, RS_EVENTS = 96;  // RS_MAX: 63 terms a lane
+// Terms up to which the serial loop is taken: its step is 78 cycles from shared memory (SH), 112 else.
+template <bool SH> constexpr int rs_serial() { return SH ? 544 : 320; }
 
 // The serial loop, by lane 0 of a warp: 78 cycles a step with the rows in shared memory (SH), 112
 // through generic addresses.
@@ -187,7 +190,7 @@ __device__ int running_sums4(const double* src, int sld, double* dst, int dld, i
         const double* s = src + (size_t)warp * sld;
         double* d = dst + (size_t)warp * dld;
         if (lane == 0) flags[warp] = 0;
-        if (n <= RS_SERIAL || n > RS_MAX || !running_sum_warp<SH>(s, d, n, start[warp], base[warp])) {
+        if (n <= rs_serial<SH>() || n > RS_MAX || !running_sum_warp<SH>(s, d, n, start[warp], base[warp])) {
             __syncwarp();
             running_sum_serial<SH>(s, d, n);
         }
@@ -195,7 +198,7 @@ __device__ int running_sums4(const double* src, int sld, double* dst, int dld, i
         idle(tid - 128, blockDim.x - 128);
     }
     __syncthreads();
-    if (n <= RS_SERIAL) return 0;
+    if (n <= rs_serial<SH>()) return 0;
     for (int j = tid; j < 4 * n; j += blockDim.x) {
         const int q = j / n, k = j - q * n;
         if (k + 1 < n) {
