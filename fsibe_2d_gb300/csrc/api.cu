@@ -3040,10 +3040,10 @@ int fsibe_drag_gradient(fsibe_ctx* c, const double* vort0, double nu, int nsteps
 // streams, and a join.  A batch is up to kBatch runs whose steps are the same launches, each of them made
 // once for all (Batch, ens_groups); the other runs' steps stay their own.  The GPU starts a graph's
 // kernels at one in 1.3 us however small they are, so that 48 runs of 256^2, 14 kernels each, took
-// 876 us a step where their work is 400; batched they take 399, and the 64-run batch (48 x 256^2,
-// 12 x 512^2, 4 x 1024^2) 1024 instead of 1569.  One batch a shape: smaller ones, which would
-// overlap more, measured no better (64-run batch with at most 0.25 / 1 / 2 million cells a batch 1248 /
-// 1192 / 1181 us, without that limit 1149).
+// 876 us a step where their work is 400; in three batches they take 394, and the 64-run ensemble
+// (48 x 256^2, 12 x 512^2, 4 x 1024^2) 1014 instead of 1569.  As few batches a shape as kBatch allows:
+// smaller ones, which would overlap more, were no better (the 64-run ensemble 3 to 9% slower with at
+// most 2 to 0.25 million cells a batch).
 struct fsibe_ensemble {
     std::vector<fsibe_ctx*> runs;
     cudaStream_t master = nullptr;
@@ -3196,17 +3196,19 @@ int fsibe_ensemble_create(const fsibe_params* params, int nruns, fsibe_ensemble*
         e->runs.push_back(c);
     }
     // The beams of many runs fill the GPU by themselves: above two cluster CTAs an SM the single-CTA beam
-    // kernel gives as much (us a step with clusters / single CTAs: 48 runs of 256^2, 384 CTAs, 470 / 425,
-    // 32, 256 CTAs, 333 / 331; the 64-run batch, 544 CTAs, 1072 / 1065), below it the clusters do, whose
-    // beams end sooner (24 of 256^2 253 / 289, 8 of 512^2 244 / 339, 8 + 4 + 2 of 256^2, 512^2 and 1024^2
-    // 384 / 504).  FSIBE_BEAM_CLUSTER, when set, decides.
+    // kernel gives as much or more (us a step with clusters / single CTAs: 48 runs of 256^2, 384 CTAs,
+    // 438 / 394; the 64-run ensemble, 544 CTAs, 1017 / 1014), below it the clusters do, whose beams end
+    // sooner (32 of 256^2, 256 CTAs, 313 / 311, 24 240 / 274, 16 200 / 235, 8 of 512^2 234 / 337, 8 + 4 + 2 of
+    // 256^2, 512^2 and 1024^2 368 / 490).  FSIBE_BEAM_CLUSTER, when set, decides.
     int ctas = 0;
     for (fsibe_ctx* c : e->runs) ctas += c->beam_cl;
     if (ctas > 2 * e->runs[0]->nsm && !std::getenv("FSIBE_BEAM_CLUSTER"))
         for (fsibe_ctx* c : e->runs) c->beam_cl = 0;
-    // In a batch of many runs the launches that take work off one run's critical path (the split
-    // nonlinear term, the stresses beside k_press_x) only add launches (64-run batch: 1587 us
-    // a step with them, 1024 without).  FSIBE_NL_SPLIT / FSIBE_STRESS_SPLIT decide when set.
+    // The launches that take work off one run's critical path (the split nonlinear term, the stresses
+    // beside k_press_x) have no batched form: with either, every run makes its own launches (the 64-run
+    // ensemble 1568 us a step with the stresses apart, 1596 with both, 1014 in batches without), and
+    // without batches they gained nothing either (1569).  FSIBE_NL_SPLIT / FSIBE_STRESS_SPLIT decide when
+    // set.
     if (nruns >= 8) {
         for (fsibe_ctx* c : e->runs) {
             if (!std::getenv("FSIBE_NL_SPLIT")) c->nl_split = false;

@@ -18,9 +18,15 @@
 // The error relative to the row's result is that of the FP64 stages or less: a flat row keeps some
 // 60 significant bits of its largest result, FP64 53 (measured against 64-bit transforms in
 // extended precision over the row shapes of the solver: tests/test_fx_algorithm.py).
-// Measured (GB300, 1024^2, ns = 256, the coupled FP64 step): k_nl_y 325 -> 181 us, k_press_x 334 -> 153,
-// k_press_y 145 -> 70, k_nl_x's advection part 148 -> 62, the step 1142 -> 601; at 256^2 the step
-// 323 -> 256 us.
+// It holds relative to the row, not element by element: where a row's large part cancels exactly (equal
+// values at every second place, say) and its small part does not, FP64 gives the small part's
+// modes to 53 bits of their own and this to some 2^-57 of the large part.
+// Measured (GB300, 1024^2, ns = 256, the coupled FP64 step; the transforms alone): k_nl_y 325 -> 181 us,
+// k_press_x 334 -> 153, k_press_y 145 -> 70, k_nl_x's advection part 148 -> 62, the step 1142 -> 601, at 256^2
+// 323 -> 256; with the pointwise work off the FP64 pipe as well (over_k2) 533 and 232 us a step, and
+// with a group of threads a transform (fluid_fx.cuh) 447 and 165.  What bounds the kernels then
+// (1024^2): k_nl_y's ALU pipe is busy 44% of the time, the FP64 pipe 29%, with 28 warps an SM that wait
+// at their barriers and on those two; k_press_x 35% and 34%.
 // Range.  The transforms that take or give a caller's arrays (WIDE) take every finite row: one whose largest
 // value is below 2^-927 is scaled up by a power of two as it enters, and results near the ends of the
 // exponent range are scaled as they leave (to zero, a denormal or infinity, rounded as any FP64 result).

@@ -264,10 +264,11 @@ __device__ __forceinline__ void row_r2c_reg(C2<R> (&v)[NBA][8], C2<R>* rb, int b
     }
 }
 // The same in the time step's fused kernels.  FP64 rows of 4096 real values (H = 2048) keep the
-// FP64 stages there.  Fixed point is the more exact at that length too (4096^2, three steps: the
-// pressure within 3.7e-16 of the CPU's, 4.0e-16 with the FP64 stages), but at 4096^2 the pressure
-// jump at the beam's free end is what is left of two values 2 10^7 times as large, one or two units
-// of their last place, and the comparison on record at that size holds that last place.
+// FP64 stages there, which makes the largest FP64 grids slower than fixed point would: of the results
+// that the three-step comparison with the CPU at 4096^2 holds to 1e-11, fixed point is the nearer in
+// all that are not differences (pressure 3.7e-16, with the FP64 stages 4.0e-16; vorticity 3.7e-16), but
+// the pressure jump at the beam's free end is what is left of two values 2 10^7 times as large, and
+// there one unit of their last place is 2e-9 (fixed point 2.9e-9, the FP64 stages the CPU's own bits).
 template <typename R, int H> constexpr bool step_fp() { return !kIsF32<R> && H == 2048; }
 // The step's x kernels with a group of threads a transform (fluid_fx.cuh): the FP64 form up to 2048,
 // where the integer chains want the warps; the FP32 form up to 512, where one block's latency is the

@@ -266,9 +266,7 @@ __device__ __forceinline__ bool hinge_inside(T gamma, T beta1, T beta2, T margin
     return in1 && in2;
 }
 
-// SmoothStep in FP32 from the FP64 distance: the FP32 form's value of the sharp end, and for the FP64
-// form an estimate within 4e-6 of the FP64 value (the arguments are rounded once or twice, |erf'| <=
-// 2/sqrt(pi) where erf is not flat, erff is within 2 ulp).
+// SmoothStep in FP32 from the FP64 distance: the FP32 form's value of the sharp end.
 __device__ __forceinline__ float smooth_step_f(double x, double t, double inv_delta, int sharp) {
     if (sharp) return (x <= t) ? 1.f : 0.f;
     const float a1 = (float)((t - x) * inv_delta), a2 = (float)((x + t) * inv_delta);
@@ -341,6 +339,11 @@ struct MaskNear {
     int q;
     bool known;
 };
+// The estimate is 0.5 (erff(u idf) + erff((2 tf - u) idf)) with u = t - d rounded to FP32: its arguments
+// have relative errors of at most 3 and 5 + |u| / (t + d) units of 2^-24, the second's two parts
+// cancelling no further than to t + d >= t whatever the body's thickness; an error r of an argument a
+// moves erf by 2/sqrt(pi) a e^(-a^2) r <= 0.49 r, and erff is within 2 ulp.  Together below 5e-7, so that
+// two estimates further apart than MASK_NEAR are in the FP64 values' order with room to spare.
 constexpr float MASK_NEAR = 2.0e-5f;
 // A lower bound of SmoothStep's fall over the distance x delta from d outwards (up to 0.1 delta of it):
 // its slope in units of 1/delta rises to its largest value and falls, so over an interval it is at

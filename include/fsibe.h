@@ -125,6 +125,11 @@ const char* fsibe_strerror(int status);
 const char* fsibe_last_error(const fsibe_ctx* ctx);
 
 /* ---- spectral operators on packed arrays (host in, host out) ------------------ */
+/* The FP64 form's transforms (these two, the initial vorticity, the field read back) take every finite
+ * value and are exact to 3 2^-53 of the result's 2-norm, below what FP64 stages give; that is relative to
+ * the rows they transform, whose values share an exponent: where the large part of a row cancels
+ * exactly, the small part left is known to some 2^-57 of the large one, and not to 53 bits of its own.
+ * The time step and the adjoint hold rows from 2^-985 to 2^1006 (one above is reported as NaN). */
 int fsibe_fft_forward(fsibe_ctx* ctx, const double* f, double* fk);      /* coftxy  cof_fftw33.f90:142-193 */
 int fsibe_fft_inverse(fsibe_ctx* ctx, const double* fk, double* f);      /* cofitxy cof_fftw33.f90:197-243 */
 int fsibe_cofdx(fsibe_ctx* ctx, const double* fk, double* out);          /* cofdx.f90:1-29   */
@@ -287,7 +292,9 @@ int fsibe_running_sums(const double* terms, int32_t n, double* out, int32_t* nse
  * registers capped for two resident blocks an SM -- and, for press_x in the FP32 form, the
  * paired kernel (two adjacent butterflies a thread) -- and keeps the fastest (cached per
  * precision and grid size for the process; FSIBE_AUTOTUNE=0 in the environment keeps the
- * defaults; FSIBE_PX_PAIRED=1 / 0 forces / forbids the paired press_x).  fsibe_tile_config
+ * defaults; FSIBE_PX_PAIRED=1 / 0 forces / forbids the paired press_x, which runs where the stresses
+ * are not formed in it).  press_x's choice is timed with or without the stresses, as the
+ * context's steps run it.  fsibe_tile_config
  * gives the rows and the blocks-per-SM bound (0: the kernel's default; 16 marks the paired
  * press_x) of each: out6 = {rows, bound} for nl_x, press_x, press_fin. */
 int fsibe_tiles(fsibe_ctx* ctx, int32_t* rows3);
