@@ -20,7 +20,8 @@
 // extended precision over the row shapes of the solver: tests/test_fx_algorithm.py).
 // It holds relative to the row, not element by element: where a row's large part cancels exactly (equal
 // values at every second place, say) and its small part does not, FP64 gives the small part's
-// modes to 53 bits of their own and this to some 2^-57 of the large part.
+// modes to 53 bits of their own and this to some 2^-59 of the large part's (256 values, ones and 10^-12
+// noise in turn: 2^-59.2 at most).
 // Measured (GB300, 1024^2, ns = 256, the coupled FP64 step; the transforms alone): k_nl_y 325 -> 181 us,
 // k_press_x 334 -> 153, k_press_y 145 -> 70, k_nl_x's advection part 148 -> 62, the step 1142 -> 601, at 256^2
 // 323 -> 256; with the pointwise work off the FP64 pipe as well (over_k2) 533 and 232 us a step, and

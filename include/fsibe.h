@@ -128,7 +128,8 @@ const char* fsibe_last_error(const fsibe_ctx* ctx);
 /* The FP64 form's transforms (these two, the initial vorticity, the field read back) take every finite
  * value and are exact to 3 2^-53 of the result's 2-norm, below what FP64 stages give; that is relative to
  * the rows they transform, whose values share an exponent: where the large part of a row cancels
- * exactly, the small part left is known to some 2^-57 of the large one, and not to 53 bits of its own.
+ * exactly, the small part's modes are known to some 2^-59 of the large part's own, and not to 53 bits
+ * of theirs.
  * The time step and the adjoint hold rows from 2^-985 to 2^1006 (one above is reported as NaN). */
 int fsibe_fft_forward(fsibe_ctx* ctx, const double* f, double* fk);      /* coftxy  cof_fftw33.f90:142-193 */
 int fsibe_fft_inverse(fsibe_ctx* ctx, const double* fk, double* f);      /* cofitxy cof_fftw33.f90:197-243 */

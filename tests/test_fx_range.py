@@ -98,25 +98,6 @@ def test_results_beyond_the_largest_double_are_infinite():
     assert got[0] == np.inf and not got[1:].any()
 
 
-@pytest.mark.parametrize("small", [1e-3, 1e-12, 1e-18])
-def test_the_part_beside_a_cancelling_one(small):
-    """Ones at every second place cancel in all but two modes; what the other places leave there is known
-    to 2^-57 of the ones: n elements rounded to the row's unit (2^-58 at most) or less, and as much again
-    in the stages, a sum of some sqrt(n) of it."""
-    n = 256
-    rng = np.random.default_rng(8)
-    z = np.where(np.arange(n) % 2 == 0, 1.0, small * rng.standard_normal(n)) + 1j * small * rng.standard_normal(n)
-    q, em = enter(np.concatenate([z.real, z.imag]))
-    v, d = stages(list(zip(q[:n], q[n:])), False, BITS, True, sum(l1(a) for a in q))
-    e = em - 1022 - BITS + d
-    got = leave([a for a, _ in v], e), leave([b for _, b in v], e)
-    ref = dft_ld(z.astype(np.clongdouble), -1)
-    err = np.sqrt((got[0] - ref[0])**2 + (got[1] - ref[1])**2)
-    k = np.arange(n) % (n // 2) != 0
-    own = np.sqrt(ref[0]**2 + ref[1]**2) * np.longdouble(2.0)**-53
-    assert (err[k] <= np.sqrt(n) * np.longdouble(2.0)**-57 + own[k]).all(), float(err[k].max() / np.sqrt(n) * 2.0**57)
-
-
 def test_zero_rows_stay_zero():
     q, em = enter(np.array([0.0, -0.0] * 8))
     assert em == 1 and not any(q)
